@@ -6,109 +6,296 @@
 // float32 path exists to show faults that bfloat16 hides, so its arithmetic must be beyond doubt:
 // on the software stack this engine was developed on (cuBLAS 12.8, B200) the library's float32
 // product with TF32 switched off returned, in some processes, pairs of wrong output columns for
-// products of a few rows (16 x 320 x 192 and the like).  And an output element here is the sum of
-// its K terms in ascending order, whatever M and N are: the same token gives the same bits in a
-// step of one token and in a step of a thousand, which the library does not promise.
+// products of a few rows (16 x 320 x 192 and the like).  And an output element here is summed in
+// an order that K alone fixes: the same token gives the same bits in a step of one token and in a
+// step of a thousand, which the library does not promise.
 //
-// One CTA computes a BM x 128 tile with 256 threads (a 16 x 16 grid of threads, BM/16 x 8 outputs
-// each); K goes through shared memory in slices of 8, both operands transposed there so that a
-// thread reads its BM/16 + 8 values of a slice as vectors.  BM is 128, or 32 for steps of few
-// rows.  Any M, N, K; rows are read as float4 where K is a multiple of 4.
+// The order: K is cut into 1, 2, 4 or 8 ranges (`sg_ranges`); inside a range the even and the odd
+// terms are two chains of FMAs in ascending order (one `fma.rn.f32x2` advances both), whose sum is
+// the range's; the ranges are added in ascending order, the bias last.  So a step whose outputs are
+// too few to fill the chip gives every range a CTA of its own (a thread-block cluster; the ranges'
+// tiles are added over distributed shared memory), a step with enough tiles lets one CTA walk
+// through all ranges, and both give the same bits.
+//
+// What bounds it: a few rows stream the weights, so the tile is 64 weight rows by the rows rounded up
+// to 2, 4, 8, 16 or 32, with four 32-deep stages of cp.async in flight per CTA and the first ones
+// issued before the dependency wait (weights are constants).  More rows are bound by the FMA pipe: a
+// 64 x 64 tile, 8 x 4 outputs a thread, operands read from shared memory four k at a time as one
+// 16-byte access (rows 36 floats apart, so eight neighbouring rows lie in different banks).  Up to 256 rows
+// a 32-row tile, of which there are twice as many, is the faster (896 x 4,864 at 207 rows 63 against 79 us,
+// 9,728 x 896 115 against 130), from 512 rows on the 64-row tile (1,024 rows 258 against 316 us).
+// Measured in chains of products: 4 rows by 9,728 x 896 8.5 us (4.1 TB/s), 1 row by 151,936 x 896 93 us
+// (5.8 TB/s), 1,024 rows by 9,728 x 896 425 us (42 TFLOP/s; the FMA pipe is busy 63 % of the cycles).  A
+// step of the 0.5B shape with 203 prompt tokens and 4 single ones, which runs 97 such products, took
+// 46.1 ms while one CTA computed 32 or 128 rows by 128 columns over all of K.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace somi {
 
-constexpr int kSgBN = 128;
-constexpr int kSgBK = 8;
-constexpr int kSgThreads = 256;
+constexpr int kSgBK = 32;             // k per stage
+constexpr int kSgPitch = kSgBK + 4;   // floats between rows of a stage
+constexpr int kSgBN = 64;
+constexpr int kSgStages = 4;
 
+// Tiles from which on one CTA walks through all ranges.  Tiles of few rows stream weights, and two an SM
+// are enough to do so; taller ones need the FMA pipe filled to the end of the last wave: 9,728 x 896 at 64
+// rows takes 60 us with 304 walking CTAs and 38 us with four times as many short ones.
+constexpr long long sg_fill_tiles(int rows) { return rows < 32 ? 148 * 2 : 148 * 8; }
+
+// Into how many ranges K is cut: a function of K alone (see above), for ranges of at least 64 terms
+// and of about 224 to 608 at the model sizes this path runs.
+inline int sg_ranges(int K) { return K >= 2048 ? 8 : (K >= 512 ? 4 : (K >= 128 ? 2 : 1)); }
+inline int sg_range_length(int K, int ranges) {
+    return (K + ranges * kSgBK - 1) / (ranges * kSgBK) * kSgBK;
+}
+
+__device__ __forceinline__ void sg_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float sg_sum2(unsigned long long d) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
+    return __fadd_rn(lo, hi);
+}
+template <int BYTES>
+__device__ __forceinline__ void sg_copy(uint32_t dst, const float* src, bool in) {
+    // (a source size of 0 writes zeros and reads nothing)
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+
+// What a thread copies of rows [row0, row0 + ROWS) of a matrix, 32 columns at a time: the same
+// columns of every row it visits, so a stage costs it one pointer addition a copy.
+template <int ROWS, int THREADS, bool VEC>
+struct SgLoader {
+    static constexpr int PER = VEC ? 4 : 1, ACROSS = kSgBK / PER;      // copies a row
+    static constexpr int APART = THREADS / ACROSS;                     // rows between a thread's copies
+    static constexpr int COPIES = (ROWS + APART - 1) / APART;
+    static_assert(THREADS % ACROSS == 0 && COPIES <= 32, "a thread stays in its columns");
+    const float* src;
+    const float* safe;
+    long long step;
+    uint32_t dst, live;
+    int k;
+
+    __device__ __forceinline__ SgLoader(float* stage, const float* m, long long ld, int row0, int n_rows, int k0) {
+        const int r = threadIdx.x / ACROSS;
+        k = k0 + threadIdx.x % ACROSS * PER;
+        safe = m;
+        src = m + static_cast<long long>(row0 + r) * ld + k;
+        step = ld * APART;
+        dst = static_cast<uint32_t>(__cvta_generic_to_shared(stage + r * kSgPitch + threadIdx.x % ACROSS * PER));
+        live = 0;
+#pragma unroll
+        for (int c = 0; c < COPIES; ++c)
+            if (r + c * APART < ROWS && row0 + r + c * APART < n_rows) live |= 1u << c;
+    }
+    // columns k0 + 32 s .. of the range that ends at k_end, into the stage `at` bytes further on
+    __device__ __forceinline__ void copy(int s, int k_end, uint32_t at) const {
+        const float* p = src + s * kSgBK;
+        const uint32_t mask = k + s * kSgBK < k_end ? live : 0u;
+#pragma unroll
+        for (int c = 0; c < COPIES; ++c) {
+            const bool in = (mask >> c) & 1u;
+            if (ROWS % APART == 0 || threadIdx.x / ACROSS + c * APART < ROWS)
+                sg_copy<4 * PER>(dst + at + c * APART * kSgPitch * 4, in ? p : safe, in);
+            p += step;
+        }
+    }
+};
+
+template <int BM, int TM, int TN>
+__host__ __device__ constexpr int sg_threads() { return (BM / TM) * (kSgBN / TN); }
 template <int BM>
-__global__ void __launch_bounds__(kSgThreads)
-sgemm_nt_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                const float* __restrict__ bias, float* __restrict__ y, int M, int N, int K,
-                long long ldx, long long ldy, long long bsx, long long bsw, long long bsy, int vec4) {
-    constexpr int TM = BM / 16;          // rows per thread
-    constexpr int TN = kSgBN / 16;       // columns per thread (8)
-    __shared__ __align__(16) float xs[kSgBK][BM];
-    __shared__ __align__(16) float ws[kSgBK][kSgBN];
+constexpr int sg_smem() { return kSgStages * (BM + kSgBN) * kSgPitch * 4; }
+
+// CLUSTER: the CTA computes one range, blockIdx.x % ranges; else all of them.
+template <int BM, int TM, int TN, bool VEC, bool CLUSTER>
+__global__ void __launch_bounds__(sg_threads<BM, TM, TN>())
+sgemm_nt_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+                float* __restrict__ y, int M, int N, int K, int ranges, int range_length, long long ldx,
+                long long ldy, long long bsx, long long bsw, long long bsy) {
+    constexpr int THREADS = sg_threads<BM, TM, TN>();
+    constexpr int ROWS_APART = BM / TM, COLS_APART = kSgBN / TN;
+    extern __shared__ __align__(16) float sg_buf[];      // [stage][x rows | w rows][pitch]
+    constexpr int STAGE = (BM + kSgBN) * kSgPitch;
     pdl_launch_dependents();
-    pdl_wait();
     // blockIdx.z is the product's index in a batch: operands of product b start b * bs{x,w,y}
     // elements further on; rows of x and y lie ldx and ldy elements apart (w's rows K)
     x += blockIdx.z * bsx;
     w += blockIdx.z * bsw;
     y += blockIdx.z * bsy;
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * kSgBN;
-    const int tr = tid / 16, tc = tid % 16;       // this thread's rows tr*TM.., columns tc*TN..
-    float acc[TM][TN];
+    const int n0 = (CLUSTER ? blockIdx.x / ranges : blockIdx.x) * kSgBN, m0 = blockIdx.y * BM;
+    const int first = CLUSTER ? blockIdx.x % ranges : 0;
+    const int k_begin = min(K, first * range_length);
+    const int k_end = CLUSTER ? min(K, k_begin + range_length) : K;
+    const int steps = (k_end - k_begin + kSgBK - 1) / kSgBK;
+    // a warp's lanes share as few rows of either operand as they can: 4 x 8 outputs apart
+    constexpr bool SQUARE = ROWS_APART % 4 == 0;
+    constexpr int WARP_COLS = COLS_APART / 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tr = SQUARE ? warp / WARP_COLS * 4 + lane / 8 : threadIdx.x / COLS_APART;
+    const int tc = SQUARE ? warp % WARP_COLS * 8 + lane % 8 : threadIdx.x % COLS_APART;
+
+    const SgLoader<kSgBN, THREADS, VEC> w_rows(sg_buf + BM * kSgPitch, w, K, n0, N, k_begin);
+    const SgLoader<BM, THREADS, VEC> x_rows(sg_buf, x, ldx, m0, M, k_begin);
+    auto load_w = [&](int s) { w_rows.copy(s, k_end, s % kSgStages * (STAGE * 4)); };
+    auto load_x = [&](int s) { x_rows.copy(s, k_end, s % kSgStages * (STAGE * 4)); };
+#pragma unroll
+    for (int s = 0; s < kSgStages - 1; ++s)
+        if (s < steps) load_w(s);                        // [constant]
+    pdl_wait();
+#pragma unroll
+    for (int s = 0; s < kSgStages - 1; ++s) {
+        if (s < steps) load_x(s);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    unsigned long long acc[TM][TN];
+    float total[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-    const bool vec = vec4 != 0;
-    // loading: a slice is BM (or 128) rows of 8 floats = two float4 per row
-    for (int k0 = 0; k0 < K; k0 += kSgBK) {
-        for (int idx = tid; idx < BM * 2; idx += kSgThreads) {
-            const int r = idx >> 1, h = (idx & 1) * 4;
-            const int gm = m0 + r, gk = k0 + h;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (gm < M) {
-                const float* p = x + static_cast<size_t>(gm) * ldx + gk;
-                if (vec && gk + 3 < K) v = *reinterpret_cast<const float4*>(p);
-                else {
-                    if (gk < K) v.x = p[0];
-                    if (gk + 1 < K) v.y = p[1];
-                    if (gk + 2 < K) v.z = p[2];
-                    if (gk + 3 < K) v.w = p[3];
-                }
+        for (int j = 0; j < TN; ++j) { acc[i][j] = 0ull; total[i][j] = 0.f; }
+    const int steps_per_range = range_length / kSgBK;
+    int left = steps_per_range;
+    bool started = false;
+    auto close_range = [&]() {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const float r = sg_sum2(acc[i][j]);
+                total[i][j] = started ? __fadd_rn(total[i][j], r) : r;
+                acc[i][j] = 0ull;
             }
-            xs[h][r] = v.x; xs[h + 1][r] = v.y; xs[h + 2][r] = v.z; xs[h + 3][r] = v.w;
+        started = true;
+    };
+    for (int s = 0; s < steps; ++s) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kSgStages - 2) : "memory");
+        __syncthreads();                                 // stage s is here; stage s - 1 has been read
+        if (s + kSgStages - 1 < steps) {
+            load_w(s + kSgStages - 1);
+            load_x(s + kSgStages - 1);
         }
-        for (int idx = tid; idx < kSgBN * 2; idx += kSgThreads) {
-            const int r = idx >> 1, h = (idx & 1) * 4;
-            const int gn = n0 + r, gk = k0 + h;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (gn < N) {
-                const float* p = w + static_cast<size_t>(gn) * K + gk;
-                if (vec && gk + 3 < K) v = *reinterpret_cast<const float4*>(p);
-                else {
-                    if (gk < K) v.x = p[0];
-                    if (gk + 1 < K) v.y = p[1];
-                    if (gk + 2 < K) v.z = p[2];
-                    if (gk + 3 < K) v.w = p[3];
-                }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const float* xs = sg_buf + (s % kSgStages) * STAGE + tr * kSgPitch;
+        const float* ws = sg_buf + (s % kSgStages) * STAGE + (BM + tc) * kSgPitch;
+#pragma unroll(TM * TN >= 32 ? 4 : 8)
+        for (int k = 0; k < kSgBK; k += 4) {
+            ulonglong2 b[TN];
+#pragma unroll
+            for (int j = 0; j < TN; ++j)
+                b[j] = *reinterpret_cast<const ulonglong2*>(ws + j * COLS_APART * kSgPitch + k);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(xs + i * ROWS_APART * kSgPitch + k);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) sg_fma2(acc[i][j], a.x, b[j].x);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) sg_fma2(acc[i][j], a.y, b[j].y);
             }
-            ws[h][r] = v.x; ws[h + 1][r] = v.y; ws[h + 2][r] = v.z; ws[h + 3][r] = v.w;
         }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < kSgBK; ++kk) {
-            float a[TM], b[TN];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = xs[kk][tr * TM + i];
-#pragma unroll
-            for (int j = 0; j < TN; j += 4) {
-                const float4 t = *reinterpret_cast<const float4*>(&ws[kk][tc * TN + j]);
-                b[j] = t.x; b[j + 1] = t.y; b[j + 2] = t.z; b[j + 3] = t.w;
-            }
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = __fmaf_rn(a[i], b[j], acc[i][j]);
+        if (!CLUSTER && --left == 0) {
+            close_range();
+            left = steps_per_range;
         }
-        __syncthreads();
     }
+    if (CLUSTER || left != steps_per_range) close_range();
+    if (!CLUSTER) {
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + tr * TM + i;
+        for (int i = 0; i < TM; ++i) {
+            const int gm = m0 + tr + i * ROWS_APART;
+            if (gm >= M) continue;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int gn = n0 + tc + j * COLS_APART;
+                if (gn < N) y[gm * ldy + gn] = bias ? __fadd_rn(total[i][j], bias[gn]) : total[i][j];
+            }
+        }
+        return;
+    }
+    // the ranges' tiles, each in its CTA's shared memory; every CTA of the cluster adds up a share of
+    // the elements in the order of the ranges (those that a short K leaves empty are left out, as
+    // the walk above never gets to them)
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();                                     // the stages are free
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j)
+            sg_buf[(tr + i * ROWS_APART) * kSgBN + tc + j * COLS_APART] = total[i][j];
+    cluster.sync();
+    constexpr int QUADS = BM * kSgBN / 4;
+    const bool wide = (ldy & 3) == 0 && (bsy & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+    for (int idx = first * THREADS + threadIdx.x; idx < QUADS; idx += ranges * THREADS) {
+        const int gm = m0 + idx / (kSgBN / 4), gn = n0 + idx % (kSgBN / 4) * 4;
+        float4 part[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+            if (r < ranges) part[r] = *cluster.map_shared_rank(reinterpret_cast<const float4*>(sg_buf) + idx, r);
+        float4 sum = part[0];
+#pragma unroll
+        for (int r = 1; r < 8; ++r)
+            if (r < ranges && r * range_length < K)
+                sum = make_float4(__fadd_rn(sum.x, part[r].x), __fadd_rn(sum.y, part[r].y),
+                                  __fadd_rn(sum.z, part[r].z), __fadd_rn(sum.w, part[r].w));
         if (gm >= M) continue;
+        float out[4] = {sum.x, sum.y, sum.z, sum.w};
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int gn = n0 + tc * TN + j;
-            if (gn < N) y[static_cast<size_t>(gm) * ldy + gn] = acc[i][j] + (bias ? bias[gn] : 0.f);
+        for (int e = 0; e < 4; ++e)
+            if (bias != nullptr && gn + e < N) out[e] = __fadd_rn(out[e], bias[gn + e]);
+        float* dst = y + gm * ldy + gn;
+        if (wide && gn + 3 < N) {
+            *reinterpret_cast<float4*>(dst) = make_float4(out[0], out[1], out[2], out[3]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (gn + e < N) dst[e] = out[e];
         }
     }
+    cluster.sync();                                      // no CTA leaves while its tile is read
+}
+
+struct SgArgs {
+    const float *x, *w, *bias;
+    float* y;
+    int M, N, K, batch;
+    long long ldx, ldy, bsx, bsw, bsy;
+};
+
+template <int BM, int TM, int TN, bool VEC, bool CLUSTER>
+int sg_launch_one(const SgArgs& a, int ranges, cudaStream_t stream) {
+    auto kernel = sgemm_nt_kernel<BM, TM, TN, VEC, CLUSTER>;
+    constexpr int smem = sg_smem<BM>();
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const unsigned tiles_n = static_cast<unsigned>((a.N + kSgBN - 1) / kSgBN);
+    const unsigned tiles_m = static_cast<unsigned>((a.M + BM - 1) / BM);
+    if (tiles_m > 65535u) return SOMI_ERR_UNSUPPORTED;
+    launch_pdl_cluster(kernel, dim3(tiles_n * (CLUSTER ? ranges : 1), tiles_m, a.batch),
+                       dim3(sg_threads<BM, TM, TN>()), smem, CLUSTER ? ranges : 1, stream, a.x, a.w, a.bias,
+                       a.y, a.M, a.N, a.K, ranges, sg_range_length(a.K, ranges), a.ldx, a.ldy, a.bsx, a.bsw,
+                       a.bsy);
+    return launch_status();
+}
+
+template <int BM, int TM, int TN>
+int sg_launch(const SgArgs& a, cudaStream_t stream) {
+    const int ranges = sg_ranges(a.K);
+    const long long tiles = static_cast<long long>((a.N + kSgBN - 1) / kSgBN) * ((a.M + BM - 1) / BM) * a.batch;
+    const bool cluster = ranges > 1 && tiles < sg_fill_tiles(BM);
+    const bool vec = ((a.K | a.ldx | a.bsx | a.bsw) & 3) == 0 &&
+                     ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) & 15) == 0;
+    if (vec) return cluster ? sg_launch_one<BM, TM, TN, true, true>(a, ranges, stream)
+                            : sg_launch_one<BM, TM, TN, true, false>(a, ranges, stream);
+    return cluster ? sg_launch_one<BM, TM, TN, false, true>(a, ranges, stream)
+                   : sg_launch_one<BM, TM, TN, false, false>(a, ranges, stream);
 }
 
 }  // namespace somi
@@ -118,24 +305,19 @@ using namespace somi;
 // y_b[M, N] = x_b[M, K] w_b[N, K]^T (+ bias) for b in [0, batch), all float32.  Rows of x_b and y_b lie
 // ldx and ldy elements apart, rows of w_b K; product b's operands start b * bs{x,w,y} elements
 // after product 0's (so the heads of a [tokens, heads, width] tensor are a batch without a copy).
+// w must not be written by a kernel of the same step: it is read before the dependency wait.
 SOMI_API int somi_gemm_f32_batched(const float* x, const float* w, const float* bias, float* y, int M,
                                    int N, int K, int batch, long long ldx, long long ldy,
                                    long long bsx, long long bsw, long long bsy, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || batch <= 0) return 0;
     if (K <= 0 || batch > 65535 || ldx < K || ldy < N) return SOMI_ERR_UNSUPPORTED;
-    const int vec4 = ((K | ldx | bsx | bsw) & 3) == 0 &&
-                     ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
-    const unsigned tiles_n = static_cast<unsigned>((N + kSgBN - 1) / kSgBN);
-    if (M <= 32) {
-        launch_pdl(sgemm_nt_kernel<32>, dim3(tiles_n, (M + 31) / 32, batch), dim3(kSgThreads), 0, stream,
-                   x, w, bias, y, M, N, K, ldx, ldy, bsx, bsw, bsy, vec4);
-    } else {
-        const unsigned tiles_m = static_cast<unsigned>((M + 127) / 128);
-        if (tiles_m > 65535u) return SOMI_ERR_UNSUPPORTED;
-        launch_pdl(sgemm_nt_kernel<128>, dim3(tiles_n, tiles_m, batch), dim3(kSgThreads), 0, stream,
-                   x, w, bias, y, M, N, K, ldx, ldy, bsx, bsw, bsy, vec4);
-    }
-    return launch_status();
+    const SgArgs a{x, w, bias, y, M, N, K, batch, ldx, ldy, bsx, bsw, bsy};
+    if (M <= 2) return sg_launch<2, 2, 1>(a, stream);
+    if (M <= 4) return sg_launch<4, 4, 1>(a, stream);
+    if (M <= 8) return sg_launch<8, 2, 2>(a, stream);
+    if (M <= 16) return sg_launch<16, 4, 2>(a, stream);
+    if (M <= 256) return sg_launch<32, 8, 2>(a, stream);
+    return sg_launch<64, 8, 4>(a, stream);
 }
 
 // y[M, N] = x[M, K] w[N, K]^T (+ bias), all float32, row-major.
