@@ -76,6 +76,8 @@ class CudaOps:
         self.use_pp_prefill = True
         self.pp_prefill_min_ctas = torch.cuda.get_device_properties(0).multi_processor_count
         self.use_tc_prefill = True
+        self.use_f32_attention = True
+        self.f32_chunk = int(self.lib.somi_attention_f32_chunk())
         self._q_maps: dict = {}
         self.lib.somi_decode_chunk.restype = ctypes.c_int
         self.decode_chunk = int(self.lib.somi_decode_chunk())
@@ -298,7 +300,8 @@ class CudaOps:
 
         In bfloat16 with head sizes 32/64/128, portions of prompts go to the tensor-core
         prefill kernel and single-token requests to the split-KV kernel (at most 16 query
-        heads per kv head); float32 and every other size go to the generic kernel.  So do values
+        heads per kv head); float32 with head sizes 64/128 under a plain causal mask or a window goes to
+        kernels of its own; every other size goes to the generic kernel.  So do values
         of another width than the keys (`value_dim`) and a chunked mask (`chunk`: a token sees
         the earlier tokens of its own chunk of that many positions).  `gate`: logits [T, nq *
         value width] (rows may lie further apart); the output is multiplied by their sigmoid;
@@ -447,9 +450,46 @@ class CudaOps:
             if trace.active():
                 trace.note(kernel, *self._attention_work(batch, 0, batch.num_prefill_requests, nq,
                                                          nkv, hd, qkv.element_size(), win))
+        # float32 under a plain causal mask or a window, head sizes 64 and 128: kernels of their own,
+        # which read a chunk of keys once for a group's heads and share a request's chunks over CTAs
+        own_f32 = (qkv.dtype == torch.float32 and self.use_f32_attention and vd == hd and not chunk
+                   and not shaped and gate is None
+                   and bool(self.lib.somi_attention_f32_supported(
+                       _ptr(qkv), _ptr(kcache), _ptr(vcache), _ptr(out), ctypes.c_int(qkv.shape[1]),
+                       ctypes.c_int(nq), ctypes.c_int(nkv), ctypes.c_int(hd))))
+        if own_f32:
+            tiles = batch.tiles[self.prefill_q_tile]
+            if tiles.shape[0]:
+                rc = self.lib.somi_attention_f32_portion(
+                    _ptr(qkv), ctypes.c_int(qkv.shape[1]), _ptr(kcache), _ptr(vcache),
+                    _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
+                    _ptr(batch.ctx_len), _ptr(tiles), ctypes.c_int(tiles.shape[0]), ctypes.c_int(nq),
+                    ctypes.c_int(nkv), ctypes.c_int(hd), ctypes.c_int(page_size), ctypes.c_float(scale),
+                    ctypes.c_int(win), _ptr(out), self._stream())
+                self._done(rc, "attention_f32_portion")
+                if trace.active():
+                    trace.note("attention_f32_portion", *self._attention_work(
+                        batch, 0, batch.num_prefill_requests, nq, nkv, hd, 4, win))
+            if n_decode:
+                max_chunks = -(-group.width * page_size // self.f32_chunk)
+                part = torch.empty(n_decode * nq * max_chunks * (hd + 2), dtype=torch.float32,
+                                   device=qkv.device)
+                rc = self.lib.somi_attention_f32_single(
+                    _ptr(qkv), ctypes.c_int(qkv.shape[1]), ctypes.c_int(batch.num_prefill_tokens),
+                    ctypes.c_int(batch.num_prefill_requests), ctypes.c_int(n_decode), _ptr(kcache),
+                    _ptr(vcache), _ptr(group.block_table), ctypes.c_int(group.width),
+                    _ptr(batch.ctx_len), ctypes.c_int(nq), ctypes.c_int(nkv), ctypes.c_int(hd),
+                    ctypes.c_int(page_size), ctypes.c_float(scale), ctypes.c_int(win), _ptr(part),
+                    ctypes.c_int(max_chunks), _ptr(out), self._stream())
+                self._done(rc, "attention_f32_single")
+                self.launches += 1
+                if trace.active():
+                    trace.note("attention_f32_single", *self._attention_work(
+                        batch, batch.num_prefill_requests, batch.num_requests, nq, nkv, hd, 4, win),
+                        detail="with merge")
         tiles = batch.tiles[self.generic_q_tile]
-        n_generic_tiles = 0 if tensor_core_prefill else tiles.shape[0]
-        n_generic_decode = 0 if split else n_decode
+        n_generic_tiles = 0 if tensor_core_prefill or own_f32 else tiles.shape[0]
+        n_generic_decode = 0 if split or own_f32 else n_decode
         if n_generic_tiles + n_generic_decode > 0:
             rc = self.lib.somi_paged_attention_generic(
                 _ptr(qkv), _code(qkv), ctypes.c_int(qkv.shape[1]), _ptr(kcache), _ptr(vcache),
@@ -1804,8 +1844,9 @@ class CudaOps:
         return out
 
     def gemm_f32(self, x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
-        """x[M, K] @ w[N, K]^T (+ bias) in float32 FMAs, each output summed over K in ascending
-        order (the float32 path's product; the library's is not used there)."""
+        """x[M, K] @ w[N, K]^T (+ bias) in float32 FMAs, each output summed over K in an order
+        that K alone fixes (the float32 path's product; the library's is not used there).  `w` is read before
+        the kernel waits for its predecessors: no kernel of the same step may write it."""
         _check(x, w, bias)
         M, K = x.shape
         N = w.shape[0]

@@ -1,10 +1,14 @@
-"""The float32 path's product at the sizes where its kernel changes shape: the bounds of the row tiles
-and of the ranges of K; and that a row's bits depend on none of it."""
+"""The float32 path's product and attention at the sizes where their kernels change shape: the bounds
+of the row tiles, of the ranges of K and of the chunks of keys; and that a row's bits depend on none of it."""
 
 import pytest
 import torch
 
+from tests.gpu_util import attention_case, batch_to_cpu
+from tests.plain.host_ops import HostOps
+
 pytestmark = pytest.mark.gpu
+HOST = HostOps()
 
 
 @pytest.fixture(scope="module")
@@ -29,3 +33,47 @@ def test_product_at_the_bounds_of_tiles_and_ranges(ops, K, N):
     assert ((whole.double() - want).abs() <= bound).all()
     for m in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65):
         assert torch.equal(ops.gemm_f32(x[130 - m:].contiguous(), w, b), whole[130 - m:]), m
+
+
+def run(ops, case, nq, nkv, hd, window):
+    mgr, batch, qkv, view, order = case
+    out = torch.full((batch.num_tokens, nq * hd), float("nan"), device="cuda")
+    ops.paged_attention(qkv, view.keys, view.values, batch, batch.groups[0], nq, nkv, hd, hd ** -0.5, window, out)
+    return out
+
+
+@pytest.mark.parametrize("nq,nkv,hd,ps,window", [(14, 2, 64, 16, None), (3, 3, 128, 8, None), (18, 2, 64, 32, 70),
+                                                 (16, 1, 128, 16, 64), (4, 2, 64, 16, 1)])
+def test_attention_at_the_bounds_of_chunks(ops, nq, nkv, hd, ps, window):
+    """Portions and single tokens that end on, before and behind a chunk of 64 keys and a tile of 64 rows."""
+    reqs = [(0, 2), (0, 63), (0, 64), (1, 64), (0, 65), (63, 2), (130, 129), (0, 1), (62, 1), (63, 1), (64, 1),
+            (65, 1), (127, 1), (128, 1), (700, 1)]
+    case = attention_case(ops, nq=nq, nkv=nkv, hd=hd, page_size=ps, window=window, requests=reqs, dtype=torch.float32)
+    mgr, batch, qkv, view, _ = case
+    out = run(ops, case, nq, nkv, hd, window)
+    ref = torch.empty_like(out, device="cpu")
+    host = batch_to_cpu(batch)
+    HOST.paged_attention(qkv.cpu(), view.keys.cpu(), view.values.cpu(), host, host.groups[0], nq, nkv, hd,
+                         hd ** -0.5, window, ref)
+    # both sides are float32: a few hundred roundings of values about 1
+    torch.testing.assert_close(out.cpu(), ref, rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("window", [None, 100])
+def test_attention_does_not_depend_on_the_cut(ops, window):
+    """The last 140 rows of a request of 271 give the same bits as one portion, and each as a single token."""
+    nq, nkv, hd = 6, 2, 64
+    whole = attention_case(ops, nq=nq, nkv=nkv, hd=hd, page_size=16, window=window, requests=[(131, 140)],
+                           dtype=torch.float32, seed=1)
+    store, table = whole[3], whole[1].groups[0].block_table[0]
+    want = run(ops, whole, nq, nkv, hd, window)
+    for r in (0, 60, 61, 139):
+        mgr, batch, qkv, view, _ = attention_case(ops, nq=nq, nkv=nkv, hd=hd, page_size=16, window=window,
+                                                  requests=[(131 + r, 1)], dtype=torch.float32, seed=2)
+        n = -(-(132 + r) // 16)
+        live = batch.groups[0].block_table[0, :n] >= 0
+        for mine, theirs in ((view.keys, store.keys), (view.values, store.values)):
+            mine[batch.groups[0].block_table[0, :n][live].long()] = theirs[table[:n][live].long()]
+        qkv.copy_(whole[2][r:r + 1])
+        got = run(ops, (mgr, batch, qkv, view, None), nq, nkv, hd, window)
+        assert torch.equal(got[0], want[r]), r
