@@ -159,9 +159,87 @@ latent_attention_generic_kernel(const T* __restrict__ q, long long q_tok_stride,
     }
 }
 
+// The cached rows that a step's prompt portions read, side by side, so that one product can expand them to
+// keys and values: request r's tiles of kLatentTile positions, aligned to position 0, from the one of its
+// first row's first visible key to the one of its newest, kGatherShares CTAs per tile.  `rows` [tiles, kLatentTile, R];
+// table[r, p] is the tile in `rows` of positions p kLatentTile ...  Positions outside the visible range are
+// zeros.  Tiles beyond the requests' own (the caller's bound is the layout's) are left alone.
+constexpr int kLatentTile = 128;
+constexpr int kGatherShares = 16;     // CTAs that share a tile (16 tiles of 1,024 bytes a row: 22 us with one each, 8 with 16)
+
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const uint4* __restrict__ cache, const int* __restrict__ block_table, int bt_stride,
+                     const int* __restrict__ cu_q, const int* __restrict__ ctx_len, int n_req, int quads,
+                     int page_size, int window, uint4* __restrict__ rows, int* __restrict__ table,
+                     int table_stride) {
+    __shared__ int req_s, tile_s;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (threadIdx.x < 32) {
+        // the request whose tiles this CTA's index falls into, 32 requests at a time
+        const int lane = threadIdx.x;
+        int before = 0, found = -1, tile = 0;
+        for (int r0 = 0; r0 < n_req && found < 0; r0 += 32) {
+            const int r = r0 + lane;
+            int first = 0, n = 0;
+            if (r < n_req) {
+                first = first_visible_key(ctx_len[r], window) / kLatentTile;
+                n = (ctx_len[r] + cu_q[r + 1] - cu_q[r] - 1) / kLatentTile + 1 - first;
+            }
+            int sum = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += x;
+            }
+            const int at = static_cast<int>(blockIdx.x) - before - (sum - n);
+            const unsigned hit = __ballot_sync(0xffffffffu, at >= 0 && at < n);
+            if (hit) {
+                const int who = __ffs(hit) - 1;
+                found = r0 + who;
+                tile = __shfl_sync(0xffffffffu, first + at, who);
+            }
+            before += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) { req_s = found; tile_s = tile; }
+    }
+    __syncthreads();
+    const int r = req_s, tile = tile_s;
+    if (r < 0) return;
+    if (threadIdx.x == 0 && blockIdx.y == 0) table[static_cast<size_t>(r) * table_stride + tile] = blockIdx.x;
+    const int first = first_visible_key(ctx_len[r], window), end = ctx_len[r] + cu_q[r + 1] - cu_q[r];
+    const int* bt = block_table + static_cast<size_t>(r) * bt_stride;
+    uint4* dst = rows + static_cast<size_t>(blockIdx.x) * kLatentTile * quads;
+    constexpr int share = kLatentTile / kGatherShares;
+    const int from = blockIdx.y * share * quads;
+    for (int i = from + threadIdx.x; i < from + share * quads; i += blockDim.x) {
+        const int n = i / quads, pos = tile * kLatentTile + n;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (pos >= first && pos < end)
+            v = cache[(static_cast<size_t>(bt[pos / page_size]) * page_size + pos % page_size) * quads + i % quads];
+        dst[i] = v;
+    }
+}
+
 }  // namespace somi
 
 using namespace somi;
+
+SOMI_API int somi_latent_tile() { return kLatentTile; }
+
+// bfloat16, R a multiple of 8.  `table_stride` at least the tiles of the longest request.
+SOMI_API int somi_latent_gather(const void* cache, const int* block_table, int bt_stride, const int* cu_q,
+                                const int* ctx_len, int n_req, int R, int page_size, int window, void* rows,
+                                int n_tiles, int* table, int table_stride, cudaStream_t stream) {
+    if (n_req <= 0 || n_tiles <= 0) return 0;
+    if (R <= 0 || R % 8 || page_size <= 0 || window < 0 ||
+        ((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(rows)) & 15))
+        return SOMI_ERR_UNSUPPORTED;
+    launch_pdl(latent_gather_kernel, dim3(n_tiles, kGatherShares), dim3(256), 0, stream, static_cast<const uint4*>(cache),
+               block_table, bt_stride, cu_q, ctx_len, n_req, R / 8, page_size, window, static_cast<uint4*>(rows),
+               table, table_stride);
+    return launch_status();
+}
 
 SOMI_API int somi_latent_attention_generic_q_tile() { return kLBM; }
 

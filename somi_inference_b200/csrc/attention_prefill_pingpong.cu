@@ -72,7 +72,7 @@ paged_prefill_pp_kernel(const __grid_constant__ CUtensorMap q_map,
                         const int* __restrict__ tiles, int nq, int nkv, int page_size,
                         float scale_log2e, int window, const float* __restrict__ sinks,
                         const float2* __restrict__ turn, __nv_bfloat16* __restrict__ out,
-                        int n_q_tiles, int keep, TwoMaps two) {
+                        int n_q_tiles, int keep, TwoMaps two, int head_cols, int v_col0) {
     constexpr int HALVES = HD / 64;
     constexpr int QTILE = HALVES * kPpQHalf;
     constexpr int TILE = HALVES * kPpKvHalf;
@@ -191,11 +191,14 @@ paged_prefill_pp_kernel(const __grid_constant__ CUtensorMap q_map,
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) break;
             if (my_page >= 0) {
-                const long long prow = (static_cast<long long>(my_page) * nkv + kvh) * page_size;
+                // a page of a head is rows of its own, or columns of rows that all heads share
+                const long long prow = head_cols > 0 ? static_cast<long long>(my_page) * page_size
+                                                     : (static_cast<long long>(my_page) * nkv + kvh) * page_size;
+                const int col0 = head_cols > 0 ? kvh * head_cols + which * v_col0 : 0;
                 unsigned char* dst = (which ? Vs : Ks) + st * TILE + lane * page_size * 128;
 #pragma unroll
                 for (int h = 0; h < HALVES; ++h)
-                    tma_load_2d(smem_u32(dst + h * kPpKvHalf), &kv_map, h * 64,
+                    tma_load_2d(smem_u32(dst + h * kPpKvHalf), &kv_map, col0 + h * 64,
                                 static_cast<int>((which ? v_row0 : k_row0) + prow), bar);
             }
         }
@@ -534,7 +537,8 @@ int launch_prefill_pp(const CUtensorMap* q_map, const CUtensorMap* kv_map, long 
                       long long v_row0, const int* block_table, int bt_stride, const int* cu_q,
                       const int* ctx_len, const int* tiles, int n_tiles, int nq, int nkv,
                       int page_size, float scale, int window, const float* sinks, const float* turn,
-                      void* out, cudaStream_t stream, int keep = 0, const TwoMaps& two = TwoMaps{}) {
+                      void* out, cudaStream_t stream, int keep = 0, const TwoMaps& two = TwoMaps{},
+                      int head_cols = 0, int v_col0 = 0) {
     const size_t smem = (TWO_MAPS ? 1 : 2) * (HD / 64) * kPpQHalf +
                         (pp_k_stages(HD) + pp_v_stages(HD)) * (HD / 64) * kPpKvHalf + 1024;
     cudaFuncSetAttribute(paged_prefill_pp_kernel<HD, TWO_MAPS>,
@@ -543,7 +547,7 @@ int launch_prefill_pp(const CUtensorMap* q_map, const CUtensorMap* kv_map, long 
     launch_pdl(paged_prefill_pp_kernel<HD, TWO_MAPS>, grid, dim3(kPpThreads), smem, stream, *q_map, *kv_map,
                k_row0, v_row0, block_table, bt_stride, cu_q, ctx_len, tiles, nq, nkv, page_size,
                scale * 1.4426950408889634f, window, sinks, reinterpret_cast<const float2*>(turn),
-               static_cast<__nv_bfloat16*>(out), n_tiles, keep, two);
+               static_cast<__nv_bfloat16*>(out), n_tiles, keep, two, head_cols, v_col0);
     return launch_status();
 }
 
@@ -584,6 +588,24 @@ SOMI_API int somi_paged_attention_prefill_pp(
                                      stream);
     return launch_prefill_pp<128>(qm, km, k_row0, v_row0, block_table, bt_stride, cu_q, ctx_len, tiles,
                                   n_tiles, nq, nkv, page_size, scale, window, sinks, turn, out, stream);
+}
+
+// The same over keys and values that lie in the columns of one matrix [rows, columns] and not in a
+// cache: head h's keys are columns h hd .. of its rows, its values v_col0 further on, and a page is
+// 128 rows (`kv_map`: that matrix with boxes of 128 rows x 64 columns).  Every head has keys of its own.
+SOMI_API int somi_attention_prefill_pp_columns(
+    const void* q_map, const void* kv_map, int v_col0, const int* block_table, int bt_stride,
+    const int* cu_q, const int* ctx_len, const int* tiles, int n_tiles, int heads, int hd, float scale,
+    int window, const float* sinks, void* out, cudaStream_t stream) {
+    if (n_tiles <= 0) return 0;
+    if (!somi_prefill_pp_supported(heads, heads, hd, kPpBN) || v_col0 % 8) return SOMI_ERR_UNSUPPORTED;
+    const CUtensorMap* qm = static_cast<const CUtensorMap*>(q_map);
+    const CUtensorMap* km = static_cast<const CUtensorMap*>(kv_map);
+    auto go = [&](auto launch) {
+        return launch(qm, km, 0, 0, block_table, bt_stride, cu_q, ctx_len, tiles, n_tiles, heads, heads, kPpBN,
+                      scale, window, sinks, nullptr, out, stream, 0, TwoMaps{}, hd, v_col0);
+    };
+    return hd == 64 ? go(launch_prefill_pp<64>) : go(launch_prefill_pp<128>);
 }
 
 // Attention in two maps (two_maps.cuh) of prompt portions.  hd (64 or 128): the width of a value and of

@@ -72,6 +72,8 @@ class CudaOps:
             self.prefill_pp_q_tile, self.latent_q_tile)))
         self.max_taps = int(self.lib.somi_causal_taps_max())
         self.use_mma_latent = True
+        self.use_expanded_latent = True
+        self.latent_tile = int(self.lib.somi_latent_tile())
         assert int(self.lib.somi_latent_attention_mma_q_tile()) == self.latent_q_tile
         self.use_pp_prefill = True
         self.pp_prefill_min_ctas = torch.cuda.get_device_properties(0).multi_processor_count
@@ -813,8 +815,8 @@ class CudaOps:
 
         `heads_first`: x is [T, heads, K] (a view of a [T, heads * K] projection) and y comes
         back as [heads, T, N]; otherwise x is [heads, T, K] and y is [T, heads, N], so that the
-        next projection reads [T, heads * N] without a copy.  x may be a view of wider rows; `out`
-        (heads_first only): a [heads, T, N] view that receives y.  float32: the engine's own product,
+        next projection reads [T, heads * N] without a copy.  x may be a view of wider rows; `out`: a
+        view of y's shape that receives it.  float32: the engine's own product,
         batched over heads; bfloat16: the library's batched product."""
         H, N, K = w.shape
         if heads_first:
@@ -824,10 +826,10 @@ class CudaOps:
             ys = y
             assert ys.shape == (H, T, N) and ys.stride(2) == 1 and ys.dtype == x.dtype
         else:
-            assert out is None
             T = x.shape[1]
             xs = x
-            y = torch.empty((T, H, N), dtype=x.dtype, device=x.device)
+            y = torch.empty((T, H, N), dtype=x.dtype, device=x.device) if out is None else out
+            assert y.shape == (T, H, N) and y.stride(2) == 1 and y.dtype == x.dtype
             ys = y.transpose(0, 1)                               # [H, T, N] view
         assert xs.shape == (H, T, K) and xs.stride(2) == 1 and w.is_contiguous()
         if x.dtype == torch.float32:
@@ -880,9 +882,82 @@ class CudaOps:
         if trace.active():
             trace.note("latent_rotary_store", 2 * T * (heads * rot + rank + rot) * x.element_size())
 
+    # A step's portions read expanded keys and values from this many rows a request on.  Per row and
+    # position read, attention over the latents takes rank / width times the operations, on the slower
+    # tensor path; expanding takes a fixed number per position.  The layer in us over the latents /
+    # expanded, 28 heads of 128 and rank 512 under a window of 1,024, portions from a prompt's start: 32 rows
+    # 40.6 / 37.0, 128 52.9 / 43.3, 512 126 / 68, 2,048 576 / 167; behind 3,000 positions: 32 rows 123 / 62, 512
+    # 242 / 95.  14 heads of 64, rank 128: 64 rows 24.8 / 26.8, 96 28.9 / 26.9, 2,048 104 / 56.
+    LATENT_EXPAND_ROWS = 96
+    LATENT_EXPAND_POSITIONS = 32768     # the most that are expanded side by side (28 heads of 128: 470 MB)
+
+    def latent_expand_tiles(self, batch, group, page_size: int, window) -> int:
+        """Tiles of positions that the step's portions may read, by the layout alone (a captured step is
+        replayed with other cached lengths): a request of q rows sees at most window - 1 + q
+        positions, which fall into (that + 254) / 128 aligned tiles, and never more than its table has."""
+        n = batch.num_prefill_requests
+        longest = -(-group.width * page_size // self.latent_tile)
+        if not window:
+            return n * longest
+        t = self.latent_tile
+        return min(n * longest, (n * (int(window) - 1 + 2 * t - 2) + batch.num_prefill_tokens) // t)
+
+    def latent_expands(self, batch, group, cache, heads: int, rank: int, key_dim: int, value_dim: int,
+                       window, dtype) -> bool:
+        """Whether the step's prompt portions read expanded keys and values (see `latent_portions`)."""
+        n = batch.num_prefill_requests
+        if not (self.use_expanded_latent and n and dtype == torch.bfloat16 and rank % 8 == 0
+                and cache.shape[3] == rank and key_dim == value_dim
+                and bool(self.lib.somi_prefill_pp_supported(ctypes.c_int(heads), ctypes.c_int(heads),
+                                                            ctypes.c_int(key_dim), ctypes.c_int(self.latent_tile)))):
+            return False
+        return (batch.num_prefill_tokens >= self.LATENT_EXPAND_ROWS * n
+                and self.latent_expand_tiles(batch, group, cache.shape[2], window) * self.latent_tile
+                <= self.LATENT_EXPAND_POSITIONS)
+
+    def latent_portions(self, q, cache, kv_up, batch, group, heads, rank, dim, scale, window, sinks, out) -> None:
+        """Attention of the step's prompt portions with keys and values expanded from the cached latents:
+        the latents that they read are gathered, one library product with `kv_up` [2 * heads * dim, rank]
+        (all heads' keys, then all heads' values) expands them, and the two-tile tcgen05 kernel
+        reads a head's keys and values as columns of the result.  `q`, `out`: [T, heads * dim], of which the
+        portions' rows are read and written."""
+        _check(q, cache, kv_up, out, group.block_table, sinks)
+        page_size, n, t = cache.shape[2], batch.num_prefill_requests, self.latent_tile
+        assert q.dtype == cache.dtype == kv_up.dtype == out.dtype == torch.bfloat16
+        assert tuple(kv_up.shape) == (2 * heads * dim, rank) and cache.shape[3] == rank
+        assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == heads)
+        n_tiles = self.latent_expand_tiles(batch, group, page_size, window)
+        longest = -(-group.width * page_size // t)
+        rows = torch.empty((n_tiles * t, rank), dtype=q.dtype, device=q.device)
+        table = torch.empty((n, longest), dtype=torch.int32, device=q.device)
+        win = int(window) if window else 0
+        rc = self.lib.somi_latent_gather(
+            _ptr(cache), _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
+            _ptr(batch.ctx_len), ctypes.c_int(n), ctypes.c_int(rank), ctypes.c_int(page_size), ctypes.c_int(win),
+            _ptr(rows), ctypes.c_int(n_tiles), _ptr(table), ctypes.c_int(longest), self._stream())
+        self._done(rc, "latent_gather")
+        if trace.active():
+            trace.note("latent_gather", 2 * rows.numel() * rows.element_size())
+        expanded = torch.nn.functional.linear(rows, kv_up)
+        if trace.active():
+            trace.note("library_gemm", (rows.numel() + kv_up.numel() + expanded.numel()) * 2,
+                       2.0 * rows.numel() * kv_up.shape[0],
+                       detail=f"M={rows.shape[0]} N={kv_up.shape[0]} K={rank}")
+        tiles = batch.tiles[self.prefill_pp_q_tile]
+        rc = self.lib.somi_attention_prefill_pp_columns(
+            ctypes.c_void_p(self._q_tensor_map(q)), ctypes.c_void_p(self._q_tensor_map(expanded)),
+            ctypes.c_int(heads * dim), _ptr(table), ctypes.c_int(longest), _ptr(batch.cu_q), _ptr(batch.ctx_len),
+            _ptr(tiles), ctypes.c_int(tiles.shape[0]), ctypes.c_int(heads), ctypes.c_int(dim),
+            ctypes.c_float(scale), ctypes.c_int(win), _ptr(sinks), _ptr(out), self._stream())
+        self._done(rc, "attention_prefill_pp_columns")
+        if trace.active():
+            trace.note("attention_prefill_tcgen05_pingpong", *self._attention_work(
+                batch, 0, n, heads, heads, dim, 2, win), detail="expanded latents")
+
     def latent_attention(self, q, cache, batch, group, heads, rank, scale, window, sinks, out,
-                         tail: int = 0) -> None:
-        """Attention of every token of the step over a cache of latents that serve as keys and
+                         tail: int = 0, singles: bool = False) -> None:
+        """Attention of every token of the step (`singles`: of its single-token requests alone, whose rows
+        `q` and `out` hold) over a cache of latents that serve as keys and
         as values for every head (`q`, `out`: [heads, T, rank]; cache [pages, 1, page, rank]).
         `tail`: elements behind the latent in q's and the cache's rows that only the scores read;
         `sinks`: float32 [heads] scores that join every softmax's denominator, or None."""
@@ -893,8 +968,12 @@ class CudaOps:
         assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == heads)
         page_size = cache.shape[2]
         T = q.shape[1]
-        tiles = batch.tiles[self.latent_q_tile]
+        tiles = batch.tiles[self.latent_q_tile][:0] if singles else batch.tiles[self.latent_q_tile]
         n_decode = batch.num_requests - batch.num_prefill_requests
+        # the kernels count rows from the step's first: without the portions' rows, from that far in front
+        skipped = (batch.num_prefill_tokens if singles else 0) * q.element_size()
+        q_at = ctypes.c_void_p(q.data_ptr() - skipped * wide)
+        out_at = ctypes.c_void_p(out.data_ptr() - skipped * rank)
         win = int(window) if window else 0
         if (self.use_mma_latent and q.dtype == torch.bfloat16
                 and bool(self.lib.somi_latent_attention_mma_supported(
@@ -906,13 +985,13 @@ class CudaOps:
                 ctypes.c_int(max_kv), ctypes.c_int(win), ctypes.c_int(n_decode), ctypes.c_int(heads)))
             ws = self._scratch(n_decode * heads * splits * (rank + 2), q.device) if splits > 1 and n_decode else None
             rc = self.lib.somi_latent_attention_mma(
-                _ptr(q), ctypes.c_longlong(wide), ctypes.c_longlong(T * wide), _ptr(cache),
+                q_at, ctypes.c_longlong(wide), ctypes.c_longlong(T * wide), _ptr(cache),
                 _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
                 _ptr(batch.ctx_len), _ptr(tiles), ctypes.c_int(tiles.shape[0]),
                 ctypes.c_int(batch.num_prefill_requests), ctypes.c_int(batch.num_prefill_tokens),
                 ctypes.c_int(n_decode), ctypes.c_int(max_kv), ctypes.c_int(heads),
                 ctypes.c_int(wide), ctypes.c_int(rank), ctypes.c_int(page_size), ctypes.c_float(scale),
-                ctypes.c_int(win), _ptr(sinks), _ptr(out), ctypes.c_longlong(rank),
+                ctypes.c_int(win), _ptr(sinks), out_at, ctypes.c_longlong(rank),
                 ctypes.c_longlong(T * rank), _ptr(ws), self._stream())
             self._done(rc, "latent_attention_mma")
             self.launches += (1 if tiles.shape[0] and n_decode else 0) + (1 if splits > 1 and n_decode else 0)
@@ -924,13 +1003,13 @@ class CudaOps:
                            detail=f"splits={splits}" if n_decode else "")
             return
         rc = self.lib.somi_latent_attention_generic(
-            _ptr(q), _code(q), ctypes.c_longlong(wide), ctypes.c_longlong(T * wide), _ptr(cache),
+            q_at, _code(q), ctypes.c_longlong(wide), ctypes.c_longlong(T * wide), _ptr(cache),
             _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
             _ptr(batch.ctx_len), _ptr(tiles), ctypes.c_int(tiles.shape[0]),
             ctypes.c_int(batch.num_prefill_requests), ctypes.c_int(batch.num_prefill_tokens),
             ctypes.c_int(n_decode), ctypes.c_int(heads), ctypes.c_int(wide), ctypes.c_int(rank),
             ctypes.c_int(page_size), ctypes.c_float(scale), ctypes.c_int(int(window) if window else 0),
-            _ptr(sinks), _ptr(out), ctypes.c_longlong(rank), ctypes.c_longlong(T * rank),
+            _ptr(sinks), out_at, ctypes.c_longlong(rank), ctypes.c_longlong(T * rank),
             self._stream())
         self._done(rc, "latent_attention")
         if trace.active():

@@ -14,8 +14,10 @@ run reads the cache of an earlier run (same kv_rank) with its own W_uk, W_uv, wi
 Because k and v are linear in c, the expansions are moved to the query side and behind the sum:
     q_h . k_h = (W_uk,h^T q_h) . c,        sum_j p_j v_h,j = W_uv,h (sum_j p_j c_j),
 so the attention kernel is multi-query attention over the latent cache itself (key = value = c,
-kv_rank wide), and no step ever expands cached positions again.  The two per-head products are
-batched products over heads.  The norms, scores, softmax and sink are float32.
+kv_rank wide), and a step of few tokens never expands cached positions.  The two per-head products are
+batched products over heads.  Prompt portions of some length (bfloat16, q and k straight from their
+latents) do expand the positions they read, once for all their rows (`latent_portions`).  The norms,
+scores, softmax and sink are float32.
 `gate` = "head": W_g has a row per head, and the logit of a head multiplies all its elements.
 
 Without a query latent (`q_rank` None) queries come straight from the input, q = W_q h, and one product
@@ -101,6 +103,9 @@ class LatentAttentionMixer:
         self.down = Linear(torch.cat(down, 0).contiguous(), None, ctx.ops)
         self.q_norm = tensors[n["q_norm"]]
         self.q_up = Linear(tensors[n["q_up"]], None, ctx.ops)
+        # all heads' W_uk, then all heads' W_uv, for portions that read expanded keys and values
+        self.kv_up = (torch.cat([tensors[n["k_up"]], tensors[n["v_up"]]], 0).contiguous()
+                      if ctx.dtype == torch.bfloat16 and self.key_dim == self.value_dim else None)
         self.gate = Linear(tensors[n["gate"]], None, ctx.ops) if params.get("gate") else None
 
     def _build_direct(self, params, tensors, n) -> None:
@@ -170,12 +175,20 @@ class LatentAttentionMixer:
                               group.slot_map if self.own_latent else None,
                               paged.keys if self.own_latent else None)
         q = self.q_up(cq)                                           # [T, H * key_dim]
-        qa = ops.head_product(q.view(T, H, self.key_dim), self.k_up_t, heads_first=True)   # [H, T, R]
-        o_lat = torch.empty_like(qa)
-        ops.latent_attention(qa, paged.keys, batch, group, H, R, self.scale, self.window,
-                             self.sinks, o_lat)
-        o = ops.head_product(o_lat, self.v_up, heads_first=False)    # [T, H, value_dim]
-        o = o.view(T, H * self.value_dim)
+        expand = self.kv_up is not None and ops.latent_expands(
+            batch, group, paged.keys, H, R, self.key_dim, self.value_dim, self.window, x.dtype)
+        first = batch.num_prefill_tokens if expand else 0           # rows from here on read the latents
+        o = torch.empty((T, H * self.value_dim), dtype=x.dtype, device=x.device)
+        if expand:
+            ops.latent_portions(q, paged.keys, self.kv_up, batch, group, H, R, self.key_dim, self.scale,
+                                self.window, self.sinks, o)
+        if first < T:
+            qa = ops.head_product(q[first:].view(T - first, H, self.key_dim), self.k_up_t, heads_first=True)
+            o_lat = torch.empty_like(qa)                            # [H, rows, R]
+            ops.latent_attention(qa, paged.keys, batch, group, H, R, self.scale, self.window,
+                                 self.sinks, o_lat, singles=expand)
+            ops.head_product(o_lat, self.v_up, heads_first=False,
+                             out=o[first:].view(T - first, H, self.value_dim))
         if self.gate is not None and self.head_gate:
             ops.head_gate_mul(o, self.gate(x), H)
         elif self.gate is not None:
