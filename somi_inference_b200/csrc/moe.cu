@@ -15,8 +15,9 @@
 //             entry's result does not depend on the tile it fell into or on the rest of the step.
 //             Epilogues: the experts' gated activation over row-interleaved gate/up weights, or
 //             float32 rows scattered back to the entries' places.
-//   matrix-vector: a step of few entries needs no grouping: every entry streams the rows of its
-//             own expert (bfloat16, 16-byte loads, two rows a warp), with the same two epilogues.
+//   matrix-vector: a step of few entries needs no grouping in memory: the first of an expert's entries
+//             streams its rows for up to four of them (bfloat16, 16-byte loads, four rows a warp), with
+//             the same two epilogues.
 //   gather / activation: what stands around the library's grouped product in prompt-sized
 //             bfloat16 steps: the rows in the grouped order, and the experts' gated activation.
 //   combine:  out[t] = weight * sum_k y[row of entry t * top + k] (+ the shared expert's rows), float32;
@@ -164,68 +165,138 @@ __global__ void clamped_gate_up_kernel(const T* __restrict__ gu, T* __restrict__
     }
 }
 
-// A step of few tokens: every (token, k) entry streams the rows of its own expert.
-// grid (row blocks, entries); a warp computes two weight rows at a time (a gate row and its up
-// row, or two output rows), lanes stride over K with 16-byte loads; x of the entry sits in shared
-// memory as float32.  MODE 1: the gated activation, out [entries, N / 2] bfloat16;
-// MODE 0: out [entries, N] float32; MODE 2: an activation without a gate (`act`), out [entries, N]
-// bfloat16.
+// A step of few tokens: the (token, k) entries of an expert stream its rows together, up to
+// kGemvEntries at a time.  grid (row blocks, entries): the CTAs of an entry that is not the first of
+// such a group of its expert's entries leave at once.  A warp computes four weight rows at a time (two
+// gate rows and their up rows, or four output rows) for all entries of the group, lanes stride over K
+// with 16-byte loads; the entries' x sit in shared memory, read in the same 16-byte pieces (eight lanes
+// cover all banks).  MODE 1: the gated activation, out [entries, N / 2] bfloat16; MODE 0: out
+// [entries, N] float32; MODE 2: an activation without a gate (`act`), out [entries, N] bfloat16.
+//
+// Bound by the experts' bytes: 8 tokens of 4 choices among 16 experts hit about 14 of them with 2.2 entries
+// each, which a CTA per entry read 2.2 times, through L2 mostly, with x as float32 eight words apart a
+// lane.  16 experts, 9,472 x 3,584 and 3,584 x 4,736, 32 entries: 303 + 174 us then, 201 + 102 now (5.4 TB/s of
+// the matrices that are hit).  Per entry every sum keeps its order (lane chains, then the butterfly), so results do not depend
+// on what else is in the step.
 constexpr int kGemvWarps = 8;
 constexpr int kGemvRowsPerCta = 64;
+constexpr int kGemvRows = 4;          // rows a warp streams at a time
+constexpr int kGemvEntries = 4;
+
+template <int MODE, int NE>
+__device__ __forceinline__ void gemv_rows(const __nv_bfloat16* __restrict__ Wm, const __nv_bfloat16* xs,
+                                          const int* entries, void* __restrict__ out, int row_begin,
+                                          int row_end, int N, int K, const GluForm& form, int act) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int row = row_begin + warp * kGemvRows; row < row_end; row += kGemvWarps * kGemvRows) {
+        const __nv_bfloat16* w = Wm + static_cast<size_t>(row) * K;
+        const int live = min(kGemvRows, N - row);
+        float a[NE][kGemvRows];
+#pragma unroll
+        for (int e = 0; e < NE; ++e)
+#pragma unroll
+            for (int r = 0; r < kGemvRows; ++r) a[e][r] = 0.f;
+#pragma unroll 2
+        for (int k = lane * 8; k < K; k += 256) {
+            uint4 u[kGemvRows];
+#pragma unroll
+            for (int r = 0; r < kGemvRows; ++r)
+                u[r] = r < live ? __ldg(reinterpret_cast<const uint4*>(w + static_cast<size_t>(r) * K + k))
+                                : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int e = 0; e < NE; ++e) {
+                const uint4 v = *reinterpret_cast<const uint4*>(xs + static_cast<size_t>(e) * K + k);
+                const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+                for (int r = 0; r < kGemvRows; ++r) {
+                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u[r]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        a[e][r] = fmaf(__low2float(h[i]), __low2float(x[i]), a[e][r]);
+                        a[e][r] = fmaf(__high2float(h[i]), __high2float(x[i]), a[e][r]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < NE; ++e) {
+#pragma unroll
+            for (int r = 0; r < kGemvRows; ++r) a[e][r] = warp_sum(a[e][r]);
+            if (lane == e) {
+                const size_t entry = entries[e];
+                if (MODE == 1) {
+                    __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + entry * (N / 2) + row / 2;
+#pragma unroll
+                    for (int r = 0; r < kGemvRows; r += 2)
+                        if (r < live) o[r / 2] = __float2bfloat16_rn(glu(a[e][r], a[e][r + 1], form));
+                } else if (MODE == 2) {
+                    __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + entry * N + row;
+#pragma unroll
+                    for (int r = 0; r < kGemvRows; ++r)
+                        if (r < live) o[r] = __float2bfloat16_rn(unary_act(a[e][r], act));
+                } else {
+                    float* o = static_cast<float*>(out) + entry * N + row;
+#pragma unroll
+                    for (int r = 0; r < kGemvRows; ++r)
+                        if (r < live) o[r] = a[e][r];
+                }
+            }
+        }
+    }
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(kGemvWarps * 32)
 moe_gemv_kernel(const __nv_bfloat16* __restrict__ A, long long a_stride, int a_div,
                 const __nv_bfloat16* __restrict__ W, const int* __restrict__ ids,
-                const int* __restrict__ table, int top, int E, void* __restrict__ out, int N, int K,
-                GluForm form, int act) {
-    extern __shared__ float xs[];                          // [K]
+                const int* __restrict__ table, int top, int E, int n_entries, int most,
+                void* __restrict__ out, int N, int K, GluForm form, int act) {
+    extern __shared__ __align__(16) __nv_bfloat16 gemv_xs[];       // [most][K]
+    __shared__ int entries_s[kGemvEntries], count_s;
     pdl_launch_dependents();
     pdl_wait();
-    const int entry = blockIdx.y;
-    const int expert = table[static_cast<size_t>(ids != nullptr ? ids[entry / top] : entry / top) * top + entry % top];
+    auto expert_of = [&](int e) {
+        return table[static_cast<size_t>(ids != nullptr ? ids[e / top] : e / top) * top + e % top];
+    };
+    const int entry = blockIdx.y, expert = expert_of(entry);
     if (expert < 0 || expert >= E) return;
-    const __nv_bfloat16* x = A + static_cast<size_t>(entry / a_div) * a_stride;
-    for (int i = threadIdx.x; i < K; i += blockDim.x) xs[i] = __bfloat162float(x[i]);
+    if (threadIdx.x < 32) {
+        // the entry's place among its expert's entries, and the group it leads if that is a first place
+        const int lane = threadIdx.x;
+        int before = 0, n = 0;
+        for (int e0 = 0; e0 < n_entries && n < most; e0 += 32) {
+            const int e = e0 + lane;
+            const bool same = e < n_entries && expert_of(e) == expert;
+            before += __popc(__ballot_sync(0xffffffffu, same && e < entry));
+            const unsigned from = __ballot_sync(0xffffffffu, same && e >= entry);
+            const int at = n + __popc(from & ((1u << lane) - 1u));
+            if (same && e >= entry && at < most) entries_s[at] = e;
+            n += __popc(from);
+        }
+        if (lane == 0) count_s = before % most == 0 ? min(n, most) : 0;
+    }
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const __nv_bfloat16* Wm = W + static_cast<size_t>(expert) * N * K;
-    const int row_end = min(N, (static_cast<int>(blockIdx.x) + 1) * kGemvRowsPerCta);
-    for (int row = blockIdx.x * kGemvRowsPerCta + warp * 2; row < row_end; row += kGemvWarps * 2) {
-        const __nv_bfloat16* w0 = Wm + static_cast<size_t>(row) * K;
-        const __nv_bfloat16* w1 = w0 + K;
-        const bool two = row + 1 < N;
-        float a0 = 0.f, a1 = 0.f;
-#pragma unroll 2
-        for (int k = lane * 8; k < K; k += 256) {
-            const uint4 u0 = *reinterpret_cast<const uint4*>(w0 + k);
-            const uint4 u1 = two ? *reinterpret_cast<const uint4*>(w1 + k) : make_uint4(0, 0, 0, 0);
-            const __nv_bfloat162* h0 = reinterpret_cast<const __nv_bfloat162*>(&u0);
-            const __nv_bfloat162* h1 = reinterpret_cast<const __nv_bfloat162*>(&u1);
+    const int count = count_s;
+    if (count == 0) return;
+    for (int i = threadIdx.x; i < count * (K / 8); i += blockDim.x) {
+        const int e = i / (K / 8), k = i % (K / 8) * 8;
+        const __nv_bfloat16* x = A + static_cast<size_t>(entries_s[e] / a_div) * a_stride + k;
+        __nv_bfloat16* dst = gemv_xs + static_cast<size_t>(e) * K + k;
+        if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+            *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(x);
+        } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float x0 = xs[k + 2 * e], x1 = xs[k + 2 * e + 1];
-                a0 = fmaf(__low2float(h0[e]), x0, a0);
-                a0 = fmaf(__high2float(h0[e]), x1, a0);
-                a1 = fmaf(__low2float(h1[e]), x0, a1);
-                a1 = fmaf(__high2float(h1[e]), x1, a1);
-            }
+            for (int j = 0; j < 8; ++j) dst[j] = x[j];
         }
-        a0 = warp_sum(a0);
-        a1 = warp_sum(a1);
-        if (lane == 0) {
-            if (MODE == 1) {
-                static_cast<__nv_bfloat16*>(out)[static_cast<size_t>(entry) * (N / 2) + row / 2] =
-                    __float2bfloat16_rn(glu(a0, a1, form));
-            } else if (MODE == 2) {
-                __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + static_cast<size_t>(entry) * N;
-                o[row] = __float2bfloat16_rn(unary_act(a0, act));
-                if (two) o[row + 1] = __float2bfloat16_rn(unary_act(a1, act));
-            } else {
-                float* o = static_cast<float*>(out) + static_cast<size_t>(entry) * N;
-                o[row] = a0;
-                if (two) o[row + 1] = a1;
-            }
-        }
+    }
+    __syncthreads();
+    const __nv_bfloat16* Wm = W + static_cast<size_t>(expert) * N * K;
+    const int row_begin = blockIdx.x * kGemvRowsPerCta, row_end = min(N, row_begin + kGemvRowsPerCta);
+    switch (count) {
+        case 1: gemv_rows<MODE, 1>(Wm, gemv_xs, entries_s, out, row_begin, row_end, N, K, form, act); break;
+        case 2: gemv_rows<MODE, 2>(Wm, gemv_xs, entries_s, out, row_begin, row_end, N, K, form, act); break;
+        case 3: gemv_rows<MODE, 3>(Wm, gemv_xs, entries_s, out, row_begin, row_end, N, K, form, act); break;
+        default: gemv_rows<MODE, 4>(Wm, gemv_xs, entries_s, out, row_begin, row_end, N, K, form, act); break;
     }
 }
 
@@ -648,30 +719,17 @@ SOMI_API int somi_moe_gemv(const void* A, long long a_stride, int a_div, const v
         (reinterpret_cast<uintptr_t>(W) & 15))
         return SOMI_ERR_UNSUPPORTED;
     dim3 grid((N + kGemvRowsPerCta - 1) / kGemvRowsPerCta, n_entries);
-    const size_t smem = sizeof(float) * K;
-    if (mode == 1) {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(moe_gemv_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(moe_gemv_kernel<1>, grid, dim3(kGemvWarps * 32), smem, stream,
-                   static_cast<const __nv_bfloat16*>(A), a_stride, a_div,
-                   static_cast<const __nv_bfloat16*>(W), ids, table, top, E, out, N, K,
+    const int most = min(kGemvEntries, 200 * 1024 / (2 * K));     // (2 or more: K is at most 40 Ki)
+    const size_t smem = sizeof(__nv_bfloat16) * most * K;
+    if (n_entries > 65535) return SOMI_ERR_UNSUPPORTED;
+    auto go = [&](auto kernel) {
+        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        launch_pdl(kernel, grid, dim3(kGemvWarps * 32), smem, stream, static_cast<const __nv_bfloat16*>(A), a_stride,
+                   a_div, static_cast<const __nv_bfloat16*>(W), ids, table, top, E, n_entries, most, out, N, K,
                    GluForm{limit, alpha, shift, cubic}, act);
-    } else if (mode == 2) {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(moe_gemv_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(moe_gemv_kernel<2>, grid, dim3(kGemvWarps * 32), smem, stream,
-                   static_cast<const __nv_bfloat16*>(A), a_stride, a_div,
-                   static_cast<const __nv_bfloat16*>(W), ids, table, top, E, out, N, K,
-                   GluForm{limit, alpha, shift, cubic}, act);
-    } else {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(moe_gemv_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(moe_gemv_kernel<0>, grid, dim3(kGemvWarps * 32), smem, stream,
-                   static_cast<const __nv_bfloat16*>(A), a_stride, a_div,
-                   static_cast<const __nv_bfloat16*>(W), ids, table, top, E, out, N, K,
-                   GluForm{limit, alpha, shift, cubic}, act);
-    }
-    return launch_status();
+        return launch_status();
+    };
+    return mode == 1 ? go(moe_gemv_kernel<1>) : (mode == 2 ? go(moe_gemv_kernel<2>) : go(moe_gemv_kernel<0>));
 }
 
 // mode 0: out[scatter ? scatter[pos] : pos] = A W^T rows (out_dtype 0: float32, 1: as A);
