@@ -73,6 +73,7 @@ class CudaOps:
         self.max_taps = int(self.lib.somi_causal_taps_max())
         self.use_mma_latent = True
         self.use_expanded_latent = True
+        self.use_scan_chunks = True
         self.latent_tile = int(self.lib.somi_latent_tile())
         assert int(self.lib.somi_latent_attention_mma_q_tile()) == self.latent_q_tile
         self.use_pp_prefill = True
@@ -1602,6 +1603,26 @@ class CudaOps:
     SCAN_PREPARE_ROWS = 16
     SCAN_TURN_ROWS = 4          # the most rows a request may have where the scan itself rotates q and k
 
+    # portions go in chunks from rows = this * state width on, on average (both sides measured in
+    # `csrc/recurrent_chunks.cu`: they meet at 128 to 256 rows for a width of 128, at 32 to 64 for 64)
+    SCAN_CHUNK_ROWS = 1
+    SCAN_CHUNK_BYTES = 1 << 29  # the most that the chunks' states may take
+
+    def scan_in_chunks(self, q, k, v, batch, heads, qk_heads, dk, dv, act_silu, unit_eps, beta, decay_logits,
+                       rotary) -> bool:
+        """Whether the step's prompt portions go through the recurrence in chunks of rows
+        (`csrc/recurrent_chunks.cu`): bfloat16, a constant decay per head, square states of 64 or 128.
+        (float32 stays with the step by step form, whose sums do not depend on the cut.)"""
+        n = getattr(batch, "num_prefill_requests", 0)
+        if not (n and self.use_scan_chunks and q.dtype == torch.bfloat16 and dk == dv and dk in (64, 128)
+                and unit_eps is None and beta is None and decay_logits is None):
+            return False
+        rot = rotary[2] if rotary is not None else 0
+        if rot % 8 or (rot and act_silu) or any(t.stride(0) % 4 or t.data_ptr() % 8 for t in (q, k, v)):
+            return False
+        return (batch.num_prefill_tokens >= self.SCAN_CHUNK_ROWS * dk * n
+                and batch.tiles[self.prefill_q_tile].shape[0] * heads * dk * dk * 4 <= self.SCAN_CHUNK_BYTES)
+
     def matrix_state_scan(self, q, k, v, state, batch, y, heads, qk_heads, dk, dv, *,
                           act_silu=False, unit_eps=None, q_scale=1.0, beta=None, decay_logits=None,
                           dt_bias=None, a_log=None, decay=None, rotary=None, prepare=None) -> None:
@@ -1616,7 +1637,8 @@ class CudaOps:
         q is multiplied by `q_scale` either way.  `rotary` = (positions [T], float64 inv_freq, dims): the
         pairs (i, i + dims / 2) of every q and k head turn by position * inv_freq[i] first.  y: float32
         [T, heads * dv].  `prepare` (None: by the
-        step's longest request) only chooses where q, k and g are computed; y is the same."""
+        step's longest request) only chooses where q, k and g are computed; y is the same.  Where it is
+        None, portions may go in chunks of rows (`scan_in_chunks`), which sum in another order."""
         _check(state, y, dt_bias, a_log, decay)
         for t in (q, k, v, beta, decay_logits):
             if t is not None and not (t.is_cuda and t.stride(1) == 1):
@@ -1627,6 +1649,8 @@ class CudaOps:
         for t in (dt_bias, a_log, decay):
             assert t is None or t.dtype == torch.float32
         max_rows = int(getattr(batch, "max_q_len", 0) or 0)
+        chunks = prepare is None and self.scan_in_chunks(q, k, v, batch, heads, qk_heads, dk, dv, act_silu,
+                                                         unit_eps, beta, decay_logits, rotary)
         if prepare is None:
             prepare = max_rows > self.SCAN_PREPARE_ROWS
         pos, freq, rot = rotary if rotary is not None else (None, None, 0)
@@ -1637,6 +1661,28 @@ class CudaOps:
             prepare = prepare or not 0 < max_rows <= self.SCAN_TURN_ROWS
         act, unit, ready = (3 if act_silu else 0), (0 if unit_eps is None else 1), 0
         vb_code = _code(v)
+        first = 0                     # requests in front of the ones that are left to the scan
+        if chunks:
+            n, heads_apart = batch.num_prefill_requests, heads // qk_heads
+            tiles = batch.tiles[self.prefill_q_tile]
+            n_rows = batch.num_prefill_tokens
+            angles = torch.empty(n_rows * rot, dtype=torch.float32, device=q.device) if rot else None
+            u = torch.empty(tiles.shape[0] * heads * dk * dk, dtype=torch.float32, device=q.device)
+            rc = self.lib.somi_matrix_state_chunks(
+                _ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(q.stride(0)), ctypes.c_longlong(k.stride(0)),
+                ctypes.c_longlong(v.stride(0)), ctypes.c_int(act), ctypes.c_float(q_scale), _ptr(decay),
+                _ptr(state), _ptr(batch.cu_q), _ptr(batch.state_slot), _ptr(tiles), ctypes.c_int(tiles.shape[0]),
+                ctypes.c_int(n), ctypes.c_int(n_rows), ctypes.c_int(heads), ctypes.c_int(heads_apart),
+                ctypes.c_int(dk), _ptr(pos), _ptr(freq), ctypes.c_int(rot), _ptr(angles), _ptr(u), _ptr(y),
+                self._stream())
+            self._done(rc, "matrix_state_chunks")
+            self.launches += 3 if rot else 2
+            if trace.active():
+                trace.note("matrix_state_chunks", n_rows * (2 * qk_heads * dk + heads * dv) * 2 + n_rows * heads * dv * 4
+                           + 2 * n * heads * dk * dv * 4, 5.0 * n_rows * heads * dk * dv)
+            if n == batch.num_requests:
+                return
+            first, max_rows, prepare = n, 1, False               # the single tokens
         if prepare:
             T, n = q.shape[0], q.shape[0] * qk_heads * dk
             n_g = T * heads * dk if decay_logits is not None else 0
@@ -1666,8 +1712,8 @@ class CudaOps:
             ctypes.c_longlong(beta.stride(0) if beta is not None else 0), _ptr(decay_logits),
             ctypes.c_longlong(decay_logits.stride(0) if decay_logits is not None else 0),
             ctypes.c_int(ready),
-            _ptr(dt_bias), _ptr(a_log), _ptr(decay), _ptr(state), _ptr(batch.cu_q),
-            _ptr(batch.state_slot), _ptr(y), ctypes.c_int(batch.num_requests), ctypes.c_int(heads),
+            _ptr(dt_bias), _ptr(a_log), _ptr(decay), _ptr(state), _ptr(batch.cu_q[first:]),
+            _ptr(batch.state_slot[first:]), _ptr(y), ctypes.c_int(batch.num_requests - first), ctypes.c_int(heads),
             ctypes.c_int(qk_heads), ctypes.c_int(dk), ctypes.c_int(dv),
             ctypes.c_int(max_rows), _ptr(pos), _ptr(freq), ctypes.c_int(rot), self._stream())
         self._done(rc, "matrix_state_scan")

@@ -1,0 +1,69 @@
+"""The recurrence with a constant decay in chunks of 64 rows, against the recurrence itself in 64 bits and
+against the step by step kernel: portions that end around a chunk, states that an earlier step left, single
+tokens beside them, rotated or activated inputs, grouped query and key heads."""
+
+import pytest
+import torch
+
+from tests.gpu_util import Steps
+from somi_inference_b200.parts.base import StateNeeds
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from somi_inference_b200.ops import cuda_ops
+    return cuda_ops()
+
+
+def turned(x, pos, freq):
+    half = freq.numel()
+    angle = pos.double()[:, None, None] * freq
+    c, s, a, b = torch.cos(angle), torch.sin(angle), x[..., :half], x[..., half:2 * half]
+    return torch.cat([a * c - b * s, b * c + a * s, x[..., 2 * half:]], -1)
+
+
+@pytest.mark.parametrize("H,G,d,rot,silu", [(3, 3, 128, 128, False), (4, 2, 64, 0, True), (2, 2, 64, 16, False), (2, 1, 128, 0, False)])
+def test_portions_in_chunks(ops, H, G, d, rot, silu):
+    g = torch.Generator().manual_seed(d + rot)
+    steps = Steps(ops, 6, state=StateNeeds({"s": ((H, d, d), torch.float32)}), dtype=torch.bfloat16, max_len=2048)
+    decay = torch.tensor([0.5, 0.97, 0.9995, 1.0][:H])
+    freq = 10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64) / max(1, rot // 2))
+    states = torch.zeros(6, H, d, d, dtype=torch.float64)
+    state = steps.mgr.view(0).state["s"]
+    for counts in ({0: 63, 1: 64, 2: 65, 3: 200, 4: 2, 5: 1000}, {0: 1, 1: 128, 2: 67, 3: 257, 4: 1, 5: 64}):
+        batch, where = steps.step(counts)
+        T = batch.num_tokens
+        x = torch.randn(T, 2 * G * d + H * d, generator=g).bfloat16()
+        q, k, v = x[:, :G * d].cuda(), x[:, G * d:2 * G * d].cuda(), x[:, 2 * G * d:].cuda()
+        args = (q, k, v)
+        kw = dict(act_silu=silu, q_scale=0.25, decay=decay.cuda(),
+                  rotary=(batch.positions, freq.cuda(), rot) if rot else None)
+        assert ops.scan_in_chunks(*args, batch, H, G, d, d, silu, None, None, None, kw["rotary"])
+        y, before = torch.full((T, H * d), float("nan"), device="cuda"), state.clone()
+        ops.matrix_state_scan(*args, state, batch, y, H, G, d, d, **kw)
+        by_step, s_step = torch.empty_like(y), before.clone()
+        ops.matrix_state_scan(*args, s_step, batch, by_step, H, G, d, d, prepare=True, **kw)
+        want = torch.empty(T, H, d, dtype=torch.float64)
+        act = torch.nn.functional.silu if silu else (lambda t: t)
+        for r, (row, n, ctx) in where.items():
+            xs = x[row:row + n].double()
+            qq, kk, vv = (t.reshape(n, -1, d) for t in (xs[:, :G * d], xs[:, G * d:2 * G * d], xs[:, 2 * G * d:]))
+            pos = torch.arange(ctx, ctx + n)
+            qq, kk, vv = act(turned(qq, pos, freq)) * 0.25, act(turned(kk, pos, freq)), act(vv)
+            qq, kk = qq.repeat_interleave(H // G, 1), kk.repeat_interleave(H // G, 1)
+            m = states[r]
+            for t in range(n):
+                m = decay.double()[:, None, None] * m + kk[t][:, :, None] * vv[t][:, None, :]
+                want[row + t] = torch.einsum("hk,hkv->hv", qq[t], m)
+            states[r] = m
+        slots = {r: int(batch.host.state_slot[j]) for j, r in enumerate(batch.host.requests)}
+        want = want.reshape(T, -1)
+        got_s = torch.stack([state[slots[r]].double().cpu().transpose(1, 2) for r in range(6)])
+        step_s = torch.stack([s_step[slots[r]].double().cpu().transpose(1, 2) for r in range(6)])
+        # float32 sums either way: no further off than the step by step form by more than a few roundings
+        for got, step, ref in ((y.double().cpu(), by_step.double().cpu(), want), (got_s, step_s, states)):
+            off, limit = (got - ref).norm() / ref.norm(), (step - ref).norm() / ref.norm()
+            assert off <= 1.5 * limit + 2e-7, (off, limit)
+            assert (got - ref).abs().max() <= 2e-5 * ref.abs().max()
