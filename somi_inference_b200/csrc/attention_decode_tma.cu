@@ -121,9 +121,10 @@ paged_decode_tma_kernel(const __grid_constant__ CUtensorMap kv_map,
     const int chunk_page0 = k0 / page_size;
     const int newest_page = (rg.kv_len - 1) / page_size;                  // written by the predecessor
 
-    // Warp 0 starts the copies before anything else: lane 0 arms both barriers with the byte
-    // counts, then one lane per page looks its page up and issues that page's copies, so the
-    // page-table reads run side by side instead of one after another.
+    // The copies start before anything else: one thread arms both barriers with the byte counts, then
+    // every warp issues a quarter of the copies (keys or values, a half of the head or every other
+    // page), one lane per page, so the page-table reads run side by side and no thread has more than a few
+    // copies to issue (a warp issues one every hundred-odd cycles).
     if (warp == 0) {
         const unsigned used = __ballot_sync(0xffffffffu, lane < pages_in_chunk && rg.needs(chunk_page0 + lane, page_size));
         if (lane == 0) {
@@ -134,22 +135,18 @@ paged_decode_tma_kernel(const __grid_constant__ CUtensorMap kv_map,
             mbar_expect_tx(bar_k, bytes);
             mbar_expect_tx(bar_v, bytes);
         }
-        __syncwarp();
-        for (int p = lane; p < pages_in_chunk; p += 32) {
-            const int ap = chunk_page0 + p;
-            if (!rg.needs(ap, page_size) || ap == newest_page) continue;
-            const long long prow = (static_cast<long long>(ld_step(bt + ap)) * nkv + kvh) * page_size;
-            const int r = p * page_size;
-#pragma unroll
-            for (int h = 0; h < HALVES; ++h)
-                tma_load_2d(smem_u32(Ks + h * kHalfBytes + r * 128), &kv_map, h * 64,
-                            static_cast<int>(k_row0 + prow), bar_k);
-#pragma unroll
-            for (int h = 0; h < HALVES; ++h)
-                tma_load_2d(smem_u32(Vs + h * kHalfBytes + r * 128), &kv_map, h * 64,
-                            static_cast<int>(v_row0 + prow), bar_v);
-        }
     }
+    __syncthreads();       // no copy before its bytes are announced
+    const bool values = warp >= 2;
+    const int half = HALVES == 2 ? warp & 1 : 0;
+    auto copy_page = [&](int p) {
+        const long long prow = (static_cast<long long>(ld_step(bt + chunk_page0 + p)) * nkv + kvh) * page_size;
+        tma_load_2d(smem_u32((values ? Vs : Ks) + half * kHalfBytes + p * page_size * 128), &kv_map, half * 64,
+                    static_cast<int>((values ? v_row0 : k_row0) + prow), values ? bar_v : bar_k);
+    };
+    const bool my_page = lane < pages_in_chunk && (HALVES == 2 || (lane & 1) == (warp & 1)) &&
+                         rg.needs(chunk_page0 + lane, page_size);
+    if (my_page && chunk_page0 + lane != newest_page) copy_page(lane);
     // V rows of pages that are not loaded must not hold stale non-finite bit patterns
     for (int p = 0; p < pages_in_chunk; ++p) {
         const int ap = chunk_page0 + p;
@@ -160,20 +157,7 @@ paged_decode_tma_kernel(const __grid_constant__ CUtensorMap kv_map,
         }
     }
     pdl_wait();
-    if (warp == 0 && newest_page >= chunk_page0 && newest_page < chunk_page0 + pages_in_chunk &&
-        lane == newest_page - chunk_page0) {
-        const int p = newest_page - chunk_page0;
-        const long long prow = (static_cast<long long>(ld_step(bt + newest_page)) * nkv + kvh) * page_size;
-        const int r = p * page_size;
-#pragma unroll
-        for (int h = 0; h < HALVES; ++h)
-            tma_load_2d(smem_u32(Ks + h * kHalfBytes + r * 128), &kv_map, h * 64,
-                        static_cast<int>(k_row0 + prow), bar_k);
-#pragma unroll
-        for (int h = 0; h < HALVES; ++h)
-            tma_load_2d(smem_u32(Vs + h * kHalfBytes + r * 128), &kv_map, h * 64,
-                        static_cast<int>(v_row0 + prow), bar_v);
-    }
+    if (my_page && chunk_page0 + lane == newest_page) copy_page(lane);
     // Q: rows of the group's heads, zero rows up to 16
     const __nv_bfloat16* qrow = qkv + static_cast<size_t>(row) * row_stride + static_cast<size_t>(kvh) * (nq / nkv) * HD;
     for (int c = tid; c < kTdRows * CPR; c += kTdThreads) {
