@@ -22,7 +22,7 @@
 namespace somi {
 
 constexpr int kF32Chunk = 64;         // keys per chunk
-constexpr int kF32Rows = 64;          // query rows of a portion's CTA
+constexpr int kF32Rows = 64;          // query rows of a tile of the list
 constexpr int kF32Heads = 8;          // query heads a split CTA takes at a time
 
 __device__ __forceinline__ void f32_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
@@ -62,27 +62,31 @@ __device__ __forceinline__ float f32_merge_out(float o, float oc, float2 f) {
 }
 
 // ------------------------------------------------------------------------- prompt portions
-template <int HD>
+// A CTA takes 16 RI rows of a tile of 64: share blockIdx.z of it.
+template <int HD, int RI>
 __global__ void __launch_bounds__(256)
 attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, const float* __restrict__ kcache,
                              const float* __restrict__ vcache, const int* __restrict__ block_table,
                              int bt_stride, const int* __restrict__ cu_q, const int* __restrict__ ctx_len,
                              const int* __restrict__ tiles, int n_tiles, int nq, int nkv, int page_size,
                              float scale, int window, float* __restrict__ out) {
+    constexpr int ROWS = 16 * RI;
     constexpr int P = HD + 4;            // floats between rows of Q and K: neighbours in different banks
     constexpr int PP = kF32Chunk + 4;
     constexpr int COLS = HD / 16;        // output columns a thread
     extern __shared__ __align__(16) float f32_smem[];
-    float* Qs = f32_smem;                // [64][P]
-    float* Ks = Qs + kF32Rows * P;       // [64][P]
+    float* Qs = f32_smem;                // [ROWS][P]
+    float* Ks = Qs + ROWS * P;       // [64][P]
     float* Vs = Ks + kF32Chunk * P;      // [64][HD]
-    float* Ps = Vs + kF32Chunk * HD;     // [64][PP]
-    __shared__ float M_s[kF32Rows], L_s[kF32Rows];
-    __shared__ float2 f_s[kF32Rows];
+    float* Ps = Vs + kF32Chunk * HD;     // [ROWS][PP]
+    __shared__ float M_s[ROWS], L_s[ROWS];
+    __shared__ float2 f_s[ROWS];
     pdl_launch_dependents();
     pdl_wait();
     const int* tile = tiles + 3 * (n_tiles - 1 - static_cast<int>(blockIdx.x));   // a prompt's last rows first
-    const int req = tile[0], row0 = tile[1], rows = tile[2], head = blockIdx.y;
+    const int req = tile[0], row0 = tile[1] + blockIdx.z * ROWS, head = blockIdx.y;
+    const int rows = min(ROWS, tile[2] - static_cast<int>(blockIdx.z) * ROWS);
+    if (rows <= 0) return;
     const int kvh = head / (nq / nkv);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int pos0 = ctx_len[req] + (row0 - cu_q[req]);
@@ -102,20 +106,20 @@ attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, cons
     const int c_first = first_key / kF32Chunk, c_end = (end_key + kF32Chunk - 1) / kF32Chunk;
     load(Ks, P, kcache, c_first);
     load(Vs, HD, vcache, c_first);
-    for (int idx = tid; idx < kF32Rows * (HD / 4); idx += 256) {
+    for (int idx = tid; idx < ROWS * (HD / 4); idx += 256) {
         const int r = idx / (HD / 4), d = idx % (HD / 4) * 4;
         float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < rows)
             q = *reinterpret_cast<const float4*>(qkv + static_cast<size_t>(row0 + r) * row_stride + head * HD + d);
         *reinterpret_cast<float4*>(Qs + r * P + d) = make_float4(q.x * scale, q.y * scale, q.z * scale, q.w * scale);
     }
-    if (tid < kF32Rows) { M_s[tid] = -INFINITY; L_s[tid] = 0.f; }
+    if (tid < ROWS) { M_s[tid] = -INFINITY; L_s[tid] = 0.f; }
     // scores: rows tr + 16 i, keys tc + 16 j, the lanes of a warp 4 x 8 of them; outputs: rows
     // tr + 16 i, columns four neighbours from 4 tc (and 64 further on)
     const int tr = warp / 2 * 4 + lane / 8, tc = warp % 2 * 8 + lane % 8;
-    float O[4][COLS];
+    float O[RI][COLS];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
         for (int e = 0; e < COLS; ++e) O[i][e] = 0.f;
 
@@ -123,9 +127,9 @@ attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, cons
         f32_wait<1>();                                   // the keys; the values may be under way
         __syncthreads();
         {
-            unsigned long long acc[4][4];
+            unsigned long long acc[RI][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RI; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
 #pragma unroll 4
@@ -134,7 +138,7 @@ attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, cons
 #pragma unroll
                 for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const ulonglong2*>(Ks + (tc + 16 * j) * P + d);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < RI; ++i) {
                     const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(Qs + (tr + 16 * i) * P + d);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) f32_fma2(acc[i][j], q.x, k[j].x);
@@ -143,7 +147,7 @@ attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, cons
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RI; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int r = tr + 16 * i, n = tc + 16 * j, key = c * kF32Chunk + n, pos = pos0 + r;
@@ -154,7 +158,7 @@ attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, cons
         __syncthreads();
         const bool more = c + 1 < c_end;
         if (more) load(Ks, P, kcache, c + 1);
-        for (int r = warp * 8; r < warp * 8 + 8; ++r) {
+        for (int r = warp * 2 * RI; r < (warp + 1) * 2 * RI; ++r) {
             float s0 = Ps[r * PP + lane], s1 = Ps[r * PP + lane + 32];
             const float2 ml = f32_chunk_softmax(s0, s1);
             Ps[r * PP + lane] = s0;
@@ -168,16 +172,16 @@ attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, cons
         }
         if (more) f32_wait<1>(); else f32_wait<0>();     // the values
         __syncthreads();
-        float oc[4][COLS];
+        float oc[RI][COLS];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < RI; ++i)
 #pragma unroll
             for (int e = 0; e < COLS; ++e) oc[i][e] = 0.f;
 #pragma unroll 4
         for (int n = 0; n < kF32Chunk; n += 4) {
-            float4 p[4];
+            float4 p[RI];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(Ps + (tr + 16 * i) * PP + n);
+            for (int i = 0; i < RI; ++i) p[i] = *reinterpret_cast<const float4*>(Ps + (tr + 16 * i) * PP + n);
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
                 float v[COLS];
@@ -187,7 +191,7 @@ attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, cons
                     v[e] = t.x; v[e + 1] = t.y; v[e + 2] = t.z; v[e + 3] = t.w;
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < RI; ++i) {
                     const float w = m == 0 ? p[i].x : (m == 1 ? p[i].y : (m == 2 ? p[i].z : p[i].w));
 #pragma unroll
                     for (int e = 0; e < COLS; ++e) oc[i][e] = __fmaf_rn(w, v[e], oc[i][e]);
@@ -195,7 +199,7 @@ attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, cons
             }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < RI; ++i) {
             const float2 f = f_s[tr + 16 * i];
 #pragma unroll
             for (int e = 0; e < COLS; ++e) O[i][e] = f32_merge_out(O[i][e], oc[i][e], f);
@@ -204,7 +208,7 @@ attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, cons
         if (more) load(Vs, HD, vcache, c + 1);
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < RI; ++i) {
         const int r = tr + 16 * i;
         if (r >= rows) continue;
         const float L = L_s[r];
@@ -355,7 +359,7 @@ attention_f32_merge_kernel(const float* __restrict__ part_o, const float2* __res
 }
 
 template <int HD>
-constexpr int f32_portion_smem() { return 4 * (2 * 64 * (HD + 4) + 64 * HD + 64 * (kF32Chunk + 4)); }
+constexpr int f32_portion_smem(int rows) { return 4 * ((rows + 64) * (HD + 4) + 64 * HD + rows * (kF32Chunk + 4)); }
 template <int HD>
 constexpr int f32_split_smem() { return 4 * (64 * (HD + 4) + 64 * HD + kF32Heads * (HD + 4 + kF32Chunk + 4)); }
 
@@ -381,14 +385,25 @@ SOMI_API int somi_attention_f32_portion(const float* qkv, int row_stride, const 
     if (n_tiles <= 0) return 0;
     if (!somi_attention_f32_supported(qkv, kcache, vcache, out, row_stride, nq, nkv, hd) || page_size <= 0)
         return SOMI_ERR_UNSUPPORTED;
+    // Few tiles: two or four CTAs share one, each with a part of its rows (the same bits).  Layer of 14 heads over 2
+    // of 64 with 1 / 2 / 4 shares: 64 rows behind 2,000 positions (14 CTAs of 64 rows) 312 / 222 / 189 us, 203 rows
+    // (56) 79 / 76 / 79, 1,024 (224) 333 / 311 / 351, 2,048 (448) 737 / 781 / 935.
+    const long long ctas = static_cast<long long>(n_tiles) * nq;
+    const int shares = ctas <= 148 / 4 ? 4 : (ctas <= 148 * 2 ? 2 : 1);
     auto go = [&](auto kernel, int smem) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        launch_pdl(kernel, dim3(n_tiles, nq), dim3(256), smem, stream, qkv, row_stride, kcache, vcache, block_table,
+        launch_pdl(kernel, dim3(n_tiles, nq, shares), dim3(256), smem, stream, qkv, row_stride, kcache, vcache, block_table,
                    bt_stride, cu_q, ctx_len, tiles, n_tiles, nq, nkv, page_size, scale, window, out);
         return launch_status();
     };
-    return hd == 64 ? go(attention_f32_portion_kernel<64>, f32_portion_smem<64>())
-                    : go(attention_f32_portion_kernel<128>, f32_portion_smem<128>());
+    const int rows = kF32Rows / shares;
+    if (hd == 64)
+        return shares == 1 ? go(attention_f32_portion_kernel<64, 4>, f32_portion_smem<64>(rows))
+             : shares == 2 ? go(attention_f32_portion_kernel<64, 2>, f32_portion_smem<64>(rows))
+                           : go(attention_f32_portion_kernel<64, 1>, f32_portion_smem<64>(rows));
+    return shares == 1 ? go(attention_f32_portion_kernel<128, 4>, f32_portion_smem<128>(rows))
+         : shares == 2 ? go(attention_f32_portion_kernel<128, 2>, f32_portion_smem<128>(rows))
+                       : go(attention_f32_portion_kernel<128, 1>, f32_portion_smem<128>(rows));
 }
 
 // Single-token requests: request req_base + i, row row_base + i.  part: n_decode * nq * max_chunks * (hd + 2)
