@@ -9,8 +9,8 @@
 // window, the keys at positions below `keep` stay visible to all later tokens.  `maps`: a key/value
 // head holds that many keys of `hd` elements side by side in one cache row; query head i reads key
 // i % maps of key/value head i / (nq / nkv) (maps neighbouring query heads share a value head's keys).
-// It is the float32 path's attention and the fallback of the bfloat16 path for
-// sizes that the tensor-core kernels refuse.  Products are accumulated with
+// It is the attention of the float32 path where attention_f32.cu does not take the sizes, the mask or the
+// epilogue, and the fallback of the bfloat16 path for sizes that the tensor-core kernels refuse.  Products are accumulated with
 // float32 FMAs, softmax is float32 and online, key tiles are aligned to
 // multiples of BN from position 0, so the arithmetic on one query row does not
 // depend on how its request was cut into steps or on what else is in the batch.

@@ -23,7 +23,8 @@ gate.  `retention` (at the end of the file): rotated queries and keys, a constan
 Products run in the compute dtype with float32 accumulation; unit norms, beta, the decays with
 their softplus and exponentials, the recurrence, the norms and the gates' sigmoids are float32 in
 the kernels.  One kernel walks through a request's rows of the step, so a sequence may arrive
-in portions of any size.
+in portions of any size; portions of some length with a constant decay (bfloat16) go in chunks of
+rows instead (`csrc/recurrent_chunks.cu`), whose sums group differently from cut to cut (rounding only).
 """
 
 from __future__ import annotations

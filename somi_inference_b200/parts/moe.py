@@ -9,8 +9,8 @@
           sizes and limit of its own, that every token passes)
 There is no router product.  Gate and up rows are interleaved, so that the activation can be a
 product's epilogue.  Three ways through the routed experts, by the step's size and dtype:
-  * few (token, expert) pairs, bfloat16: every pair streams the rows of its own expert (a
-    matrix-vector kernel; nothing is sorted);
+  * few (token, expert) pairs, bfloat16: up to four pairs of an expert stream its rows together (a
+    matrix-vector kernel; nothing is sorted in memory);
   * many pairs, bfloat16: the pairs are grouped by expert on the device, the rows gathered in that
     order, and the library's grouped product runs over them, as the engine's prompt-sized products
     run in the library; the activation is a kernel between the two products;
