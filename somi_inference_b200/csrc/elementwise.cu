@@ -303,8 +303,8 @@ __global__ void rope_store_kernel(T* __restrict__ qkv, const int* __restrict__ p
     }
 }
 
-// The bfloat16 case for many tokens: four tokens per CTA (one, while that still leaves fewer
-// CTAs than four per SM: steps of a few dozen decode tokens), 16-byte accesses.
+// The bfloat16 case for many tokens: four tokens per CTA (one or two, while that still leaves fewer
+// CTAs than four per SM: steps of a few dozen decode tokens, short prompts), 16-byte accesses.
 // A work item is 8 consecutive dims of one head: a rotated pair of 8-dim groups (i, i + rot/2)
 // of a query or key head, 8 unrotated key dims, or 8 value dims.  Needs rot/2, hd - rot and hd
 // to be multiples of 8 and 16-byte aligned rows.
@@ -679,8 +679,12 @@ SOMI_API int somi_rope_store(void* qkv, int dtype, const int* positions, const f
     const auto aligned16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (dtype == SOMI_BF16 && T > 32 && rot > 0 && (rot & 15) == 0 && ((hd - rot) & 7) == 0 &&
         (hd & 7) == 0 && aligned16(qkv) && aligned16(kcache) && aligned16(vcache)) {
-        const int toks = T <= 4 * 148 ? 1 : kRopeToks;
-        launch_pdl(rope_store_bf16x8_kernel, dim3((T + toks - 1) / toks), dim3(256),
+        // 28 heads over 4 of 128: 1,000 tokens 5.3 us with two a CTA against 6.3 with four, 2,048 8.3 against 7.6;
+        // 14 over 2 of 64, where four tokens are 320 items, 8,111 tokens 9.3 us with 128 threads against 10.7
+        const int toks = T <= 4 * 148 ? 1 : (T <= 8 * 148 ? 2 : kRopeToks);
+        const int items = (nq + nkv) * (rot >> 4) + nkv * ((hd - rot) >> 3) + nkv * (hd >> 3);
+        const int threads = toks * items <= 512 && toks == kRopeToks ? 128 : 256;
+        launch_pdl(rope_store_bf16x8_kernel, dim3((T + toks - 1) / toks), dim3(threads),
                    smem * toks, stream, static_cast<__nv_bfloat16*>(qkv), positions, inv_freq, T,
                    nq, nkv, hd, rot, slot_map, static_cast<__nv_bfloat16*>(kcache),
                    static_cast<__nv_bfloat16*>(vcache), page_size, toks);
