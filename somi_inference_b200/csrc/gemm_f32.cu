@@ -19,7 +19,7 @@
 //
 // What bounds it: a few rows stream the weights, so the tile is 64 weight rows by the rows rounded up
 // to 2, 4, 8, 16 or 32, with four 32-deep stages of cp.async in flight per CTA and the first ones
-// issued before the dependency wait (weights are constants).  More rows are bound by the FMA pipe: a
+// issued before the dependency wait (a model's weights are constants).  More rows are bound by the FMA pipe: a
 // 64 x 64 tile, 8 x 4 outputs a thread, operands read from shared memory four k at a time as one
 // 16-byte access (rows 36 floats apart, so eight neighbouring rows lie in different banks).  Up to 256 rows
 // a 32-row tile, of which there are twice as many, is the faster (896 x 4,864 at 207 rows 63 against 79 us,
@@ -118,7 +118,7 @@ template <int BM, int TM, int TN, bool VEC, bool CLUSTER>
 __global__ void __launch_bounds__(sg_threads<BM, TM, TN>())
 sgemm_nt_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                 float* __restrict__ y, int M, int N, int K, int ranges, int range_length, long long ldx,
-                long long ldy, long long bsx, long long bsw, long long bsy) {
+                long long ldy, long long bsx, long long bsw, long long bsy, int w_constant) {
     constexpr int THREADS = sg_threads<BM, TM, TN>();
     constexpr int ROWS_APART = BM / TM, COLS_APART = kSgBN / TN;
     extern __shared__ __align__(16) float sg_buf[];      // [stage][x rows | w rows][pitch]
@@ -145,9 +145,10 @@ sgemm_nt_kernel(const float* __restrict__ x, const float* __restrict__ w, const 
     const SgLoader<BM, THREADS, VEC> x_rows(sg_buf, x, ldx, m0, M, k_begin);
     auto load_w = [&](int s) { w_rows.copy(s, k_end, s % kSgStages * (STAGE * 4)); };
     auto load_x = [&](int s) { x_rows.copy(s, k_end, s % kSgStages * (STAGE * 4)); };
+    if (!w_constant) pdl_wait();
 #pragma unroll
     for (int s = 0; s < kSgStages - 1; ++s)
-        if (s < steps) load_w(s);                        // [constant]
+        if (s < steps) load_w(s);                        // [constant], or behind the wait
     pdl_wait();
 #pragma unroll
     for (int s = 0; s < kSgStages - 1; ++s) {
@@ -265,7 +266,7 @@ sgemm_nt_kernel(const float* __restrict__ x, const float* __restrict__ w, const 
 struct SgArgs {
     const float *x, *w, *bias;
     float* y;
-    int M, N, K, batch;
+    int M, N, K, batch, w_constant;
     long long ldx, ldy, bsx, bsw, bsy;
 };
 
@@ -281,7 +282,7 @@ int sg_launch_one(const SgArgs& a, int ranges, cudaStream_t stream) {
     launch_pdl_cluster(kernel, dim3(tiles_n * (CLUSTER ? ranges : 1), tiles_m, a.batch),
                        dim3(sg_threads<BM, TM, TN>()), smem, CLUSTER ? ranges : 1, stream, a.x, a.w, a.bias,
                        a.y, a.M, a.N, a.K, ranges, sg_range_length(a.K, ranges), a.ldx, a.ldy, a.bsx, a.bsw,
-                       a.bsy);
+                       a.bsy, a.w_constant);
     return launch_status();
 }
 
@@ -305,13 +306,15 @@ using namespace somi;
 // y_b[M, N] = x_b[M, K] w_b[N, K]^T (+ bias) for b in [0, batch), all float32.  Rows of x_b and y_b lie
 // ldx and ldy elements apart, rows of w_b K; product b's operands start b * bs{x,w,y} elements
 // after product 0's (so the heads of a [tokens, heads, width] tensor are a batch without a copy).
-// w must not be written by a kernel of the same step: it is read before the dependency wait.
+// w_constant: no kernel of the same step writes w (a model's weights), so it is read before the
+// dependency wait.
 SOMI_API int somi_gemm_f32_batched(const float* x, const float* w, const float* bias, float* y, int M,
                                    int N, int K, int batch, long long ldx, long long ldy,
-                                   long long bsx, long long bsw, long long bsy, cudaStream_t stream) {
+                                   long long bsx, long long bsw, long long bsy, int w_constant,
+                                   cudaStream_t stream) {
     if (M <= 0 || N <= 0 || batch <= 0) return 0;
     if (K <= 0 || batch > 65535 || ldx < K || ldy < N) return SOMI_ERR_UNSUPPORTED;
-    const SgArgs a{x, w, bias, y, M, N, K, batch, ldx, ldy, bsx, bsw, bsy};
+    const SgArgs a{x, w, bias, y, M, N, K, batch, w_constant, ldx, ldy, bsx, bsw, bsy};
     if (M <= 2) return sg_launch<2, 2, 1>(a, stream);
     if (M <= 4) return sg_launch<4, 4, 1>(a, stream);
     if (M <= 8) return sg_launch<8, 2, 2>(a, stream);
@@ -322,6 +325,6 @@ SOMI_API int somi_gemm_f32_batched(const float* x, const float* w, const float* 
 
 // y[M, N] = x[M, K] w[N, K]^T (+ bias), all float32, row-major.
 SOMI_API int somi_gemm_f32(const float* x, const float* w, const float* bias, float* y, int M, int N,
-                           int K, cudaStream_t stream) {
-    return somi_gemm_f32_batched(x, w, bias, y, M, N, K, 1, K, N, 0, 0, 0, stream);
+                           int K, int w_constant, cudaStream_t stream) {
+    return somi_gemm_f32_batched(x, w, bias, y, M, N, K, 1, K, N, 0, 0, 0, w_constant, stream);
 }

@@ -313,8 +313,10 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
 #pragma unroll
                 for (int j = 0; j < C; ++j) {
                     const float x = xs[(s + m) * D + tc + 16 * j];
+                    // (on the diagonal a later row's infinity must not meet a probability of zero)
+                    if (s + m <= tr + 16 * b) o[b][j] = fmaf(p[b].v[m], x, o[b][j]);
 #pragma unroll
-                    for (int i = b; i < 4; ++i) o[i][j] = fmaf(p[i].v[m], x, o[i][j]);
+                    for (int i = b + 1; i < 4; ++i) o[i][j] = fmaf(p[i].v[m], x, o[i][j]);
                 }
         }
     }

@@ -838,7 +838,7 @@ class CudaOps:
                 _ptr(xs), _ptr(w), None, _ptr(ys), ctypes.c_int(T), ctypes.c_int(N),
                 ctypes.c_int(K), ctypes.c_int(H), ctypes.c_longlong(xs.stride(1)),
                 ctypes.c_longlong(ys.stride(1)), ctypes.c_longlong(xs.stride(0)),
-                ctypes.c_longlong(N * K), ctypes.c_longlong(ys.stride(0)), self._stream())
+                ctypes.c_longlong(N * K), ctypes.c_longlong(ys.stride(0)), ctypes.c_int(0), self._stream())
             self._done(rc, "gemm_f32_batched")
             name = "gemm_f32_batched"
         else:
@@ -1968,10 +1968,11 @@ class CudaOps:
             return out, out2
         return out
 
-    def gemm_f32(self, x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+    def gemm_f32(self, x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
+                 constant: bool = False) -> torch.Tensor:
         """x[M, K] @ w[N, K]^T (+ bias) in float32 FMAs, each output summed over K in an order
-        that K alone fixes (the float32 path's product; the library's is not used there).  `w` is read before
-        the kernel waits for its predecessors: no kernel of the same step may write it."""
+        that K alone fixes (the float32 path's product; the library's is not used there).  `constant`: no
+        kernel of the same step writes `w` (a model's weights), and the kernel may read it before it waits."""
         _check(x, w, bias)
         M, K = x.shape
         N = w.shape[0]
@@ -1980,7 +1981,7 @@ class CudaOps:
             raise KernelError("gemm_f32 takes float32 x[M, K], w[N, K] and bias[N]")
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
         rc = self.lib.somi_gemm_f32(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), ctypes.c_int(M),
-                                    ctypes.c_int(N), ctypes.c_int(K), self._stream())
+                                    ctypes.c_int(N), ctypes.c_int(K), ctypes.c_int(1 if constant else 0), self._stream())
         self._done(rc, "gemm_f32")
         if trace.active():
             trace.note("gemm_f32", (N * K + M * K + M * N) * 4, 2.0 * M * N * K, detail=f"M={M} N={N} K={K}")

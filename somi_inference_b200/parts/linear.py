@@ -37,7 +37,7 @@ class Linear:
         if self.skinny(x):
             return self.ops.skinny_gemm(x, self.weight, self.bias, self.ops.GEMM_BF16)
         if self.own_f32(x):
-            return self.ops.gemm_f32(x, self.weight, self.bias)
+            return self.ops.gemm_f32(x, self.weight, self.bias, constant=True)
         y = F.linear(x, self.weight, self.bias)
         self._note(x, y)
         return y
@@ -81,7 +81,7 @@ class Linear:
         if self.skinny(x):
             return self.ops.skinny_gemm(x, self.weight, None, self.ops.GEMM_F32)
         if self.own_f32(x):
-            return self.ops.gemm_f32(x, self.weight, None)
+            return self.ops.gemm_f32(x, self.weight, None, constant=True)
         if x.dtype == torch.float32:
             y = F.linear(x, self.weight)
         elif _MM_TAKES_OUT_DTYPE:

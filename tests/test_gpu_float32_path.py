@@ -77,3 +77,30 @@ def test_attention_does_not_depend_on_the_cut(ops, window):
         qkv.copy_(whole[2][r:r + 1])
         got = run(ops, (mgr, batch, qkv, view, None), nq, nkv, hd, window)
         assert torch.equal(got[0], want[r]), r
+
+
+@pytest.mark.parametrize("window", [None, 40])
+def test_a_later_value_that_is_infinite_reaches_no_earlier_row(ops, window):
+    """The value of position 150 is infinite: rows in front of it (in its chunk and tile, too) and, under the
+    window, rows that have passed it keep their bits."""
+    nq, nkv, hd = 4, 2, 64
+    case = attention_case(ops, nq=nq, nkv=nkv, hd=hd, page_size=16, window=window, requests=[(100, 120)], dtype=torch.float32)
+    want = run(ops, case, nq, nkv, hd, window)
+    table = case[1].groups[0].block_table[0]
+    case[3].values[int(table[150 // 16]), :, 150 % 16] = float("inf")
+    got = run(ops, case, nq, nkv, hd, window)
+    sees = torch.arange(100, 220) >= 150
+    if window:
+        sees &= torch.arange(100, 220) < 150 + window
+    assert torch.equal(got[~sees.cuda()], want[~sees.cuda()])
+    assert not got[sees.cuda()].isfinite().any()
+
+
+def test_product_with_a_matrix_made_in_the_same_step(ops):
+    """`w` is an output of the kernel in front: without `constant` it is read behind that kernel."""
+    g = torch.Generator().manual_seed(4)
+    a, b, x = (torch.randn(n, 256, generator=g).cuda() for n in (256, 300, 5))
+    for _ in range(20):
+        w = ops.gemm_f32(b, a, constant=True)
+        y = ops.gemm_f32(x, w)
+        torch.testing.assert_close(y.double(), x.double() @ w.double().T, rtol=1e-4, atol=1e-2)

@@ -67,3 +67,21 @@ def test_portions_in_chunks(ops, H, G, d, rot, silu):
             off, limit = (got - ref).norm() / ref.norm(), (step - ref).norm() / ref.norm()
             assert off <= 1.5 * limit + 2e-7, (off, limit)
             assert (got - ref).abs().max() <= 2e-5 * ref.abs().max()
+
+
+def test_a_later_value_that_is_infinite_reaches_no_earlier_row(ops):
+    H, d, T = 2, 64, 200
+    g = torch.Generator().manual_seed(9)
+    x, decay = torch.randn(T, 3 * H * d, generator=g).bfloat16().cuda(), torch.full((H,), 0.9, device="cuda")
+    out = []
+    for value in (None, float("inf")):
+        steps = Steps(ops, 1, state=StateNeeds({"s": ((H, d, d), torch.float32)}), dtype=torch.bfloat16)
+        batch, _ = steps.step({0: T})
+        if value is not None:
+            x[75, 2 * H * d:] = value
+        y = torch.empty(T, H * d, device="cuda")
+        q, k, v = x[:, :H * d], x[:, H * d:2 * H * d], x[:, 2 * H * d:]
+        assert ops.scan_in_chunks(q, k, v, batch, H, H, d, d, False, None, None, None, None)
+        ops.matrix_state_scan(q, k, v, steps.mgr.view(0).state["s"], batch, y, H, H, d, d, decay=decay)
+        out.append(y)
+    assert torch.equal(out[0][:75], out[1][:75]) and not out[1][75].isfinite().any()
