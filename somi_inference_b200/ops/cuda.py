@@ -46,6 +46,18 @@ def _check(*tensors: torch.Tensor | None) -> None:
             raise KernelError("kernel arguments must be contiguous")
 
 
+class _TensorMap:
+    """A CUtensorMap in host memory, 128-byte aligned.  It goes into a call as the argument itself and not
+    as its address, so that the call holds it until the launch has copied it: the tables below
+    forget their maps when they are full, in the middle of a call that takes two as well."""
+
+    __slots__ = ("raw", "_as_parameter_")
+
+    def __init__(self) -> None:
+        self.raw = (ctypes.c_ubyte * 256)()
+        self._as_parameter_ = ctypes.c_void_p((ctypes.addressof(self.raw) + 127) & ~127)
+
+
 class CudaOps:
     name = "cuda"
 
@@ -210,21 +222,19 @@ class CudaOps:
         return dtype == torch.bfloat16 and bool(self.lib.somi_decode_supported(
             ctypes.c_int(nq), ctypes.c_int(nkv), ctypes.c_int(hd)))
 
-    def _kv_tensor_map(self, storage: torch.Tensor, hd: int, page_size: int):
+    def _kv_tensor_map(self, storage: torch.Tensor, hd: int, page_size: int) -> _TensorMap:
         """A TMA tensor map over a cache group's whole storage, seen as [rows, hd] bfloat16."""
         key = (storage.data_ptr(), storage.numel(), hd, page_size)
         entry = self._tensor_maps.get(key)
         if entry is None:
-            raw = (ctypes.c_ubyte * 256)()
-            addr = (ctypes.addressof(raw) + 127) & ~127
-            rc = self.lib.somi_make_kv_tensor_map(ctypes.c_void_p(addr), _ptr(storage),
+            entry = _TensorMap()
+            rc = self.lib.somi_make_kv_tensor_map(entry, _ptr(storage),
                                                   ctypes.c_longlong(storage.numel() // hd),
                                                   ctypes.c_int(hd), ctypes.c_int(page_size))
             if rc != 0:
                 raise KernelError(f"could not encode a tensor map over the cache (code {rc})")
-            entry = (raw, addr)
             self._tensor_maps[key] = entry
-        return entry[1]
+        return entry
 
     def set_decode_ring_chunks(self, chunks: int) -> None:
         """Chunks of 128 keys that one CTA of the TMA decode kernel walks through: 0 lets the
@@ -236,22 +246,20 @@ class CudaOps:
         """Programmatic dependent launch for all kernels of the library (on by default)."""
         self.lib.somi_set_pdl(ctypes.c_int(1 if on else 0))
 
-    def _q_tensor_map(self, qkv: torch.Tensor) -> int:
+    def _q_tensor_map(self, qkv: torch.Tensor) -> _TensorMap:
         key = (qkv.data_ptr(), qkv.shape[0], qkv.shape[1])
         entry = self._q_maps.get(key)
         if entry is None:
             if len(self._q_maps) > 4096:
                 self._q_maps.clear()
-            raw = (ctypes.c_ubyte * 256)()
-            addr = (ctypes.addressof(raw) + 127) & ~127
-            rc = self.lib.somi_make_q_tensor_map(ctypes.c_void_p(addr), _ptr(qkv),
+            entry = _TensorMap()
+            rc = self.lib.somi_make_q_tensor_map(entry, _ptr(qkv),
                                                  ctypes.c_longlong(qkv.shape[0]),
                                                  ctypes.c_longlong(qkv.shape[1]))
             if rc != 0:
                 raise KernelError(f"could not encode a tensor map over the projection buffer (code {rc})")
-            entry = (raw, addr)
             self._q_maps[key] = entry
-        return entry[1]
+        return entry
 
     def check_errors(self) -> None:
         """Raise if a kernel recorded that one of its bounded waits ran out (synchronises)."""
@@ -378,8 +386,8 @@ class CudaOps:
                 prefill_turned = True
                 tiles = batch.tiles[self.prefill_tc_q_tile]
                 rc = self.lib.somi_paged_attention_prefill_tc_shaped(
-                    ctypes.c_void_p(self._q_tensor_map(qkv)),
-                    ctypes.c_void_p(self._kv_tensor_map(storage, hd, page_size)),
+                    self._q_tensor_map(qkv),
+                    self._kv_tensor_map(storage, hd, page_size),
                     ctypes.c_longlong((kcache.data_ptr() - storage.data_ptr()) // row_bytes),
                     ctypes.c_longlong((vcache.data_ptr() - storage.data_ptr()) // row_bytes),
                     _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
@@ -391,7 +399,7 @@ class CudaOps:
             elif shaped and not two_tiles:
                 tiles = batch.tiles[self.prefill_q_tile]
                 rc = self.lib.somi_paged_attention_prefill_tma_shaped(
-                    ctypes.c_void_p(self._kv_tensor_map(storage, hd, page_size)), _ptr(qkv),
+                    self._kv_tensor_map(storage, hd, page_size), _ptr(qkv),
                     ctypes.c_int(qkv.shape[1]),
                     ctypes.c_longlong((kcache.data_ptr() - storage.data_ptr()) // row_bytes),
                     ctypes.c_longlong((vcache.data_ptr() - storage.data_ptr()) // row_bytes),
@@ -405,8 +413,8 @@ class CudaOps:
                 prefill_turned = True
                 tiles = batch.tiles[self.prefill_pp_q_tile]
                 rc = self.lib.somi_paged_attention_prefill_pp(
-                    ctypes.c_void_p(self._q_tensor_map(qkv)),
-                    ctypes.c_void_p(self._kv_tensor_map(storage, hd, page_size)),
+                    self._q_tensor_map(qkv),
+                    self._kv_tensor_map(storage, hd, page_size),
                     ctypes.c_longlong((kcache.data_ptr() - storage.data_ptr()) // row_bytes),
                     ctypes.c_longlong((vcache.data_ptr() - storage.data_ptr()) // row_bytes),
                     _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
@@ -419,8 +427,8 @@ class CudaOps:
                     and bool(self.lib.somi_prefill_tc_supported(*sizes))):
                 tiles = batch.tiles[self.prefill_tc_q_tile]
                 rc = self.lib.somi_paged_attention_prefill_tc(
-                    ctypes.c_void_p(self._q_tensor_map(qkv)),
-                    ctypes.c_void_p(self._kv_tensor_map(storage, hd, page_size)),
+                    self._q_tensor_map(qkv),
+                    self._kv_tensor_map(storage, hd, page_size),
                     ctypes.c_longlong((kcache.data_ptr() - storage.data_ptr()) // row_bytes),
                     ctypes.c_longlong((vcache.data_ptr() - storage.data_ptr()) // row_bytes),
                     _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
@@ -432,7 +440,7 @@ class CudaOps:
                   and bool(self.lib.somi_prefill_tma_supported(*sizes))):
                 tiles = batch.tiles[self.prefill_q_tile]
                 rc = self.lib.somi_paged_attention_prefill_tma(
-                    ctypes.c_void_p(self._kv_tensor_map(storage, hd, page_size)), _ptr(qkv),
+                    self._kv_tensor_map(storage, hd, page_size), _ptr(qkv),
                     ctypes.c_int(qkv.shape[1]),
                     ctypes.c_longlong((kcache.data_ptr() - storage.data_ptr()) // row_bytes),
                     ctypes.c_longlong((vcache.data_ptr() - storage.data_ptr()) // row_bytes),
@@ -525,7 +533,7 @@ class CudaOps:
                 k_row0 = (kcache.data_ptr() - storage.data_ptr()) // row_bytes
                 v_row0 = (vcache.data_ptr() - storage.data_ptr()) // row_bytes
                 rc = self.lib.somi_paged_attention_decode_tma(
-                    ctypes.c_void_p(self._kv_tensor_map(storage, hd, page_size)), _ptr(qkv),
+                    self._kv_tensor_map(storage, hd, page_size), _ptr(qkv),
                     ctypes.c_int(qkv.shape[1]), ctypes.c_int(batch.num_prefill_tokens),
                     ctypes.c_int(batch.num_prefill_requests), ctypes.c_int(n_decode),
                     ctypes.c_longlong(k_row0), ctypes.c_longlong(v_row0),
@@ -604,7 +612,7 @@ class CudaOps:
         decode = (paired and self.use_tma_decode and n_decode > 0
                   and bool(self.lib.somi_two_map_decode_supported(*sizes)))
         if prefill or decode:
-            kv_map = ctypes.c_void_p(self._kv_tensor_map(storage, vd, page_size))
+            kv_map = self._kv_tensor_map(storage, vd, page_size)
             rows = (ctypes.c_longlong((kcache.data_ptr() - storage.data_ptr()) // (vd * 2)),
                     ctypes.c_longlong((vcache.data_ptr() - storage.data_ptr()) // (vd * 2)))
 
@@ -616,7 +624,7 @@ class CudaOps:
         if prefill:
             tiles = batch.tiles[self.prefill_tc_q_tile]
             rc = self.lib.somi_two_map_attention_prefill(
-                ctypes.c_void_p(self._q_tensor_map(qkv)), kv_map, *rows, _ptr(group.block_table),
+                self._q_tensor_map(qkv), kv_map, *rows, _ptr(group.block_table),
                 ctypes.c_int(group.width), _ptr(batch.cu_q), _ptr(batch.ctx_len), _ptr(tiles),
                 ctypes.c_int(tiles.shape[0]), *sizes, *mask, *form, _ptr(gate),
                 ctypes.c_longlong(gate_stride), _ptr(out), self._stream())
@@ -946,7 +954,7 @@ class CudaOps:
                        detail=f"M={rows.shape[0]} N={kv_up.shape[0]} K={rank}")
         tiles = batch.tiles[self.prefill_pp_q_tile]
         rc = self.lib.somi_attention_prefill_pp_columns(
-            ctypes.c_void_p(self._q_tensor_map(q)), ctypes.c_void_p(self._q_tensor_map(expanded)),
+            self._q_tensor_map(q), self._q_tensor_map(expanded),
             ctypes.c_int(heads * dim), _ptr(table), ctypes.c_int(longest), _ptr(batch.cu_q), _ptr(batch.ctx_len),
             _ptr(tiles), ctypes.c_int(tiles.shape[0]), ctypes.c_int(heads), ctypes.c_int(dim),
             ctypes.c_float(scale), ctypes.c_int(win), _ptr(sinks), _ptr(out), self._stream())
@@ -1889,23 +1897,21 @@ class CudaOps:
         # 11.4-11.7); short K (few stages per CTA) and small matrices go to the library
         return M <= 16 or (K >= 2048 and (N * K >= (32 << 20) or K >= 4 * N))
 
-    def _gemm_map(self, t: torch.Tensor, box_rows: int) -> int:
+    def _gemm_map(self, t: torch.Tensor, box_rows: int) -> _TensorMap:
         key = (t.data_ptr(), t.shape[0], t.shape[1], box_rows)
         entry = self._gemm_maps.get(key)
         if entry is None:
             if len(self._gemm_maps) > 8192:
                 self._gemm_maps.clear()
-            raw = (ctypes.c_ubyte * 256)()
-            addr = (ctypes.addressof(raw) + 127) & ~127
-            rc = self.lib.somi_make_gemm_tensor_map(ctypes.c_void_p(addr), _ptr(t),
+            entry = _TensorMap()
+            rc = self.lib.somi_make_gemm_tensor_map(entry, _ptr(t),
                                                     ctypes.c_longlong(t.shape[0]),
                                                     ctypes.c_longlong(t.shape[1]),
                                                     ctypes.c_int(box_rows))
             if rc != 0:
                 raise KernelError(f"could not encode a tensor map over a {tuple(t.shape)} matrix (code {rc})")
-            entry = (raw, addr)
             self._gemm_maps[key] = entry
-        return entry[1]
+        return entry
 
     def skinny_gemm(self, x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
                     mode: int = 0, splits: int = 1, deep_ring: bool = False,
@@ -1946,7 +1952,7 @@ class CudaOps:
         deep_ring = deep_ring or ctas <= 148
         if mode == self.GEMM_XIELU_SIDE:
             rc = self.lib.somi_skinny_gemm_act(
-                ctypes.c_void_p(self._gemm_map(w, 128)), ctypes.c_void_p(self._gemm_map(x, box)),
+                self._gemm_map(w, 128), self._gemm_map(x, box),
                 ctypes.c_int(box), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
                 ctypes.c_int(1), ctypes.c_int(mode), _ptr(bias),
                 _code(bias) if bias is not None else _F32, _ptr(out), _ptr(out2),
@@ -1954,7 +1960,7 @@ class CudaOps:
                 ctypes.c_int(1 if deep_ring else 0), self._stream())
         else:
             rc = self.lib.somi_skinny_gemm(
-                ctypes.c_void_p(self._gemm_map(w, 128)), ctypes.c_void_p(self._gemm_map(x, box)),
+                self._gemm_map(w, 128), self._gemm_map(x, box),
                 ctypes.c_int(box), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
                 ctypes.c_int(splits), ctypes.c_int(mode), _ptr(bias),
                 _code(bias) if bias is not None else _F32, _ptr(out),
