@@ -371,6 +371,8 @@ SOMI_API int somi_matrix_state_chunks(const void* q, const void* k, const void* 
                                       float* y, cudaStream_t stream) {
     if (n_tiles <= 0 || n_req <= 0) return 0;
     const uintptr_t bits = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v);
+    if (decay == nullptr || (rot > 0 && (positions == nullptr || rot_freq == nullptr || angles == nullptr)))
+        return SOMI_ERR_UNSUPPORTED;
     if ((D != 64 && D != 128) || heads <= 0 || heads > 65535 || n_req > 65535 || group <= 0 || heads % group ||
         ((q_stride | k_stride | v_stride) & 3) || (bits & 7) || rot < 0 || rot > D || rot % 8 || (rot > 0 && (silu & 1)) ||
         ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(u)) & 15) || (reinterpret_cast<uintptr_t>(angles) & 15))

@@ -1656,6 +1656,8 @@ class CudaOps:
         assert decay_logits is None or decay_logits.dtype == torch.float32
         for t in (dt_bias, a_log, decay):
             assert t is None or t.dtype == torch.float32
+        if decay is None and decay_logits is None:
+            raise KernelError("matrix_state_scan takes a decay per head, or decay logits")
         max_rows = int(getattr(batch, "max_q_len", 0) or 0)
         chunks = prepare is None and self.scan_in_chunks(q, k, v, batch, heads, qk_heads, dk, dv, act_silu,
                                                          unit_eps, beta, decay_logits, rotary)

@@ -2,11 +2,13 @@
 refuses before it launches anything.  The library is a stand-in whose functions are called through ctypes."""
 
 import ctypes
+from types import SimpleNamespace
 
 import pytest
 import torch
 
 from somi_inference_b200.ops import cuda
+from somi_inference_b200.ops.build import build
 
 P, I, L, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 
@@ -48,3 +50,42 @@ def test_maps_stay_alive_until_their_launch_returns(ops):
         w, x = store[2 * i:2 * i + 1], store[2 * i + 1:2 * i + 2]
         ops.skinny_gemm(x, w)
     assert len(launches) == 4200 and churn and not bad
+
+
+class OnDevice(torch.Tensor):
+    """A CPU tensor that the host side takes for one of the device's."""
+    is_cuda = True
+
+
+def on_device(*shape, dtype=torch.float32):
+    return torch.zeros(*shape, dtype=dtype).as_subclass(OnDevice)
+
+
+def test_a_recurrence_without_a_decay_is_refused(ops):
+    """Neither a decay per head nor decay logits, whichever way the rows would go: portions in chunks, short
+    portions, single tokens."""
+    launches = []
+    for name in ("somi_matrix_state_chunks", "somi_matrix_state_prepare", "somi_matrix_state_scan"):
+        setattr(ops.lib, name, lambda *args: launches.append(args) or 0)
+    ops.use_scan_chunks, ops.prefill_q_tile = True, 64
+    H, d, T = 2, 64, 80
+    for n_portions in (1, 0):
+        batch = SimpleNamespace(num_tokens=T, num_requests=1, num_prefill_requests=n_portions, max_q_len=T,
+                                num_prefill_tokens=T * n_portions, cu_q=on_device(2), state_slot=on_device(1),
+                                tiles={64: torch.zeros(2 * n_portions, 3)})
+        qkv, state, y = on_device(T, 3 * H * d, dtype=torch.bfloat16), on_device(1, H, d, d), on_device(T, H * d)
+        with pytest.raises(cuda.KernelError, match="decay"):
+            ops.matrix_state_scan(qkv[:, :H * d], qkv[:, H * d:2 * H * d], qkv[:, 2 * H * d:], state, batch, y, H, H, d, d)
+    assert not launches
+
+
+def test_the_chunks_launcher_refuses_null_arguments():
+    """A launcher's checks come before its first launch, so they are the same without a device."""
+    lib = ctypes.CDLL(build(verbose=False))
+    at = P(1 << 16)
+
+    def call(decay=at, positions=at, freq=at, angles=at, rot=16):
+        return lib.somi_matrix_state_chunks(at, at, at, L(256), L(256), L(256), I(0), F(1), decay, at, at, at, at, I(1), I(1),
+                                            I(64), I(2), I(1), I(64), positions, freq, I(rot), angles, at, at, P(0))
+    assert call(decay=P(0)) == call(decay=P(0), rot=0) == cuda.ERR_UNSUPPORTED
+    assert call(positions=P(0)) == call(freq=P(0)) == call(angles=P(0)) == cuda.ERR_UNSUPPORTED
