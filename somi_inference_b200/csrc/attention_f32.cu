@@ -41,16 +41,18 @@ __device__ __forceinline__ void f32_commit() { asm volatile("cp.async.commit_gro
 template <int N>
 __device__ __forceinline__ void f32_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// The 64 probabilities of a row, two a lane, from its scores: maximum and sum over the chunk.
+// The 64 probabilities of a row, two a lane, from its scores: maximum and sum over the chunk.  A hidden key's
+// score is -infinity.  The maximum passes over a score that is not a number, so what a key adds is decided
+// by its own score: a NaN among hidden keys (m = -infinity) makes p and the sum NaN.
 __device__ __forceinline__ float2 f32_chunk_softmax(float& s0, float& s1) {
     const float m = warp_max(fmaxf(s0, s1));
-    s0 = m == -INFINITY ? 0.f : expf(s0 - m);
-    s1 = m == -INFINITY ? 0.f : expf(s1 - m);
+    s0 = s0 == -INFINITY ? 0.f : expf(s0 - m);
+    s1 = s1 == -INFINITY ? 0.f : expf(s1 - m);
     return make_float2(m, warp_sum(__fadd_rn(s0, s1)));
 }
 // (M, L) <- (M, L) merged with a chunk's; returns the factors of the old output and of the chunk's.
 __device__ __forceinline__ float2 f32_merge(float& M, float& L, float m, float l) {
-    if (m == -INFINITY) return make_float2(1.f, 0.f);            // the row sees nothing of the chunk
+    if (m == -INFINITY && l == 0.f) return make_float2(1.f, 0.f);     // the row sees nothing of the chunk
     const float top = fmaxf(M, m);
     const float2 f = make_float2(expf(M - top), expf(m - top));  // (M = -inf before the first chunk: 0)
     L = __fmaf_rn(l, f.y, __fmul_rn(L, f.x));

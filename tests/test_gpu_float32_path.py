@@ -104,3 +104,26 @@ def test_product_with_a_matrix_made_in_the_same_step(ops):
         w = ops.gemm_f32(b, a, constant=True)
         y = ops.gemm_f32(x, w)
         torch.testing.assert_close(y.double(), x.double() @ w.double().T, rtol=1e-4, atol=1e-2)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("window", [None, 67])
+@pytest.mark.parametrize("at", [0, 63, 64, 128])
+def test_a_score_that_is_no_number_reaches_every_row_that_sees_it(ops, hd, window, at):
+    """The key of position `at` is NaN: also where it is the only visible key of its chunk (the row at a chunk's
+    first position, a window's last key), the rows that see it are NaN, and the others keep their bits."""
+    nq, nkv, ps = 4, 2, 16
+    reqs = [(0, 200), (60, 10)] + [(n, 1) for n in (0, 63, 64, 128, 129, 130, 150)]
+    case = attention_case(ops, nq=nq, nkv=nkv, hd=hd, page_size=ps, window=window, requests=reqs, dtype=torch.float32)
+    batch = case[1]
+    want = run(ops, case, nq, nkv, hd, window)
+    sees, tables = [], batch.groups[0].block_table.cpu()
+    for i, (c, q) in enumerate(reqs):
+        page = int(tables[i, at // ps]) if at < c + q else -1
+        if page >= 0:                                    # (a window has taken back what nobody sees)
+            case[3].keys[page, :, at % ps] = float("nan")
+        sees += [at <= p and (window is None or at > p - window) for p in range(c, c + q)]
+    sees = torch.tensor(sees).cuda()
+    got = run(ops, case, nq, nkv, hd, window)
+    assert got[sees].isnan().all()
+    assert torch.equal(got[~sees], want[~sees])
