@@ -130,11 +130,9 @@ paged_attention_generic_kernel(const T* __restrict__ qkv, int row_stride,
                 const float s = Ss[m * (kBN + 1) + lane];
                 const float m_old = m_s[m];
                 const float m_new = fmaxf(m_old, warp_max(s));
-                float p = 0.f, alpha = 1.f;
-                if (m_new != -INFINITY) {
-                    alpha = expf(m_old - m_new);          // m_old = -inf gives 0
-                    p = expf(s - m_new);                   // s = -inf gives 0
-                }
+                // (the maximum passes over a NaN: what a key adds is decided by its own score)
+                const float alpha = m_new == -INFINITY ? 1.f : expf(m_old - m_new);    // m_old = -inf gives 0
+                const float p = s == -INFINITY ? 0.f : expf(s - m_new);
                 const float psum = warp_sum(p);
                 Ss[m * (kBN + 1) + lane] = p;
                 if (lane == 0) {

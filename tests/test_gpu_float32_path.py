@@ -106,12 +106,13 @@ def test_product_with_a_matrix_made_in_the_same_step(ops):
         torch.testing.assert_close(y.double(), x.double() @ w.double().T, rtol=1e-4, atol=1e-2)
 
 
-@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("hd", [64, 128, 32])
 @pytest.mark.parametrize("window", [None, 67])
 @pytest.mark.parametrize("at", [0, 63, 64, 128])
 def test_a_score_that_is_no_number_reaches_every_row_that_sees_it(ops, hd, window, at):
     """The key of position `at` is NaN: also where it is the only visible key of its chunk (the row at a chunk's
-    first position, a window's last key), the rows that see it are NaN, and the others keep their bits."""
+    first position, a window's last key), the rows that see it are NaN, and the others keep their bits.  (Head size
+    32 runs the kernel for any size.)"""
     nq, nkv, ps = 4, 2, 16
     reqs = [(0, 200), (60, 10)] + [(n, 1) for n in (0, 63, 64, 128, 129, 130, 150)]
     case = attention_case(ops, nq=nq, nkv=nkv, hd=hd, page_size=ps, window=window, requests=reqs, dtype=torch.float32)
