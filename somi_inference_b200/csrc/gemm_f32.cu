@@ -277,12 +277,15 @@ int sg_launch_one(const SgArgs& a, int ranges, cudaStream_t stream) {
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     const unsigned tiles_n = static_cast<unsigned>((a.N + kSgBN - 1) / kSgBN);
-    const unsigned tiles_m = static_cast<unsigned>((a.M + BM - 1) / BM);
-    if (tiles_m > 65535u) return SOMI_ERR_UNSUPPORTED;
-    launch_pdl_cluster(kernel, dim3(tiles_n * (CLUSTER ? ranges : 1), tiles_m, a.batch),
-                       dim3(sg_threads<BM, TM, TN>()), smem, CLUSTER ? ranges : 1, stream, a.x, a.w, a.bias,
-                       a.y, a.M, a.N, a.K, ranges, sg_range_length(a.K, ranges), a.ldx, a.ldy, a.bsx, a.bsw,
-                       a.bsy, a.w_constant);
+    // (a grid has at most 65,535 tiles of rows: 4.19 M rows go in one launch)
+    for (int m = 0; m < a.M;) {
+        const int rows = a.M - m < 65535 * BM ? a.M - m : 65535 * BM;
+        launch_pdl_cluster(kernel, dim3(tiles_n * (CLUSTER ? ranges : 1), (rows + BM - 1) / BM, a.batch),
+                           dim3(sg_threads<BM, TM, TN>()), smem, CLUSTER ? ranges : 1, stream, a.x + m * a.ldx, a.w,
+                           a.bias, a.y + m * a.ldy, rows, a.N, a.K, ranges, sg_range_length(a.K, ranges), a.ldx,
+                           a.ldy, a.bsx, a.bsw, a.bsy, a.w_constant);
+        m += rows;
+    }
     return launch_status();
 }
 

@@ -35,6 +35,15 @@ def test_product_at_the_bounds_of_tiles_and_ranges(ops, K, N):
         assert torch.equal(ops.gemm_f32(x[130 - m:].contiguous(), w, b), whole[130 - m:]), m
 
 
+def test_product_with_more_rows_than_a_grid_has_tiles(ops):
+    """65,535 tiles of 64 rows and 70 rows more: each product is a sum of four terms (five roundings)."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    M, K, N = 65535 * 64 + 70, 4, 3
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    y, bound = ops.gemm_f32(x, w), 5 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert ((y.double() - x.double() @ w.double().T).abs() <= bound).all()
+
+
 def run(ops, case, nq, nkv, hd, window):
     mgr, batch, qkv, view, order = case
     out = torch.full((batch.num_tokens, nq * hd), float("nan"), device="cuda")
