@@ -251,7 +251,8 @@ attention_f32_portion_kernel(const float* __restrict__ qkv, int row_stride, cons
 }
 
 // ------------------------------------------------------------------- single-token requests
-// part_o [request][query head][chunk][HD], part_ml likewise with (m, l); chunks counted from 0.
+// part_o [request][query head][chunk][HD], part_ml likewise with (m, l); a request's chunks are counted from the
+// one of its first visible key, so that a window needs no more of them than it reaches.
 template <int HD>
 __global__ void __launch_bounds__(128)
 attention_f32_split_kernel(const float* __restrict__ qkv, int row_stride, int row_base, int req_base,
@@ -267,11 +268,12 @@ attention_f32_split_kernel(const float* __restrict__ qkv, int row_stride, int ro
     float* Qs = Vs + kF32Chunk * HD;     // [8][P]
     float* Ps = Qs + kF32Heads * P;      // [8][PP]
     pdl_launch_dependents();
-    const int c = blockIdx.x, kvh = blockIdx.y, i = blockIdx.z, req = req_base + i;
+    const int kvh = blockIdx.y, i = blockIdx.z, req = req_base + i;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int pos = ld_step(ctx_len + req);              // [descriptor]
     const int first_key = window > 0 ? max(0, pos - window + 1) : 0;
-    if (c * kF32Chunk > pos || (c + 1) * kF32Chunk <= first_key) {
+    const int at = blockIdx.x, c = first_key / kF32Chunk + at;
+    if (c * kF32Chunk > pos) {
         pdl_wait();
         return;
     }
@@ -331,7 +333,7 @@ attention_f32_split_kernel(const float* __restrict__ qkv, int row_stride, int ro
             Ps[r * PP + lane] = s0;
             Ps[r * PP + lane + 32] = s1;
             if (lane == 0 && r < heads)
-                part_ml[(static_cast<size_t>(i) * nq + kvh * group + h0 + r) * max_chunks + c] = ml;
+                part_ml[(static_cast<size_t>(i) * nq + kvh * group + h0 + r) * max_chunks + at] = ml;
         }
         __syncthreads();
         const int d = tid % HD, r0 = tid / HD * OUT_ROWS;
@@ -355,7 +357,7 @@ attention_f32_split_kernel(const float* __restrict__ qkv, int row_stride, int ro
 #pragma unroll
         for (int r = 0; r < OUT_ROWS; ++r)
             if (r0 + r < heads)
-                part_o[((static_cast<size_t>(i) * nq + kvh * group + h0 + r0 + r) * max_chunks + c) * HD + d] = o[r];
+                part_o[((static_cast<size_t>(i) * nq + kvh * group + h0 + r0 + r) * max_chunks + at) * HD + d] = o[r];
     }
 }
 
@@ -368,10 +370,10 @@ attention_f32_merge_kernel(const float* __restrict__ part_o, const float2* __res
     pdl_launch_dependents();
     pdl_wait();
     const int pos = ctx_len[req_base + i];
-    const int first = (window > 0 ? max(0, pos - window + 1) : 0) / kF32Chunk, end = pos / kF32Chunk + 1;
+    const int end = pos / kF32Chunk + 1 - (window > 0 ? max(0, pos - window + 1) : 0) / kF32Chunk;
     const size_t base = (static_cast<size_t>(i) * nq + head) * max_chunks;
     float M = -INFINITY, L = 0.f, O = 0.f;
-    for (int c0 = first; c0 < end; c0 += 8) {            // eight chunks' loads in flight
+    for (int c0 = 0; c0 < end; c0 += 8) {            // eight chunks' loads in flight
         float2 ml[8];
         float o[8];
 #pragma unroll
@@ -438,7 +440,7 @@ SOMI_API int somi_attention_f32_portion(const float* qkv, int row_stride, const 
 }
 
 // Single-token requests: request req_base + i, row row_base + i.  part: n_decode * nq * max_chunks * (hd + 2)
-// floats, max_chunks at least the chunks of the longest request.
+// floats, max_chunks at least the chunks that the longest request's token sees keys of.
 SOMI_API int somi_attention_f32_single(const float* qkv, int row_stride, int row_base, int req_base, int n_decode,
                                        const float* kcache, const float* vcache, const int* block_table,
                                        int bt_stride, const int* ctx_len, int nq, int nkv, int hd, int page_size,

@@ -304,6 +304,10 @@ class CudaOps:
             flops += 4.0 * nq * hd * pairs
         return moved, flops
 
+    # The most that single tokens' partial results may take in float32 attention (a request at least): more
+    # requests go one group behind the other.  64 requests of 40 heads of 128 at 32,768 positions need 681 MB.
+    F32_PART_FLOATS = 1 << 25
+
     def paged_attention(self, qkv, kcache, vcache, batch, group, nq, nkv, hd, scale, window,
                         out, storage=None, value_dim=None, chunk=None, gate=None,
                         gate_per_head=False, softcap=None, sinks=None, turn=None) -> None:
@@ -482,18 +486,23 @@ class CudaOps:
                     trace.note("attention_f32_portion", *self._attention_work(
                         batch, 0, batch.num_prefill_requests, nq, nkv, hd, 4, win))
             if n_decode:
+                # (a window of n positions meets at most (n + 62) / 64 + 1 chunks of 64)
                 max_chunks = -(-group.width * page_size // self.f32_chunk)
-                part = torch.empty(n_decode * nq * max_chunks * (hd + 2), dtype=torch.float32,
-                                   device=qkv.device)
-                rc = self.lib.somi_attention_f32_single(
-                    _ptr(qkv), ctypes.c_int(qkv.shape[1]), ctypes.c_int(batch.num_prefill_tokens),
-                    ctypes.c_int(batch.num_prefill_requests), ctypes.c_int(n_decode), _ptr(kcache),
-                    _ptr(vcache), _ptr(group.block_table), ctypes.c_int(group.width),
-                    _ptr(batch.ctx_len), ctypes.c_int(nq), ctypes.c_int(nkv), ctypes.c_int(hd),
-                    ctypes.c_int(page_size), ctypes.c_float(scale), ctypes.c_int(win), _ptr(part),
-                    ctypes.c_int(max_chunks), _ptr(out), self._stream())
-                self._done(rc, "attention_f32_single")
-                self.launches += 1
+                if win:
+                    max_chunks = min(max_chunks, (win + self.f32_chunk - 2) // self.f32_chunk + 1)
+                each = nq * max_chunks * (hd + 2)
+                most = min(n_decode, max(1, self.F32_PART_FLOATS // each))
+                part = torch.empty(most * each, dtype=torch.float32, device=qkv.device)
+                for at in range(0, n_decode, most):
+                    rc = self.lib.somi_attention_f32_single(
+                        _ptr(qkv), ctypes.c_int(qkv.shape[1]), ctypes.c_int(batch.num_prefill_tokens + at),
+                        ctypes.c_int(batch.num_prefill_requests + at), ctypes.c_int(min(most, n_decode - at)),
+                        _ptr(kcache), _ptr(vcache), _ptr(group.block_table), ctypes.c_int(group.width),
+                        _ptr(batch.ctx_len), ctypes.c_int(nq), ctypes.c_int(nkv), ctypes.c_int(hd),
+                        ctypes.c_int(page_size), ctypes.c_float(scale), ctypes.c_int(win), _ptr(part),
+                        ctypes.c_int(max_chunks), _ptr(out), self._stream())
+                    self._done(rc, "attention_f32_single")
+                    self.launches += 1
                 if trace.active():
                     trace.note("attention_f32_single", *self._attention_work(
                         batch, batch.num_prefill_requests, batch.num_requests, nq, nkv, hd, 4, win),

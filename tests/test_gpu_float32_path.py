@@ -137,3 +137,15 @@ def test_a_score_that_is_no_number_reaches_every_row_that_sees_it(ops, hd, windo
     got = run(ops, case, nq, nkv, hd, window)
     assert got[sees].isnan().all()
     assert torch.equal(got[~sees], want[~sees])
+
+
+@pytest.mark.parametrize("window", [None, 1, 65, 70])
+def test_attention_of_single_tokens_in_groups(ops, monkeypatch, window):
+    """Requests one group behind the other over the same scratch: the same bits as all in one launch."""
+    nq, nkv, hd = 6, 2, 64
+    reqs = [(0, 70)] + [(n, 1) for n in (0, 63, 64, 65, 127, 128, 129, 130, 700)]
+    case = attention_case(ops, nq=nq, nkv=nkv, hd=hd, page_size=16, window=window, requests=reqs, dtype=torch.float32)
+    want = run(ops, case, nq, nkv, hd, window)
+    for requests in (1, 2, 4):
+        monkeypatch.setattr(ops, "F32_PART_FLOATS", requests * nq * (12 if window is None else (window + 62) // 64 + 1) * (hd + 2))
+        assert torch.equal(run(ops, case, nq, nkv, hd, window), want)

@@ -89,3 +89,28 @@ def test_the_chunks_launcher_refuses_null_arguments():
                                             I(64), I(2), I(1), I(64), positions, freq, I(rot), angles, at, at, P(0))
     assert call(decay=P(0)) == call(decay=P(0), rot=0) == cuda.ERR_UNSUPPORTED
     assert call(positions=P(0)) == call(freq=P(0)) == call(angles=P(0)) == cuda.ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("n,nq,nkv,hd,positions,window", [(64, 40, 8, 128, 32768, None), (64, 40, 8, 128, 32768, 1024),
+                                                          (3, 14, 2, 64, 512, None), (3, 14, 2, 64, 131072, 65)])
+def test_scratch_of_float32_single_tokens_is_bounded(ops, monkeypatch, n, nq, nkv, hd, positions, window):
+    """Every request is in one launch, no launch's partial results take more than 128 MB, and a window needs
+    only the chunks that it meets."""
+    calls, sizes = [], []
+    ops.lib.somi_attention_f32_supported = lambda *args: 1
+    ops.lib.somi_attention_f32_single = lambda *args: calls.append([getattr(a, "value", a) for a in args]) or 0
+    ops.use_f32_attention, ops.f32_chunk, ops.prefill_q_tile, ops.generic_q_tile = True, 64, 64, 16
+    kv = on_device(1, nkv, 16, hd)
+    group = SimpleNamespace(block_table=on_device(1, 1), width=positions // 16)
+    batch = SimpleNamespace(num_requests=n + 2, num_prefill_requests=2, num_prefill_tokens=70, cu_q=on_device(1),
+                            ctx_len=on_device(1), tiles={64: torch.zeros(0, 3), 16: torch.zeros(0, 3)})
+    real = torch.empty
+    monkeypatch.setattr(cuda.torch, "empty", lambda size, **kw: sizes.append(size) or real(1, **kw))
+    ops.paged_attention(on_device(1, (nq + 2 * nkv) * hd), kv, kv, batch, group, nq, nkv, hd, 1.0, window, on_device(1, nq * hd))
+    chunks = -(-positions // 64) if window is None else max((p + window - 1) // 64 - p // 64 + 1 for p in range(64))
+    at = 0
+    for row, request, count, most in ((c[2], c[3], c[4], c[-3]) for c in calls):
+        assert (row, request, most) == (70 + at, 2 + at, chunks)
+        assert count * nq * chunks * (hd + 2) <= sizes[0] <= (1 << 25)
+        at += count
+    assert at == n and len(sizes) == 1
