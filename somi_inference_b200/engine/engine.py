@@ -196,8 +196,8 @@ class Engine:
         """Forward pass of one batch.  A step is a sequence of a few hundred kernels; for
         single-token steps and for portions of a small model the host cannot issue them as fast
         as the GPU runs them.  So the kernel sequence is captured in a CUDA graph the second time
-        a layout (tokens and rows of every request class, tiles, table width, wanted rows) is
-        seen and replayed from then on; the batch descriptor lives at fixed device addresses, so
+        a layout (tokens and rows of every request class, tiles, table width, wanted rows, and what
+        parts enter beside it) is seen and replayed from then on; the batch descriptor lives at fixed device addresses, so
         a replay reads the new step's data."""
         self.last_batch = batch
         graphable = (self.use_graphs and self.device.type == "cuda" and self.model.graph_safe
@@ -209,7 +209,7 @@ class Engine:
             # the descriptor buffer moved: graphs captured over the old addresses are void
             self._graphs.clear()
             self._graph_generation = self.builder.generation
-        key = batch.layout_key
+        key = batch.layout_key + self.model.layout_facts(batch)
         entry = self._graphs.get(key)
         if entry is not None:
             graph, logits, launches = entry

@@ -909,16 +909,17 @@ class CudaOps:
     LATENT_EXPAND_ROWS = 96
     LATENT_EXPAND_POSITIONS = 32768     # the most that are expanded side by side (28 heads of 128: 470 MB)
 
-    def latent_expand_tiles(self, batch, group, page_size: int, window) -> int:
-        """Tiles of positions that the step's portions may read, by the layout alone (a captured step is
-        replayed with other cached lengths): a request of q rows sees at most window - 1 + q
-        positions, which fall into (that + 254) / 128 aligned tiles, and never more than its table has."""
-        n = batch.num_prefill_requests
-        longest = -(-group.width * page_size // self.latent_tile)
-        if not window:
-            return n * longest
-        t = self.latent_tile
-        return min(n * longest, (n * (int(window) - 1 + 2 * t - 2) + batch.num_prefill_tokens) // t)
+    def latent_expand_tiles(self, batch, window) -> int:
+        """Tiles of positions that the step's portions read, by their own lengths, rounded up to one of four
+        sizes per power of two.  A captured step is replayed with other lengths: the number belongs to what
+        its layout is told apart by (`BuildContext.layout_facts`)."""
+        t, win, n = self.latent_tile, int(window) if window else 0, 0
+        cu, ctx = batch.host.cu_q, batch.host.ctx_len
+        for r in range(batch.num_prefill_requests):
+            cached = int(ctx[r])
+            n += (cached + int(cu[r + 1] - cu[r]) - 1) // t + 1 - (max(0, cached - win + 1) // t if win else 0)
+        step = 1 << max(0, n.bit_length() - 3)
+        return -(-n // step) * step
 
     def latent_expands(self, batch, group, cache, heads: int, rank: int, key_dim: int, value_dim: int,
                        window, dtype) -> bool:
@@ -930,7 +931,7 @@ class CudaOps:
                                                             ctypes.c_int(key_dim), ctypes.c_int(self.latent_tile)))):
             return False
         return (batch.num_prefill_tokens >= self.LATENT_EXPAND_ROWS * n
-                and self.latent_expand_tiles(batch, group, cache.shape[2], window) * self.latent_tile
+                and self.latent_expand_tiles(batch, window) * self.latent_tile
                 <= self.LATENT_EXPAND_POSITIONS)
 
     def latent_portions(self, q, cache, kv_up, batch, group, heads, rank, dim, scale, window, sinks, out) -> None:
@@ -944,7 +945,7 @@ class CudaOps:
         assert q.dtype == cache.dtype == kv_up.dtype == out.dtype == torch.bfloat16
         assert tuple(kv_up.shape) == (2 * heads * dim, rank) and cache.shape[3] == rank
         assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == heads)
-        n_tiles = self.latent_expand_tiles(batch, group, page_size, window)
+        n_tiles = self.latent_expand_tiles(batch, window)
         longest = -(-group.width * page_size // t)
         rows = torch.empty((n_tiles * t, rank), dtype=q.dtype, device=q.device)
         table = torch.empty((n, longest), dtype=torch.int32, device=q.device)

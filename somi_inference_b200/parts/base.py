@@ -64,6 +64,10 @@ class BuildContext:
     dtype: torch.dtype            # compute dtype: torch.bfloat16 or torch.float32
     device: torch.device
     ops: Any                      # kernel table (ops.CudaOps on the product path)
+    # What a part's launches depend on beside a step's layout (its sizes): name -> function of the batch
+    # with a hashable result.  Parts that are alike enter the same name.  A captured step is replayed only
+    # for batches with equal layouts and equal facts.
+    layout_facts: dict = field(default_factory=dict)
 
     def place(self, t: torch.Tensor, *, matrix: bool) -> torch.Tensor:
         """Move a loaded tensor to the device in the precision it is held in.

@@ -106,6 +106,8 @@ class LatentAttentionMixer:
         # all heads' W_uk, then all heads' W_uv, for portions that read expanded keys and values
         self.kv_up = (torch.cat([tensors[n["k_up"]], tensors[n["v_up"]]], 0).contiguous()
                       if ctx.dtype == torch.bfloat16 and self.key_dim == self.value_dim else None)
+        if self.kv_up is not None:
+            ctx.layout_facts["latents", self.window] = lambda batch: ctx.ops.latent_expand_tiles(batch, self.window)
         self.gate = Linear(tensors[n["gate"]], None, ctx.ops) if params.get("gate") else None
 
     def _build_direct(self, params, tensors, n) -> None:

@@ -99,6 +99,12 @@ class Decoder:
         owners = [run.cache_of for run in self.schedule]
         return needs, owners
 
+    def layout_facts(self, batch) -> tuple:
+        """What the step's launches depend on beside its layout (nothing in a step of single tokens)."""
+        if not batch.num_prefill_requests:
+            return ()
+        return tuple(fact(batch) for fact in self.ctx.layout_facts.values())
+
     def forward(self, batch, cache) -> torch.Tensor:
         """Run the step's tokens; return float32 logits [len(batch.logit_rows), vocab]."""
         residual = self.embedding.forward(batch)

@@ -2,13 +2,17 @@
 refuses before it launches anything.  The library is a stand-in whose functions are called through ctypes."""
 
 import ctypes
+import random
 from types import SimpleNamespace
 
+import numpy as np
 import pytest
 import torch
 
+from somi_inference_b200.config.spec import PartSpec
 from somi_inference_b200.ops import cuda
 from somi_inference_b200.ops.build import build
+from somi_inference_b200.parts import MIXERS, BuildContext, Decoder
 
 P, I, L, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 
@@ -114,3 +118,74 @@ def test_scratch_of_float32_single_tokens_is_bounded(ops, monkeypatch, n, nq, nk
         assert count * nq * chunks * (hd + 2) <= sizes[0] <= (1 << 25)
         at += count
     assert at == n and len(sizes) == 1
+
+
+def portions(*lengths, singles=()):
+    """A step of portions (cached tokens, tokens) and single tokens behind them, as the kernel table reads it."""
+    reqs = [*lengths, *((c, 1) for c in singles)]
+    cu = np.cumsum([0] + [q for _, q in reqs])
+    T, widest = int(cu[-1]), max(c + q for c, q in reqs)
+    tiles = {t: torch.tensor([(r, cu[r] + i, min(t, q - i)) for r, (_, q) in enumerate(lengths) for i in range(0, q, t)],
+                             dtype=torch.int32).view(-1, 3) for t in (16, 64, 128, 256)}
+    return SimpleNamespace(
+        num_tokens=T, num_requests=len(reqs), num_prefill_requests=len(lengths), num_prefill_tokens=int(cu[len(lengths)]),
+        max_q_len=max(q for _, q in reqs), cu_q=on_device(len(reqs) + 1), ctx_len=on_device(len(reqs)),
+        state_slot=on_device(len(reqs)), positions=on_device(T, dtype=torch.int32), tiles=tiles,
+        groups=[SimpleNamespace(block_table=on_device(len(reqs), 1), width=-(-widest // 16))],
+        host=SimpleNamespace(cu_q=cu, ctx_len=np.array([c for c, _ in reqs])))
+
+
+@pytest.fixture
+def latents(ops):
+    """The kernel table with stand-ins behind latent attention; `calls` names them with their numbers."""
+    ops.calls = []
+    for name in ("somi_latent_gather", "somi_attention_prefill_pp_columns", "somi_latent_attention_mma"):
+        setattr(ops.lib, name, lambda *args, name=name: ops.calls.append((name, [getattr(a, "value", a) for a in args])) or 0)
+    ops.lib.somi_prefill_pp_supported = ops.lib.somi_latent_attention_mma_supported = lambda *args: 1
+    ops.lib.somi_latent_attention_splits = lambda *args: 1
+    ops._q_tensor_map = lambda t: P(0)
+    ops.use_expanded_latent, ops.use_mma_latent = True, True
+    ops.latent_tile, ops.prefill_pp_q_tile, ops.latent_q_tile = 128, 256, 16
+    return ops
+
+
+def expanded_tiles(ops, batch, window=None, heads=1, rank=8, dim=64):
+    """Tiles that each product over expanded latents runs over."""
+    T = batch.num_tokens
+    q, out = (on_device(T, heads * dim, dtype=torch.bfloat16) for _ in range(2))
+    ops.calls.clear()
+    ops.latent_portions(q, on_device(1, 1, 16, rank, dtype=torch.bfloat16), on_device(2 * heads * dim, rank, dtype=torch.bfloat16),
+                        batch, batch.groups[0], heads, rank, dim, 1.0, window, None, out)
+    return [args[10] for name, args in ops.calls if name == "somi_latent_gather"]
+
+
+def test_expanded_positions_are_the_portions_own(latents):
+    """A prompt beside a long request expands its own positions; other lengths that round to the same
+    number give the same launches, and no number is short."""
+    assert expanded_tiles(latents, portions((0, 96), singles=(16000,))) == [1]
+    assert expanded_tiles(latents, portions((3000, 100), singles=(16000,)), window=128) == [3]
+    rng = random.Random(1)
+    for _ in range(300):
+        reqs = [(rng.randrange(0, 3000), rng.randrange(2, 700)) for _ in range(rng.randrange(1, 6))]
+        window = rng.choice((None, 1, 127, 128, 129, 1000))
+        read = sum(len({p // 128 for p in range(0 if window is None else max(0, c - window + 1), c + q)}) for c, q in reqs)
+        (tiles,) = expanded_tiles(latents, portions(*reqs, singles=(9000,)), window)
+        assert read <= tiles <= 1.25 * read
+    assert len({expanded_tiles(latents, portions((0, q)))[0] for q in range(2, 8192, 32)}) <= 24
+
+
+def test_the_number_of_expanded_tiles_is_a_fact_of_the_layout(latents):
+    """Two steps of equal sizes whose portions read another number of tiles are told apart; layers that are
+    alike enter one fact."""
+    latents.check_latent_geometry = lambda *args: None
+    names = ("q_down", "q_norm", "q_up", "k_up", "v_up", "out", "kv_down", "kv_norm")
+    ctx = BuildContext(dtype=torch.bfloat16, device=torch.device("cpu"), ops=latents)
+    for window in (None, None, 256):
+        spec = PartSpec("latent_attention", {
+            "hidden_size": 64, "heads": 1, "key_dim": 64, "value_dim": 64, "q_rank": 8, "kv_rank": 8, "scale": 1.0,
+            "window": window, "own_latent": True, "eps": 1e-5, "names": {n: n for n in names}})
+        MIXERS.build(spec, {d.name: torch.zeros(d.shape, dtype=torch.bfloat16) for d in MIXERS.declare(spec)}, ctx)
+    model = SimpleNamespace(ctx=ctx)
+    facts = [Decoder.layout_facts(model, portions((c, 100), singles=(5000,))) for c in (0, 28, 29, 2000)]
+    assert len(facts[0]) == 2 and facts[0] == facts[1] and len(set(facts)) == 3
+    assert Decoder.layout_facts(model, portions(singles=(5000,))) == ()
