@@ -31,8 +31,15 @@ def _code(t: torch.Tensor) -> int:
     raise TypeError(f"kernels take float32 or bfloat16 tensors, got {t.dtype}")
 
 
-def _ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t: torch.Tensor | None, at: int = 0) -> ctypes.c_void_p:
+    """The address of `t`'s element `at`."""
+    return ctypes.c_void_p(0 if t is None else t.data_ptr() + at * t.element_size() if at else t.data_ptr())
+
+
+def _rounded_up(n: int) -> int:
+    """The next of four sizes per power of two, so that few layouts differ in it."""
+    step = 1 << max(0, n.bit_length() - 3)
+    return -(-n // step) * step
 
 
 def _check(*tensors: torch.Tensor | None) -> None:
@@ -121,6 +128,26 @@ class CudaOps:
             raise KernelError(f"{what}: these sizes are not supported by the kernel")
         if rc != 0:
             raise KernelError(f"{what}: CUDA error {rc}")
+
+    @staticmethod
+    def _tiles_of(batch, size: int, first: int, end: int) -> tuple[ctypes.c_void_p, int]:
+        """The query tiles of `size` rows of the portions among requests [first, end): address and number."""
+        tiles, n = batch.tiles[size], batch.num_prefill_requests
+        if first <= 0 and end >= n:
+            return _ptr(tiles), tiles.shape[0]
+        ends, at = batch.host.cu_q, []
+        for stop in (min(first, n), min(end, n)):
+            at.append(sum(-(-int(ends[r + 1] - ends[r]) // size) for r in range(stop)))
+        return _ptr(tiles, 3 * at[0]), at[1] - at[0]
+
+    @staticmethod
+    def run_facts(batch, runs) -> tuple:
+        """What tells a step's launches apart beside its layout, for portions that go in `runs`: these, and
+        the portions' lengths where a run ends among them (its rows and tiles follow from them)."""
+        n, cu = batch.num_prefill_requests, batch.host.cu_q
+        if any(0 < first < n for first, _, _ in runs):
+            return runs, tuple(int(cu[r]) for r in range(1, n))
+        return runs, ()
 
     def check_attention_geometry(self, num_heads: int, num_kv_heads: int, head_dim: int) -> None:
         if head_dim % 16 or not 16 <= head_dim <= 256:
@@ -900,7 +927,7 @@ class CudaOps:
         if trace.active():
             trace.note("latent_rotary_store", 2 * T * (heads * rot + rank + rot) * x.element_size())
 
-    # A step's portions read expanded keys and values from this many rows a request on.  Per row and
+    # A portion reads expanded keys and values from this many rows on.  Per row and
     # position read, attention over the latents takes rank / width times the operations, on the slower
     # tensor path; expanding takes a fixed number per position.  The layer in us over the latents /
     # expanded, 28 heads of 128 and rank 512 under a window of 1,024, portions from a prompt's start: 32 rows
@@ -909,51 +936,61 @@ class CudaOps:
     LATENT_EXPAND_ROWS = 96
     LATENT_EXPAND_POSITIONS = 32768     # the most that are expanded side by side (28 heads of 128: 470 MB)
 
-    def latent_expand_tiles(self, batch, window) -> int:
-        """Tiles of positions that the step's portions read, by their own lengths, rounded up to one of four
-        sizes per power of two.  A captured step is replayed with other lengths: the number belongs to what
-        its layout is told apart by (`BuildContext.layout_facts`)."""
-        t, win, n = self.latent_tile, int(window) if window else 0, 0
+    def latent_runs(self, batch, window) -> tuple:
+        """The step's requests as runs (first, end, tiles): neighbouring portions that read expanded keys and
+        values, with the tiles of positions that they read, and neighbours that read the latents (0 tiles;
+        single tokens always do).  A portion's own rows and positions decide, so it goes the same way
+        whatever else is in the step.  Tiles are rounded up to one of four sizes per power of two.  A captured
+        step is replayed with other lengths: the runs belong to what its layout is told apart by (`run_facts`)."""
+        t, win = self.latent_tile, int(window) if window else 0
+        most = self.LATENT_EXPAND_POSITIONS // t
         cu, ctx = batch.host.cu_q, batch.host.ctx_len
+        runs = []                                        # [first, end, tiles]
         for r in range(batch.num_prefill_requests):
-            cached = int(ctx[r])
-            n += (cached + int(cu[r + 1] - cu[r]) - 1) // t + 1 - (max(0, cached - win + 1) // t if win else 0)
-        step = 1 << max(0, n.bit_length() - 3)
-        return -(-n // step) * step
+            rows, cached = int(cu[r + 1] - cu[r]), int(ctx[r])
+            n = (cached + rows - 1) // t + 1 - (max(0, cached - win + 1) // t if win else 0)
+            if rows < self.LATENT_EXPAND_ROWS or _rounded_up(n) > most:
+                n = 0
+            if runs and (n > 0) == (runs[-1][2] > 0) and _rounded_up(runs[-1][2] + n) <= most:
+                runs[-1][1:] = r + 1, runs[-1][2] + n
+            else:
+                runs.append([r, r + 1, n])
+        if runs and not runs[-1][2]:
+            runs[-1][1] = batch.num_requests
+        elif batch.num_requests > batch.num_prefill_requests:
+            runs.append([batch.num_prefill_requests, batch.num_requests, 0])
+        return tuple((a, b, _rounded_up(n)) for a, b, n in runs)
 
     def latent_expands(self, batch, group, cache, heads: int, rank: int, key_dim: int, value_dim: int,
                        window, dtype) -> bool:
-        """Whether the step's prompt portions read expanded keys and values (see `latent_portions`)."""
-        n = batch.num_prefill_requests
-        if not (self.use_expanded_latent and n and dtype == torch.bfloat16 and rank % 8 == 0
+        """Whether portions of the step may read expanded keys and values (`latent_runs` says which)."""
+        return (self.use_expanded_latent and batch.max_q_len >= self.LATENT_EXPAND_ROWS and dtype == torch.bfloat16 and rank % 8 == 0
                 and cache.shape[3] == rank and key_dim == value_dim
                 and bool(self.lib.somi_prefill_pp_supported(ctypes.c_int(heads), ctypes.c_int(heads),
-                                                            ctypes.c_int(key_dim), ctypes.c_int(self.latent_tile)))):
-            return False
-        return (batch.num_prefill_tokens >= self.LATENT_EXPAND_ROWS * n
-                and self.latent_expand_tiles(batch, window) * self.latent_tile
-                <= self.LATENT_EXPAND_POSITIONS)
+                                                            ctypes.c_int(key_dim), ctypes.c_int(self.latent_tile))))
 
-    def latent_portions(self, q, cache, kv_up, batch, group, heads, rank, dim, scale, window, sinks, out) -> None:
-        """Attention of the step's prompt portions with keys and values expanded from the cached latents:
-        the latents that they read are gathered, one library product with `kv_up` [2 * heads * dim, rank]
+    def latent_portions(self, q, cache, kv_up, batch, group, heads, rank, dim, scale, window, sinks, out, run) -> None:
+        """Attention of a run of prompt portions (`latent_runs`) with keys and values expanded from the cached
+        latents: the latents that they read are gathered, one library product with `kv_up` [2 * heads * dim, rank]
         (all heads' keys, then all heads' values) expands them, and the two-tile tcgen05 kernel
         reads a head's keys and values as columns of the result.  `q`, `out`: [T, heads * dim], of which the
-        portions' rows are read and written."""
+        run's rows are read and written."""
         _check(q, cache, kv_up, out, group.block_table, sinks)
-        page_size, n, t = cache.shape[2], batch.num_prefill_requests, self.latent_tile
+        page_size, t = cache.shape[2], self.latent_tile
+        first, end, n_tiles = run
         assert q.dtype == cache.dtype == kv_up.dtype == out.dtype == torch.bfloat16
         assert tuple(kv_up.shape) == (2 * heads * dim, rank) and cache.shape[3] == rank
         assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == heads)
-        n_tiles = self.latent_expand_tiles(batch, window)
         longest = -(-group.width * page_size // t)
         rows = torch.empty((n_tiles * t, rank), dtype=q.dtype, device=q.device)
-        table = torch.empty((n, longest), dtype=torch.int32, device=q.device)
+        # (requests keep their numbers in the tables: rows in front of the run's are not written or read)
+        table = torch.empty((end, longest), dtype=torch.int32, device=q.device)
         win = int(window) if window else 0
         rc = self.lib.somi_latent_gather(
-            _ptr(cache), _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
-            _ptr(batch.ctx_len), ctypes.c_int(n), ctypes.c_int(rank), ctypes.c_int(page_size), ctypes.c_int(win),
-            _ptr(rows), ctypes.c_int(n_tiles), _ptr(table), ctypes.c_int(longest), self._stream())
+            _ptr(cache), _ptr(group.block_table, first * group.width), ctypes.c_int(group.width), _ptr(batch.cu_q, first),
+            _ptr(batch.ctx_len, first), ctypes.c_int(end - first), ctypes.c_int(rank), ctypes.c_int(page_size),
+            ctypes.c_int(win), _ptr(rows), ctypes.c_int(n_tiles), _ptr(table, first * longest), ctypes.c_int(longest),
+            self._stream())
         self._done(rc, "latent_gather")
         if trace.active():
             trace.note("latent_gather", 2 * rows.numel() * rows.element_size())
@@ -962,22 +999,22 @@ class CudaOps:
             trace.note("library_gemm", (rows.numel() + kv_up.numel() + expanded.numel()) * 2,
                        2.0 * rows.numel() * kv_up.shape[0],
                        detail=f"M={rows.shape[0]} N={kv_up.shape[0]} K={rank}")
-        tiles = batch.tiles[self.prefill_pp_q_tile]
+        tiles, n = self._tiles_of(batch, self.prefill_pp_q_tile, first, end)
         rc = self.lib.somi_attention_prefill_pp_columns(
             self._q_tensor_map(q), self._q_tensor_map(expanded),
             ctypes.c_int(heads * dim), _ptr(table), ctypes.c_int(longest), _ptr(batch.cu_q), _ptr(batch.ctx_len),
-            _ptr(tiles), ctypes.c_int(tiles.shape[0]), ctypes.c_int(heads), ctypes.c_int(dim),
+            tiles, ctypes.c_int(n), ctypes.c_int(heads), ctypes.c_int(dim),
             ctypes.c_float(scale), ctypes.c_int(win), _ptr(sinks), _ptr(out), self._stream())
         self._done(rc, "attention_prefill_pp_columns")
         if trace.active():
             trace.note("attention_prefill_tcgen05_pingpong", *self._attention_work(
-                batch, 0, n, heads, heads, dim, 2, win), detail="expanded latents")
+                batch, first, end, heads, heads, dim, 2, win), detail="expanded latents")
 
     def latent_attention(self, q, cache, batch, group, heads, rank, scale, window, sinks, out,
-                         tail: int = 0, singles: bool = False) -> None:
-        """Attention of every token of the step (`singles`: of its single-token requests alone, whose rows
-        `q` and `out` hold) over a cache of latents that serve as keys and
-        as values for every head (`q`, `out`: [heads, T, rank]; cache [pages, 1, page, rank]).
+                         tail: int = 0, first: int = 0, end: int | None = None) -> None:
+        """Attention of every token of the step (of requests [`first`, `end`) alone, whose rows `q` and `out`
+        hold) over a cache of latents that serve as keys and
+        as values for every head (`q`, `out`: [heads, rows, rank]; cache [pages, 1, page, rank]).
         `tail`: elements behind the latent in q's and the cache's rows that only the scores read;
         `sinks`: float32 [heads] scores that join every softmax's denominator, or None."""
         _check(q, cache, out, group.block_table, sinks)
@@ -987,10 +1024,12 @@ class CudaOps:
         assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == heads)
         page_size = cache.shape[2]
         T = q.shape[1]
-        tiles = batch.tiles[self.latent_q_tile][:0] if singles else batch.tiles[self.latent_q_tile]
-        n_decode = batch.num_requests - batch.num_prefill_requests
-        # the kernels count rows from the step's first: without the portions' rows, from that far in front
-        skipped = (batch.num_prefill_tokens if singles else 0) * q.element_size()
+        n_prefill = batch.num_prefill_requests
+        end = batch.num_requests if end is None else end
+        tiles, n_tiles = self._tiles_of(batch, self.latent_q_tile, first, end)
+        n_decode = max(0, end - n_prefill)
+        # the kernels count rows from the step's first: without the rows in front, from that far in front
+        skipped = (int(batch.host.cu_q[first]) if first else 0) * q.element_size()
         q_at = ctypes.c_void_p(q.data_ptr() - skipped * wide)
         out_at = ctypes.c_void_p(out.data_ptr() - skipped * rank)
         win = int(window) if window else 0
@@ -1006,16 +1045,16 @@ class CudaOps:
             rc = self.lib.somi_latent_attention_mma(
                 q_at, ctypes.c_longlong(wide), ctypes.c_longlong(T * wide), _ptr(cache),
                 _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
-                _ptr(batch.ctx_len), _ptr(tiles), ctypes.c_int(tiles.shape[0]),
+                _ptr(batch.ctx_len), tiles, ctypes.c_int(n_tiles),
                 ctypes.c_int(batch.num_prefill_requests), ctypes.c_int(batch.num_prefill_tokens),
                 ctypes.c_int(n_decode), ctypes.c_int(max_kv), ctypes.c_int(heads),
                 ctypes.c_int(wide), ctypes.c_int(rank), ctypes.c_int(page_size), ctypes.c_float(scale),
                 ctypes.c_int(win), _ptr(sinks), out_at, ctypes.c_longlong(rank),
                 ctypes.c_longlong(T * rank), _ptr(ws), self._stream())
             self._done(rc, "latent_attention_mma")
-            self.launches += (1 if tiles.shape[0] and n_decode else 0) + (1 if splits > 1 and n_decode else 0)
+            self.launches += (1 if n_tiles and n_decode else 0) + (1 if splits > 1 and n_decode else 0)
             if trace.active():
-                moved, flops = self._attention_work(batch, 0, batch.num_requests, heads, 1, rank,
+                moved, flops = self._attention_work(batch, first, end, heads, 1, rank,
                                                     q.element_size(), win)
                 moved, flops = moved / 2 * (wide / rank), flops / 2 * (1 + wide / rank)
                 trace.note("latent_attention_mma", moved + heads * T * rank * q.element_size(), flops,
@@ -1024,7 +1063,7 @@ class CudaOps:
         rc = self.lib.somi_latent_attention_generic(
             q_at, _code(q), ctypes.c_longlong(wide), ctypes.c_longlong(T * wide), _ptr(cache),
             _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
-            _ptr(batch.ctx_len), _ptr(tiles), ctypes.c_int(tiles.shape[0]),
+            _ptr(batch.ctx_len), tiles, ctypes.c_int(n_tiles),
             ctypes.c_int(batch.num_prefill_requests), ctypes.c_int(batch.num_prefill_tokens),
             ctypes.c_int(n_decode), ctypes.c_int(heads), ctypes.c_int(wide), ctypes.c_int(rank),
             ctypes.c_int(page_size), ctypes.c_float(scale), ctypes.c_int(int(window) if window else 0),
@@ -1032,7 +1071,7 @@ class CudaOps:
             self._stream())
         self._done(rc, "latent_attention")
         if trace.active():
-            moved, flops = self._attention_work(batch, 0, batch.num_requests, heads, 1, rank,
+            moved, flops = self._attention_work(batch, first, end, heads, 1, rank,
                                                 q.element_size(), int(window) if window else 0)
             moved, flops = moved / 2 * (wide / rank), flops / 2 * (1 + wide / rank)
             trace.note("latent_attention_generic", moved + heads * T * rank * q.element_size(), flops)

@@ -107,7 +107,8 @@ class LatentAttentionMixer:
         self.kv_up = (torch.cat([tensors[n["k_up"]], tensors[n["v_up"]]], 0).contiguous()
                       if ctx.dtype == torch.bfloat16 and self.key_dim == self.value_dim else None)
         if self.kv_up is not None:
-            ctx.layout_facts["latents", self.window] = lambda batch: ctx.ops.latent_expand_tiles(batch, self.window)
+            ctx.layout_facts["latents", self.window] = lambda batch: ctx.ops.run_facts(
+                batch, ctx.ops.latent_runs(batch, self.window))
         self.gate = Linear(tensors[n["gate"]], None, ctx.ops) if params.get("gate") else None
 
     def _build_direct(self, params, tensors, n) -> None:
@@ -177,20 +178,27 @@ class LatentAttentionMixer:
                               group.slot_map if self.own_latent else None,
                               paged.keys if self.own_latent else None)
         q = self.q_up(cq)                                           # [T, H * key_dim]
-        expand = self.kv_up is not None and ops.latent_expands(
-            batch, group, paged.keys, H, R, self.key_dim, self.value_dim, self.window, x.dtype)
-        first = batch.num_prefill_tokens if expand else 0           # rows from here on read the latents
         o = torch.empty((T, H * self.value_dim), dtype=x.dtype, device=x.device)
-        if expand:
-            ops.latent_portions(q, paged.keys, self.kv_up, batch, group, H, R, self.key_dim, self.scale,
-                                self.window, self.sinks, o)
-        if first < T:
-            qa = ops.head_product(q[first:].view(T - first, H, self.key_dim), self.k_up_t, heads_first=True)
+        # portions of some length read expanded keys and values, everything else the latents
+        runs = ((0, batch.num_requests, 0),)
+        if self.kv_up is not None and ops.latent_expands(batch, group, paged.keys, H, R, self.key_dim, self.value_dim,
+                                                         self.window, x.dtype):
+            runs = ops.latent_runs(batch, self.window)
+        for run in runs:
+            if run[2]:
+                ops.latent_portions(q, paged.keys, self.kv_up, batch, group, H, R, self.key_dim, self.scale,
+                                    self.window, self.sinks, o, run)
+                continue
+            first, end, _ = run
+            q_run, o_run = q, o
+            if len(runs) > 1:
+                rows = slice(int(batch.host.cu_q[first]), int(batch.host.cu_q[end]))
+                q_run, o_run = q[rows], o[rows]
+            qa = ops.head_product(q_run.view(-1, H, self.key_dim), self.k_up_t, heads_first=True)
             o_lat = torch.empty_like(qa)                            # [H, rows, R]
             ops.latent_attention(qa, paged.keys, batch, group, H, R, self.scale, self.window,
-                                 self.sinks, o_lat, singles=expand)
-            ops.head_product(o_lat, self.v_up, heads_first=False,
-                             out=o[first:].view(T - first, H, self.value_dim))
+                                 self.sinks, o_lat, first=first, end=end)
+            ops.head_product(o_lat, self.v_up, heads_first=False, out=o_run.view(-1, H, self.value_dim))
         if self.gate is not None and self.head_gate:
             ops.head_gate_mul(o, self.gate(x), H)
         elif self.gate is not None:

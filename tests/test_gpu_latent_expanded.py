@@ -35,12 +35,17 @@ def layers(ops, dim, window):
     return out
 
 
+ENDS = [{0: 127, 1: 128, 2: 129, 3: 300, 4: 385, 5: 5}, {0: 1, 1: 1, 2: 257, 3: 130, 4: 255, 5: 200}]
+RUNS = [{0: 40, 1: 150, 2: 2, 3: 95, 4: 96, 5: 200}, {0: 300, 1: 1, 2: 97, 3: 20, 4: 130, 5: 1}]
+
+
+@pytest.mark.parametrize("steps,expansions", [(ENDS, 2), (RUNS, 4)])
 @pytest.mark.parametrize("dim,window,page", [(64, None, 16), (128, None, 8), (64, 127, 32), (128, 300, 16), (64, 1, 16)])
-def test_expanded_portions(ops, dim, window, page):
+def test_expanded_portions(ops, dim, window, page, steps, expansions):
     """Two steps: portions that end around a tile of 128 positions, then portions and single tokens behind
-    them (their first visible key in, on and behind a tile's first position)."""
+    them (their first visible key in, on and behind a tile's first position); or portions of 96 rows and
+    more between shorter ones, which read the latents."""
     mixers = layers(ops, dim, window)
-    steps = [{0: 127, 1: 128, 2: 129, 3: 300, 4: 385, 5: 5}, {0: 1, 1: 1, 2: 257, 3: 130, 4: 255, 5: 200}]
     paged = PagedKVNeeds(1, RANK, window, value_dim=0)
     error, route = {}, []
     real = ops.latent_portions
@@ -65,7 +70,7 @@ def test_expanded_portions(ops, dim, window, page):
         ops.check_errors()
     finally:
         ops.latent_portions, ops.use_expanded_latent = real, was
-    assert len(route) == 2
+    assert len(route) == expansions
     # bfloat16 either way: an operand of each of the two per-head products is rounded to 2^-9 of itself
     for plain, expanded in zip(error[False], error[True]):
         assert expanded.mean() <= 1.3 * plain.mean() + 1e-4
@@ -75,10 +80,10 @@ def test_expanded_portions(ops, dim, window, page):
 def test_short_portions_read_the_latents(ops):
     mixer = layers(ops, 64, None)[torch.bfloat16]
     cache = Steps(ops, 2, paged=PagedKVNeeds(1, RANK, None, value_dim=0), dtype=torch.bfloat16)
-    batch, _ = cache.step({0: 40, 1: 151})
+    batch, _ = cache.step({0: 95, 1: 40})
     args = (batch, batch.groups[0], cache.mgr.view(0).paged.keys, HEADS, RANK)
     assert not ops.latent_expands(*args, 64, 64, None, torch.bfloat16)
-    batch, _ = cache.step({0: 42, 1: 150})
+    batch, _ = cache.step({0: 2, 1: 96})
     args = (batch, batch.groups[0], cache.mgr.view(0).paged.keys, HEADS, RANK)
     assert ops.latent_expands(*args, 64, 64, None, torch.bfloat16)
     assert not ops.latent_expands(*args, 64, 128, None, torch.bfloat16)

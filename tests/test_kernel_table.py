@@ -154,8 +154,11 @@ def expanded_tiles(ops, batch, window=None, heads=1, rank=8, dim=64):
     T = batch.num_tokens
     q, out = (on_device(T, heads * dim, dtype=torch.bfloat16) for _ in range(2))
     ops.calls.clear()
-    ops.latent_portions(q, on_device(1, 1, 16, rank, dtype=torch.bfloat16), on_device(2 * heads * dim, rank, dtype=torch.bfloat16),
-                        batch, batch.groups[0], heads, rank, dim, 1.0, window, None, out)
+    for run in ops.latent_runs(batch, window):
+        if run[2]:
+            ops.latent_portions(q, on_device(1, 1, 16, rank, dtype=torch.bfloat16),
+                                on_device(2 * heads * dim, rank, dtype=torch.bfloat16), batch, batch.groups[0], heads,
+                                rank, dim, 1.0, window, None, out, run)
     return [args[10] for name, args in ops.calls if name == "somi_latent_gather"]
 
 
@@ -166,12 +169,35 @@ def test_expanded_positions_are_the_portions_own(latents):
     assert expanded_tiles(latents, portions((3000, 100), singles=(16000,)), window=128) == [3]
     rng = random.Random(1)
     for _ in range(300):
-        reqs = [(rng.randrange(0, 3000), rng.randrange(2, 700)) for _ in range(rng.randrange(1, 6))]
+        reqs = [(rng.randrange(0, 3000), rng.randrange(96, 700)) for _ in range(rng.randrange(1, 6))]
         window = rng.choice((None, 1, 127, 128, 129, 1000))
         read = sum(len({p // 128 for p in range(0 if window is None else max(0, c - window + 1), c + q)}) for c, q in reqs)
         (tiles,) = expanded_tiles(latents, portions(*reqs, singles=(9000,)), window)
         assert read <= tiles <= 1.25 * read
-    assert len({expanded_tiles(latents, portions((0, q)))[0] for q in range(2, 8192, 32)}) <= 24
+    assert len({expanded_tiles(latents, portions((0, q)))[0] for q in range(96, 8192, 32)}) <= 24
+
+
+@pytest.mark.parametrize("window", [None, 300])
+def test_a_portion_goes_its_own_way_whatever_else_is_in_the_step(latents, window):
+    """Latent attention: whether a portion reads expanded keys and values follows from its rows and positions; the
+    runs go through all requests in order, and each launch reaches its run's tiles and rows."""
+    rng = random.Random(2)
+    sizes = [(0, 95), (0, 96), (0, 40), (500, 300), (0, 2), (latents.LATENT_EXPAND_POSITIONS, 200), (20000, 96)]
+
+    def alone(size):
+        return latents.latent_runs(portions(size), window)[0][2] > 0
+    assert [alone(s) for s in sizes] == [False, True, False, True, False, window is not None, True]
+    for _ in range(100):
+        reqs = [rng.choice(sizes) for _ in range(rng.randrange(1, 7))]
+        batch = portions(*reqs, singles=rng.choice(((), (7, 9000))))
+        runs = latents.latent_runs(batch, window)
+        assert [r for a, b, _ in runs for r in range(a, b)] == list(range(batch.num_requests))
+        for a, b, tiles in runs:
+            assert all(r < len(reqs) and alone(reqs[r]) if tiles else r >= len(reqs) or not alone(reqs[r]) for r in range(a, b))
+            assert 0 <= tiles * 128 <= latents.LATENT_EXPAND_POSITIONS
+            at, n = latents._tiles_of(batch, 64, a, b)
+            mine = [t for t in batch.tiles[64].tolist() if a <= t[0] < b]
+            assert n == len(mine) and (not n or batch.tiles[64][(at.value - batch.tiles[64].data_ptr()) // 12].tolist() == mine[0])
 
 
 def test_the_number_of_expanded_tiles_is_a_fact_of_the_layout(latents):
@@ -189,3 +215,7 @@ def test_the_number_of_expanded_tiles_is_a_fact_of_the_layout(latents):
     facts = [Decoder.layout_facts(model, portions((c, 100), singles=(5000,))) for c in (0, 28, 29, 2000)]
     assert len(facts[0]) == 2 and facts[0] == facts[1] and len(set(facts)) == 3
     assert Decoder.layout_facts(model, portions(singles=(5000,))) == ()
+    # equal numbers of rows and tiles, but the run of short portions is at other rows
+    a, b = portions((0, 110), (0, 60)), portions((0, 112), (0, 58))
+    assert all(a.tiles[t].shape == b.tiles[t].shape for t in a.tiles) and a.num_tokens == b.num_tokens
+    assert Decoder.layout_facts(model, a) != Decoder.layout_facts(model, b)
