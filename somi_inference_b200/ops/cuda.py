@@ -934,16 +934,17 @@ class CudaOps:
     # 40.6 / 37.0, 128 52.9 / 43.3, 512 126 / 68, 2,048 576 / 167; behind 3,000 positions: 32 rows 123 / 62, 512
     # 242 / 95.  14 heads of 64, rank 128: 64 rows 24.8 / 26.8, 96 28.9 / 26.9, 2,048 104 / 56.
     LATENT_EXPAND_ROWS = 96
-    LATENT_EXPAND_POSITIONS = 32768     # the most that are expanded side by side (28 heads of 128: 470 MB)
+    LATENT_EXPAND_BYTES = 1 << 29       # the most that a run's latents, keys and values may take
 
-    def latent_runs(self, batch, window) -> tuple:
+    def latent_runs(self, batch, window, heads: int, rank: int, dim: int) -> tuple:
         """The step's requests as runs (first, end, tiles): neighbouring portions that read expanded keys and
         values, with the tiles of positions that they read, and neighbours that read the latents (0 tiles;
         single tokens always do).  A portion's own rows and positions decide, so it goes the same way
-        whatever else is in the step.  Tiles are rounded up to one of four sizes per power of two.  A captured
+        whatever else is in the step.  A run's workspace is bounded (more portions are another run; one portion of
+        more positions reads the latents).  Tiles are rounded up to one of four sizes per power of two.  A captured
         step is replayed with other lengths: the runs belong to what its layout is told apart by (`run_facts`)."""
         t, win = self.latent_tile, int(window) if window else 0
-        most = self.LATENT_EXPAND_POSITIONS // t
+        most = self.LATENT_EXPAND_BYTES // (t * (rank + 2 * heads * dim) * 2)      # tiles
         cu, ctx = batch.host.cu_q, batch.host.ctx_len
         runs = []                                        # [first, end, tiles]
         for r in range(batch.num_prefill_requests):

@@ -107,8 +107,9 @@ class LatentAttentionMixer:
         self.kv_up = (torch.cat([tensors[n["k_up"]], tensors[n["v_up"]]], 0).contiguous()
                       if ctx.dtype == torch.bfloat16 and self.key_dim == self.value_dim else None)
         if self.kv_up is not None:
-            ctx.layout_facts["latents", self.window] = lambda batch: ctx.ops.run_facts(
-                batch, ctx.ops.latent_runs(batch, self.window))
+            sizes = self.window, self.heads, self.kv_rank, self.key_dim
+            ctx.layout_facts["latents", *sizes] = lambda batch: ctx.ops.run_facts(
+                batch, ctx.ops.latent_runs(batch, *sizes))
         self.gate = Linear(tensors[n["gate"]], None, ctx.ops) if params.get("gate") else None
 
     def _build_direct(self, params, tensors, n) -> None:
@@ -183,7 +184,7 @@ class LatentAttentionMixer:
         runs = ((0, batch.num_requests, 0),)
         if self.kv_up is not None and ops.latent_expands(batch, group, paged.keys, H, R, self.key_dim, self.value_dim,
                                                          self.window, x.dtype):
-            runs = ops.latent_runs(batch, self.window)
+            runs = ops.latent_runs(batch, self.window, H, R, self.key_dim)
         for run in runs:
             if run[2]:
                 ops.latent_portions(q, paged.keys, self.kv_up, batch, group, H, R, self.key_dim, self.scale,

@@ -154,7 +154,7 @@ def expanded_tiles(ops, batch, window=None, heads=1, rank=8, dim=64):
     T = batch.num_tokens
     q, out = (on_device(T, heads * dim, dtype=torch.bfloat16) for _ in range(2))
     ops.calls.clear()
-    for run in ops.latent_runs(batch, window):
+    for run in ops.latent_runs(batch, window, heads, rank, dim):
         if run[2]:
             ops.latent_portions(q, on_device(1, 1, 16, rank, dtype=torch.bfloat16),
                                 on_device(2 * heads * dim, rank, dtype=torch.bfloat16), batch, batch.groups[0], heads,
@@ -182,22 +182,36 @@ def test_a_portion_goes_its_own_way_whatever_else_is_in_the_step(latents, window
     """Latent attention: whether a portion reads expanded keys and values follows from its rows and positions; the
     runs go through all requests in order, and each launch reaches its run's tiles and rows."""
     rng = random.Random(2)
-    sizes = [(0, 95), (0, 96), (0, 40), (500, 300), (0, 2), (latents.LATENT_EXPAND_POSITIONS, 200), (20000, 96)]
+    sizes = [(0, 95), (0, 96), (0, 40), (500, 300), (0, 2), (40000, 200), (20000, 96)]
+    heads, rank, dim = 28, 512, 128
+    position = 2 * (rank + 2 * heads * dim)              # bytes
 
     def alone(size):
-        return latents.latent_runs(portions(size), window)[0][2] > 0
+        return latents.latent_runs(portions(size), window, heads, rank, dim)[0][2] > 0
     assert [alone(s) for s in sizes] == [False, True, False, True, False, window is not None, True]
     for _ in range(100):
         reqs = [rng.choice(sizes) for _ in range(rng.randrange(1, 7))]
         batch = portions(*reqs, singles=rng.choice(((), (7, 9000))))
-        runs = latents.latent_runs(batch, window)
+        runs = latents.latent_runs(batch, window, heads, rank, dim)
         assert [r for a, b, _ in runs for r in range(a, b)] == list(range(batch.num_requests))
         for a, b, tiles in runs:
             assert all(r < len(reqs) and alone(reqs[r]) if tiles else r >= len(reqs) or not alone(reqs[r]) for r in range(a, b))
-            assert 0 <= tiles * 128 <= latents.LATENT_EXPAND_POSITIONS
+            assert 0 <= tiles * 128 * position <= 1 << 29
             at, n = latents._tiles_of(batch, 64, a, b)
             mine = [t for t in batch.tiles[64].tolist() if a <= t[0] < b]
             assert n == len(mine) and (not n or batch.tiles[64][(at.value - batch.tiles[64].data_ptr()) // 12].tolist() == mine[0])
+
+
+@pytest.mark.parametrize("heads,dim", [(128, 128), (16, 64)])
+def test_the_workspace_of_expanded_latents_is_bounded_in_bytes(latents, monkeypatch, heads, dim):
+    """Many heads expand fewer positions side by side: no workspace takes more than 512 MB."""
+    rank, real, sizes = 512, torch.empty, []
+    monkeypatch.setattr(cuda.torch, "empty", lambda size, **kw: sizes.append(size) or real(1, **kw))
+    monkeypatch.setattr(cuda.torch.nn.functional, "linear", lambda x, w: torch.zeros(1, 1, dtype=torch.bfloat16))
+    batch = portions(*((3000, 500),) * 12, (30000, 100))
+    expanded_tiles(latents, batch, None, heads, rank, dim)
+    rows = [s[0] for s in sizes if s[1] == rank]
+    assert rows and all(r * (rank + 2 * heads * dim) * 2 <= 1 << 29 for r in rows)
 
 
 def test_the_number_of_expanded_tiles_is_a_fact_of_the_layout(latents):
