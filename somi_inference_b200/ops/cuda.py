@@ -962,13 +962,16 @@ class CudaOps:
             runs.append([batch.num_prefill_requests, batch.num_requests, 0])
         return tuple((a, b, _rounded_up(n)) for a, b, n in runs)
 
+    def latent_expand_supported(self, heads: int, rank: int, key_dim: int, value_dim: int) -> bool:
+        """Whether portions of a bfloat16 layer of these sizes can read expanded keys and values."""
+        return rank % 8 == 0 and key_dim == value_dim and bool(self.lib.somi_prefill_pp_supported(
+            ctypes.c_int(heads), ctypes.c_int(heads), ctypes.c_int(key_dim), ctypes.c_int(self.latent_tile)))
+
     def latent_expands(self, batch, group, cache, heads: int, rank: int, key_dim: int, value_dim: int,
                        window, dtype) -> bool:
         """Whether portions of the step may read expanded keys and values (`latent_runs` says which)."""
-        return (self.use_expanded_latent and batch.max_q_len >= self.LATENT_EXPAND_ROWS and dtype == torch.bfloat16 and rank % 8 == 0
-                and cache.shape[3] == rank and key_dim == value_dim
-                and bool(self.lib.somi_prefill_pp_supported(ctypes.c_int(heads), ctypes.c_int(heads),
-                                                            ctypes.c_int(key_dim), ctypes.c_int(self.latent_tile))))
+        return (self.use_expanded_latent and batch.max_q_len >= self.LATENT_EXPAND_ROWS and dtype == torch.bfloat16
+                and cache.shape[3] == rank and self.latent_expand_supported(heads, rank, key_dim, value_dim))
 
     def latent_portions(self, q, cache, kv_up, batch, group, heads, rank, dim, scale, window, sinks, out, run) -> None:
         """Attention of a run of prompt portions (`latent_runs`) with keys and values expanded from the cached

@@ -103,10 +103,12 @@ class LatentAttentionMixer:
         self.down = Linear(torch.cat(down, 0).contiguous(), None, ctx.ops)
         self.q_norm = tensors[n["q_norm"]]
         self.q_up = Linear(tensors[n["q_up"]], None, ctx.ops)
-        # all heads' W_uk, then all heads' W_uv, for portions that read expanded keys and values
-        self.kv_up = (torch.cat([tensors[n["k_up"]], tensors[n["v_up"]]], 0).contiguous()
-                      if ctx.dtype == torch.bfloat16 and self.key_dim == self.value_dim else None)
-        if self.kv_up is not None:
+        # all heads' W_uk, then all heads' W_uv, for portions that read expanded keys and values; only where the
+        # sizes allow it, and W_uv in one copy for both ways
+        self.kv_up = None
+        if ctx.dtype == torch.bfloat16 and ctx.ops.latent_expand_supported(H, self.kv_rank, self.key_dim, self.value_dim):
+            self.kv_up = torch.cat([tensors[n["k_up"]], tensors[n["v_up"]]], 0).contiguous()
+            self.v_up = self.kv_up[H * self.key_dim:].view(H, self.value_dim, self.kv_rank)
             sizes = self.window, self.heads, self.kv_rank, self.key_dim
             ctx.layout_facts["latents", *sizes] = lambda batch: ctx.ops.run_facts(
                 batch, ctx.ops.latent_runs(batch, *sizes))

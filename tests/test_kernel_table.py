@@ -214,17 +214,34 @@ def test_the_workspace_of_expanded_latents_is_bounded_in_bytes(latents, monkeypa
     assert rows and all(r * (rank + 2 * heads * dim) * 2 <= 1 << 29 for r in rows)
 
 
+def latent_layer(ops, windows, dim=64):
+    """The last of a model's latent layers, one per window, and the context that they were built in."""
+    ops.check_latent_geometry = lambda *args: None
+    names = ("q_down", "q_norm", "q_up", "k_up", "v_up", "out", "kv_down", "kv_norm")
+    ctx = BuildContext(dtype=torch.bfloat16, device=torch.device("cpu"), ops=ops)
+    for window in windows:
+        spec = PartSpec("latent_attention", {
+            "hidden_size": 64, "heads": 2, "key_dim": dim, "value_dim": dim, "q_rank": 8, "kv_rank": 8, "scale": 1.0,
+            "window": window, "own_latent": True, "eps": 1e-5, "names": {n: n for n in names}})
+        mixer = MIXERS.build(spec, {d.name: torch.ones(d.shape, dtype=torch.bfloat16) for d in MIXERS.declare(spec)}, ctx)
+    return mixer, ctx
+
+
+def test_expansion_weights_are_held_where_they_are_read(latents):
+    """Sizes that never read expanded keys and values hold no matrix for them; where they do, W_uv lies in
+    memory once."""
+    latents.lib.somi_prefill_pp_supported = lambda nq, nkv, hd, page: hd.value in (64, 128)
+    mixer, ctx = latent_layer(latents, [None], dim=32)
+    assert mixer.kv_up is None and not ctx.layout_facts
+    mixer, _ = latent_layer(latents, [None])
+    assert mixer.kv_up.shape == (2 * 2 * 64, 8) and mixer.v_up.shape == (2, 64, 8)
+    assert mixer.v_up.data_ptr() == mixer.kv_up[2 * 64:].data_ptr()
+
+
 def test_the_number_of_expanded_tiles_is_a_fact_of_the_layout(latents):
     """Two steps of equal sizes whose portions read another number of tiles are told apart; layers that are
     alike enter one fact."""
-    latents.check_latent_geometry = lambda *args: None
-    names = ("q_down", "q_norm", "q_up", "k_up", "v_up", "out", "kv_down", "kv_norm")
-    ctx = BuildContext(dtype=torch.bfloat16, device=torch.device("cpu"), ops=latents)
-    for window in (None, None, 256):
-        spec = PartSpec("latent_attention", {
-            "hidden_size": 64, "heads": 1, "key_dim": 64, "value_dim": 64, "q_rank": 8, "kv_rank": 8, "scale": 1.0,
-            "window": window, "own_latent": True, "eps": 1e-5, "names": {n: n for n in names}})
-        MIXERS.build(spec, {d.name: torch.zeros(d.shape, dtype=torch.bfloat16) for d in MIXERS.declare(spec)}, ctx)
+    _, ctx = latent_layer(latents, (None, None, 256))
     model = SimpleNamespace(ctx=ctx)
     facts = [Decoder.layout_facts(model, portions((c, 100), singles=(5000,))) for c in (0, 28, 29, 2000)]
     assert len(facts[0]) == 2 and facts[0] == facts[1] and len(set(facts)) == 3
