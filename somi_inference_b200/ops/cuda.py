@@ -141,6 +141,27 @@ class CudaOps:
         return _ptr(tiles, 3 * at[0]), at[1] - at[0]
 
     @staticmethod
+    def _portion_runs(batch, tiles, most: int, rounded=int) -> tuple:
+        """The step's requests as runs (first, end, tiles): neighbouring portions that a kernel over tiles
+        takes, with the sum of their `tiles(rows, cached)` (at most `most`, as `rounded`), and neighbours that
+        it leaves (0 tiles; single tokens always are)."""
+        cu, ctx = batch.host.cu_q, batch.host.ctx_len
+        runs = []
+        for r in range(batch.num_prefill_requests):
+            n = tiles(int(cu[r + 1] - cu[r]), int(ctx[r]))
+            if rounded(n) > most:
+                n = 0
+            if runs and (n > 0) == (runs[-1][2] > 0) and rounded(runs[-1][2] + n) <= most:
+                runs[-1][1:] = r + 1, runs[-1][2] + n
+            else:
+                runs.append([r, r + 1, n])
+        if runs and not runs[-1][2]:
+            runs[-1][1] = batch.num_requests
+        elif batch.num_requests > batch.num_prefill_requests:
+            runs.append([batch.num_prefill_requests, batch.num_requests, 0])
+        return tuple((first, end, rounded(n)) for first, end, n in runs)
+
+    @staticmethod
     def run_facts(batch, runs) -> tuple:
         """What tells a step's launches apart beside its layout, for portions that go in `runs`: these, and
         the portions' lengths where a run ends among them (its rows and tiles follow from them)."""
@@ -944,23 +965,12 @@ class CudaOps:
         more positions reads the latents).  Tiles are rounded up to one of four sizes per power of two.  A captured
         step is replayed with other lengths: the runs belong to what its layout is told apart by (`run_facts`)."""
         t, win = self.latent_tile, int(window) if window else 0
-        most = self.LATENT_EXPAND_BYTES // (t * (rank + 2 * heads * dim) * 2)      # tiles
-        cu, ctx = batch.host.cu_q, batch.host.ctx_len
-        runs = []                                        # [first, end, tiles]
-        for r in range(batch.num_prefill_requests):
-            rows, cached = int(cu[r + 1] - cu[r]), int(ctx[r])
-            n = (cached + rows - 1) // t + 1 - (max(0, cached - win + 1) // t if win else 0)
-            if rows < self.LATENT_EXPAND_ROWS or _rounded_up(n) > most:
-                n = 0
-            if runs and (n > 0) == (runs[-1][2] > 0) and _rounded_up(runs[-1][2] + n) <= most:
-                runs[-1][1:] = r + 1, runs[-1][2] + n
-            else:
-                runs.append([r, r + 1, n])
-        if runs and not runs[-1][2]:
-            runs[-1][1] = batch.num_requests
-        elif batch.num_requests > batch.num_prefill_requests:
-            runs.append([batch.num_prefill_requests, batch.num_requests, 0])
-        return tuple((a, b, _rounded_up(n)) for a, b, n in runs)
+
+        def tiles(rows: int, cached: int) -> int:
+            if rows < self.LATENT_EXPAND_ROWS:
+                return 0
+            return (cached + rows - 1) // t + 1 - (max(0, cached - win + 1) // t if win else 0)
+        return self._portion_runs(batch, tiles, self.LATENT_EXPAND_BYTES // (t * (rank + 2 * heads * dim) * 2), _rounded_up)
 
     def latent_expand_supported(self, heads: int, rank: int, key_dim: int, value_dim: int) -> bool:
         """Whether portions of a bfloat16 layer of these sizes can read expanded keys and values."""
@@ -1664,25 +1674,30 @@ class CudaOps:
     SCAN_PREPARE_ROWS = 16
     SCAN_TURN_ROWS = 4          # the most rows a request may have where the scan itself rotates q and k
 
-    # portions go in chunks from rows = this * state width on, on average (both sides measured in
+    # a portion goes in chunks from rows = this * state width on (both sides measured in
     # `csrc/recurrent_chunks.cu`: they meet at 128 to 256 rows for a width of 128, at 32 to 64 for 64)
     SCAN_CHUNK_ROWS = 1
-    SCAN_CHUNK_BYTES = 1 << 29  # the most that the chunks' states may take
+    SCAN_CHUNK_BYTES = 1 << 29  # the most that the chunks' states of a run of portions may take
 
     def scan_in_chunks(self, q, k, v, batch, heads, qk_heads, dk, dv, act_silu, unit_eps, beta, decay_logits,
                        rotary) -> bool:
-        """Whether the step's prompt portions go through the recurrence in chunks of rows
+        """Whether some of the step's prompt portions go through the recurrence in chunks of rows
         (`csrc/recurrent_chunks.cu`): bfloat16, a constant decay per head, square states of 64 or 128.
         (float32 stays with the step by step form, whose sums do not depend on the cut.)"""
         n = getattr(batch, "num_prefill_requests", 0)
-        if not (n and self.use_scan_chunks and q.dtype == torch.bfloat16 and dk == dv and dk in (64, 128)
-                and unit_eps is None and beta is None and decay_logits is None):
+        if not (n and self.use_scan_chunks and batch.max_q_len >= self.SCAN_CHUNK_ROWS * dk and q.dtype == torch.bfloat16
+                and dk == dv and dk in (64, 128) and unit_eps is None and beta is None and decay_logits is None):
             return False
         rot = rotary[2] if rotary is not None else 0
-        if rot % 8 or (rot and act_silu) or any(t.stride(0) % 4 or t.data_ptr() % 8 for t in (q, k, v)):
-            return False
-        return (batch.num_prefill_tokens >= self.SCAN_CHUNK_ROWS * dk * n
-                and batch.tiles[self.prefill_q_tile].shape[0] * heads * dk * dk * 4 <= self.SCAN_CHUNK_BYTES)
+        return not (rot % 8 or (rot and act_silu) or any(t.stride(0) % 4 or t.data_ptr() % 8 for t in (q, k, v)))
+
+    def scan_runs(self, batch, heads: int, dk: int) -> tuple:
+        """The step's requests as runs (first, end, tiles of 64 rows): neighbouring portions that go through the
+        recurrence in chunks, and neighbours that go step by step (0 tiles).  A portion's own rows decide,
+        so it goes the same way whatever else is in the step.  A run's workspace is bounded (more portions are
+        another run; one portion of more rows goes step by step)."""
+        return self._portion_runs(batch, lambda rows, cached: -(-rows // 64) if rows >= self.SCAN_CHUNK_ROWS * dk else 0,
+                                  self.SCAN_CHUNK_BYTES // (heads * dk * dk * 4))
 
     def matrix_state_scan(self, q, k, v, state, batch, y, heads, qk_heads, dk, dv, *,
                           act_silu=False, unit_eps=None, q_scale=1.0, beta=None, decay_logits=None,
@@ -1711,82 +1726,102 @@ class CudaOps:
             assert t is None or t.dtype == torch.float32
         if decay is None and decay_logits is None:
             raise KernelError("matrix_state_scan takes a decay per head, or decay logits")
-        max_rows = int(getattr(batch, "max_q_len", 0) or 0)
-        chunks = prepare is None and self.scan_in_chunks(q, k, v, batch, heads, qk_heads, dk, dv, act_silu,
-                                                         unit_eps, beta, decay_logits, rotary)
-        if prepare is None:
-            prepare = max_rows > self.SCAN_PREPARE_ROWS
         pos, freq, rot = rotary if rotary is not None else (None, None, 0)
         if rot:
             _check(pos, freq)
             assert pos.dtype == torch.int32 and freq.dtype == torch.float64 and freq.numel() >= rot // 2
-            # the scan turns q and k itself only in steps of a few rows
-            prepare = prepare or not 0 < max_rows <= self.SCAN_TURN_ROWS
+        runs = ((0, batch.num_requests, 0),)
+        if prepare is None and self.scan_in_chunks(q, k, v, batch, heads, qk_heads, dk, dv, act_silu, unit_eps, beta,
+                                                   decay_logits, rotary):
+            runs = self.scan_runs(batch, heads, dk)
+        for run in runs:
+            if run[2]:
+                self._scan_chunks(q, k, v, state, batch, y, heads, qk_heads, dk, act_silu, q_scale, decay, rotary, run)
+            else:
+                self._scan_steps(q, k, v, state, batch, y, heads, qk_heads, dk, dv, act_silu, unit_eps, q_scale, beta,
+                                 decay_logits, dt_bias, a_log, decay, rotary, prepare, run[0], run[1])
+
+    def _scan_chunks(self, q, k, v, state, batch, y, heads, qk_heads, dk, act_silu, q_scale, decay, rotary, run) -> None:
+        pos, freq, rot = rotary if rotary is not None else (None, None, 0)
+        first, end, n_tiles = run
+        rows = int(batch.host.cu_q[end])                     # (angles of the rows in front are made too)
+        tiles, _ = self._tiles_of(batch, self.prefill_q_tile, first, end)
+        angles = torch.empty(rows * rot, dtype=torch.float32, device=q.device) if rot else None
+        u = torch.empty(n_tiles * heads * dk * dk, dtype=torch.float32, device=q.device)
+        rc = self.lib.somi_matrix_state_chunks(
+            _ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(q.stride(0)), ctypes.c_longlong(k.stride(0)),
+            ctypes.c_longlong(v.stride(0)), ctypes.c_int(3 if act_silu else 0), ctypes.c_float(q_scale), _ptr(decay),
+            _ptr(state), _ptr(batch.cu_q, first), _ptr(batch.state_slot, first), tiles, ctypes.c_int(n_tiles),
+            ctypes.c_int(end - first), ctypes.c_int(rows), ctypes.c_int(heads), ctypes.c_int(heads // qk_heads),
+            ctypes.c_int(dk), _ptr(pos), _ptr(freq), ctypes.c_int(rot), _ptr(angles), _ptr(u), _ptr(y),
+            self._stream())
+        self._done(rc, "matrix_state_chunks")
+        self.launches += 3 if rot else 2
+        if trace.active():
+            rows -= int(batch.host.cu_q[first])
+            trace.note("matrix_state_chunks", rows * (2 * qk_heads * dk + heads * dk) * 2 + rows * heads * dk * 4
+                       + 2 * (end - first) * heads * dk * dk * 4, 5.0 * rows * heads * dk * dk)
+
+    def _scan_steps(self, q, k, v, state, batch, y, heads, qk_heads, dk, dv, act_silu, unit_eps, q_scale, beta,
+                    decay_logits, dt_bias, a_log, decay, rotary, prepare, first, end) -> None:
+        """The scan over requests [first, end) of the step."""
+        pos, freq, rot = rotary if rotary is not None else (None, None, 0)
+        row, rows = 0, q.shape[0]
+        max_rows = int(getattr(batch, "max_q_len", 0) or 0)
+        if end - first < batch.num_requests:
+            cu = batch.host.cu_q
+            row, rows = int(cu[first]), int(cu[end] - cu[first])
+            max_rows = max(int(cu[r + 1] - cu[r]) for r in range(first, end))
+        if prepare is None:
+            prepare = max_rows > self.SCAN_PREPARE_ROWS
+        # the scan turns q and k itself only in steps of a few rows
+        prepare = prepare or bool(rot and not 0 < max_rows <= self.SCAN_TURN_ROWS)
         act, unit, ready = (3 if act_silu else 0), (0 if unit_eps is None else 1), 0
-        vb_code = _code(v)
-        first = 0                     # requests in front of the ones that are left to the scan
-        if chunks:
-            n, heads_apart = batch.num_prefill_requests, heads // qk_heads
-            tiles = batch.tiles[self.prefill_q_tile]
-            n_rows = batch.num_prefill_tokens
-            angles = torch.empty(n_rows * rot, dtype=torch.float32, device=q.device) if rot else None
-            u = torch.empty(tiles.shape[0] * heads * dk * dk, dtype=torch.float32, device=q.device)
-            rc = self.lib.somi_matrix_state_chunks(
-                _ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(q.stride(0)), ctypes.c_longlong(k.stride(0)),
-                ctypes.c_longlong(v.stride(0)), ctypes.c_int(act), ctypes.c_float(q_scale), _ptr(decay),
-                _ptr(state), _ptr(batch.cu_q), _ptr(batch.state_slot), _ptr(tiles), ctypes.c_int(tiles.shape[0]),
-                ctypes.c_int(n), ctypes.c_int(n_rows), ctypes.c_int(heads), ctypes.c_int(heads_apart),
-                ctypes.c_int(dk), _ptr(pos), _ptr(freq), ctypes.c_int(rot), _ptr(angles), _ptr(u), _ptr(y),
-                self._stream())
-            self._done(rc, "matrix_state_chunks")
-            self.launches += 3 if rot else 2
-            if trace.active():
-                trace.note("matrix_state_chunks", n_rows * (2 * qk_heads * dk + heads * dv) * 2 + n_rows * heads * dv * 4
-                           + 2 * n * heads * dk * dv * 4, 5.0 * n_rows * heads * dk * dv)
-            if n == batch.num_requests:
-                return
-            first, max_rows, prepare = n, 1, False               # the single tokens
+        vb_code, elt = _code(v), q.element_size()
+        q_at, k_at, logits_at = _ptr(q), _ptr(k), _ptr(decay_logits)
         if prepare:
-            T, n = q.shape[0], q.shape[0] * qk_heads * dk
-            n_g = T * heads * dk if decay_logits is not None else 0
+            n = rows * qk_heads * dk
+            n_g = rows * heads * dk if decay_logits is not None else 0
             buf = torch.empty(2 * n + n_g, dtype=torch.float32, device=q.device)
-            qn, kn = buf[:n].view(T, -1), buf[n:2 * n].view(T, -1)
-            gd = buf[2 * n:].view(T, -1) if n_g else None
+            qn, kn = buf[:n].view(rows, -1), buf[n:2 * n].view(rows, -1)
+            gd = buf[2 * n:].view(rows, -1) if n_g else None
             rc = self.lib.somi_matrix_state_prepare(
-                _ptr(q), _ptr(k), _code(q), ctypes.c_longlong(q.stride(0)), ctypes.c_longlong(k.stride(0)),
-                ctypes.c_int(act), ctypes.c_int(unit), ctypes.c_float(unit_eps or 0.0),
-                ctypes.c_float(q_scale), _ptr(decay_logits),
+                _ptr(q, row * q.stride(0)), _ptr(k, row * k.stride(0)), _code(q), ctypes.c_longlong(q.stride(0)),
+                ctypes.c_longlong(k.stride(0)), ctypes.c_int(act), ctypes.c_int(unit), ctypes.c_float(unit_eps or 0.0),
+                ctypes.c_float(q_scale), _ptr(decay_logits, row * decay_logits.stride(0) if n_g else 0),
                 ctypes.c_longlong(decay_logits.stride(0) if decay_logits is not None else 0),
-                _ptr(dt_bias), _ptr(a_log), _ptr(qn), _ptr(kn), _ptr(gd), ctypes.c_int(T),
-                ctypes.c_int(heads), ctypes.c_int(qk_heads), ctypes.c_int(dk), _ptr(pos), _ptr(freq),
+                _ptr(dt_bias), _ptr(a_log), _ptr(qn), _ptr(kn), _ptr(gd), ctypes.c_int(rows),
+                ctypes.c_int(heads), ctypes.c_int(qk_heads), ctypes.c_int(dk), _ptr(pos, row), _ptr(freq),
                 ctypes.c_int(rot), self._stream())
             self._done(rc, "matrix_state_prepare")
             if trace.active():
-                trace.note("matrix_state_prepare", 2 * n * (q.element_size() + 4) + 2 * n_g * 4)
+                trace.note("matrix_state_prepare", 2 * n * (elt + 4) + 2 * n_g * 4)
             q, k, decay_logits = qn, kn, gd
             act, unit, ready, q_scale = act & 2, 0, 1, 1.0      # q is scaled already
             pos, freq, rot = None, None, 0                      # and q and k are turned
+            # (the scan counts rows from the step's first: from that far in front)
+            q_at, k_at = _ptr(q, -row * q.stride(0)), _ptr(k, -row * k.stride(0))
+            logits_at = _ptr(gd, -row * gd.stride(0) if n_g else 0)
         rc = self.lib.somi_matrix_state_scan(
-            _ptr(q), _ptr(k), _ptr(v), _code(q), vb_code, ctypes.c_longlong(q.stride(0)),
+            q_at, k_at, _ptr(v), _code(q), vb_code, ctypes.c_longlong(q.stride(0)),
             ctypes.c_longlong(k.stride(0)), ctypes.c_longlong(v.stride(0)),
             ctypes.c_int(act), ctypes.c_int(unit),
             ctypes.c_float(unit_eps or 0.0), ctypes.c_float(q_scale),
             ctypes.c_int(0 if beta is None else 1), _ptr(beta),
-            ctypes.c_longlong(beta.stride(0) if beta is not None else 0), _ptr(decay_logits),
+            ctypes.c_longlong(beta.stride(0) if beta is not None else 0), logits_at,
             ctypes.c_longlong(decay_logits.stride(0) if decay_logits is not None else 0),
             ctypes.c_int(ready),
-            _ptr(dt_bias), _ptr(a_log), _ptr(decay), _ptr(state), _ptr(batch.cu_q[first:]),
-            _ptr(batch.state_slot[first:]), _ptr(y), ctypes.c_int(batch.num_requests - first), ctypes.c_int(heads),
+            _ptr(dt_bias), _ptr(a_log), _ptr(decay), _ptr(state), _ptr(batch.cu_q, first),
+            _ptr(batch.state_slot, first), _ptr(y), ctypes.c_int(end - first), ctypes.c_int(heads),
             ctypes.c_int(qk_heads), ctypes.c_int(dk), ctypes.c_int(dv),
             ctypes.c_int(max_rows), _ptr(pos), _ptr(freq), ctypes.c_int(rot), self._stream())
         self._done(rc, "matrix_state_scan")
         if trace.active():
-            T = q.shape[0]
-            moved = T * (2 * qk_heads * dk + heads * dv) * q.element_size() + T * heads * dv * 4 \
-                + 2 * batch.num_requests * heads * dk * dv * 4
+            moved = rows * (2 * qk_heads * dk + heads * dv) * q.element_size() + rows * heads * dv * 4 \
+                + 2 * (end - first) * heads * dk * dv * 4
             if decay_logits is not None:
-                moved += T * heads * dk * 4
-            trace.note("matrix_state_scan", moved, (8.0 if beta is not None else 5.0) * T * heads * dk * dv,
+                moved += rows * heads * dk * 4
+            trace.note("matrix_state_scan", moved, (8.0 if beta is not None else 5.0) * rows * heads * dk * dv,
                        detail="delta rule" if beta is not None else "decayed sum")
 
     def group_rmsnorm_gate(self, y, gate, weight, eps, groups, out, gate_act: str = "sigmoid") -> None:

@@ -133,6 +133,13 @@ class DeltaRuleMixer:
         return partial if partial is not None else self.out(gated)
 
 
+def _enter_runs(ctx: BuildContext, heads: int, key_dim: int, value_dim: int) -> None:
+    """Which portions go in chunks of rows depends on their lengths: a fact of a step's layout."""
+    if ctx.dtype == torch.bfloat16 and key_dim == value_dim and key_dim in (64, 128):
+        ctx.layout_facts["recurrence", heads, key_dim] = lambda batch: ctx.ops.run_facts(
+            batch, ctx.ops.scan_runs(batch, heads, key_dim))
+
+
 @MIXERS.register("decay_sum")
 class DecaySumMixer:
     graph_safe = True
@@ -158,6 +165,7 @@ class DecaySumMixer:
         if len(decay) != self.heads:
             raise ValueError(f"{len(decay)} decays for {self.heads} heads")
         self.decay = torch.tensor(decay, dtype=torch.float32, device=ctx.device)
+        _enter_runs(ctx, self.heads, self.key_dim, self.value_dim)
         self.eps = float(params["eps"])
         self.qk_width = self.heads * self.key_dim
         self.inner = self.heads * self.value_dim
@@ -295,6 +303,7 @@ class RetentionMixer:
         if len(decay) != self.heads:
             raise ValueError(f"{len(decay)} decays for {self.heads} heads")
         self.decay = torch.tensor(decay, dtype=torch.float32, device=ctx.device)
+        _enter_runs(ctx, self.heads, self.key_dim, self.value_dim)
         rotary = params.get("rotary") or {}
         self.rotary_dim = int(rotary.get("dims", 0))
         if self.rotary_dim % 2 or self.rotary_dim > self.key_dim:

@@ -85,3 +85,27 @@ def test_a_later_value_that_is_infinite_reaches_no_earlier_row(ops):
         ops.matrix_state_scan(q, k, v, steps.mgr.view(0).state["s"], batch, y, H, H, d, d, decay=decay)
         out.append(y)
     assert torch.equal(out[0][:75], out[1][:75]) and not out[1][75].isfinite().any()
+
+
+@pytest.mark.parametrize("d,rot", [(64, 64), (128, 0)])
+def test_a_portion_alone_gives_the_same_bits(ops, d, rot):
+    """Portions that go in chunks between such as do not, and single tokens: outputs and states are those of the
+    request by itself."""
+    H, counts = 2, {0: 2, 1: 300, 2: 63, 3: 128, 4: 30, 5: 257, 6: 1}
+    g = torch.Generator().manual_seed(d)
+    decay, freq = torch.tensor([0.9, 0.999]).cuda(), (10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64) / 64)).cuda()
+    x = {r: torch.randn(n, 3 * H * d, generator=g).bfloat16().cuda() for r, n in counts.items()}
+
+    def run(which):
+        steps = Steps(ops, 7, state=StateNeeds({"s": ((H, d, d), torch.float32)}), dtype=torch.bfloat16)
+        batch, where = steps.step({r: counts[r] for r in which})
+        rows = torch.cat([x[r] for r in which if counts[r] > 1] + [x[r] for r in which if counts[r] == 1])
+        y, state = torch.full((rows.shape[0], H * d), float("nan"), device="cuda"), steps.mgr.view(0).state["s"]
+        ops.matrix_state_scan(rows[:, :H * d], rows[:, H * d:2 * H * d], rows[:, 2 * H * d:], state, batch, y, H, H, d, d,
+                              decay=decay, rotary=(batch.positions, freq, rot) if rot else None)
+        slots = dict(zip(batch.host.requests, batch.host.state_slot))
+        return {r: (y[where[r][0]:where[r][0] + counts[r]], state[int(slots[r])]) for r in which}
+    together = run(list(counts))
+    for r in counts:
+        for a, b in zip(together[r], run([r])[r]):
+            assert torch.equal(a, b), r

@@ -250,3 +250,44 @@ def test_the_number_of_expanded_tiles_is_a_fact_of_the_layout(latents):
     a, b = portions((0, 110), (0, 60)), portions((0, 112), (0, 58))
     assert all(a.tiles[t].shape == b.tiles[t].shape for t in a.tiles) and a.num_tokens == b.num_tokens
     assert Decoder.layout_facts(model, a) != Decoder.layout_facts(model, b)
+
+
+def test_a_portion_goes_through_the_recurrence_its_own_way(ops):
+    """In chunks or step by step by its own rows; the launches cover all requests in order, with their rows."""
+    calls = []
+    for name in ("chunks", "prepare", "scan"):
+        setattr(ops.lib, f"somi_matrix_state_{name}",
+                lambda *args, name=name: calls.append((name, [getattr(a, "value", a) for a in args])) or 0)
+    ops.use_scan_chunks, ops.prefill_q_tile = True, 64
+    H, d, rng = 2, 64, random.Random(3)
+    least = ops.SCAN_CHUNK_ROWS * d
+    for _ in range(100):
+        lengths = [rng.choice((2, 17, least - 1, least, least + 1, 5 * least)) for _ in range(rng.randrange(1, 6))]
+        batch = portions(*((0, n) for n in lengths), singles=rng.choice(((), (5, 9))))
+        T, R = batch.num_tokens, batch.num_requests
+        qkv = on_device(T, 3 * H * d, dtype=torch.bfloat16)
+        calls.clear()
+        ops.matrix_state_scan(qkv[:, :H * d], qkv[:, H * d:2 * H * d], qkv[:, 2 * H * d:], on_device(R, H, d, d), batch,
+                              on_device(T, H * d), H, H, d, d, decay=on_device(H))
+        at, cu = 0, batch.cu_q.data_ptr()
+        for name, args in calls:
+            if name == "prepare":
+                continue
+            n = args[14] if name == "chunks" else args[-10]
+            first = ((args[10] if name == "chunks" else args[-13]) - cu) // 4
+            assert first == at and n >= 1
+            for r in range(at, at + n):
+                assert (r < len(lengths) and lengths[r] >= least) == (name == "chunks")
+            if name == "chunks":
+                assert args[13] == sum(-(-q // 64) for q in lengths[at:at + n]) and args[15] == batch.host.cu_q[at + n]
+            at += n
+        assert at == R
+
+
+def test_the_chunks_workspace_is_bounded(ops):
+    """Portions whose chunks' states together take more than 512 MB go one run behind the other, one that
+    takes more by itself step by step."""
+    heads, d = 28, 128
+    runs = ops.scan_runs(portions((0, 10000), (0, 10000), (0, 20000), singles=(4,)), heads, d)
+    assert runs == ((0, 1, 157), (1, 2, 157), (2, 4, 0))
+    assert all(n * heads * d * d * 4 <= 1 << 29 for _, _, n in runs)
