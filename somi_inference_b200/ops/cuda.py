@@ -1674,9 +1674,11 @@ class CudaOps:
     SCAN_PREPARE_ROWS = 16
     SCAN_TURN_ROWS = 4          # the most rows a request may have where the scan itself rotates q and k
 
-    # a portion goes in chunks from rows = this * state width on (both sides measured in
-    # `csrc/recurrent_chunks.cu`: they meet at 128 to 256 rows for a width of 128, at 32 to 64 for 64)
-    SCAN_CHUNK_ROWS = 1
+    # A portion goes in chunks from rows = this * state width on.  The layer in us step by step / in chunks,
+    # captured: 14 heads of 64: 64 rows 38.9 / 36.9, 84 beside 11 single tokens 43.1 / 43.1, 96 45.2 / 36.9, 256 79.8 /
+    # 39.0; 28 of 128: 128 rows 94.0 / 96.4, 160 100.5 / 100.8, 192 110.5 / 102.5, 256 129.1 / 113.9.  Launched one by one
+    # both are bound by the host up to about 256 rows, and the 84 rows beside single tokens took 130.1 / 145.7.
+    SCAN_CHUNK_ROWS = 1.5
     SCAN_CHUNK_BYTES = 1 << 29  # the most that the chunks' states of a run of portions may take
 
     def scan_in_chunks(self, q, k, v, batch, heads, qk_heads, dk, dv, act_silu, unit_eps, beta, decay_logits,
@@ -1746,14 +1748,14 @@ class CudaOps:
         first, end, n_tiles = run
         rows = int(batch.host.cu_q[end])                     # (angles of the rows in front are made too)
         tiles, _ = self._tiles_of(batch, self.prefill_q_tile, first, end)
-        angles = torch.empty(rows * rot, dtype=torch.float32, device=q.device) if rot else None
-        u = torch.empty(n_tiles * heads * dk * dk, dtype=torch.float32, device=q.device)
+        n_u = n_tiles * heads * dk * dk                      # the chunks' states, and the angles behind them
+        u = torch.empty(n_u + rows * rot, dtype=torch.float32, device=q.device)
         rc = self.lib.somi_matrix_state_chunks(
             _ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(q.stride(0)), ctypes.c_longlong(k.stride(0)),
             ctypes.c_longlong(v.stride(0)), ctypes.c_int(3 if act_silu else 0), ctypes.c_float(q_scale), _ptr(decay),
             _ptr(state), _ptr(batch.cu_q, first), _ptr(batch.state_slot, first), tiles, ctypes.c_int(n_tiles),
             ctypes.c_int(end - first), ctypes.c_int(rows), ctypes.c_int(heads), ctypes.c_int(heads // qk_heads),
-            ctypes.c_int(dk), _ptr(pos), _ptr(freq), ctypes.c_int(rot), _ptr(angles), _ptr(u), _ptr(y),
+            ctypes.c_int(dk), _ptr(pos), _ptr(freq), ctypes.c_int(rot), _ptr(u, n_u), _ptr(u), _ptr(y),
             self._stream())
         self._done(rc, "matrix_state_chunks")
         self.launches += 3 if rot else 2
@@ -1771,7 +1773,7 @@ class CudaOps:
         if end - first < batch.num_requests:
             cu = batch.host.cu_q
             row, rows = int(cu[first]), int(cu[end] - cu[first])
-            max_rows = max(int(cu[r + 1] - cu[r]) for r in range(first, end))
+            max_rows = max((int(cu[r + 1] - cu[r]) for r in range(first, min(end, batch.num_prefill_requests))), default=1)
         if prepare is None:
             prepare = max_rows > self.SCAN_PREPARE_ROWS
         # the scan turns q and k itself only in steps of a few rows

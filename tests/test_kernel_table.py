@@ -260,7 +260,7 @@ def test_a_portion_goes_through_the_recurrence_its_own_way(ops):
                 lambda *args, name=name: calls.append((name, [getattr(a, "value", a) for a in args])) or 0)
     ops.use_scan_chunks, ops.prefill_q_tile = True, 64
     H, d, rng = 2, 64, random.Random(3)
-    least = ops.SCAN_CHUNK_ROWS * d
+    least = int(ops.SCAN_CHUNK_ROWS * d)
     for _ in range(100):
         lengths = [rng.choice((2, 17, least - 1, least, least + 1, 5 * least)) for _ in range(rng.randrange(1, 6))]
         batch = portions(*((0, n) for n in lengths), singles=rng.choice(((), (5, 9))))
