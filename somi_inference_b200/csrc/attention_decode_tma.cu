@@ -603,11 +603,15 @@ int launch_tma_decode(const CUtensorMap* map, const void* qkv, int row_stride, i
             sm_count = 148;
     }
     const long long units = static_cast<long long>(max_splits) * nkv * n_decode;
-    // (up to five chunks a CTA the one-chunk kernel is the faster: 64 requests of 28 heads over 4 of 128 at
-    // 2,048 positions 68.7 us for the layer against 72.8 with four chunks and 70.6 with six, 32 of 40 over 8
-    // 87.3 against 89.3 and 90.2; at 8,192 positions 183 against 171 with eight)
+    // Where few chunks fall to a CTA the one-chunk kernel is the faster, unless its merge gets long (more than 32
+    // chunks a request).  The layer in us, one chunk / as many as fit, contexts from half the given length up:
+    // 28 heads over 4 of 128, 64 requests: 2 at 1,260 positions 53.3 / 59.9, 4 at 2,412 73.9 / 76.8, 5 at 3,052 84.5 /
+    // 85.8, 6 at 3,692 95.5 / 96.4, 7 at 4,204 105.5 / 103.4; 16 requests: 4 at 10,092 84.4 / 84.5, 5 at 12,524 99.8 / 96.4, 6 at 14,828
+    // 113.5 / 106.6.  14 over 2 of 64, 64 requests: 3 at 3,820 37.1 / 37.0, 4 at 4,972 45.0 / 44.8, 5 at 6,252 50.7 / 49.2, 6 at 7,404 57.5 /
+    // 55.1.  40 over 8 of 128, 32 requests: 3 at 1,900 84.8 / 91.5, 5 at 3,052 103.4 / 105.1, 6 at 3,692 113.7 / 116.6, 7 at 4,204 128.8 / 125.0.
     const int fitting = static_cast<int>(std::min<long long>(kRingMaxCpc, units / (8LL * sm_count)));
-    const int cpc = g_ring_chunks > 0 ? std::min(g_ring_chunks, kRingMaxCpc) : (fitting >= 6 ? fitting : 1);
+    const int cpc = g_ring_chunks > 0 ? std::min(g_ring_chunks, kRingMaxCpc)
+                    : (fitting >= 6 || (fitting == 5 && max_splits > 32) ? fitting : 1);
     if (cpc >= 2) {
         const size_t ring_smem = (kRingK + kRingV) * TILE + kTdRows * HD * 2 + kTdRows * kTdChunk * 2 + 1024;
         cudaFuncSetAttribute(paged_decode_ring_kernel<HD, TWO_MAPS>,
