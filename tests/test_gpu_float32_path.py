@@ -149,3 +149,38 @@ def test_attention_of_single_tokens_in_groups(ops, monkeypatch, window):
     for requests in (1, 2, 4):
         monkeypatch.setattr(ops, "F32_PART_FLOATS", requests * nq * (12 if window is None else (window + 62) // 64 + 1) * (hd + 2))
         assert torch.equal(run(ops, case, nq, nkv, hd, window), want)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("window,infinite", [(None, False), (100, False), (None, True), (100, True)])
+def test_shares_of_a_tile_give_the_same_bits(ops, hd, window, infinite):
+    """A tile of 64 rows is one CTA's, or shared by two or four where a step has few: a request of 140 rows alone
+    (18 tiles and heads: four), among 5 (90: two) and among 20 like it (360: one), with an infinite value too."""
+    nq, nkv, ps = 6, 2, 16
+    got, first = [], None
+    for n in (1, 5, 20):
+        case = attention_case(ops, nq=nq, nkv=nkv, hd=hd, page_size=ps, window=window, requests=[(131, 140)] * n,
+                              dtype=torch.float32)
+        _, batch, qkv, view, _ = case
+        assert batch.tiles[64].shape[0] * nq == 18 * n
+        table = batch.groups[0].block_table[:, :17].long()
+        if first is None:
+            if infinite:
+                view.values[table[0, 150 // ps], :, 150 % ps] = float("inf")
+            live = table[0] >= 0
+            first = qkv.clone(), view.keys[table[0][live]].clone(), view.values[table[0][live]].clone()
+        for i in range(n):
+            assert torch.equal(table[i] >= 0, live)
+            view.keys[table[i][live]], view.values[table[i][live]] = first[1], first[2]
+            qkv[140 * i:140 * (i + 1)] = first[0]
+        got.append(run(ops, case, nq, nkv, hd, window))
+    sees = torch.arange(131, 271) >= 150
+    if window:
+        sees &= torch.arange(131, 271) < 150 + window
+    for out in got:
+        for part in out.split(140):
+            assert torch.equal(part[~sees.cuda()], got[0][~sees.cuda()])
+            if not infinite:
+                assert torch.equal(part, got[0])
+            else:
+                assert not part[sees.cuda()].isfinite().any()
