@@ -220,8 +220,7 @@ sgemm_nt_kernel(const float* __restrict__ x, const float* __restrict__ w, const 
         return;
     }
     // the ranges' tiles, each in its CTA's shared memory; every CTA of the cluster adds up a share of
-    // the elements in the order of the ranges (those that a short K leaves empty are left out, as
-    // the walk above never gets to them)
+    // the elements in the order of the ranges (no K leaves one empty)
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -243,7 +242,7 @@ sgemm_nt_kernel(const float* __restrict__ x, const float* __restrict__ w, const 
         float4 sum = part[0];
 #pragma unroll
         for (int r = 1; r < 8; ++r)
-            if (r < ranges && r * range_length < K)
+            if (r < ranges)
                 sum = make_float4(__fadd_rn(sum.x, part[r].x), __fadd_rn(sum.y, part[r].y),
                                   __fadd_rn(sum.z, part[r].z), __fadd_rn(sum.w, part[r].w));
         if (gm >= M) continue;

@@ -10,8 +10,8 @@
 //
 // Why: step by step, a portion is one chain of rows per (head, 16 columns) with two sums over a warp each:
 // 224 CTAs for 28 heads of 128, 522 us for 2,048 rows behind 43 us of preparation.  In chunks a row
-// costs no more operations (64 x 2 x (5/8) + 128 x 2 per column against 128 x 2 and the sums), nothing waits
-// for anything but the second kernel, and the FMA pipe is the bound: thread tiles of 8 x 8 and 4 x 8 from
+// costs a third more FMAs (64 x 2 x (5/8) + 128 x 2 per column against 128 x 2 and the sums over warps), but nothing
+// waits for anything but the second kernel, and the FMA pipe is the bound: thread tiles of 8 x 8 and 4 x 8 from
 // shared memory, the upper triangle left out in blocks of 16.  The same rows: angles 5, U 70, states 36,
 // y 123 us (0.92 and 1.5 G FMAs at 26 and 24 TFLOP/s; scalar and paired FMAs take the same time).  The layer
 // with it, step by step / in chunks, 28 heads of 128: 128 rows 98 / 99 us, 256 132 / 115, 2,048 796 / 446, 8,192
