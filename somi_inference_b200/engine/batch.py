@@ -48,6 +48,8 @@ class HostBatch:
     ctx_len: np.ndarray
     state_slot: np.ndarray
     requests: list
+    # what parts work out from these arrays for the step, once for all layers that are alike
+    plans: dict = field(default_factory=dict)
 
 
 @dataclass

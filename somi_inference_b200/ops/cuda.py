@@ -9,6 +9,7 @@ compiled library, construction fails.
 from __future__ import annotations
 
 import ctypes
+from functools import lru_cache
 
 import torch
 
@@ -135,6 +136,8 @@ class CudaOps:
         tiles, n = batch.tiles[size], batch.num_prefill_requests
         if first <= 0 and end >= n:
             return _ptr(tiles), tiles.shape[0]
+        if first >= n:
+            return _ptr(tiles), 0
         ends, at = batch.host.cu_q, []
         for stop in (min(first, n), min(end, n)):
             at.append(sum(-(-int(ends[r + 1] - ends[r]) // size) for r in range(stop)))
@@ -145,10 +148,11 @@ class CudaOps:
         """The step's requests as runs (first, end, tiles): neighbouring portions that a kernel over tiles
         takes, with the sum of their `tiles(rows, cached)` (at most `most`, as `rounded`), and neighbours that
         it leaves (0 tiles; single tokens always are)."""
-        cu, ctx = batch.host.cu_q, batch.host.ctx_len
-        runs = []
-        for r in range(batch.num_prefill_requests):
-            n = tiles(int(cu[r + 1] - cu[r]), int(ctx[r]))
+        runs, row = [], 0
+        for r, (end, cached) in enumerate(zip(batch.host.cu_q[1:batch.num_prefill_requests + 1].tolist(),
+                                              batch.host.ctx_len.tolist())):
+            n = tiles(end - row, cached)
+            row = end
             if rounded(n) > most:
                 n = 0
             if runs and (n > 0) == (runs[-1][2] > 0) and rounded(runs[-1][2] + n) <= most:
@@ -964,14 +968,20 @@ class CudaOps:
         whatever else is in the step.  A run's workspace is bounded (more portions are another run; one portion of
         more positions reads the latents).  Tiles are rounded up to one of four sizes per power of two.  A captured
         step is replayed with other lengths: the runs belong to what its layout is told apart by (`run_facts`)."""
+        runs = batch.host.plans.get(("latents", window, heads, rank, dim))
+        if runs is not None:
+            return runs
         t, win = self.latent_tile, int(window) if window else 0
 
         def tiles(rows: int, cached: int) -> int:
             if rows < self.LATENT_EXPAND_ROWS:
                 return 0
             return (cached + rows - 1) // t + 1 - (max(0, cached - win + 1) // t if win else 0)
-        return self._portion_runs(batch, tiles, self.LATENT_EXPAND_BYTES // (t * (rank + 2 * heads * dim) * 2), _rounded_up)
+        runs = self._portion_runs(batch, tiles, self.LATENT_EXPAND_BYTES // (t * (rank + 2 * heads * dim) * 2), _rounded_up)
+        batch.host.plans["latents", window, heads, rank, dim] = runs
+        return runs
 
+    @lru_cache(maxsize=256)
     def latent_expand_supported(self, heads: int, rank: int, key_dim: int, value_dim: int) -> bool:
         """Whether portions of a bfloat16 layer of these sizes can read expanded keys and values."""
         return rank % 8 == 0 and key_dim == value_dim and bool(self.lib.somi_prefill_pp_supported(
@@ -1698,8 +1708,12 @@ class CudaOps:
         recurrence in chunks, and neighbours that go step by step (0 tiles).  A portion's own rows decide,
         so it goes the same way whatever else is in the step.  A run's workspace is bounded (more portions are
         another run; one portion of more rows goes step by step)."""
-        return self._portion_runs(batch, lambda rows, cached: -(-rows // 64) if rows >= self.SCAN_CHUNK_ROWS * dk else 0,
-                                  self.SCAN_CHUNK_BYTES // (heads * dk * dk * 4))
+        runs = batch.host.plans.get(("recurrence", heads, dk))
+        if runs is None:
+            runs = self._portion_runs(batch, lambda rows, cached: -(-rows // 64) if rows >= self.SCAN_CHUNK_ROWS * dk else 0,
+                                      self.SCAN_CHUNK_BYTES // (heads * dk * dk * 4))
+            batch.host.plans["recurrence", heads, dk] = runs
+        return runs
 
     def matrix_state_scan(self, q, k, v, state, batch, y, heads, qk_heads, dk, dv, *,
                           act_silu=False, unit_eps=None, q_scale=1.0, beta=None, decay_logits=None,

@@ -132,7 +132,7 @@ def portions(*lengths, singles=()):
         max_q_len=max(q for _, q in reqs), cu_q=on_device(len(reqs) + 1), ctx_len=on_device(len(reqs)),
         state_slot=on_device(len(reqs)), positions=on_device(T, dtype=torch.int32), tiles=tiles,
         groups=[SimpleNamespace(block_table=on_device(len(reqs), 1), width=-(-widest // 16))],
-        host=SimpleNamespace(cu_q=cu, ctx_len=np.array([c for c, _ in reqs])))
+        host=SimpleNamespace(cu_q=cu, ctx_len=np.array([c for c, _ in reqs]), plans={}))
 
 
 @pytest.fixture
