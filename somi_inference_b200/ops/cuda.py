@@ -954,10 +954,11 @@ class CudaOps:
 
     # A portion reads expanded keys and values from this many rows on.  Per row and
     # position read, attention over the latents takes rank / width times the operations, on the slower
-    # tensor path; expanding takes a fixed number per position.  The layer in us over the latents /
-    # expanded, 28 heads of 128 and rank 512 under a window of 1,024, portions from a prompt's start: 32 rows
-    # 40.6 / 37.0, 128 52.9 / 43.3, 512 126 / 68, 2,048 576 / 167; behind 3,000 positions: 32 rows 123 / 62, 512
-    # 242 / 95.  14 heads of 64, rank 128: 64 rows 24.8 / 26.8, 96 28.9 / 26.9, 2,048 104 / 56.
+    # tensor path; expanding takes a fixed number per position.  The layer, captured in a graph, in us over the
+    # latents / expanded, 28 heads of 128 and rank 512 under a window of 1,024, portions from a prompt's start:
+    # 32 rows 40.6 / 37.0, 96 48.7 / 39.9, 512 126 / 68, 2,048 571 / 160; behind 3,000 positions: 32 rows 123 / 62, 512
+    # 242 / 95; without a window beside single tokens at 16,000 positions: 96 rows and one 203.0 / 204.5, 500 and one 277 /
+    # 227, 300 behind 4,000 and eight 507 / 268.  14 heads of 64, rank 128: 64 rows 24.8 / 26.8, 96 28.9 / 26.9, 2,048 104 / 56.
     LATENT_EXPAND_ROWS = 96
     LATENT_EXPAND_BYTES = 1 << 29       # the most that a run's latents, keys and values may take
 
