@@ -21,9 +21,11 @@
 // to 2, 4, 8, 16 or 32, with four 32-deep stages of cp.async in flight per CTA and the first ones
 // issued before the dependency wait (a model's weights are constants).  More rows are bound by the FMA pipe: a
 // 64 x 64 tile, 8 x 4 outputs a thread, operands read from shared memory four k at a time as one
-// 16-byte access (rows 36 floats apart, so eight neighbouring rows lie in different banks).  Up to 256 rows
-// a 32-row tile, of which there are twice as many, is the faster (896 x 4,864 at 207 rows 63 against 79 us,
-// 9,728 x 896 115 against 130), from 512 rows on the 64-row tile (1,024 rows 258 against 316 us).
+// 16-byte access (rows 36 floats apart, so eight neighbouring rows lie in different banks).  Up to 384 rows
+// a 32-row tile, of which there are twice as many, is the faster: 32 / 64 rows a tile in us, at 257, 384 and 448 rows:
+// 896 x 4,864 82.4 / 98.1, 101.1 / 116.8, 120.1 / 127.3; 9,728 x 896 144.3 / 156.4, 185.8 / 188.4, 212.5 / 217.7; 1,152 x 896 23.6 /
+// 25.6, 30.4 / 32.9, 34.6 / 34.1; 896 x 896 18.8 / 24.4, 23.9 / 25.6, 27.3 / 25.7.  From there on they take turns, and at 512
+// rows 9,728 x 896, the largest share of a step, is ahead with 64 (239.9 / 229.6; 1,024 x 896 x 4,864 316 / 258).
 // Measured in chains of products: 4 rows by 9,728 x 896 8.5 us (4.1 TB/s), 1 row by 151,936 x 896 93 us
 // (5.8 TB/s), 1,024 rows by 9,728 x 896 425 us (42 TFLOP/s; the FMA pipe is busy 63 % of the cycles).  A
 // step of the 0.5B shape with 203 prompt tokens and 4 single ones, which runs 97 such products, took
@@ -321,7 +323,7 @@ SOMI_API int somi_gemm_f32_batched(const float* x, const float* w, const float* 
     if (M <= 4) return sg_launch<4, 4, 1>(a, stream);
     if (M <= 8) return sg_launch<8, 2, 2>(a, stream);
     if (M <= 16) return sg_launch<16, 4, 2>(a, stream);
-    if (M <= 256) return sg_launch<32, 8, 2>(a, stream);
+    if (M <= 384) return sg_launch<32, 8, 2>(a, stream);
     return sg_launch<64, 8, 4>(a, stream);
 }
 

@@ -35,6 +35,16 @@ def test_product_at_the_bounds_of_tiles_and_ranges(ops, K, N):
         assert torch.equal(ops.gemm_f32(x[130 - m:].contiguous(), w, b), whole[130 - m:]), m
 
 
+@pytest.mark.parametrize("N,K", [(65, 548), (9728, 130)])
+def test_product_around_the_switch_of_row_tiles(ops, N, K):
+    """Up to 384 rows a tile has 32 rows, from there on 64: a row gives the same bits in either."""
+    g = torch.Generator().manual_seed(N)
+    x, w = torch.randn(449, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    whole = ops.gemm_f32(x, w)
+    for m in (256, 257, 383, 384, 385):
+        assert torch.equal(ops.gemm_f32(x[:m].contiguous(), w), whole[:m]), m
+
+
 def test_product_with_more_rows_than_a_grid_has_tiles(ops):
     """65,535 tiles of 64 rows and 70 rows more: each product is a sum of four terms (five roundings)."""
     g = torch.Generator(device="cuda").manual_seed(3)
