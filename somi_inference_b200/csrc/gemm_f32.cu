@@ -1,5 +1,7 @@
-// The float32 path's matrix product: y[M, N] = x[M, K] w[N, K]^T (+ bias[N]), every product and
-// sum a float32 FMA on the CUDA cores (no tensor cores, no reduced-precision mode of any kind).
+// The float32 path's matrix product: y[M, N] = x[M, K] w[N, K]^T (+ bias[N]).  From 512 terms on, where rows can be
+// read 16 bytes at a time, the product goes to tensor cores in exact bfloat16 parts (gemm_f32_split.cuh, gemm_f32_rows.cu,
+// gemm_f32_tcgen05.cu); this file takes the others, every product and sum a float32 FMA on the CUDA cores.
+// Neither uses a reduced-precision mode of any kind.
 //
 // The reference's engine uses the library product here (nn.Linear,
 // somi_inference/models/qwen2.py:221-222,268-271).  This engine does not, for two reasons.  The
@@ -19,20 +21,15 @@
 //
 // What bounds it: a few rows stream the weights, so the tile is 64 weight rows by the rows rounded up
 // to 2, 4, 8, 16 or 32, with four 32-deep stages of cp.async in flight per CTA and the first ones
-// issued before the dependency wait (a model's weights are constants).  More rows are bound by the FMA pipe: a
-// 64 x 64 tile, 8 x 4 outputs a thread, operands read from shared memory four k at a time as one
+// issued before the dependency wait (a model's weights are constants).  More rows are bound by shared memory and the FMA
+// pipe in turn: a 64 x 64 tile, 8 x 4 outputs a thread, operands read from shared memory four k at a time as one
 // 16-byte access (rows 36 floats apart, so eight neighbouring rows lie in different banks).  Up to 384 rows
-// a 32-row tile, of which there are twice as many, is the faster: 32 / 64 rows a tile in us, at 257, 384 and 448 rows:
-// 896 x 4,864 82.4 / 98.1, 101.1 / 116.8, 120.1 / 127.3; 9,728 x 896 144.3 / 156.4, 185.8 / 188.4, 212.5 / 217.7; 1,152 x 896 23.6 /
-// 25.6, 30.4 / 32.9, 34.6 / 34.1; 896 x 896 18.8 / 24.4, 23.9 / 25.6, 27.3 / 25.7.  From there on they take turns, and at 512
-// rows 9,728 x 896, the largest share of a step, is ahead with 64 (239.9 / 229.6; 1,024 x 896 x 4,864 316 / 258).
-// Measured in chains of products: 4 rows by 9,728 x 896 8.5 us (4.1 TB/s), 1 row by 151,936 x 896 93 us
-// (5.8 TB/s), 1,024 rows by 9,728 x 896 425 us (42 TFLOP/s; the FMA pipe is busy 63 % of the cycles).  A
-// step of the 0.5B shape with 203 prompt tokens and 4 single ones, which runs 97 such products, took
-// 46.1 ms while one CTA computed 32 or 128 rows by 128 columns over all of K.
+// a 32-row tile, of which there are twice as many, is the faster.  Measured with 896 terms, when those came here too:
+// 32 / 64 rows a tile, 9,728 x 896, 257, 384 and 448 rows 144.3 / 156.4, 185.8 / 188.4, 212.5 / 217.7 us, 512 rows
+// 239.9 / 229.6; 1,024 rows 425 us (42 TFLOP/s; the tensor cores take 113).
 #include <cooperative_groups.h>
 
-#include "common.cuh"
+#include "gemm_f32_split.cuh"
 
 namespace somi {
 
@@ -264,15 +261,8 @@ sgemm_nt_kernel(const float* __restrict__ x, const float* __restrict__ w, const 
     cluster.sync();                                      // no CTA leaves while its tile is read
 }
 
-struct SgArgs {
-    const float *x, *w, *bias;
-    float* y;
-    int M, N, K, batch, w_constant;
-    long long ldx, ldy, bsx, bsw, bsy;
-};
-
 template <int BM, int TM, int TN, bool VEC, bool CLUSTER>
-int sg_launch_one(const SgArgs& a, int ranges, cudaStream_t stream) {
+int sg_launch_one(const FsArgs& a, int ranges, cudaStream_t stream) {
     auto kernel = sgemm_nt_kernel<BM, TM, TN, VEC, CLUSTER>;
     constexpr int smem = sg_smem<BM>();
     if (smem > 48 * 1024)
@@ -291,7 +281,7 @@ int sg_launch_one(const SgArgs& a, int ranges, cudaStream_t stream) {
 }
 
 template <int BM, int TM, int TN>
-int sg_launch(const SgArgs& a, cudaStream_t stream) {
+int sg_launch(const FsArgs& a, cudaStream_t stream) {
     const int ranges = sg_ranges(a.K);
     const long long tiles = static_cast<long long>((a.N + kSgBN - 1) / kSgBN) * ((a.M + BM - 1) / BM) * a.batch;
     const bool cluster = ranges > 1 && tiles < sg_fill_tiles(BM);
@@ -318,7 +308,8 @@ SOMI_API int somi_gemm_f32_batched(const float* x, const float* w, const float* 
                                    cudaStream_t stream) {
     if (M <= 0 || N <= 0 || batch <= 0) return 0;
     if (K <= 0 || batch > 65535 || ldx < K || ldy < N) return SOMI_ERR_UNSUPPORTED;
-    const SgArgs a{x, w, bias, y, M, N, K, batch, w_constant, ldx, ldy, bsx, bsw, bsy};
+    const FsArgs a{x, w, bias, y, M, N, K, batch, w_constant, ldx, ldy, bsx, bsw, bsy};
+    if (fs_takes(a)) return M <= 16 ? fs_launch_rows(a, stream) : fs_launch_tiles(a, stream);
     if (M <= 2) return sg_launch<2, 2, 1>(a, stream);
     if (M <= 4) return sg_launch<4, 4, 1>(a, stream);
     if (M <= 8) return sg_launch<8, 2, 2>(a, stream);

@@ -330,6 +330,9 @@ class CudaOps:
         if int(self.lib.somi_gemm_error()) != 0:
             raise KernelError("the tcgen05 matrix product gave up waiting on a barrier; "
                               "its results are not valid")
+        if int(self.lib.somi_gemm_f32_error()) != 0:
+            raise KernelError("the float32 tcgen05 matrix product gave up waiting on a barrier; "
+                              "its results are not valid")
 
     @staticmethod
     def _attention_work(batch, first: int, last: int, nq: int, nkv: int, hd: int, elt: int,
@@ -2083,7 +2086,8 @@ class CudaOps:
 
     def gemm_f32(self, x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
                  constant: bool = False) -> torch.Tensor:
-        """x[M, K] @ w[N, K]^T (+ bias) in float32 FMAs, each output summed over K in an order
+        """x[M, K] @ w[N, K]^T (+ bias) in float32: FMAs, or from 512 terms on products of exact bfloat16 parts
+        on tensor cores with float32 sums (`csrc/gemm_f32_split.cuh`); each output summed over K in an order
         that K alone fixes (the float32 path's product; the library's is not used there).  `constant`: no
         kernel of the same step writes `w` (a model's weights), and the kernel may read it before it waits."""
         _check(x, w, bias)

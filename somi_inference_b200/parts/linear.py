@@ -5,8 +5,9 @@ The reference's engine uses `nn.Linear` for every projection
 tokens (bfloat16, at most `ops.skinny_max_tokens` rows) runs the engine's own tcgen05 kernel,
 which streams the weight once through TMA and tensor memory and can leave split-K partial sums
 or apply SiLU(gate)*up in its epilogue; larger bfloat16 steps (prompt portions) go to the library
-product.  float32 goes to the engine's own float32 kernel (`csrc/gemm_f32.cu`: plain FMAs, every
-output summed over K in an order that K alone fixes, whatever the step's size), not to the library.
+product.  float32 goes to the engine's own float32 kernels (`csrc/gemm_f32.cu`: plain FMAs, or exact
+bfloat16 parts on tensor cores with float32 sums, by the matrix's sizes alone; every output summed over K
+in an order that K alone fixes, whatever the step's size), not to the library.
 """
 
 from __future__ import annotations

@@ -1,0 +1,68 @@
+"""The float32 product in bfloat16 parts (from 512 terms on): the sizes where its kernels and tiles change, in rows, features
+and terms; that a row's bits depend on none of them; and operands that have no parts."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from somi_inference_b200.ops import cuda_ops
+    return cuda_ops()
+
+
+@pytest.mark.parametrize("K", [512, 516, 896, 1024, 1088, 2044, 4864, 20480])
+@pytest.mark.parametrize("N", [64, 333, 1152, 5000])
+def test_rows_and_error(ops, N, K):
+    """One error bound for all forms: six products of parts leave out less than 2^-25 of a term; a block's last four steps (and
+    20 that are 2^-8 as large) lose less than two units of 2^-24 of the terms' magnitudes each, and the sums over
+    blocks and ranges round K / 64 + 9 times.  Each row gives the bits that it gives alone."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    x = torch.randn(700, K, generator=g, device="cuda")
+    w, b = torch.randn(N, K, generator=g, device="cuda"), torch.randn(N, generator=g, device="cuda")
+    whole = ops.gemm_f32(x, w, b)
+    want, size = x.double() @ w.double().T + b.double(), x.double().abs() @ w.double().abs().T + b.double().abs()
+    assert ((whole.double() - want).abs() <= (K / 64 + 9 + 8 + 2) * 2.0 ** -24 * size).all()
+    for m in (1, 8, 9, 16, 17, 64, 65, 129, 207, 257, 513):
+        assert torch.equal(ops.gemm_f32(x[700 - m:].contiguous(), w, b), whole[700 - m:]), m
+    ops.check_errors()
+
+
+@pytest.mark.parametrize("M", [3, 11, 40, 300, 1500])
+@pytest.mark.parametrize("N", [80, 6000])
+def test_operands_without_parts(ops, M, N):
+    """Infinities, NaN and numbers that bfloat16 rounds to infinity: the outputs that meet them are what float32
+    FMAs give, the others keep their bits."""
+    K = 640
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    x[:, 3] *= 0.1                                       # (its product with the largest numbers stays finite)
+    before = ops.gemm_f32(x, w)
+    x[1, 70], x[2, 71] = float("inf"), 3.4e38
+    w[5, 600], w[77, 3] = float("nan"), -3.4e38
+    w[5 + 1:, 71].clamp_(-0.5, 0.5)
+    w[:, 70].abs_()
+    touched = torch.zeros(M, N, dtype=torch.bool, device="cuda")
+    touched[1:3], touched[:, 5], touched[:, 77] = True, True, True
+    after, clean = ops.gemm_f32(x, w), w.clone()
+    clean[5], clean[77] = 0, 0
+    rest = ops.gemm_f32(x, clean)
+    assert torch.equal(after[~touched], rest[~touched]) and before.isfinite().all()
+    assert after[:, 5].isnan().all() and (after[1, 6:77] == float("inf")).all()
+    want = (x[2].double() * w[6:77].double()).sum(1)
+    torch.testing.assert_close(after[2, 6:77].double(), want, rtol=1e-4, atol=0)
+    torch.testing.assert_close(after[0, 77].double(), (x[0].double() * w[77].double()).sum(), rtol=1e-4, atol=0)
+
+
+def test_products_of_a_batch_and_strided_rows(ops):
+    """A product per head over views of wider rows, few rows and many: the bits of each head by itself."""
+    H, K, N = 3, 512, 128
+    g = torch.Generator(device="cuda").manual_seed(2)
+    w = torch.randn(H, N, K, generator=g, device="cuda")
+    for T in (5, 200):
+        x = torch.randn(T, H * K + 8, generator=g, device="cuda")[:, 4:4 + H * K].view(T, H, K)
+        y = ops.head_product(x, w, heads_first=True)
+        for h in range(H):
+            assert torch.equal(y[h], ops.gemm_f32(x[:, h].contiguous(), w[h]))
