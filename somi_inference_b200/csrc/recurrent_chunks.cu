@@ -1,40 +1,37 @@
 // The matrix-state recurrence with a constant decay per head, S <- g S + k v^T, y = S^T q, for prompt portions
-// in chunks of 64 rows (bfloat16 inputs; the step by step form in recurrent_parts.cu serves single
+// in chunks of 128 rows (bfloat16 inputs; the step by step form in recurrent_parts.cu serves single
 // tokens, short portions, float32 inputs, decays per channel and the delta rule).  With S_0 the state in
 // front of a chunk, t and s rows of it counted from 0, and n rows:
 //     y_t = g^(t + 1) S_0^T q_t + sum over s <= t of g^(t - s) (q_t . k_s) v_s
 //     S_n = g^n S_0 + U,   U = sum over s of g^(n - 1 - s) k_s v_s^T
 // Three kernels: U of every chunk and head; the states in front of every chunk, from U in place and in
-// order (and the last one to the request's slot); y.  Everything is float32: the products are FMAs on the
-// CUDA cores, the powers of g are powf, q and k are activated and rotated in float32 as they are read.
+// order (and the last one to the request's slot); y.  Everything is float32: q and k are activated and rotated in float32 as they
+// are read, the powers of g are powf, and the products take every float32 operand as three bfloat16 numbers whose sum it
+// is (gemm_f32_split.cuh; v as it is, where it is not activated), summed in float32 by `tcgen05.mma`.
 //
 // Why: step by step, a portion is one chain of rows per (head, 16 columns) with two sums over a warp each:
-// 224 CTAs for 28 heads of 128, 522 us for 2,048 rows behind 43 us of preparation.  In chunks a row
-// costs a third more FMAs (64 x 2 x (5/8) + 128 x 2 per column against 128 x 2 and the sums over warps), but nothing
-// waits for anything but the second kernel, and the FMA pipe is the bound: thread tiles of 8 x 8 and 4 x 8 from
-// shared memory, the upper triangle left out in blocks of 16.  The same rows: angles 5, U 70, states 36,
-// y 123 us (0.92 and 1.5 G FMAs at 26 and 24 TFLOP/s; scalar and paired FMAs take the same time).  The layer
-// with it, step by step / in chunks, 28 heads of 128: 128 rows 98 / 99 us, 256 132 / 115, 2,048 796 / 446, 8,192
-// 3,053 / 1,669; 14 heads of 64: 32 rows 33 / 37, 64 40 / 37, 2,048 467 / 92.
-#include "common.cuh"
+// 224 CTAs for 28 heads of 128, 522 us for 2,048 rows behind 43 us of preparation.  In chunks nothing
+// waits for anything but the second kernel.  As FMAs on the CUDA cores, in chunks of 64 rows, the products took U 70 and y 123 us
+// (25 TFLOP/s); on tensor cores, with half as many states in between, the same rows take: angles 3, U 28, states 18 (36), y 66 us,
+// each with nothing in L2.  What bounds them now: a CTA's phases (load and split, multiply, load and split, ..) one behind the
+// other, two CTAs to an SM, with the tensor pipe busy a quarter of the time, and 448 CTAs in two rounds of 296.  Fetching
+// a phase ahead did not shorten y, U by 1 us.
+// The layer with it, 28 heads of 128, 2,048 rows: step by step 796, FMAs 462, now 365 us.
+#include "gemm_f32_split.cuh"
 #include "rotation.cuh"
+#include "tcgen05.cuh"
 #include "vec4.cuh"
 
 namespace somi {
 
-constexpr int kChRows = 64;           // rows per chunk (the tile list's query tiles of 64)
+constexpr int kChRows = 128;          // rows per chunk: two tiles of the tile list, the MMA's M
+constexpr int kChTile = 64;
 constexpr int kChThreads = 256;
-constexpr int kChBK = 32;             // key channels of the state staged at a time
+constexpr int kChHalf = 64;           // rows or channels of one swizzled tile's other side: 128 bytes
+
+__device__ int g_chunks_error = 0;
 
 __device__ __forceinline__ float ch_silu(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ void ch_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ float ch_sum2(unsigned long long d) {
-    float lo, hi;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
-    return lo + hi;
-}
 
 // Cosine and sine of every pair of the portions' rows, once for all heads.
 __global__ void chunk_angles_kernel(const int* __restrict__ positions, const double* __restrict__ freq, int half,
@@ -45,6 +42,18 @@ __global__ void chunk_angles_kernel(const int* __restrict__ positions, const dou
     if (i < n) cs[i] = turn_by(static_cast<double>(positions[i / half]), freq[i % half]);
 }
 
+// The chunks of a run of requests, as its tiles of 64 rows give them: each pair of a request's tiles, at the pair's first.
+struct ChTiles {
+    const int *tiles, *cu_q;          // (request, first row, rows); the run's requests' first rows
+    int first;                        // the run's first request
+    // The chunk that begins with tile i: its first row, and how many it has (0: the tile is another chunk's second).
+    __device__ __forceinline__ int rows_of(int i, int& row0) const {
+        const int r = ld_step(tiles + 3 * i) - first;     // [descriptor]
+        row0 = ld_step(tiles + 3 * i + 1);
+        return (row0 - ld_step(cu_q + r)) / kChTile & 1 ? 0 : min(kChRows, ld_step(cu_q + r + 1) - row0);
+    }
+};
+
 struct ChRows {                       // rows of q, k or v of one head
     const __nv_bfloat16* p;           // row 0 of the step, the head's first element
     long long stride;
@@ -53,108 +62,288 @@ struct ChRows {                       // rows of q, k or v of one head
     int half;
 };
 
-// Rows [row0, row0 + rows) into shared memory as float32 times `factor(row)`, zeros up to 64 rows.  A thread
-// takes two quads of a row at a time, the two that turn together where the row turns; all its loads are
-// under way before the first value is used (one after the other they took longer than the products).
-template <int D, typename F>
-__device__ __forceinline__ void ch_load(float* dst, int pitch, const ChRows& m, int row0, int rows, F factor) {
-    constexpr int ACROSS = D / 8, APART = kChThreads / ACROSS, N = kChRows / APART;
-    const int r0 = threadIdx.x / ACROSS, p = threadIdx.x % ACROSS, turning = m.cs != nullptr ? m.half / 4 : 0;
-    const bool turn = p < turning;
-    const int c = turn ? 4 * p : 8 * turning + 8 * (p - turning), c2 = turn ? c + m.half : c + 4;
-    uint2 x[N], o[N];
-    float4 a[N], b[N];
+// Two quads of a row, activated, turned against each other where the row turns, times f.
+__device__ __forceinline__ void ch_values(const uint2& x, const uint2& o, bool turn, const float4& a, const float4& b, int silu,
+                                          float f, F4& u, F4& v) {
+    u = load4(reinterpret_cast<const __nv_bfloat16*>(&x));
+    v = load4(reinterpret_cast<const __nv_bfloat16*>(&o));
+    if (silu) {
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const int r = r0 + i * APART;
-        x[i] = o[i] = make_uint2(0, 0);
-        a[i] = b[i] = make_float4(1.f, 0.f, 1.f, 0.f);
-        if (r < rows) {
-            const __nv_bfloat16* row = m.p + static_cast<size_t>(row0 + r) * m.stride;
-            x[i] = __ldg(reinterpret_cast<const uint2*>(row + c));
-            o[i] = __ldg(reinterpret_cast<const uint2*>(row + c2));
-            if (turn) {
-                const float4* cs = reinterpret_cast<const float4*>(m.cs + static_cast<size_t>(row0 + r) * m.half + c);
-                a[i] = cs[0];
-                b[i] = cs[1];
-            }
+        for (int e = 0; e < 4; ++e) { u.v[e] = ch_silu(u.v[e]); v.v[e] = ch_silu(v.v[e]); }
+    }
+    if (turn) {
+        const float cs[4] = {a.x, a.z, b.x, b.z}, sn[4] = {a.y, a.w, b.y, b.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float lo = fmaf(u.v[e], cs[e], -(v.v[e] * sn[e]));
+            v.v[e] = fmaf(v.v[e], cs[e], u.v[e] * sn[e]);
+            u.v[e] = lo;
         }
     }
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const int r = r0 + i * APART;
-        F4 u = load4(reinterpret_cast<const __nv_bfloat16*>(&x[i])), v = load4(reinterpret_cast<const __nv_bfloat16*>(&o[i]));
-        if (m.silu) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) { u.v[e] = ch_silu(u.v[e]); v.v[e] = ch_silu(v.v[e]); }
-        }
-        if (turn) {
-            const float cs[4] = {a[i].x, a[i].z, b[i].x, b[i].z}, sn[4] = {a[i].y, a[i].w, b[i].y, b[i].w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float lo = fmaf(u.v[e], cs[e], -(v.v[e] * sn[e]));
-                v.v[e] = fmaf(v.v[e], cs[e], u.v[e] * sn[e]);
-                u.v[e] = lo;
-            }
-        }
-        const float f = r < rows ? factor(r) : 0.f;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { u.v[e] *= f; v.v[e] *= f; }
-        store4(dst + r * pitch + c, u);
-        store4(dst + r * pitch + c2, v);
-    }
+    for (int e = 0; e < 4; ++e) { u.v[e] *= f; v.v[e] *= f; }
+}
+// A row's channels in pairs of quads: pair p is the quads at c and c2, which turn against each other or are neighbours.
+__device__ __forceinline__ void ch_pair(const ChRows& m, int p, bool& turn, int& c, int& c2) {
+    const int turning = m.cs != nullptr ? m.half / 4 : 0;
+    turn = p < turning;
+    c = turn ? 4 * p : 8 * turning + 8 * (p - turning);
+    c2 = turn ? c + m.half : c + 4;
+}
+// The three parts of a quad (gemm_f32_split.cuh), as 8 bytes each.
+__device__ __forceinline__ void ch_split(const F4& u, uint2 (&part)[3]) {
+    fs_split(u.v[0], u.v[1], part[0].x, part[1].x, part[2].x);
+    fs_split(u.v[2], u.v[3], part[0].y, part[1].y, part[2].y);
 }
 
-// U [tile][head][value channel][key channel].  A CTA per (tile, head); a thread owns C x C elements.
-template <int D>
-__global__ void __launch_bounds__(kChThreads)
-chunk_update_kernel(ChRows k, ChRows v, const float* __restrict__ decay, const int* __restrict__ tiles, int heads,
+// What a thread reads of ROWS rows of one or two matrices (q and k turn by the same angles): pair `pl` of every APART-th row.
+// Fetched a phase before it is used, so that the loads run under the MMAs of the phase before.
+template <int ROWS, int PAIRS, int MATS>
+struct ChFetch {
+    static constexpr int APART = kChThreads / PAIRS, N = ROWS / APART;
+    static_assert(ROWS % APART == 0, "whole passes");
+    uint2 x[MATS][N], o[MATS][N];
+    float4 a[N], b[N];
+    int c, c2;
+    bool turn;
+    __device__ __forceinline__ void fetch(const ChRows* const (&m)[MATS], int row0, int at, int rows, int p0) {
+        ch_pair(*m[0], p0 + static_cast<int>(threadIdx.x) % PAIRS, turn, c, c2);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int r = at + threadIdx.x / PAIRS + i * APART;
+            a[i] = b[i] = make_float4(1.f, 0.f, 1.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < MATS; ++k) x[k][i] = o[k][i] = make_uint2(0, 0);
+            if (r < rows) {
+#pragma unroll
+                for (int k = 0; k < MATS; ++k) {
+                    const __nv_bfloat16* row = m[k]->p + static_cast<size_t>(row0 + r) * m[k]->stride;
+                    x[k][i] = __ldg(reinterpret_cast<const uint2*>(row + c));
+                    o[k][i] = __ldg(reinterpret_cast<const uint2*>(row + c2));
+                }
+                if (turn) {
+                    const float4* cs = reinterpret_cast<const float4*>(m[0]->cs + static_cast<size_t>(row0 + r) * m[0]->half + c);
+                    a[i] = cs[0];
+                    b[i] = cs[1];
+                }
+            }
+        }
+    }
+    // The parts of matrix K times factor(row).  FLAT: tiles of [ROWS][8 pairs], a pair's eight numbers together: 64 channels in
+    // an order that q, k and the state share, for products over channels.  Else tiles of [ROWS][64 channels] in the rows'
+    // order, a block of 64 channels behind the other.
+    template <int K, bool FLAT, typename F>
+    __device__ __forceinline__ void put(unsigned char* dst, int plane, int silu, int at, F factor) const {
+        static_assert(!FLAT || PAIRS == 8, "64 channels");
+        const int pl = threadIdx.x % PAIRS;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int rl = threadIdx.x / PAIRS + i * APART;
+            F4 u, v;
+            ch_values(x[K][i], o[K][i], turn, a[i], b[i], silu, factor(at + rl), u, v);
+            uint2 pu[3], pv[3];
+            ch_split(u, pu);
+            ch_split(v, pv);
+            auto place = [&](int channel) {
+                return dst + channel / 64 * (ROWS * 128) + rl * 128 + (((channel & 63) >> 3 ^ (rl & 7)) << 4) + (channel & 4) * 2;
+            };
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                if (FLAT) {
+                    *reinterpret_cast<uint4*>(dst + e * plane + rl * 128 + ((pl ^ (rl & 7)) << 4)) =
+                        make_uint4(pu[e].x, pu[e].y, pv[e].x, pv[e].y);
+                } else {
+                    *reinterpret_cast<uint2*>(place(c) + e * plane) = pu[e];
+                    *reinterpret_cast<uint2*>(place(c2) + e * plane) = pv[e];
+                }
+            }
+        }
+    }
+};
+// 64 rows of v from row `at` on, to tiles of [64][64 channels]: as they are, or (SILU) three parts.  A number that is
+// not finite is left out (an MMA would carry it to rows that do not see it) and its row noted in `odd`, if that is given.
+template <int D, bool SILU>
+struct ChFetchV {
+    static constexpr int ACROSS = D / 4, APART = kChThreads / ACROSS, N = 64 / APART;
+    uint2 x[N];
+    __device__ __forceinline__ void fetch(const ChRows& m, int row0, int at, int rows) {
+        const int c = threadIdx.x % ACROSS * 4;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int r = at + threadIdx.x / ACROSS + i * APART;
+            x[i] = r < rows ? __ldg(reinterpret_cast<const uint2*>(m.p + static_cast<size_t>(row0 + r) * m.stride + c)) : make_uint2(0, 0);
+        }
+    }
+    __device__ __forceinline__ void put(unsigned char* dst, int plane, int at, uint32_t* odd) const {
+        const int c = threadIdx.x % ACROSS * 4;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int rl = threadIdx.x / ACROSS + i * APART;
+            F4 u = load4(reinterpret_cast<const __nv_bfloat16*>(&x[i]));
+            bool fine = true;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (SILU) u.v[e] = ch_silu(u.v[e]);
+                fine &= fs_finite(u.v[e]);
+            }
+            if (!fine && odd != nullptr) {
+                atomicOr(odd + ((at + rl) >> 5), 1u << ((at + rl) & 31));
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (!fs_finite(u.v[e])) u.v[e] = 0.f;
+            }
+            uint2 part[3];
+            ch_split(u, part);
+            unsigned char* to = dst + c / 64 * (64 * 128) + rl * 128 + (((c & 63) >> 3 ^ (rl & 7)) << 4) + (c & 4) * 2;
+#pragma unroll
+            for (int e = 0; e < (SILU ? 3 : 1); ++e) *reinterpret_cast<uint2*>(to + e * plane) = part[e];
+        }
+    }
+};
+
+// Products of parts, the small ones first, in groups of K steps: `f(a's part, b's part, step, accumulate)`.  PB: 3, or 1 where b is bfloat16.
+template <int PB, typename F>
+__device__ __forceinline__ void ch_products(int steps, bool fresh, F f) {
+    for (int j = 0; j < steps; ++j) {
+        f(2, 0, j, !(fresh && j == 0));
+        if (PB == 3) {
+            f(0, 2, j, true);
+            f(1, 1, j, true);
+        }
+        f(1, 0, j, true);
+        if (PB == 3) f(0, 1, j, true);
+    }
+    for (int j = 0; j < steps; ++j) f(0, 0, j, true);
+}
+__host__ __device__ constexpr uint32_t ch_idesc(int n, bool a_mn, bool b_mn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u) |
+           (static_cast<uint32_t>(n >> 3) << 17) | (8u << 24);
+}
+
+// What both MMA kernels set up: one barrier, 256 columns of tensor memory.
+struct ChMma {
+    uint32_t bar, tmem, phase;
+    bool ok;
+    __device__ __forceinline__ void start(unsigned long long* bar_s, uint32_t* tmem_s) {
+        bar = smem_u32(bar_s);
+        phase = 0;
+        ok = true;
+        if (threadIdx.x == 0) {
+            mbar_init(bar, 1);
+            mbar_fence_init();
+        }
+        if (threadIdx.x < 32) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_s)), "r"(256) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+        }
+        t5::fence_before();
+        __syncthreads();
+        t5::fence_after();
+        tmem = *tmem_s;
+    }
+    // shared memory that all threads have written is the MMAs' operand from here on
+    __device__ __forceinline__ void operands_ready() {
+        fence_proxy_async();
+        t5::fence_before();
+        __syncthreads();
+        t5::fence_after();
+    }
+    __device__ __forceinline__ void wait() {              // for what thread 0 has committed
+        if (ok && !mbar_wait(bar, phase, 2000000)) {
+            ok = false;
+            atomicExch(&g_chunks_error, 1);
+        }
+        phase ^= 1;
+        __syncwarp();
+        t5::fence_after();
+    }
+    __device__ __forceinline__ void end() {
+        t5::fence_before();
+        __syncthreads();
+        if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(256) : "memory");
+    }
+};
+
+// U [tile][head][value channel][key channel].  A CTA per (tile, head), two on an SM: 64 rows at a time, k in parts and v; D = V^T K with
+// the rows as the products' K, both operands as the rows lie; the halves' sums in two accumulators.
+template <int D, bool SILU>
+__global__ void __launch_bounds__(kChThreads, 2)
+chunk_update_kernel(ChRows k, ChRows v, const float* __restrict__ decay, ChTiles tiles, int heads,
                     int group, float* __restrict__ u) {
-    constexpr int C = D / 16;
-    extern __shared__ __align__(16) float ch_smem[];
-    float* ks = ch_smem;                                  // [64][D]
-    float* vs = ks + kChRows * D;                         // [64][D]
-    pdl_launch_dependents();
-    pdl_wait();
-    const int* tile = tiles + 3 * blockIdx.x;
-    const int row0 = tile[1], rows = tile[2], h = blockIdx.y;
+    constexpr int PLANE = 64 * D * 2, PV = SILU ? 3 : 1;
+    extern __shared__ unsigned char ch_raw[];
+    unsigned char* vs = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ch_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* ks = vs + PV * PLANE;                  // (with 64 channels an MMA reads 64 more of v: into k, and not used)
     __shared__ float pow_s[kChRows];
+    __shared__ __align__(8) unsigned long long bar_s;
+    __shared__ uint32_t tmem_s;
+    pdl_launch_dependents();
+    int row0;
+    const int rows = tiles.rows_of(blockIdx.x, row0), h = blockIdx.y;
+    if (rows == 0) {
+        pdl_wait();
+        return;
+    }
+    ChMma mma;
+    mma.start(&bar_s, &tmem_s);
+    pdl_wait();
     if (threadIdx.x < kChRows) pow_s[threadIdx.x] = powf(decay[h], static_cast<float>(threadIdx.x));
     __syncthreads();
     k.p += static_cast<size_t>(h / group) * D;
     v.p += static_cast<size_t>(h) * D;
-    ch_load<D>(ks, D, k, row0, rows, [&](int r) { return pow_s[rows - 1 - r]; });
-    ch_load<D>(vs, D, v, row0, rows, [](int) { return 1.f; });
-    __syncthreads();
-    // key channels 4 ti .. (and 64 further on), value channels 4 tj .. likewise; a warp 4 x 8 of them
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ti = warp / 2 * 4 + lane / 8, tj = warp % 2 * 8 + lane % 8;
-    float acc[C][C];                                      // [value channel][key channel]
-#pragma unroll
-    for (int j = 0; j < C; ++j)
-#pragma unroll
-        for (int i = 0; i < C; ++i) acc[j][i] = 0.f;
-#pragma unroll 4
-    for (int s = 0; s < kChRows; ++s) {
-        float a[C], b[C];
-#pragma unroll
-        for (int e = 0; e < C; e += 4) {
-            const F4 x = load4(ks + s * D + 4 * ti + 16 * e), y = load4(vs + s * D + 4 * tj + 16 * e);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { a[e + i] = x.v[i]; b[e + i] = y.v[i]; }
+    const int halves = rows > 64 ? 2 : 1;
+    ChFetch<64, D / 8, 1> fk;
+    ChFetchV<D, SILU> fv;
+    fk.fetch({&k}, row0, 0, rows, 0);
+    fv.fetch(v, row0, 0, rows);
+    for (int i = 0; i < halves; ++i) {
+        if (i > 0) mma.wait();                            // the first half's operands have been read
+        fv.put(vs, PLANE, 64 * i, nullptr);
+        fk.template put<0, false>(ks, PLANE, k.silu, 64 * i, [&](int r) { return pow_s[max(rows - 1 - r, 0)]; });
+        if (i + 1 < halves) {
+            fk.fetch({&k}, row0, 64, rows, 0);
+            fv.fetch(v, row0, 64, rows);
         }
-#pragma unroll
-        for (int j = 0; j < C; ++j)
-#pragma unroll
-            for (int i = 0; i < C; ++i) acc[j][i] = fmaf(a[i], b[j], acc[j][i]);
+        mma.operands_ready();
+        if (threadIdx.x == 0) {
+            const uint64_t kd = t5::desc_mnmajor(smem_u32(ks), 64 * 128), vd = t5::desc_mnmajor(smem_u32(vs), 64 * 128);
+            ch_products<PV>(4, true, [&](int pk, int pv, int j, bool more) {
+                t5::mma_ss(mma.tmem + i * D, vd + ((pv * PLANE + j * 16 * 128) >> 4), kd + ((pk * PLANE + j * 16 * 128) >> 4),
+                           ch_idesc(D, true, true), more);
+            });
+            t5::commit(mma.bar);
+        }
     }
-    float* dst = u + (static_cast<size_t>(blockIdx.x) * heads + h) * D * D;
+    mma.wait();
+    // row 32 (warp % 4) + lane, one half of its columns, through shared memory to whole rows
+    constexpr int COLS = D / 2, PITCH = COLS + 4;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if ((warp & 3) * 32 < D) {
+        float* own = reinterpret_cast<float*>(vs) + warp * 32 * PITCH;
+        const uint32_t at = mma.tmem + (static_cast<uint32_t>(warp & 3) << 21) + (warp >> 2) * COLS;
 #pragma unroll
-    for (int j = 0; j < C; ++j)
+        for (int c = 0; c < COLS; c += 32) {
+            float x[32];
+            t5::ld32(at + c, x);
+            if (halves > 1) {
+                float z[32];
+                t5::ld32(at + D + c, z);
 #pragma unroll
-        for (int i = 0; i < C; i += 4)
-            store4(dst + (4 * tj + j % 4 + 64 * (j / 4)) * D + 4 * ti + 16 * i,
-                   F4{{acc[j][i], acc[j][i + 1], acc[j][i + 2], acc[j][i + 3]}});
+                for (int e = 0; e < 32; ++e) x[e] += z[e];
+            }
+#pragma unroll
+            for (int e = 0; e < 32; e += 4)
+                *reinterpret_cast<float4*>(own + lane * PITCH + c + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
+        }
+        __syncwarp();
+        float* dst = u + (static_cast<size_t>(blockIdx.x) * heads + h) * D * D + (warp & 3) * 32 * D + (warp >> 2) * COLS;
+#pragma unroll 4
+        for (int i = lane; i < 32 * (COLS / 4); i += 32) {
+            const int r = i / (COLS / 4), c = i % (COLS / 4) * 4;
+            *reinterpret_cast<float4*>(dst + r * D + c) = *reinterpret_cast<const float4*>(own + r * PITCH + c);
+        }
+    }
+    mma.end();
 }
 
 // U of a request's chunks -> the states in front of them, in place; the state behind the last to its slot.
@@ -167,14 +356,14 @@ chunk_states_kernel(float* __restrict__ u, const float* __restrict__ decay, cons
     pdl_wait();
     const int h = blockIdx.y, r = blockIdx.z;
     int tile = 0;                                         // the request's first
-    for (int i = 0; i < r; ++i) tile += (cu_q[i + 1] - cu_q[i] + kChRows - 1) / kChRows;
+    for (int i = 0; i < r; ++i) tile += (cu_q[i + 1] - cu_q[i] + kChTile - 1) / kChTile;
     const int rows = cu_q[r + 1] - cu_q[r], n = (rows + kChRows - 1) / kChRows;
     const float g = decay[h], full = powf(g, static_cast<float>(kChRows));
     const float tail = powf(g, static_cast<float>(rows - (n - 1) * kChRows));
     const int at = (blockIdx.x * kChThreads + threadIdx.x) * 4;
     float* own = state + (static_cast<size_t>(state_slot[r]) * heads + h) * D * D + at;
     float* p = u + (static_cast<size_t>(tile) * heads + h) * D * D + at;
-    const size_t step = static_cast<size_t>(heads) * D * D;
+    const size_t step = static_cast<size_t>(kChRows / kChTile) * heads * D * D;
     F4 s = load4(own);
     constexpr int AHEAD = 8;                              // loads in flight
     for (int c0 = 0; c0 < n; c0 += AHEAD) {
@@ -194,162 +383,198 @@ chunk_states_kernel(float* __restrict__ u, const float* __restrict__ decay, cons
     store4(own, s);
 }
 
-// y of a chunk.  A CTA per (tile, head): rows tr + 16 i; the products q . k_s for keys tc + 16 j; outputs
-// of value channels tc + 16 j (from the state) and then, with P in shared memory, the same.
-template <int D>
+// One channel of a row, activated and turned (the way of numbers that are not finite).
+__device__ float ch_value(const ChRows& m, int row, int c) {
+    const __nv_bfloat16* p = m.p + static_cast<size_t>(row) * m.stride;
+    float x = __bfloat162float(p[c]);
+    if (m.silu) x = ch_silu(x);
+    if (m.cs == nullptr || c >= 2 * m.half) return x;
+    const bool low = c < m.half;
+    const float other = __bfloat162float(p[low ? c + m.half : c - m.half]);
+    const float2 t = m.cs[static_cast<size_t>(row) * m.half + (low ? c : c - m.half)];
+    return low ? fmaf(x, t.x, -(other * t.y)) : fmaf(x, t.x, other * t.y);
+}
+
+// y of a chunk.  A CTA per (tile, head), two on an SM.  For 64 channels at a time q and k in parts, then the state over k: scores
+// q k^T and q S in two accumulators.  Then a thread takes half a row of scores, masks and decays them and writes
+// them as parts for their product with v, 64 keys at a time, into the scores' accumulator.
+template <int D, bool SILU>
 __global__ void __launch_bounds__(kChThreads, 2)
 chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* __restrict__ decay,
-                     const int* __restrict__ tiles, const float* __restrict__ states, int heads, int group,
+                     ChTiles tiles, const float* __restrict__ states, int heads, int group,
                      float* __restrict__ y) {
-    constexpr int C = D / 16, P = D + 4, PP = kChRows + 4, SP = kChBK + 4, STAGES = 2;
-    extern __shared__ __align__(16) float ch_smem[];
-    float* qs = ch_smem;                                  // [64][P]
-    float* ps = qs + kChRows * P;                         // [64][PP]
-    float* xs = ps + kChRows * PP;                        // k [64][P], then stages of the state [D][SP], then v [64][D]
+    constexpr int PLANE = kChRows * 128, VPLANE = 64 * D * 2, PV = SILU ? 3 : 1;
+    extern __shared__ unsigned char ch_raw[];
+    unsigned char* xs = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ch_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* ys = xs + 3 * PLANE;
     __shared__ float pow_s[kChRows + 1];
+    __shared__ uint32_t odd_s[kChRows / 32];
+    __shared__ __align__(8) unsigned long long bar_s;
+    __shared__ uint32_t tmem_s;
     pdl_launch_dependents();
+    int row0;
+    const int rows = tiles.rows_of(blockIdx.x, row0), h = blockIdx.y;
+    if (rows == 0) {
+        pdl_wait();
+        return;
+    }
+    ChMma mma;
+    if (threadIdx.x < kChRows / 32) odd_s[threadIdx.x] = 0;
+    mma.start(&bar_s, &tmem_s);
     pdl_wait();
-    const int* tile = tiles + 3 * blockIdx.x;
-    const int row0 = tile[1], rows = tile[2], h = blockIdx.y;
     q.p += static_cast<size_t>(h / group) * D;
     k.p += static_cast<size_t>(h / group) * D;
     v.p += static_cast<size_t>(h) * D;
     if (threadIdx.x <= kChRows) pow_s[threadIdx.x] = powf(decay[h], static_cast<float>(threadIdx.x));
-    ch_load<D>(qs, P, q, row0, rows, [&](int) { return q_scale; });
-    ch_load<D>(xs, P, k, row0, rows, [](int) { return 1.f; });
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int tr = warp / 2 * 4 + lane / 8, tc = warp % 2 * 8 + lane % 8;
-    {
-        unsigned long long acc[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-#pragma unroll 4
-        for (int d = 0; d < D; d += 4) {
-            ulonglong2 b[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(xs + (tc + 16 * j) * P + d);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(qs + (tr + 16 * i) * P + d);
-#pragma unroll
-                for (int j = 0; j <= i; ++j) ch_fma2(acc[i][j], a.x, b[j].x);
-#pragma unroll
-                for (int j = 0; j <= i; ++j) ch_fma2(acc[i][j], a.y, b[j].y);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j <= i; ++j) {
-                const int t = tr + 16 * i, s = tc + 16 * j;
-                ps[t * PP + s] = s <= t ? ch_sum2(acc[i][j]) * pow_s[t - s] : 0.f;
-            }
-    }
-    __syncthreads();                                      // k has been read
     const float* st = states + (static_cast<size_t>(blockIdx.x) * heads + h) * D * D;
-    auto stage = [&](int c) {                             // key channels 32 c .. of all value channels
-        float* dst = xs + c % STAGES * (D * SP);
-        for (int i = threadIdx.x; i < D * (kChBK / 4); i += kChThreads) {
-            const int j = i / (kChBK / 4), e = i % (kChBK / 4) * 4;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
-                             static_cast<uint32_t>(__cvta_generic_to_shared(dst + j * SP + e))),
-                         "l"(st + j * D + c * kChBK + e)
-                         : "memory");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, halves = rows > 64 ? 2 : 1;
+    const uint32_t scores = mma.tmem, carried = mma.tmem + 128;
+    const uint64_t xd = t5::desc_kmajor(smem_u32(xs)), yd = t5::desc_kmajor(smem_u32(ys));
+    ChFetch<kChRows, 8, 2> f;
+    f.fetch({&q, &k}, row0, 0, rows, 0);
+    for (int i = 0; i < D / 64; ++i) {
+        if (i > 0) mma.wait();
+        f.template put<0, true>(xs, PLANE, q.silu, 0, [&](int) { return q_scale; });
+        f.template put<1, true>(ys, PLANE, k.silu, 0, [](int) { return 1.f; });
+        mma.operands_ready();
+        if (threadIdx.x == 0) {
+            ch_products<3>(4, i == 0, [&](int pa, int pb, int j, bool more) {
+                t5::mma_ss(scores, xd + ((pa * PLANE + j * 32) >> 4), yd + ((pb * PLANE + j * 32) >> 4), ch_idesc(kChRows, false, false), more);
+            });
+            t5::commit(mma.bar);
         }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-    // even and odd terms of every output's product with the state
-    unsigned long long acc[4][C];
+        // the state's 64 key channels, in the same order
+        constexpr int N = D / (kChThreads / 8);
+        const int r0 = threadIdx.x / 8, pl = threadIdx.x % 8;
+        bool turn;
+        int c, c2;
+        ch_pair(q, 8 * i + pl, turn, c, c2);
+        F4 a[N], b[N];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < C; ++j) acc[i][j] = 0ull;
-    stage(0);
-    for (int c = 0; c < D / kChBK; ++c) {
-        if (c + 1 < D / kChBK) {
-            stage(c + 1);
-            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        for (int n = 0; n < N; ++n) {
+            const float* p = st + (r0 + n * (kChThreads / 8)) * D;
+            a[n] = load4(p + c);
+            b[n] = load4(p + c2);
         }
-        __syncthreads();
-        const float* ss = xs + c % STAGES * (D * SP);
-#pragma unroll 2
-        for (int d = 0; d < kChBK; d += 4) {
-            ulonglong2 a[4];
+        mma.wait();
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                a[i] = *reinterpret_cast<const ulonglong2*>(qs + (tr + 16 * i) * P + c * kChBK + d);
+        for (int n = 0; n < N; ++n) {
+            const int r = r0 + n * (kChThreads / 8);
+            uint2 pa[3], pb[3];
+            ch_split(a[n], pa);
+            ch_split(b[n], pb);
 #pragma unroll
-            for (int j = 0; j < C; ++j) {
-                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(ss + (tc + 16 * j) * SP + d);
+            for (int e = 0; e < 3; ++e)
+                *reinterpret_cast<uint4*>(ys + e * PLANE + r * 128 + ((pl ^ (r & 7)) << 4)) = make_uint4(pa[e].x, pa[e].y, pb[e].x, pb[e].y);
+        }
+        if (i + 1 < D / 64) f.fetch({&q, &k}, row0, 0, rows, 8 * (i + 1));
+        mma.operands_ready();
+        if (threadIdx.x == 0) {
+            ch_products<3>(4, i == 0, [&](int pa, int pb, int j, bool more) {
+                t5::mma_ss(carried, xd + ((pa * PLANE + j * 32) >> 4), yd + ((pb * PLANE + j * 32) >> 4), ch_idesc(D, false, false), more);
+            });
+            t5::commit(mma.bar);
+        }
+    }
+    ChFetchV<D, SILU> fv;
+    fv.fetch(v, row0, 0, rows);
+    // a row's scores of keys 64 (warp / 4) .., while the last MMAs run
+    const int t = (warp & 3) * 32 + lane, s0 = (warp >> 2) * 64;
+    const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;
+    float p[64];
+    t5::ld32(scores + lanes + s0, p);
+    t5::ld32(scores + lanes + s0 + 32, p + 32);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) ch_fma2(acc[i][j], a[i].x, b.x);
+    for (int s = 0; s < 64; ++s) p[s] = s0 + s <= t ? p[s] * pow_s[max(t - s0 - s, 0)] : 0.f;
+    mma.wait();                                           // q and the state have been read
+    for (int i = 0; i < halves; ++i) {
+        if (i > 0) mma.wait();
+        if (warp >> 2 == i) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) ch_fma2(acc[i][j], a[i].y, b.y);
+            for (int c = 0; c < 64; c += 8) {
+                uint4 part[3];
+                fs_split(p[c], p[c + 1], part[0].x, part[1].x, part[2].x);
+                fs_split(p[c + 2], p[c + 3], part[0].y, part[1].y, part[2].y);
+                fs_split(p[c + 4], p[c + 5], part[0].z, part[1].z, part[2].z);
+                fs_split(p[c + 6], p[c + 7], part[0].w, part[1].w, part[2].w);
+#pragma unroll
+                for (int e = 0; e < 3; ++e)
+                    *reinterpret_cast<uint4*>(xs + e * PLANE + t * 128 + ((c / 8 ^ (t & 7)) << 4)) = part[e];
             }
         }
-        __syncthreads();                                  // the stage has been read
-    }
-    float o[4][C];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < C; ++j) o[i][j] = ch_sum2(acc[i][j]) * pow_s[tr + 16 * i + 1];
-    ch_load<D>(xs, D, v, row0, rows, [](int) { return 1.f; });
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {                         // 16 keys that the rows of blocks b .. 3 see
-#pragma unroll 2
-        for (int s = 16 * b; s < 16 * b + 16; s += 4) {
-            F4 p[4];
-#pragma unroll
-            for (int i = b; i < 4; ++i) p[i] = load4(ps + (tr + 16 * i) * PP + s);
-#pragma unroll
-            for (int m = 0; m < 4; ++m)
-#pragma unroll
-                for (int j = 0; j < C; ++j) {
-                    const float x = xs[(s + m) * D + tc + 16 * j];
-                    // (on the diagonal a later row's infinity must not meet a probability of zero)
-                    if (s + m <= tr + 16 * b) o[b][j] = fmaf(p[b].v[m], x, o[b][j]);
-#pragma unroll
-                    for (int i = b + 1; i < 4; ++i) o[i][j] = fmaf(p[i].v[m], x, o[i][j]);
-                }
+        fv.put(ys, VPLANE, 64 * i, odd_s);
+        if (i + 1 < halves) fv.fetch(v, row0, 64, rows);
+        mma.operands_ready();
+        if (threadIdx.x == 0) {
+            const uint64_t vd = t5::desc_mnmajor(smem_u32(ys), 64 * 128);
+            ch_products<PV>(4, i == 0, [&](int pa, int pb, int j, bool more) {
+                t5::mma_ss(scores, xd + ((pa * PLANE + j * 32) >> 4), vd + ((pb * VPLANE + j * 16 * 128) >> 4), ch_idesc(D, false, true), more);
+            });
+            t5::commit(mma.bar);
         }
     }
+    mma.wait();
+    // y = g^(t + 1) q S + P v: half of a row's columns a thread, through shared memory to whole rows
+    constexpr int COLS = D / 2, PITCH = COLS + 4;
+    const int col0 = (warp >> 2) * COLS;
+    float* own = reinterpret_cast<float*>(xs) + warp * 32 * PITCH;
+    const uint32_t odd = odd_s[0] | odd_s[1] | odd_s[2] | odd_s[3];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = tr + 16 * i;
-        if (t >= rows) continue;
-        float* dst = y + static_cast<size_t>(row0 + t) * heads * D + static_cast<size_t>(h) * D + tc;
+    for (int c = 0; c < COLS; c += 32) {
+        float o[32], z[32];
+        t5::ld32(scores + lanes + col0 + c, o);
+        t5::ld32(carried + lanes + col0 + c, z);
 #pragma unroll
-        for (int j = 0; j < C; ++j) dst[16 * j] = o[i][j];
+        for (int e = 0; e < 32; ++e) o[e] = fmaf(z[e], pow_s[t + 1], o[e]);
+#pragma unroll
+        for (int e = 0; e < 32; e += 4)
+            *reinterpret_cast<float4*>(own + lane * PITCH + c + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
     }
+    if (odd != 0 && t < rows) {                           // values that are not finite: to the rows that see them
+#pragma unroll 1
+        for (int s = 0; s <= t; ++s) {
+            if (!(odd_s[s >> 5] >> (s & 31) & 1)) continue;
+            float dot = 0.f;
+            for (int c = 0; c < D; ++c) dot = fmaf(ch_value(q, row0 + t, c) * q_scale, ch_value(k, row0 + s, c), dot);
+            dot *= pow_s[t - s];
+            for (int c = 0; c < COLS; ++c) {
+                const float x = ch_value(v, row0 + s, col0 + c);
+                if (!fs_finite(x)) own[lane * PITCH + c] = fmaf(dot, x, own[lane * PITCH + c]);
+            }
+        }
+    }
+    __syncwarp();
+    float* dst = y + static_cast<size_t>(row0 + (warp & 3) * 32) * heads * D + static_cast<size_t>(h) * D + col0;
+    const int live = rows - (warp & 3) * 32;
+#pragma unroll 4
+    for (int i = lane; i < 32 * (COLS / 4); i += 32) {
+        const int r = i / (COLS / 4), c = i % (COLS / 4) * 4;
+        if (r < live)
+            *reinterpret_cast<float4*>(dst + static_cast<size_t>(r) * heads * D + c) = *reinterpret_cast<const float4*>(own + r * PITCH + c);
+    }
+    mma.end();
 }
 
-template <int D>
-constexpr int ch_update_smem() { return 4 * 2 * kChRows * D; }
-template <int D>
-constexpr int ch_outputs_smem() {
-    constexpr int k = kChRows * (D + 4), s = 2 * D * (kChBK + 4);
-    return 4 * (kChRows * (D + 4) + kChRows * (kChRows + 4) + (k > s ? k : s));
+template <int D, bool SILU>
+constexpr int ch_update_smem() {
+    constexpr int parts = ((SILU ? 3 : 1) + 3) * 64 * D * 2, out = 8 * 32 * (D / 2 + 4) * 4;
+    return (parts > out ? parts : out) + 1024;
 }
+constexpr int kChOutputsSmem = 6 * kChRows * 128 + 1024;
 
-template <int D>
+template <int D, bool SILU>
 int launch_chunks(const ChRows& q, const ChRows& k, const ChRows& v, float q_scale, const float* decay, float* state,
-                  const int* cu_q, const int* state_slot, const int* tiles, int n_tiles, int n_req, int heads,
+                  const int* cu_q, const int* state_slot, const int* tile_list, int n_tiles, int n_req, int first, int heads,
                   int group, float* u, float* y, cudaStream_t stream) {
-    cudaFuncSetAttribute(chunk_update_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, ch_update_smem<D>());
-    cudaFuncSetAttribute(chunk_outputs_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, ch_outputs_smem<D>());
+    const ChTiles tiles{tile_list, cu_q, first};
+    cudaFuncSetAttribute(chunk_update_kernel<D, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, ch_update_smem<D, SILU>());
+    cudaFuncSetAttribute(chunk_outputs_kernel<D, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, kChOutputsSmem);
     const dim3 grid(n_tiles, heads);
-    launch_pdl(chunk_update_kernel<D>, grid, dim3(kChThreads), ch_update_smem<D>(), stream, k, v, decay, tiles, heads,
+    launch_pdl(chunk_update_kernel<D, SILU>, grid, dim3(kChThreads), ch_update_smem<D, SILU>(), stream, k, v, decay, tiles, heads,
                group, u);
     launch_pdl(chunk_states_kernel<D>, dim3(D * D / 4 / kChThreads, heads, n_req), dim3(kChThreads), 0, stream, u, decay,
                cu_q, state_slot, state, heads);
-    launch_pdl(chunk_outputs_kernel<D>, grid, dim3(kChThreads), ch_outputs_smem<D>(), stream, q, k, v, q_scale, decay,
+    launch_pdl(chunk_outputs_kernel<D, SILU>, grid, dim3(kChThreads), kChOutputsSmem, stream, q, k, v, q_scale, decay,
                tiles, u, heads, group, y);
     return launch_status();
 }
@@ -361,14 +586,14 @@ using namespace somi;
 // q, k: bfloat16 rows of heads / group heads of D elements, `stride` apart; v: of `heads` heads; D = 64 or 128.
 // `silu`: q and k (bit 0) and v (bit 1) pass SiLU.  rot > 0: the pairs (i, i + rot / 2) of q and k turn by
 // positions * rot_freq; angles: float32 scratch [portions' rows, rot].  `tiles`: int32 [n_tiles, 3] = (request,
-// first row, rows <= 64) over the n_req multi-token requests, in order.  u: float32 scratch [n_tiles, heads, D, D].
+// first row, rows <= 64) over the n_req multi-token requests, in order, request numbers from `first` on.  u: float32 scratch [n_tiles, heads, D, D].
 // state: float32 [slots, heads, D, D] (value channel, key channel); y: float32 rows of heads * D.
 SOMI_API int somi_matrix_state_chunks(const void* q, const void* k, const void* v, long long q_stride,
                                       long long k_stride, long long v_stride, int silu, float q_scale,
                                       const float* decay, float* state, const int* cu_q, const int* state_slot,
                                       const int* tiles, int n_tiles, int n_req, int n_rows, int heads, int group, int D,
                                       const int* positions, const double* rot_freq, int rot, float* angles, float* u,
-                                      float* y, cudaStream_t stream) {
+                                      float* y, int first, cudaStream_t stream) {
     if (n_tiles <= 0 || n_req <= 0) return 0;
     const uintptr_t bits = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v);
     if (decay == nullptr || (rot > 0 && (positions == nullptr || rot_freq == nullptr || angles == nullptr)))
@@ -383,8 +608,16 @@ SOMI_API int somi_matrix_state_chunks(const void* q, const void* k, const void* 
     const ChRows qr{static_cast<const __nv_bfloat16*>(q), q_stride, silu & 1, cs, half};
     const ChRows kr{static_cast<const __nv_bfloat16*>(k), k_stride, silu & 1, cs, half};
     const ChRows vr{static_cast<const __nv_bfloat16*>(v), v_stride, silu >> 1 & 1, nullptr, 0};
-    return D == 64 ? launch_chunks<64>(qr, kr, vr, q_scale, decay, state, cu_q, state_slot, tiles, n_tiles, n_req, heads,
-                                       group, u, y, stream)
-                   : launch_chunks<128>(qr, kr, vr, q_scale, decay, state, cu_q, state_slot, tiles, n_tiles, n_req, heads,
-                                        group, u, y, stream);
+#define SOMI_CHUNKS(D_, SILU_) \
+    launch_chunks<D_, SILU_>(qr, kr, vr, q_scale, decay, state, cu_q, state_slot, tiles, n_tiles, n_req, first, heads, group, u, y, stream)
+    if (D == 64) return silu & 2 ? SOMI_CHUNKS(64, true) : SOMI_CHUNKS(64, false);
+    return silu & 2 ? SOMI_CHUNKS(128, true) : SOMI_CHUNKS(128, false);
+#undef SOMI_CHUNKS
+}
+
+SOMI_API int somi_chunks_error() {
+    int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_chunks_error, sizeof(int)) != cudaSuccess) return -1;
+    if (v) cudaMemcpyToSymbol(g_chunks_error, &zero, sizeof(int));
+    return v;
 }

@@ -333,6 +333,9 @@ class CudaOps:
         if int(self.lib.somi_gemm_f32_error()) != 0:
             raise KernelError("the float32 tcgen05 matrix product gave up waiting on a barrier; "
                               "its results are not valid")
+        if int(self.lib.somi_chunks_error()) != 0:
+            raise KernelError("the recurrence in chunks gave up waiting on a barrier; "
+                              "its results are not valid")
 
     @staticmethod
     def _attention_work(batch, first: int, last: int, nq: int, nkv: int, hd: int, elt: int,
@@ -1774,7 +1777,7 @@ class CudaOps:
             _ptr(state), _ptr(batch.cu_q, first), _ptr(batch.state_slot, first), tiles, ctypes.c_int(n_tiles),
             ctypes.c_int(end - first), ctypes.c_int(rows), ctypes.c_int(heads), ctypes.c_int(heads // qk_heads),
             ctypes.c_int(dk), _ptr(pos), _ptr(freq), ctypes.c_int(rot), _ptr(u, n_u), _ptr(u), _ptr(y),
-            self._stream())
+            ctypes.c_int(first), self._stream())
         self._done(rc, "matrix_state_chunks")
         self.launches += 3 if rot else 2
         if trace.active():
