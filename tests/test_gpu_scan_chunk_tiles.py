@@ -1,4 +1,4 @@
-"""The recurrence in chunks of 128 rows at the bounds of its tiles of 64 rows and of its chunks."""
+"""The recurrence in chunks of 128 rows at the bounds of its tiles of 64 rows and of its chunks, and the norm of parts behind it."""
 
 import pytest
 import torch
@@ -54,3 +54,27 @@ def test_what_is_not_finite_reaches_the_rows_that_see_it(ops, d, silu, what):
             assert not z[at:, :d].isfinite().any() and torch.equal(u[0, :, :, 6:], s[0, :, :, 6:])
         else:
             assert not z[at, :d].isfinite().any() and torch.equal(z[at + 1:], y[at + 1:]) and torch.equal(u, s)
+
+
+@pytest.mark.parametrize("T", [1, 3, 41, 400])
+@pytest.mark.parametrize("groups,n", [(14, 64), (28, 128), (5, 32), (3, 48), (2, 256)])
+def test_norm_of_parts(ops, T, groups, n):
+    """Few and many parts, those that go four columns at a time and those that do not, gates in either type and with rows
+    further apart: a sum of n squares in float32, then the output type's rounding."""
+    C = groups * n
+    g = torch.Generator(device="cuda").manual_seed(T + C)
+    y = torch.randn(T, C, generator=g, device="cuda")
+    for gate_type, out_type, apart, w_len in ((torch.bfloat16, torch.bfloat16, 8, n), (torch.float32, torch.float32, 4, C),
+                                              (torch.bfloat16, torch.float32, 2, n), (None, torch.bfloat16, 0, None)):
+        gate = None if gate_type is None else torch.randn(T, C + apart, generator=g, device="cuda").to(gate_type)[:, :C]
+        w = None if w_len is None else torch.randn(w_len, generator=g, device="cuda")
+        out = torch.empty(T, C, dtype=out_type, device="cuda")
+        ops.group_rmsnorm_gate(y, gate, w, 1e-5, groups, out, gate_act="silu")
+        v = y.double().view(T, groups, n)
+        want = (v / (v.square().mean(-1, keepdim=True) + 1e-5).sqrt()).reshape(T, C)
+        if w is not None:
+            want *= w.double().repeat(C // w_len)
+        if gate is not None:
+            want *= torch.nn.functional.silu(gate.double())
+        tol = 5e-6 if out_type == torch.float32 else 2.0 ** -8
+        torch.testing.assert_close(out.double(), want, rtol=tol, atol=1e-6)
