@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #define SOMI_F32 0
 #define SOMI_BF16 1
 #define SOMI_ERR_UNSUPPORTED 10001   // outside every cudaError_t value in use
@@ -95,6 +97,18 @@ __device__ __forceinline__ float glu(float gate, float up, const GluForm& f) {
     const float g = fminf(gate, f.limit);
     const float u = fminf(fmaxf(up, -f.limit), f.limit);
     return g / (1.0f + expf(-glu_argument(g, f))) * (u + f.shift);
+}
+
+// Lets `KERNEL` have `bytes` of dynamic shared memory (the same for every call): asked of the runtime once a device.
+template <auto KERNEL>
+inline void allow_smem(int bytes) {
+    static std::atomic<unsigned long long> asked{0};
+    int device = 0;
+    cudaGetDevice(&device);
+    const unsigned long long bit = 1ull << (device & 63);
+    if (device < 64 && (asked.load(std::memory_order_relaxed) & bit)) return;
+    if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess && device < 64)
+        asked.fetch_or(bit, std::memory_order_relaxed);
 }
 
 inline int launch_status() { return static_cast<int>(cudaGetLastError()); }

@@ -14,6 +14,7 @@
 namespace somi {
 
 constexpr int kFrFeatures = 16, kFrWarps = 8, kFrThreads = 32 * kFrWarps;
+constexpr int kFrMostSmem = 227 * 1024;
 constexpr int kFrPitch = 20;              // floats between tokens of a partial tile (no bank twice in a store)
 
 // A warp's blocks of the weights arrive in shared memory by cp.async, all of them or STAGES ahead, before the
@@ -295,8 +296,8 @@ template <int MT, int STAGES, bool IN_PLACE, bool CLUSTER>
 int fr_launch_one(const FsArgs& a, int cluster, int blocks, int range_blocks, int own, cudaStream_t stream) {
     const int smem = 4 * (kFrWarps * STAGES * kFrFeatures * kFsBK + (IN_PLACE ? 0 : own * 8 * MT * kFrPitch) +
                           (CLUSTER ? own / range_blocks * kFrFeatures * 8 * MT : 0));
-    auto kernel = f32_rows_kernel<MT, STAGES, IN_PLACE, CLUSTER>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    constexpr auto kernel = f32_rows_kernel<MT, STAGES, IN_PLACE, CLUSTER>;
+    allow_smem<kernel>(kFrMostSmem);
     launch_pdl_cluster(kernel, dim3((a.N + kFrFeatures - 1) / kFrFeatures * cluster, 1, a.batch), dim3(kFrThreads), smem,
                        cluster, stream, a.x, a.w, a.bias, a.y, a.M, a.N, a.K, blocks, range_blocks, own, cluster, a.ldx, a.ldy,
                        a.bsx, a.bsw, a.bsy, a.w_constant);
@@ -312,7 +313,7 @@ int fr_launch(const FsArgs& a, cudaStream_t stream) {
     // walking 86; 9,728 x 896, 8 rows: 12.1 and 9.4)
     if (MT == 1 && blocks <= 2 * kFrWarps && tiles > 148 * 2) {
         const int smem = 4 * (kFrWarps * 2 * kFrFeatures * kFsBK + 2 * blocks * 8 * kFrPitch);
-        cudaFuncSetAttribute(f32_rows_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        allow_smem<f32_rows_walk_kernel>(kFrMostSmem);
         const int all = (a.N + kFrFeatures - 1) / kFrFeatures, ctas = (148 * 2 + a.batch - 1) / a.batch;
         launch_pdl(f32_rows_walk_kernel, dim3(all < ctas ? all : ctas, 1, a.batch), dim3(kFrThreads), smem, stream, a.x, a.w,
                    a.bias, a.y, a.M, a.N, a.K, blocks, range_blocks, all, a.ldx, a.ldy, a.bsx, a.bsw, a.bsy, a.w_constant);

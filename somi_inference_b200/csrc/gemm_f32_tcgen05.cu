@@ -402,8 +402,8 @@ struct FtForm {
 
 template <int NB, bool TOKENS>
 int ft_launch_one(const FsArgs& a, int cluster, int blocks, int range_blocks, cudaStream_t stream) {
-    auto kernel = f32_tiles_kernel<NB, TOKENS>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ft_smem<NB>());
+    constexpr auto kernel = f32_tiles_kernel<NB, TOKENS>;
+    allow_smem<kernel>(ft_smem<NB>());
     constexpr int TN = TOKENS ? NB : 128, TM = TOKENS ? 128 : NB;
     for (int m = 0; m < a.M;) {                          // (a grid has at most 65,535 tiles of rows)
         const int rows = a.M - m < 65535 * TM ? a.M - m : 65535 * TM;

@@ -567,8 +567,8 @@ int launch_chunks(const ChRows& q, const ChRows& k, const ChRows& v, float q_sca
                   const int* cu_q, const int* state_slot, const int* tile_list, int n_tiles, int n_req, int first, int heads,
                   int group, float* u, float* y, cudaStream_t stream) {
     const ChTiles tiles{tile_list, cu_q, first};
-    cudaFuncSetAttribute(chunk_update_kernel<D, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, ch_update_smem<D, SILU>());
-    cudaFuncSetAttribute(chunk_outputs_kernel<D, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, kChOutputsSmem);
+    allow_smem<chunk_update_kernel<D, SILU>>(ch_update_smem<D, SILU>());
+    allow_smem<chunk_outputs_kernel<D, SILU>>(kChOutputsSmem);
     const dim3 grid(n_tiles, heads);
     launch_pdl(chunk_update_kernel<D, SILU>, grid, dim3(kChThreads), ch_update_smem<D, SILU>(), stream, k, v, decay, tiles, heads,
                group, u);
