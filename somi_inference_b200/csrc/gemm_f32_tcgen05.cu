@@ -5,9 +5,10 @@
 // 24 MMA steps in turn, each into an accumulator of its own in tensor memory; eight warps read the accumulators and
 // add them to their sums in registers (a thread has one row and half of the columns).
 //
-// What bounds it: the splitting.  Timelines (128 x 144, 14 blocks): a block every 2,600 to 2,900 cycles, of which the splitting
-// warps take 2,100 to 2,500, the MMAs 1,600 to 1,850 and the adding 500; 2,400 cycles in front of the first block and
-// 4,000 behind the last.  Issuing the next block's loads one by one between the splits took 4,500 cycles a block, with
+// What bounds it: shared memory. At 128 x 144 a block's MMAs read 206 KB of it and the split parts are 104 KB, 2,430 cycles at 128
+// bytes; timelines show a block every 2,600 to 2,900 (splitting 2,100 to 2,500, MMAs 1,600 to 1,850, adding 500, side by
+// side), 2,400 cycles in front of the first and 4,000 behind the last.  Twelve splitting and four adding warps were no
+// faster (207 rows by 9,728 features 31.8 us, 64 rows 23.1).  Issuing the next block's loads one by one between the splits took 4,500 cycles a block, with
 // every load behind all splits the loads' latency was added to them; so they go in two groups, a and b.
 // In chains of products, FMA kernel before / now, us: 9,728 x 896, 17, 64, 207, 1,024 and 4,096 rows 22, 37, 115, 424, 1,623 /
 // 17.7, 19.7, 30.8, 113, 411 (174 TFLOP/s of float32 products); 896 x 4,864 21, 39, 65, 255, 950 / 15.0, 15.5, 20.6, 83, 222;
@@ -300,32 +301,42 @@ f32_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w, const
             // the ranges' tiles [column][128 rows], each in its CTA's shared memory: every CTA adds up a share of the
             // elements in the order of the ranges
             cluster.sync();
-            for (int i = rank * kFtGroup + tid - kFtGroup; i < NB * 32; i += cluster_size * kFtGroup) {
-                const int c = i >> 5, q = (i & 31) * 4;      // column, and four rows
-                const int m = m0 + c, n = n0 + q;
-                if (m >= M || n >= N) continue;
-                const float4* mine = reinterpret_cast<const float4*>(stages) + c * 32 + (i & 31);
-                float4 part[8];
+            const int step = cluster_size * kFtGroup;
+            for (int i0 = rank * kFtGroup + tid - kFtGroup; i0 < NB * 32; i0 += 2 * step) {
+                float4 part[2][8];                       // two elements' loads in flight
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    if (k < cluster_size) part[k] = *cluster.map_shared_rank(mine, k);
-                float v[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
+                for (int u = 0; u < 2; ++u) {
+                    const int i = i0 + u * step;
+                    if (i >= NB * 32 || m0 + (i >> 5) >= M || n0 + (i & 31) * 4 >= N) continue;
+                    const float4* mine = reinterpret_cast<const float4*>(stages) + i;
 #pragma unroll
-                for (int k = 1; k < 8; ++k)
-                    if (k < cluster_size) {
-                        v[0] = __fadd_rn(v[0], part[k].x);
-                        v[1] = __fadd_rn(v[1], part[k].y);
-                        v[2] = __fadd_rn(v[2], part[k].z);
-                        v[3] = __fadd_rn(v[3], part[k].w);
-                    }
+                    for (int k = 0; k < 8; ++k)
+                        if (k < cluster_size) part[u][k] = *cluster.map_shared_rank(mine, k);
+                }
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (n + e < N) {
-                        if (!fs_finite(v[e])) v[e] = fs_plain_sum(x + m * ldx, w + static_cast<long long>(n + e) * K, K);
-                        y[m * ldy + n + e] = bias ? __fadd_rn(v[e], bias[n + e]) : v[e];
-                    }
+                for (int u = 0; u < 2; ++u) {
+                    const int i = i0 + u * step, m = m0 + (i >> 5), n = n0 + (i & 31) * 4;       // a column, four of its rows
+                    if (i >= NB * 32 || m >= M || n >= N) continue;
+                    float v[4] = {part[u][0].x, part[u][0].y, part[u][0].z, part[u][0].w};
+#pragma unroll
+                    for (int k = 1; k < 8; ++k)
+                        if (k < cluster_size) {
+                            v[0] = __fadd_rn(v[0], part[u][k].x);
+                            v[1] = __fadd_rn(v[1], part[u][k].y);
+                            v[2] = __fadd_rn(v[2], part[u][k].z);
+                            v[3] = __fadd_rn(v[3], part[u][k].w);
+                        }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (n + e < N) {
+                            if (!fs_finite(v[e])) v[e] = fs_plain_sum(x + m * ldx, w + static_cast<long long>(n + e) * K, K);
+                            y[m * ldy + n + e] = bias ? __fadd_rn(v[e], bias[n + e]) : v[e];
+                        }
+                }
             }
-            cluster.sync();                                  // no CTA leaves while its tile is read
+            // no CTA leaves while its tile is read: the stores above have taken what was read, and nobody waits for them here
+            __syncwarp();
+            asm volatile("barrier.cluster.arrive.relaxed.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
         } else if (ok && !TOKENS) {
             const int n = n0 + row, count = n < N ? min(HALF, M - m0 - col0) : 0;
             float* dst = y + (m0 + col0) * ldy + n;
