@@ -408,15 +408,14 @@ attention_f32_rows_kernel(const float* __restrict__ qkv, int row_stride, const f
     }
 }
 
-// The same for few tiles: a CTA takes 16 RI rows of a tile of 64 (share blockIdx.z of it), and 8 / RI warps share 16 rows, a
+// The same for few tiles: a CTA takes 16 RI rows of a tile of 64 (a share of it), and 8 / RI warps share 16 rows, a
 // part of the keys each, then of the columns; scores and probabilities pass through shared memory.
 template <int HD, int RI>
-__global__ void __launch_bounds__(256, HD == 64 ? 2 : 1)
-attention_f32_shares_kernel(const float* __restrict__ qkv, int row_stride, const float* __restrict__ kcache,
-                            const float* __restrict__ vcache, const int* __restrict__ block_table,
-                            int bt_stride, const int* __restrict__ cu_q, const int* __restrict__ ctx_len,
-                            const int* __restrict__ tiles, int n_tiles, int nq, int nkv, int page_size,
-                            float scale, int window, float* __restrict__ out) {
+__device__ __forceinline__ void
+f32_shares(int tile_at, int head, int part, const float* __restrict__ qkv, int row_stride, const float* __restrict__ kcache,
+           const float* __restrict__ vcache, const int* __restrict__ block_table, int bt_stride, const int* __restrict__ cu_q,
+           const int* __restrict__ ctx_len, const int* __restrict__ tiles, int nq, int nkv, int page_size, float scale,
+           int window, float* __restrict__ out) {
     constexpr int ROWS = 16 * RI, PP = kF32Chunk + 4;
     constexpr int ACROSS = 8 / RI, KT = 8 / ACROSS, OT = HD / 8 / ACROSS;          // n8 tiles of keys and columns for a warp
     constexpr int QPLANE = ROWS * HD * 2, KPLANE = kF32Chunk * HD * 2, PPLANE = ROWS * 128;
@@ -433,9 +432,9 @@ attention_f32_shares_kernel(const float* __restrict__ qkv, int row_stride, const
     __shared__ long long at_s[2][kF32Chunk];
     pdl_launch_dependents();
     pdl_wait();
-    const int* tile = tiles + 3 * (n_tiles - 1 - static_cast<int>(blockIdx.x));   // a prompt's last rows first
-    const int req = tile[0], row0 = tile[1] + blockIdx.z * ROWS, head = blockIdx.y;
-    const int rows = min(ROWS, tile[2] - static_cast<int>(blockIdx.z) * ROWS);
+    const int* tile = tiles + 3 * tile_at;
+    const int req = tile[0], row0 = tile[1] + part * ROWS;
+    const int rows = min(ROWS, tile[2] - part * ROWS);
     if (rows <= 0) return;
     const int kvh = head / (nq / nkv);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -688,27 +687,37 @@ attention_f32_shares_kernel(const float* __restrict__ qkv, int row_stride, const
     }
 }
 
+template <int HD, int RI>
+__global__ void __launch_bounds__(256, HD == 64 ? 2 : 1)
+attention_f32_shares_kernel(const float* __restrict__ qkv, int row_stride, const float* __restrict__ kcache,
+                            const float* __restrict__ vcache, const int* __restrict__ block_table,
+                            int bt_stride, const int* __restrict__ cu_q, const int* __restrict__ ctx_len,
+                            const int* __restrict__ tiles, int n_tiles, int nq, int nkv, int page_size,
+                            float scale, int window, float* __restrict__ out) {
+    f32_shares<HD, RI>(n_tiles - 1 - static_cast<int>(blockIdx.x), blockIdx.y, blockIdx.z, qkv, row_stride, kcache, vcache,
+                       block_table, bt_stride, cu_q, ctx_len, tiles, nq, nkv, page_size, scale, window, out);   // a prompt's last rows first
+}
+
 // ------------------------------------------------------------------- single-token requests
 // part_o [request][query head][chunk][HD], part_ml likewise with (m, l); a request's chunks are counted from the
 // one of its first visible key, so that a window needs no more of them than it reaches.
 template <int HD>
-__global__ void __launch_bounds__(128)
-attention_f32_split_kernel(const float* __restrict__ qkv, int row_stride, int row_base, int req_base,
-                           const float* __restrict__ kcache, const float* __restrict__ vcache,
-                           const int* __restrict__ block_table, int bt_stride, const int* __restrict__ ctx_len,
-                           int nq, int nkv, int page_size, float scale, int window, int max_chunks,
-                           float* __restrict__ part_o, float2* __restrict__ part_ml) {
+__device__ __forceinline__ void
+f32_single(int at, int kvh, int i, const float* __restrict__ qkv, int row_stride, int row_base, int req_base,
+           const float* __restrict__ kcache, const float* __restrict__ vcache, const int* __restrict__ block_table, int bt_stride,
+           const int* __restrict__ ctx_len, int nq, int nkv, int page_size, float scale, int window, int max_chunks,
+           float* __restrict__ part_o, float2* __restrict__ part_ml) {
     constexpr int P = HD + 4, PP = kF32Chunk + 4;
     constexpr int QUADS = HD / 4, OT = HD / 32;          // n8 tiles of columns a warp
     extern __shared__ __align__(16) float f32_smem[];
     float* Vs = f32_smem;                // [64][P]
     float* Ps = Vs + kF32Chunk * P;      // [8][PP]
     pdl_launch_dependents();
-    const int kvh = blockIdx.y, i = blockIdx.z, req = req_base + i;
+    const int req = req_base + i;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int pos = ld_step(ctx_len + req);              // [descriptor]
     const int first_key = window > 0 ? max(0, pos - window + 1) : 0;
-    const int at = blockIdx.x, c = first_key / kF32Chunk + at;
+    const int c = first_key / kF32Chunk + at;
     if (c * kF32Chunk > pos) {
         pdl_wait();
         return;
@@ -886,6 +895,40 @@ attention_f32_split_kernel(const float* __restrict__ qkv, int row_stride, int ro
 }
 
 template <int HD>
+__global__ void __launch_bounds__(128)
+attention_f32_split_kernel(const float* __restrict__ qkv, int row_stride, int row_base, int req_base,
+                           const float* __restrict__ kcache, const float* __restrict__ vcache,
+                           const int* __restrict__ block_table, int bt_stride, const int* __restrict__ ctx_len,
+                           int nq, int nkv, int page_size, float scale, int window, int max_chunks,
+                           float* __restrict__ part_o, float2* __restrict__ part_ml) {
+    f32_single<HD>(blockIdx.x, blockIdx.y, blockIdx.z, qkv, row_stride, row_base, req_base, kcache, vcache, block_table, bt_stride,
+                   ctx_len, nq, nkv, page_size, scale, window, max_chunks, part_o, part_ml);
+}
+
+// Portions and single tokens of a step in one launch: the portions' CTAs first, then one per (chunk, kv head, request), whose
+// upper four warps have nothing to do.
+template <int HD, int RI>
+__global__ void __launch_bounds__(256, HD == 64 ? 2 : 1)
+attention_f32_mixed_kernel(const float* __restrict__ qkv, int row_stride, const float* __restrict__ kcache,
+                           const float* __restrict__ vcache, const int* __restrict__ block_table, int bt_stride,
+                           const int* __restrict__ cu_q, const int* __restrict__ ctx_len, const int* __restrict__ tiles,
+                           int n_tiles, int nq, int nkv, int page_size, float scale, int window, float* __restrict__ out,
+                           int row_base, int req_base, int max_chunks, float* __restrict__ part_o,
+                           float2* __restrict__ part_ml) {
+    const int portion = n_tiles * nq * (4 / RI);
+    int b = blockIdx.x;
+    if (b < portion) {
+        f32_shares<HD, RI>(n_tiles - 1 - b % n_tiles, b / n_tiles % nq, b / (n_tiles * nq), qkv, row_stride, kcache, vcache,
+                           block_table, bt_stride, cu_q, ctx_len, tiles, nq, nkv, page_size, scale, window, out);
+        return;
+    }
+    if (threadIdx.x >= 128) return;                      // (whole warps: barriers count the threads that are left)
+    b -= portion;
+    f32_single<HD>(b % max_chunks, b / max_chunks % nkv, b / (max_chunks * nkv), qkv, row_stride, row_base, req_base, kcache,
+                   vcache, block_table, bt_stride, ctx_len, nq, nkv, page_size, scale, window, max_chunks, part_o, part_ml);
+}
+
+template <int HD>
 __global__ void __launch_bounds__(HD)
 attention_f32_merge_kernel(const float* __restrict__ part_o, const float2* __restrict__ part_ml, int max_chunks,
                            const int* __restrict__ ctx_len, int row_base, int req_base, int nq, int window,
@@ -922,6 +965,9 @@ constexpr int f32_shares_smem(int rows) { return f32_rows_smem<HD>(rows) + 3 * 2
 template <int HD>
 constexpr int f32_split_smem() { return 4 * (kF32Chunk * (HD + 4) + kF32Heads * (kF32Chunk + 4)); }
 
+template <int HD, int RI>
+constexpr int f32_mixed_smem() { return f32_shares_smem<HD>(16 * RI) > f32_split_smem<HD>() ? f32_shares_smem<HD>(16 * RI) : f32_split_smem<HD>(); }
+
 }  // namespace somi
 
 using namespace somi;
@@ -936,6 +982,15 @@ SOMI_API int somi_attention_f32_supported(const float* qkv, const float* kcache,
     return (hd == 64 || hd == 128) && nkv > 0 && nq % nkv == 0 && nq <= 65535 && row_stride % 4 == 0 && (bits & 15) == 0;
 }
 
+// Few tiles: two or four CTAs share one, each with a part of its rows; many: a warp keeps 16 rows to itself (the same
+// bits).  Layer of 14 heads over 2 of 64, 4 / 2 shares / rows in us: 203 rows (56 tiles and heads) 47 / 51 / 62, 64 rows behind
+// 2,000 positions (14) 170 / 197 / 266, 300 behind 100 (70) 66 / 71 / 91, 512 (112) 92 / 83 / 103, 1,024 (224) 205 / 164 /
+// 171, 2,048 (448) 585 / 413 / 365, 5,000 (1,106) 2,924 / 1,892 / 1,508.
+static int f32_shares_of(int n_tiles, int nq) {
+    const long long ctas = static_cast<long long>(n_tiles) * nq;
+    return ctas <= 100 ? 4 : (ctas <= 148 * 2 ? 2 : 1);
+}
+
 // Prompt portions: the tile list's query tiles are at most 64 rows.
 SOMI_API int somi_attention_f32_portion(const float* qkv, int row_stride, const float* kcache, const float* vcache,
                                         const int* block_table, int bt_stride, const int* cu_q, const int* ctx_len,
@@ -944,12 +999,7 @@ SOMI_API int somi_attention_f32_portion(const float* qkv, int row_stride, const 
     if (n_tiles <= 0) return 0;
     if (!somi_attention_f32_supported(qkv, kcache, vcache, out, row_stride, nq, nkv, hd) || page_size <= 0)
         return SOMI_ERR_UNSUPPORTED;
-    // Few tiles: two or four CTAs share one, each with a part of its rows; many: a warp keeps 16 rows to itself (the same
-    // bits).  Layer of 14 heads over 2 of 64, 4 / 2 shares / rows in us: 203 rows (56 tiles and heads) 47 / 51 / 62, 64 rows behind
-    // 2,000 positions (14) 170 / 197 / 266, 300 behind 100 (70) 66 / 71 / 91, 512 (112) 92 / 83 / 103, 1,024 (224) 205 / 164 /
-    // 171, 2,048 (448) 585 / 413 / 365, 5,000 (1,106) 2,924 / 1,892 / 1,508.
-    const long long ctas = static_cast<long long>(n_tiles) * nq;
-    const int shares = ctas <= 100 ? 4 : (ctas <= 148 * 2 ? 2 : 1);
+    const int shares = f32_shares_of(n_tiles, nq);
 #define SOMI_F32_PORTION(KERNEL, THREADS, SHARES, SMEM) \
     (allow_smem<KERNEL>(SMEM), launch_pdl(KERNEL, dim3(n_tiles, nq, SHARES), dim3(THREADS), SMEM, stream, qkv, row_stride, kcache, \
                                           vcache, block_table, bt_stride, cu_q, ctx_len, tiles, n_tiles, nq, nkv, page_size, \
@@ -992,4 +1042,44 @@ SOMI_API int somi_attention_f32_single(const float* qkv, int row_stride, int row
     };
     return hd == 64 ? go(attention_f32_split_kernel<64>, attention_f32_merge_kernel<64>, f32_split_smem<64>())
                     : go(attention_f32_split_kernel<128>, attention_f32_merge_kernel<128>, f32_split_smem<128>());
+}
+
+// Whether a step's portions and single tokens go in one launch: where few tiles share their rows out, and the single tokens are at most
+// four waves of CTAs as large as the portions' (two an SM at 64, one at 128).  A captured layer of 14 heads over 2 of 64, one launch / apart, us:
+// 203 rows and 4 tokens behind 1,000 (136 CTAs of single tokens) 51.2 / 57.8, 16 (544) 55.1 / 61.1, 32 (1,088) 66.0 / 68.1, 64
+// (2,176) 91.0 / 85.7; 16 behind 2,000 (1,088) 67.7 / 69.7; 64 rows behind 2,000 and 8 tokens 174 / 181; 1,024 rows and 16 tokens 171 / 180.
+SOMI_API int somi_attention_f32_mixed_takes(int n_tiles, int nq, int nkv, int hd, int n_decode, int max_chunks) {
+    return n_tiles > 0 && n_decode > 0 && nq > 0 && f32_shares_of(n_tiles, nq) > 1 &&
+           static_cast<long long>(n_decode) * max_chunks * nkv <= 4 * 148 * (hd == 64 ? 2 : 1);
+}
+
+// Both, where the rule above takes them: arguments as of the two functions in front of it.
+SOMI_API int somi_attention_f32_mixed(const float* qkv, int row_stride, const float* kcache, const float* vcache,
+                                      const int* block_table, int bt_stride, const int* cu_q, const int* ctx_len,
+                                      const int* tiles, int n_tiles, int nq, int nkv, int hd, int page_size, float scale,
+                                      int window, float* out, int row_base, int req_base, int n_decode, float* part,
+                                      int max_chunks, cudaStream_t stream) {
+    if (!somi_attention_f32_supported(qkv, kcache, vcache, out, row_stride, nq, nkv, hd) || page_size <= 0 || max_chunks <= 0 ||
+        n_decode > 65535 || (reinterpret_cast<uintptr_t>(part) & 7) ||
+        !somi_attention_f32_mixed_takes(n_tiles, nq, nkv, hd, n_decode, max_chunks))
+        return SOMI_ERR_UNSUPPORTED;
+    float2* part_ml = reinterpret_cast<float2*>(part);
+    float* part_o = part + 2 * static_cast<size_t>(n_decode) * nq * max_chunks;
+    const int shares = f32_shares_of(n_tiles, nq), singles = n_decode * max_chunks * nkv;
+#define SOMI_F32_MIXED(HD, RI) \
+    (allow_smem<attention_f32_mixed_kernel<HD, RI>>(f32_mixed_smem<HD, RI>()), \
+     launch_pdl(attention_f32_mixed_kernel<HD, RI>, dim3(n_tiles * nq * (4 / RI) + singles), dim3(256), f32_mixed_smem<HD, RI>(), \
+                stream, qkv, row_stride, kcache, vcache, block_table, bt_stride, cu_q, ctx_len, tiles, n_tiles, nq, nkv, \
+                page_size, scale, window, out, row_base, req_base, max_chunks, part_o, part_ml), \
+     launch_pdl(attention_f32_merge_kernel<HD>, dim3(n_decode, nq), dim3(HD), 0, stream, part_o, part_ml, max_chunks, ctx_len, \
+                row_base, req_base, nq, window, out))
+    if (hd == 64) {
+        if (shares == 2) SOMI_F32_MIXED(64, 2);
+        else SOMI_F32_MIXED(64, 1);
+    } else {
+        if (shares == 2) SOMI_F32_MIXED(128, 2);
+        else SOMI_F32_MIXED(128, 1);
+    }
+#undef SOMI_F32_MIXED
+    return launch_status();
 }

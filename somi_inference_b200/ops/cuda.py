@@ -532,32 +532,43 @@ class CudaOps:
                        ctypes.c_int(nq), ctypes.c_int(nkv), ctypes.c_int(hd))))
         if own_f32:
             tiles = batch.tiles[self.prefill_q_tile]
-            if tiles.shape[0]:
+            # (a window of n positions meets at most (n + 62) / 64 + 1 chunks of 64)
+            max_chunks = -(-group.width * page_size // self.f32_chunk)
+            if win:
+                max_chunks = min(max_chunks, (win + self.f32_chunk - 2) // self.f32_chunk + 1)
+            each = nq * max_chunks * (hd + 2)
+            most = min(n_decode, max(1, self.F32_PART_FLOATS // each))
+            part = torch.empty(most * each, dtype=torch.float32, device=qkv.device) if n_decode else None
+            table = (_ptr(group.block_table), ctypes.c_int(group.width))
+            shape = (ctypes.c_int(nq), ctypes.c_int(nkv), ctypes.c_int(hd), ctypes.c_int(page_size), ctypes.c_float(scale),
+                     ctypes.c_int(win))
+            together = most and most == n_decode and tiles.shape[0] and self.lib.somi_attention_f32_mixed_takes(
+                ctypes.c_int(tiles.shape[0]), *shape[:3], ctypes.c_int(n_decode), ctypes.c_int(max_chunks))
+            if together:
+                rc = self.lib.somi_attention_f32_mixed(
+                    _ptr(qkv), ctypes.c_int(qkv.shape[1]), _ptr(kcache), _ptr(vcache), *table, _ptr(batch.cu_q),
+                    _ptr(batch.ctx_len), _ptr(tiles), ctypes.c_int(tiles.shape[0]), *shape, _ptr(out),
+                    ctypes.c_int(batch.num_prefill_tokens), ctypes.c_int(batch.num_prefill_requests), ctypes.c_int(n_decode),
+                    _ptr(part), ctypes.c_int(max_chunks), self._stream())
+                self._done(rc, "attention_f32_mixed")
+                self.launches += 1
+                if trace.active():
+                    trace.note("attention_f32_mixed", *self._attention_work(batch, 0, batch.num_requests, nq, nkv, hd, 4, win),
+                               detail="with merge")
+            if tiles.shape[0] and not together:
                 rc = self.lib.somi_attention_f32_portion(
-                    _ptr(qkv), ctypes.c_int(qkv.shape[1]), _ptr(kcache), _ptr(vcache),
-                    _ptr(group.block_table), ctypes.c_int(group.width), _ptr(batch.cu_q),
-                    _ptr(batch.ctx_len), _ptr(tiles), ctypes.c_int(tiles.shape[0]), ctypes.c_int(nq),
-                    ctypes.c_int(nkv), ctypes.c_int(hd), ctypes.c_int(page_size), ctypes.c_float(scale),
-                    ctypes.c_int(win), _ptr(out), self._stream())
+                    _ptr(qkv), ctypes.c_int(qkv.shape[1]), _ptr(kcache), _ptr(vcache), *table, _ptr(batch.cu_q),
+                    _ptr(batch.ctx_len), _ptr(tiles), ctypes.c_int(tiles.shape[0]), *shape, _ptr(out), self._stream())
                 self._done(rc, "attention_f32_portion")
                 if trace.active():
                     trace.note("attention_f32_portion", *self._attention_work(
                         batch, 0, batch.num_prefill_requests, nq, nkv, hd, 4, win))
-            if n_decode:
-                # (a window of n positions meets at most (n + 62) / 64 + 1 chunks of 64)
-                max_chunks = -(-group.width * page_size // self.f32_chunk)
-                if win:
-                    max_chunks = min(max_chunks, (win + self.f32_chunk - 2) // self.f32_chunk + 1)
-                each = nq * max_chunks * (hd + 2)
-                most = min(n_decode, max(1, self.F32_PART_FLOATS // each))
-                part = torch.empty(most * each, dtype=torch.float32, device=qkv.device)
+            if n_decode and not together:
                 for at in range(0, n_decode, most):
                     rc = self.lib.somi_attention_f32_single(
                         _ptr(qkv), ctypes.c_int(qkv.shape[1]), ctypes.c_int(batch.num_prefill_tokens + at),
                         ctypes.c_int(batch.num_prefill_requests + at), ctypes.c_int(min(most, n_decode - at)),
-                        _ptr(kcache), _ptr(vcache), _ptr(group.block_table), ctypes.c_int(group.width),
-                        _ptr(batch.ctx_len), ctypes.c_int(nq), ctypes.c_int(nkv), ctypes.c_int(hd),
-                        ctypes.c_int(page_size), ctypes.c_float(scale), ctypes.c_int(win), _ptr(part),
+                        _ptr(kcache), _ptr(vcache), *table, _ptr(batch.ctx_len), *shape, _ptr(part),
                         ctypes.c_int(max_chunks), _ptr(out), self._stream())
                     self._done(rc, "attention_f32_single")
                     self.launches += 1
@@ -1691,10 +1702,10 @@ class CudaOps:
     SCAN_PREPARE_ROWS = 16
     SCAN_TURN_ROWS = 4          # the most rows a request may have where the scan itself rotates q and k
 
-    # A portion goes in chunks from rows = this * state width on.  The layer in us step by step / in chunks,
-    # captured: 14 heads of 64: 64 rows 38.9 / 36.9, 84 beside 11 single tokens 43.1 / 43.1, 96 45.2 / 36.9, 256 79.8 /
-    # 39.0; 28 of 128: 128 rows 94.0 / 96.4, 160 100.5 / 100.8, 192 110.5 / 102.5, 256 129.1 / 113.9.  Launched one by one
-    # both are bound by the host up to about 256 rows, and the 84 rows beside single tokens took 130.1 / 145.7.
+    # A portion goes in chunks from rows = this * state width on.  The layer in us, captured, step by step / in chunks:
+    # 14 heads of 64: 96 rows 45.1 / 37.7, 128 51.3 / 38.3, 256 77.9 / 40.1, 512 131 / 45.1; 28 of 128: 192 rows 111 / 92.1,
+    # 256 130 / 97.0, 512 219 / 122.  Step by step is 38.3 at 64 rows of the first and 91.2 at 128 of the second, where chunks
+    # are at best the same.  Launched one by one both are bound by the host up to about 256 rows (130 / 120).
     SCAN_CHUNK_ROWS = 1.5
     SCAN_CHUNK_BYTES = 1 << 29  # the most that the chunks' states of a run of portions may take
 

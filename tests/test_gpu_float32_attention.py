@@ -84,3 +84,26 @@ def test_error_against_64_bits(ops, hd, n):
     want = torch.einsum("hqk,khd->qhd", s.softmax(-1), v.repeat_interleave(nq // nkv, 1))
     assert (out.double() - want).norm() <= 1e-6 * want.norm()
     assert (out.double() - want).abs().max() <= 1e-5
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("window", [None, 100])
+@pytest.mark.parametrize("n", [1, 8])
+def test_one_launch_for_portions_and_single_tokens(ops, monkeypatch, hd, window, n):
+    """What one launch gives (four shares, two) is what a launch for each gives, bit for bit; more single tokens than the
+    rule takes go apart."""
+    nq, nkv, ps = 6, 2, 16
+    for singles in ([0], [63, 64, 700], [500] * 80):
+        requests = [(131, 140), (0, 3), *[(0, 64)] * (n - 1)] + [(c, 1) for c in singles]
+        if n == 8:
+            requests = [(131, 140)] * n + [(c, 1) for c in singles]
+        case = attention_case(ops, nq=nq, nkv=nkv, hd=hd, page_size=ps, window=window, requests=requests, dtype=torch.float32)
+        before = ops.launches
+        got = run(ops, case, nq, nkv, hd, window)
+        took = ops.launches - before
+        with monkeypatch.context() as m:
+            m.setattr(ops.lib, "somi_attention_f32_mixed_takes", lambda *args: 0)
+            want = run(ops, case, nq, nkv, hd, window)
+        assert took == (2 if len(singles) < 80 or window else 3)
+        assert got.isfinite().all() and torch.equal(got, want)
+    ops.check_errors()
