@@ -905,10 +905,10 @@ attention_f32_split_kernel(const float* __restrict__ qkv, int row_stride, int ro
                    ctx_len, nq, nkv, page_size, scale, window, max_chunks, part_o, part_ml);
 }
 
-// Portions and single tokens of a step in one launch: the portions' CTAs first, then one per (chunk, kv head, request), whose
+// Portions and single tokens of a step in one launch (head size 64): the portions' CTAs first, then one per (chunk, kv head, request), whose
 // upper four warps have nothing to do.
-template <int HD, int RI>
-__global__ void __launch_bounds__(256, HD == 64 ? 2 : 1)
+template <int RI>
+__global__ void __launch_bounds__(256, 2)
 attention_f32_mixed_kernel(const float* __restrict__ qkv, int row_stride, const float* __restrict__ kcache,
                            const float* __restrict__ vcache, const int* __restrict__ block_table, int bt_stride,
                            const int* __restrict__ cu_q, const int* __restrict__ ctx_len, const int* __restrict__ tiles,
@@ -918,13 +918,13 @@ attention_f32_mixed_kernel(const float* __restrict__ qkv, int row_stride, const 
     const int portion = n_tiles * nq * (4 / RI);
     int b = blockIdx.x;
     if (b < portion) {
-        f32_shares<HD, RI>(n_tiles - 1 - b % n_tiles, b / n_tiles % nq, b / (n_tiles * nq), qkv, row_stride, kcache, vcache,
+        f32_shares<64, RI>(n_tiles - 1 - b % n_tiles, b / n_tiles % nq, b / (n_tiles * nq), qkv, row_stride, kcache, vcache,
                            block_table, bt_stride, cu_q, ctx_len, tiles, nq, nkv, page_size, scale, window, out);
         return;
     }
     if (threadIdx.x >= 128) return;                      // (whole warps: barriers count the threads that are left)
     b -= portion;
-    f32_single<HD>(b % max_chunks, b / max_chunks % nkv, b / (max_chunks * nkv), qkv, row_stride, row_base, req_base, kcache,
+    f32_single<64>(b % max_chunks, b / max_chunks % nkv, b / (max_chunks * nkv), qkv, row_stride, row_base, req_base, kcache,
                    vcache, block_table, bt_stride, ctx_len, nq, nkv, page_size, scale, window, max_chunks, part_o, part_ml);
 }
 
@@ -965,8 +965,7 @@ constexpr int f32_shares_smem(int rows) { return f32_rows_smem<HD>(rows) + 3 * 2
 template <int HD>
 constexpr int f32_split_smem() { return 4 * (kF32Chunk * (HD + 4) + kF32Heads * (kF32Chunk + 4)); }
 
-template <int HD, int RI>
-constexpr int f32_mixed_smem() { return f32_shares_smem<HD>(16 * RI) > f32_split_smem<HD>() ? f32_shares_smem<HD>(16 * RI) : f32_split_smem<HD>(); }
+static_assert(f32_split_smem<64>() <= f32_shares_smem<64>(16), "a launch of both has the portions' shared memory");
 
 }  // namespace somi
 
@@ -1044,13 +1043,14 @@ SOMI_API int somi_attention_f32_single(const float* qkv, int row_stride, int row
                     : go(attention_f32_split_kernel<128>, attention_f32_merge_kernel<128>, f32_split_smem<128>());
 }
 
-// Whether a step's portions and single tokens go in one launch: where few tiles share their rows out, and the single tokens are at most
-// four waves of CTAs as large as the portions' (two an SM at 64, one at 128).  A captured layer of 14 heads over 2 of 64, one launch / apart, us:
+// Whether a step's portions and single tokens go in one launch: head size 64, where few tiles share their rows out and the single tokens
+// are at most four waves of CTAs as large as the portions', two an SM.  A captured layer of 14 heads over 2 of 64, one launch / apart, us:
 // 203 rows and 4 tokens behind 1,000 (136 CTAs of single tokens) 51.2 / 57.8, 16 (544) 55.1 / 61.1, 32 (1,088) 66.0 / 68.1, 64
 // (2,176) 91.0 / 85.7; 16 behind 2,000 (1,088) 67.7 / 69.7; 64 rows behind 2,000 and 8 tokens 174 / 181; 1,024 rows and 16 tokens 171 / 180.
+// At 128 a CTA fills an SM and the single tokens wait for the portions: 28 heads over 4, 203 rows and 4 tokens 201 / 192, 8 tokens 218 / 204.
 SOMI_API int somi_attention_f32_mixed_takes(int n_tiles, int nq, int nkv, int hd, int n_decode, int max_chunks) {
-    return n_tiles > 0 && n_decode > 0 && nq > 0 && f32_shares_of(n_tiles, nq) > 1 &&
-           static_cast<long long>(n_decode) * max_chunks * nkv <= 4 * 148 * (hd == 64 ? 2 : 1);
+    return hd == 64 && n_tiles > 0 && n_decode > 0 && nq > 0 && f32_shares_of(n_tiles, nq) > 1 &&
+           static_cast<long long>(n_decode) * max_chunks * nkv <= 4 * 2 * 148;
 }
 
 // Both, where the rule above takes them: arguments as of the two functions in front of it.
@@ -1066,20 +1066,16 @@ SOMI_API int somi_attention_f32_mixed(const float* qkv, int row_stride, const fl
     float2* part_ml = reinterpret_cast<float2*>(part);
     float* part_o = part + 2 * static_cast<size_t>(n_decode) * nq * max_chunks;
     const int shares = f32_shares_of(n_tiles, nq), singles = n_decode * max_chunks * nkv;
-#define SOMI_F32_MIXED(HD, RI) \
-    (allow_smem<attention_f32_mixed_kernel<HD, RI>>(f32_mixed_smem<HD, RI>()), \
-     launch_pdl(attention_f32_mixed_kernel<HD, RI>, dim3(n_tiles * nq * (4 / RI) + singles), dim3(256), f32_mixed_smem<HD, RI>(), \
-                stream, qkv, row_stride, kcache, vcache, block_table, bt_stride, cu_q, ctx_len, tiles, n_tiles, nq, nkv, \
-                page_size, scale, window, out, row_base, req_base, max_chunks, part_o, part_ml), \
-     launch_pdl(attention_f32_merge_kernel<HD>, dim3(n_decode, nq), dim3(HD), 0, stream, part_o, part_ml, max_chunks, ctx_len, \
-                row_base, req_base, nq, window, out))
-    if (hd == 64) {
-        if (shares == 2) SOMI_F32_MIXED(64, 2);
-        else SOMI_F32_MIXED(64, 1);
-    } else {
-        if (shares == 2) SOMI_F32_MIXED(128, 2);
-        else SOMI_F32_MIXED(128, 1);
-    }
-#undef SOMI_F32_MIXED
-    return launch_status();
+    auto go = [&](auto kernel, int smem, int ctas) {
+        launch_pdl(kernel, dim3(ctas + singles), dim3(256), smem, stream, qkv, row_stride, kcache, vcache, block_table, bt_stride,
+                   cu_q, ctx_len, tiles, n_tiles, nq, nkv, page_size, scale, window, out, row_base, req_base, max_chunks, part_o,
+                   part_ml);
+        launch_pdl(attention_f32_merge_kernel<64>, dim3(n_decode, nq), dim3(64), 0, stream, part_o, part_ml, max_chunks, ctx_len,
+                   row_base, req_base, nq, window, out);
+        return launch_status();
+    };
+    allow_smem<attention_f32_mixed_kernel<1>>(f32_shares_smem<64>(16));
+    allow_smem<attention_f32_mixed_kernel<2>>(f32_shares_smem<64>(32));
+    return shares == 2 ? go(attention_f32_mixed_kernel<2>, f32_shares_smem<64>(32), n_tiles * nq * 2)
+                       : go(attention_f32_mixed_kernel<1>, f32_shares_smem<64>(16), n_tiles * nq * 4);
 }
