@@ -10,8 +10,8 @@
 // ascending order: with M the larger maximum, L <- L e^(M_old - M) + l_c e^(m_c - M), O likewise.  The
 // prompt kernel merges in registers; the split kernel writes (m_c, l_c, o_c) and the merge kernel
 // goes through them.  So how a request was cut into steps, or what else is in a step, changes no bit.  A score that comes out
-// infinite or NaN is summed again as FMAs; a value that is not finite stays out of the products and is added to the rows
-// that see it.
+// infinite or NaN is summed again as FMAs; a value that is not finite, or so large that bfloat16 rounds it to infinity, stays out of
+// the products and is added to the rows that see it.
 //
 // Why these two shapes.  Single tokens are bound by latency and by the cache's bytes: one CTA per
 // (request, key/value head, chunk) reads keys and values once for all query heads of the group, with every
@@ -144,7 +144,7 @@ attention_f32_rows_kernel(const float* __restrict__ qkv, int row_stride, const f
     unsigned char* Qs = f32_raw;                                         // parts [3][ROWS][HD], in swizzled rows like all of them
     unsigned char* Ks = Qs + 3 * QPLANE;                                 // [3][64][HD]
     unsigned char* Vs = Ks + 3 * KPLANE;                                 // [3][64][HD]
-    __shared__ unsigned wild_s[2][2];                                    // keys of a chunk with a value that is not finite
+    __shared__ unsigned wild_s[2][2];                                    // keys of a chunk with a value that has no parts
     __shared__ long long at_s[2][kF32Chunk];                             // where a chunk's keys lie, or -1
     pdl_launch_dependents();
     pdl_wait();
@@ -187,14 +187,14 @@ attention_f32_rows_kernel(const float* __restrict__ qkv, int row_stride, const f
         for (int i = 0; i < ITEMS; ++i) {
             const int idx = tid + THREADS * i, n = idx / (HD / 8);
             float x[8] = {q[i][0].x, q[i][0].y, q[i][0].z, q[i][0].w, q[i][1].x, q[i][1].y, q[i][1].z, q[i][1].w};
-            float none = 0.f;
+            float most = 0.f;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) none = fmaf(x[e], 0.f, none);
-            if (none != 0.f) {                           // (0 times a number that is not finite is NaN)
+            for (int e = 0; e < 8; ++e) most = fs_largest(most, x[e]);
+            if (!fs_has_parts(most)) {
                 atomicOr(&wild_s[c & 1][n >> 5], 1u << (n & 31));
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
-                    if (!fs_finite(x[e])) x[e] = 0.f;
+                    if (!fs_has_parts(x[e])) x[e] = 0.f;
             }
             f32_put8(Vs + swizzled_offset<HD>(n, idx % (HD / 8)), KPLANE, make_float4(x[0], x[1], x[2], x[3]), make_float4(x[4], x[5], x[6], x[7]));
         }
@@ -362,7 +362,7 @@ attention_f32_rows_kernel(const float* __restrict__ qkv, int row_stride, const f
                     f32_main(oc[i + 1], a, b2);
                 }
             }
-            if (wild0 | wild1) {                         // values that are not finite, to the rows that see them
+            if (wild0 | wild1) {                         // values without parts, to the rows that see them
 #pragma unroll 1
                 for (int n = 0; n < kF32Chunk; ++n) {
                     if (!((n < 32 ? wild0 : wild1) >> (n & 31) & 1)) continue;
@@ -384,7 +384,7 @@ attention_f32_rows_kernel(const float* __restrict__ qkv, int row_stride, const f
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             const float x = v[8 * i + (e & 1)];
-                            if (fs_finite(x)) continue;
+                            if (fs_has_parts(x)) continue;
 #pragma unroll
                             for (int k = 0; k < 4; ++k) oc[i][k] = f32_select(k == e, __fmaf_rn(e < 2 ? p0 : p1, x, oc[i][k]), oc[i][k]);
                         }
@@ -474,14 +474,14 @@ f32_shares(int tile_at, int head, int part, const float* __restrict__ qkv, int r
         for (int i = 0; i < ITEMS; ++i) {
             const int idx = tid + 256 * i, n = idx / (HD / 8);
             float x[8] = {vq[i][0].x, vq[i][0].y, vq[i][0].z, vq[i][0].w, vq[i][1].x, vq[i][1].y, vq[i][1].z, vq[i][1].w};
-            float none = 0.f;
+            float most = 0.f;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) none = fmaf(x[e], 0.f, none);
-            if (none != 0.f) {
+            for (int e = 0; e < 8; ++e) most = fs_largest(most, x[e]);
+            if (!fs_has_parts(most)) {
                 atomicOr(&wild_s[c & 1][n >> 5], 1u << (n & 31));
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
-                    if (!fs_finite(x[e])) x[e] = 0.f;
+                    if (!fs_has_parts(x[e])) x[e] = 0.f;
             }
             f32_put8(Vs + swizzled_offset<HD>(n, idx % (HD / 8)), KPLANE, make_float4(x[0], x[1], x[2], x[3]), make_float4(x[4], x[5], x[6], x[7]));
         }
@@ -665,7 +665,7 @@ f32_shares(int tile_at, int head, int part, const float* __restrict__ qkv, int r
 #pragma unroll
                     for (int i = 0; i < OT; ++i) {
                         const float x = v[(share * OT + i) * 8 + 2 * t + (e & 1)];
-                        if (!fs_finite(x)) oc[i][e] = __fmaf_rn(p, x, oc[i][e]);
+                        if (!fs_has_parts(x)) oc[i][e] = __fmaf_rn(p, x, oc[i][e]);
                     }
                 }
             }
@@ -855,7 +855,7 @@ f32_single(int at, int kvh, int i, const float* __restrict__ qkv, int row_stride
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
                     v[m] = src[m * P];
-                    if (!fs_finite(v[m])) {
+                    if (!fs_has_parts(v[m])) {
                         wild = true;
                         v[m] = 0.f;
                     }
@@ -872,7 +872,7 @@ f32_single(int at, int kvh, int i, const float* __restrict__ qkv, int row_stride
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int n8 = 0; n8 < OT; ++n8) f32_main(o[n8], a0[j], b0[j][n8]);
-        if (__any_sync(0xffffffffu, wild)) {             // values that are not finite, one by one
+        if (__any_sync(0xffffffffu, wild)) {             // values without parts, one by one
 #pragma unroll 1
             for (int n = 0; n < kF32Chunk; ++n) {
                 const int key = c * kF32Chunk + n;
@@ -882,7 +882,7 @@ f32_single(int at, int kvh, int i, const float* __restrict__ qkv, int row_stride
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const float x = Vs[n * P + (warp * OT + n8) * 8 + 2 * t + e];
-                        if (!fs_finite(x)) o[n8][e] = __fmaf_rn(Ps[g * PP + n], x, o[n8][e]);
+                        if (!fs_has_parts(x)) o[n8][e] = __fmaf_rn(Ps[g * PP + n], x, o[n8][e]);
                     }
             }
         }

@@ -60,6 +60,14 @@ __device__ __forceinline__ float fs_plain_sum(const float* x, const float* w, in
     return (s0 + s1) + (s2 + s3);
 }
 __device__ __forceinline__ bool fs_finite(float v) { return fabsf(v) <= 3.4028234664e38f; }
+// Whether v is the sum of three parts: finite, and below (2 - 2^-8) 2^127, from where on bfloat16 rounds to infinity.
+constexpr float kFsNoParts = 3.39617752923e38f;
+__device__ __forceinline__ bool fs_has_parts(float v) { return fabsf(v) < kFsNoParts; }
+// The larger magnitude, or NaN: below kFsNoParts only where all numbers have parts.
+__device__ __forceinline__ float fs_largest(float m, float v) {
+    asm("max.NaN.f32 %0, %0, %1;\n" : "+f"(m) : "f"(fabsf(v)));
+    return m;
+}
 
 struct FsArgs {
     const float *x, *w, *bias;

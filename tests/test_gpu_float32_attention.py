@@ -27,8 +27,8 @@ def copies(ops, n, q, nq, nkv, hd, ps, window, rows, change=None):
     _, batch, qkv, view, _ = case
     table = batch.groups[0].block_table[:, :-(-(131 + q) // ps)].long()
     for i in range(n):
-        live = table[i][table[i] >= 0]
-        view.keys[live], view.values[live] = rows[1][:live.numel()], rows[2][:live.numel()]
+        live = table[i] >= 0                             # (a window's requests have given back the pages behind it)
+        view.keys[table[i][live]], view.values[table[i][live]] = rows[1][live], rows[2][live]
         if change is not None:
             change(view, table[i])
         qkv[q * i:q * (i + 1)] = rows[0][:q]
@@ -71,6 +71,54 @@ def test_kernels_give_the_same_bits(ops, hd, window, infinite):
         assert got[0][:19].isfinite().all()
 
 
+def probabilities(rows, q, nq, nkv, hd, window=None):
+    """[nq, q, 131 + q] in 64 bits."""
+    k = rows[1].transpose(1, 2).reshape(-1, nkv, hd)[:131 + q].double()
+    s = torch.einsum("qhd,khd->hqk", rows[0][:, :nq * hd].view(q, nq, hd).double(), k.repeat_interleave(nq // nkv, 1)) * hd ** -0.5
+    key, pos = torch.arange(131 + q, device="cuda"), torch.arange(131, 131 + q, device="cuda")[:, None]
+    return s.masked_fill((key > pos) | (key <= pos - (window or 10 ** 6)), float("-inf")).softmax(-1)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("window", [None, 100])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38, -3.3962e38])
+def test_values_without_parts(ops, hd, window, value):
+    """A value that is not finite, or that bfloat16 rounds to infinity, in four shares, two, a warp for 16 rows, and for single
+    tokens: rows that do not see it and the other columns keep their bits, those that see it get what FMAs give
+    (of a finite one p v, as accurate as p: a few 2^-24 of eight times a score)."""
+    nq, nkv, ps, q, at, column = 6, 2, 16, 140, 150, 3
+    rows = made(q, nq, nkv, hd, ps)
+    clean = run(ops, copies(ops, 1, q, nq, nkv, hd, ps, window, rows), nq, nkv, hd, window).view(q, nq, hd)
+
+    def change(view, table):
+        view.values[table[at // ps], :, at % ps, column] = value
+    outs = [run(ops, copies(ops, n, q, nq, nkv, hd, ps, window, rows, change), nq, nkv, hd, window) for n in (1, 8, 20)]
+    got, pos = outs[0].view(q, nq, hd), torch.arange(131, 131 + q, device="cuda")
+    sees = (pos >= at) & (pos < at + (window or 10 ** 6))
+    rest = torch.arange(hd, device="cuda") != column
+    assert clean.isfinite().all() and torch.equal(got[~sees], clean[~sees]) and torch.equal(got[..., rest], clean[..., rest])
+    if abs(value) < float("inf"):
+        want = probabilities(rows, q, nq, nkv, hd, window)[:, :, at].T[sees] * value
+        torch.testing.assert_close(got[sees][..., column].double(), want, rtol=1e-5, atol=0)
+    else:
+        assert (got[sees][..., column].isnan() if value != value else got[sees][..., column] == value).all()
+    for out in outs[1:]:
+        for part in out.view(-1, q, nq, hd):
+            assert ((part == got) | (part.isnan() & got.isnan())).all()
+    for r in (18, 19, 60, 118, 119, 139):
+        case = attention_case(ops, nq=nq, nkv=nkv, hd=hd, page_size=ps, window=window, requests=[(131 + r, 1)], dtype=torch.float32)
+        _, batch, qkv, view, _ = case
+        table = batch.groups[0].block_table[0, :-(-(132 + r) // ps)].long()
+        live = table >= 0
+        view.keys[table[live]], view.values[table[live]] = (t[:table.numel()][live] for t in rows[1:])
+        if at // ps < table.numel() and live[at // ps]:
+            change(view, table)
+        qkv[0] = rows[0][r]
+        single = run(ops, case, nq, nkv, hd, window)[0].view(nq, hd)
+        assert ((single == got[r]) | (single.isnan() & got[r].isnan())).all()
+    ops.check_errors()
+
+
 @pytest.mark.parametrize("hd,n", [(64, 1), (64, 8), (64, 20), (128, 1), (128, 20)])
 def test_error_against_64_bits(ops, hd, n):
     """Scores of a few units are off by a few 2^-24 of the sum of their terms' magnitudes (about 8 times a score), which
@@ -78,10 +126,8 @@ def test_error_against_64_bits(ops, hd, n):
     nq, nkv, ps, q = 6, 2, 16, 140
     rows = made(q, nq, nkv, hd, ps)
     out = run(ops, copies(ops, n, q, nq, nkv, hd, ps, None, rows), nq, nkv, hd, None)[:q].view(q, nq, hd)
-    k, v = (t.transpose(1, 2).reshape(-1, nkv, hd)[:131 + q].double() for t in rows[1:])
-    s = torch.einsum("qhd,khd->hqk", rows[0][:, :nq * hd].view(q, nq, hd).double(), k.repeat_interleave(nq // nkv, 1)) * hd ** -0.5
-    s.masked_fill_(torch.arange(131 + q, device="cuda") > torch.arange(131, 131 + q, device="cuda")[:, None], float("-inf"))
-    want = torch.einsum("hqk,khd->qhd", s.softmax(-1), v.repeat_interleave(nq // nkv, 1))
+    v = rows[2].transpose(1, 2).reshape(-1, nkv, hd)[:131 + q].double()
+    want = torch.einsum("hqk,khd->qhd", probabilities(rows, q, nq, nkv, hd), v.repeat_interleave(nq // nkv, 1))
     assert (out.double() - want).norm() <= 1e-6 * want.norm()
     assert (out.double() - want).abs().max() <= 1e-5
 
