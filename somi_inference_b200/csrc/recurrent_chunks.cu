@@ -7,7 +7,7 @@
 // Three kernels: U of every chunk and head; the states in front of every chunk, from U in place and in
 // order (and the last one to the request's slot); y.  Everything is float32: q and k are activated and rotated in float32 as they
 // are read, the powers of g are powf, and the products take every float32 operand as three bfloat16 numbers whose sum it
-// is (gemm_f32_split.cuh; v as it is, where it is not activated), summed in float32 by `tcgen05.mma`.
+// is (gemm_f32_split.cuh; v as it is, where it is not activated), summed in float32 by `tcgen05.mma`, 64 terms at a time.
 //
 // Why: step by step, a portion is one chain of rows per (head, 16 columns) with two sums over a warp each:
 // 224 CTAs for 28 heads of 128, 522 us for 2,048 rows behind 43 us of preparation.  In chunks nothing
@@ -201,11 +201,12 @@ struct ChFetchV {
     }
 };
 
-// Products of parts, the small ones first, in groups of K steps: `f(a's part, b's part, step, accumulate)`.  PB: 3, or 1 where b is bfloat16.
+// Products of parts, the small ones first, in groups of K steps: `f(a's part, b's part, step, accumulate)`, the first into an empty
+// accumulator.  PB: 3, or 1 where b is bfloat16.
 template <int PB, typename F>
-__device__ __forceinline__ void ch_products(int steps, bool fresh, F f) {
+__device__ __forceinline__ void ch_products(int steps, F f) {
     for (int j = 0; j < steps; ++j) {
-        f(2, 0, j, !(fresh && j == 0));
+        f(2, 0, j, j > 0);
         if (PB == 3) {
             f(0, 2, j, true);
             f(1, 1, j, true);
@@ -307,7 +308,7 @@ chunk_update_kernel(ChRows k, ChRows v, const float* __restrict__ decay, ChTiles
         mma.operands_ready();
         if (threadIdx.x == 0) {
             const uint64_t kd = t5::desc_mnmajor(smem_u32(ks), 64 * 128), vd = t5::desc_mnmajor(smem_u32(vs), 64 * 128);
-            ch_products<PV>(4, true, [&](int pk, int pv, int j, bool more) {
+            ch_products<PV>(4, [&](int pk, int pv, int j, bool more) {
                 t5::mma_ss(mma.tmem + i * D, vd + ((pv * PLANE + j * 16 * 128) >> 4), kd + ((pk * PLANE + j * 16 * 128) >> 4),
                            ch_idesc(D, true, true), more);
             });
@@ -395,15 +396,18 @@ __device__ float ch_value(const ChRows& m, int row, int c) {
     return low ? fmaf(x, t.x, -(other * t.y)) : fmaf(x, t.x, other * t.y);
 }
 
-// y of a chunk.  A CTA per (tile, head), two on an SM.  For 64 channels at a time q and k in parts, then the state over k: scores
-// q k^T and q S in two accumulators.  Then a thread takes half a row of scores, masks and decays them and writes
-// them as parts for their product with v, 64 keys at a time, into the scores' accumulator.
+// y of a chunk.  A CTA per (tile, head), two on an SM.  q S and scores q k^T, for 64 channels at a time; then a thread takes half
+// a row of scores, masks and decays them and writes them as parts for their product with v, 64 keys at a time.  Every sum
+// of 64 terms has an accumulator of its own and they are added in registers (gemm_f32_split.cuh says why: with 128 terms
+// in one, y of 28 heads of 128 was off by 6.6e-7, with 64 by 1.7e-7, as FMAs by 2.4e-7).  With 128 channels two of them fill
+// the CTA's half of tensor memory: so q S comes first, its two sums go to the state's own place, whose only reader this CTA is, and q's first
+// 64 channels are split once more for the scores.
 template <int D, bool SILU>
 __global__ void __launch_bounds__(kChThreads, 2)
 chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* __restrict__ decay,
-                     ChTiles tiles, const float* __restrict__ states, int heads, int group,
+                     ChTiles tiles, float* __restrict__ states, int heads, int group,
                      float* __restrict__ y) {
-    constexpr int PLANE = kChRows * 128, VPLANE = 64 * D * 2, PV = SILU ? 3 : 1;
+    constexpr int PLANE = kChRows * 128, VPLANE = 64 * D * 2, PV = SILU ? 3 : 1, PARTS = D / 64;
     extern __shared__ unsigned char ch_raw[];
     unsigned char* xs = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ch_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     unsigned char* ys = xs + 3 * PLANE;
@@ -426,24 +430,22 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
     k.p += static_cast<size_t>(h / group) * D;
     v.p += static_cast<size_t>(h) * D;
     if (threadIdx.x <= kChRows) pow_s[threadIdx.x] = powf(decay[h], static_cast<float>(threadIdx.x));
-    const float* st = states + (static_cast<size_t>(blockIdx.x) * heads + h) * D * D;
+    float* st = states + (static_cast<size_t>(blockIdx.x) * heads + h) * D * D;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, halves = rows > 64 ? 2 : 1;
-    const uint32_t scores = mma.tmem, carried = mma.tmem + 128;
+    const uint32_t first = mma.tmem, second = mma.tmem + 128;
     const uint64_t xd = t5::desc_kmajor(smem_u32(xs)), yd = t5::desc_kmajor(smem_u32(ys));
-    ChFetch<kChRows, 8, 2> f;
-    f.fetch({&q, &k}, row0, 0, rows, 0);
-    for (int i = 0; i < D / 64; ++i) {
-        if (i > 0) mma.wait();
-        f.template put<0, true>(xs, PLANE, q.silu, 0, [&](int) { return q_scale; });
-        f.template put<1, true>(ys, PLANE, k.silu, 0, [](int) { return 1.f; });
+    // xs (64 channels of q) by ys (of k or the state) into columns `to` on
+    auto multiply = [&](uint32_t to, int n) {
         mma.operands_ready();
         if (threadIdx.x == 0) {
-            ch_products<3>(4, i == 0, [&](int pa, int pb, int j, bool more) {
-                t5::mma_ss(scores, xd + ((pa * PLANE + j * 32) >> 4), yd + ((pb * PLANE + j * 32) >> 4), ch_idesc(kChRows, false, false), more);
+            ch_products<3>(4, [&](int pa, int pb, int j, bool more) {
+                t5::mma_ss(to, xd + ((pa * PLANE + j * 32) >> 4), yd + ((pb * PLANE + j * 32) >> 4), ch_idesc(n, false, false), more);
             });
             t5::commit(mma.bar);
         }
-        // the state's 64 key channels, in the same order
+    };
+    // the state's key channels 64 i .., in the order of q's; `ready` runs between the loads and the writes
+    auto put_state = [&](int i, auto ready) {
         constexpr int N = D / (kChThreads / 8);
         const int r0 = threadIdx.x / 8, pl = threadIdx.x % 8;
         bool turn;
@@ -456,7 +458,7 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
             a[n] = load4(p + c);
             b[n] = load4(p + c2);
         }
-        mma.wait();
+        ready();
 #pragma unroll
         for (int n = 0; n < N; ++n) {
             const int r = r0 + n * (kChThreads / 8);
@@ -467,26 +469,70 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
             for (int e = 0; e < 3; ++e)
                 *reinterpret_cast<uint4*>(ys + e * PLANE + r * 128 + ((pl ^ (r & 7)) << 4)) = make_uint4(pa[e].x, pa[e].y, pb[e].x, pb[e].y);
         }
-        if (i + 1 < D / 64) f.fetch({&q, &k}, row0, 0, rows, 8 * (i + 1));
-        mma.operands_ready();
-        if (threadIdx.x == 0) {
-            ch_products<3>(4, i == 0, [&](int pa, int pb, int j, bool more) {
-                t5::mma_ss(carried, xd + ((pa * PLANE + j * 32) >> 4), yd + ((pb * PLANE + j * 32) >> 4), ch_idesc(D, false, false), more);
-            });
-            t5::commit(mma.bar);
+    };
+    const int t = (warp & 3) * 32 + lane, s0 = (warp >> 2) * 64;         // the thread's row, its scores' first key
+    const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;
+    constexpr int COLS = D / 2, PITCH = COLS + 4;
+    const int col0 = (warp >> 2) * COLS;
+    ChFetch<kChRows, 8, 2> f;
+    float p[64];
+    if constexpr (PARTS == 1) {
+        f.fetch({&q, &k}, row0, 0, rows, 0);
+        f.template put<0, true>(xs, PLANE, q.silu, 0, [&](int) { return q_scale; });
+        f.template put<1, true>(ys, PLANE, k.silu, 0, [](int) { return 1.f; });
+        multiply(first, kChRows);
+        put_state(0, [&]() { mma.wait(); });
+        multiply(second, D);
+        t5::ld32(first + lanes + s0, p);
+        t5::ld32(first + lanes + s0 + 32, p + 32);
+    } else {
+        for (int i = 0; i < PARTS; ++i) {
+            ChFetch<kChRows, 8, 1> fq;
+            fq.fetch({&q}, row0, 0, rows, 8 * i);
+            put_state(i, [&]() { if (i > 0) mma.wait(); });
+            fq.template put<0, true>(xs, PLANE, q.silu, 0, [&](int) { return q_scale; });
+            multiply(i == 0 ? second : first, D);
         }
+        mma.wait();
+#pragma unroll
+        for (int c = 0; c < COLS; c += 32) {             // g^(t + 1) q S of this thread's row and half, where it finds it again
+            float a[32], b[32];
+            t5::ld32(second + lanes + col0 + c, a);
+            t5::ld32(first + lanes + col0 + c, b);
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) {
+                F4 z;
+#pragma unroll
+                for (int x = 0; x < 4; ++x) z.v[x] = (a[e + x] + b[e + x]) * pow_s[t + 1];
+                store4(st + ((c + e) / 4 * kChThreads + threadIdx.x) * 4, z);
+            }
+        }
+        ChFetch<kChRows, 8, 1> fk;
+        fk.fetch({&k}, row0, 0, rows, 8);                // (q's second half is there)
+        fk.template put<0, true>(ys, PLANE, k.silu, 0, [](int) { return 1.f; });
+        multiply(first, kChRows);
+        f.fetch({&q, &k}, row0, 0, rows, 0);
+        mma.wait();
+        f.template put<0, true>(xs, PLANE, q.silu, 0, [&](int) { return q_scale; });
+        f.template put<1, true>(ys, PLANE, k.silu, 0, [](int) { return 1.f; });
+        multiply(second, kChRows);
     }
     ChFetchV<D, SILU> fv;
     fv.fetch(v, row0, 0, rows);
-    // a row's scores of keys 64 (warp / 4) .., while the last MMAs run
-    const int t = (warp & 3) * 32 + lane, s0 = (warp >> 2) * 64;
-    const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;
-    float p[64];
-    t5::ld32(scores + lanes + s0, p);
-    t5::ld32(scores + lanes + s0 + 32, p + 32);
+    mma.wait();                                           // q and the state or keys have been read
+    if constexpr (PARTS == 2) {
+#pragma unroll
+        for (int c = 0; c < 64; c += 32) {
+            float b[32];
+            t5::ld32(second + lanes + s0 + c, p + c);
+            t5::ld32(first + lanes + s0 + c, b);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) p[c + e] += b[e];
+        }
+    }
 #pragma unroll
     for (int s = 0; s < 64; ++s) p[s] = s0 + s <= t ? p[s] * pow_s[max(t - s0 - s, 0)] : 0.f;
-    mma.wait();                                           // q and the state have been read
+    constexpr uint32_t NEXT = D;                          // columns from the first keys' accumulator to the others'
     for (int i = 0; i < halves; ++i) {
         if (i > 0) mma.wait();
         if (warp >> 2 == i) {
@@ -507,25 +553,39 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
         mma.operands_ready();
         if (threadIdx.x == 0) {
             const uint64_t vd = t5::desc_mnmajor(smem_u32(ys), 64 * 128);
-            ch_products<PV>(4, i == 0, [&](int pa, int pb, int j, bool more) {
-                t5::mma_ss(scores, xd + ((pa * PLANE + j * 32) >> 4), vd + ((pb * VPLANE + j * 16 * 128) >> 4), ch_idesc(D, false, true), more);
+            ch_products<PV>(4, [&](int pa, int pb, int j, bool more) {
+                t5::mma_ss(first + i * NEXT, xd + ((pa * PLANE + j * 32) >> 4), vd + ((pb * VPLANE + j * 16 * 128) >> 4), ch_idesc(D, false, true), more);
             });
             t5::commit(mma.bar);
         }
     }
     mma.wait();
     // y = g^(t + 1) q S + P v: half of a row's columns a thread, through shared memory to whole rows
-    constexpr int COLS = D / 2, PITCH = COLS + 4;
-    const int col0 = (warp >> 2) * COLS;
     float* own = reinterpret_cast<float*>(xs) + warp * 32 * PITCH;
     const uint32_t odd = odd_s[0] | odd_s[1] | odd_s[2] | odd_s[3];
 #pragma unroll
     for (int c = 0; c < COLS; c += 32) {
-        float o[32], z[32];
-        t5::ld32(scores + lanes + col0 + c, o);
-        t5::ld32(carried + lanes + col0 + c, z);
+        float o[32];
+        t5::ld32(first + lanes + col0 + c, o);
+        if (halves > 1) {
+            float z[32];
+            t5::ld32(first + NEXT + lanes + col0 + c, z);
 #pragma unroll
-        for (int e = 0; e < 32; ++e) o[e] = fmaf(z[e], pow_s[t + 1], o[e]);
+            for (int e = 0; e < 32; ++e) o[e] += z[e];
+        }
+        if constexpr (PARTS == 1) {
+            float z[32];
+            t5::ld32(second + lanes + col0 + c, z);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] = fmaf(z[e], pow_s[t + 1], o[e]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) {
+                const F4 z = load4(st + ((c + e) / 4 * kChThreads + threadIdx.x) * 4);
+#pragma unroll
+                for (int x = 0; x < 4; ++x) o[e + x] += z.v[x];
+            }
+        }
 #pragma unroll
         for (int e = 0; e < 32; e += 4)
             *reinterpret_cast<float4*>(own + lane * PITCH + c + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);

@@ -35,6 +35,34 @@ def test_rows_around_tiles_and_chunks(ops, d, silu):
         assert (got - want).norm() <= 1e-6 * want.norm() and (got - want).abs().max() <= 2e-5 * want.abs().max()
 
 
+@pytest.mark.parametrize("d,silu", [(64, False), (64, True), (128, False), (128, True)])
+def test_error_against_64_bits(ops, d, silu):
+    """Slow decays, so that all rows of a chunk and the state count.  y passes three sums (scores, q S, P v) of chains of 64
+    terms, each off by up to 6.5e-8, all of it towards zero, and their sums over 128 terms and the state's roundings add as much as
+    one of them; 128 terms in one chain were off by 5.9e-7 to 6.8e-7 with 128 channels."""
+    H, T = 3, 300
+    g = torch.Generator().manual_seed(d)
+    x = (1.2 * torch.randn(T, 3 * H * d, generator=g)).bfloat16().cuda()
+    decay, first = torch.tensor([1 - 2.0 ** -5, 1 - 2.0 ** -8, 1 - 2.0 ** -12], device="cuda"), torch.randn(H, d, d, generator=g).cuda() * 3
+    steps = Steps(ops, 1, state=StateNeeds({"s": ((H, d, d), torch.float32)}), dtype=torch.bfloat16)
+    batch, _ = steps.step({0: T})
+    y, state = torch.empty(T, H * d, device="cuda"), steps.mgr.view(0).state["s"]
+    slot = int(batch.host.state_slot[0])
+    state[slot] = first
+    parts = x[:, :H * d], x[:, H * d:2 * H * d], x[:, 2 * H * d:]
+    ops.matrix_state_scan(*parts, state, batch, y, H, H, d, d, act_silu=silu, decay=decay, q_scale=0.25)
+    ops.check_errors()
+    q, k, v = (t.double().view(T, H, d) for t in parts)
+    if silu:
+        q, k, v = (torch.nn.functional.silu(t) for t in (q, k, v))
+    m, want = first.double().transpose(1, 2), torch.empty(T, H, d, dtype=torch.float64, device="cuda")
+    for t in range(T):
+        m = decay.double()[:, None, None] * m + k[t][:, :, None] * v[t][:, None, :]
+        want[t] = torch.einsum("hk,hkv->hv", q[t] * 0.25, m)
+    for got, ref in ((y.view(T, H, d), want), (state[slot].transpose(1, 2), m)):
+        assert (got.double() - ref).norm() <= 2.6e-7 * ref.norm()
+
+
 @pytest.mark.parametrize("d,silu", [(64, True), (128, False), (128, True)])
 @pytest.mark.parametrize("what", ["v", "k", "q"])
 def test_what_is_not_finite_reaches_the_rows_that_see_it(ops, d, silu, what):
