@@ -27,7 +27,6 @@ namespace somi {
 constexpr int kChRows = 128;          // rows per chunk: two tiles of the tile list, the MMA's M
 constexpr int kChTile = 64;
 constexpr int kChThreads = 256;
-constexpr int kChHalf = 64;           // rows or channels of one swizzled tile's other side: 128 bytes
 
 __device__ int g_chunks_error = 0;
 
@@ -96,6 +95,21 @@ __device__ __forceinline__ void ch_split(const F4& u, uint2 (&part)[3]) {
     fs_split(u.v[2], u.v[3], part[0].y, part[1].y, part[2].y);
 }
 
+// Numbers of row r that have no parts (an MMA would carry what they are to rows that do not see them): 0 in their place, and
+// the row noted.
+__device__ __forceinline__ void ch_leave_out(F4& u, F4& v, int r, uint32_t* odd) {
+    float most = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) most = fs_largest(fs_largest(most, u.v[e]), v.v[e]);
+    if (fs_has_parts(most)) return;
+    atomicOr(odd + (r >> 5), 1u << (r & 31));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (!fs_has_parts(u.v[e])) u.v[e] = 0.f;
+        if (!fs_has_parts(v.v[e])) v.v[e] = 0.f;
+    }
+}
+
 // What a thread reads of ROWS rows of one or two matrices (q and k turn by the same angles): pair `pl` of every APART-th row.
 // Fetched a phase before it is used, so that the loads run under the MMAs of the phase before.
 template <int ROWS, int PAIRS, int MATS>
@@ -131,9 +145,9 @@ struct ChFetch {
     }
     // The parts of matrix K times factor(row).  FLAT: tiles of [ROWS][8 pairs], a pair's eight numbers together: 64 channels in
     // an order that q, k and the state share, for products over channels.  Else tiles of [ROWS][64 channels] in the rows'
-    // order, a block of 64 channels behind the other.
+    // order, a block of 64 channels behind the other, and numbers that have no parts are left out, their rows noted in `odd`.
     template <int K, bool FLAT, typename F>
-    __device__ __forceinline__ void put(unsigned char* dst, int plane, int silu, int at, F factor) const {
+    __device__ __forceinline__ void put(unsigned char* dst, int plane, int silu, int at, F factor, uint32_t* odd = nullptr) const {
         static_assert(!FLAT || PAIRS == 8, "64 channels");
         const int pl = threadIdx.x % PAIRS;
 #pragma unroll
@@ -141,6 +155,7 @@ struct ChFetch {
             const int rl = threadIdx.x / PAIRS + i * APART;
             F4 u, v;
             ch_values(x[K][i], o[K][i], turn, a[i], b[i], silu, factor(at + rl), u, v);
+            if (!FLAT) ch_leave_out(u, v, at + rl, odd);
             uint2 pu[3], pv[3];
             ch_split(u, pu);
             ch_split(v, pv);
@@ -160,8 +175,8 @@ struct ChFetch {
         }
     }
 };
-// 64 rows of v from row `at` on, to tiles of [64][64 channels]: as they are, or (SILU) three parts.  A number that is
-// not finite is left out (an MMA would carry it to rows that do not see it) and its row noted in `odd`, if that is given.
+// 64 rows of v from row `at` on, to tiles of [64][64 channels]: as they are, or (SILU) three parts.  Numbers that have no
+// parts are left out and their rows noted in `odd`.
 template <int D, bool SILU>
 struct ChFetchV {
     static constexpr int ACROSS = D / 4, APART = kChThreads / ACROSS, N = 64 / APART;
@@ -179,19 +194,12 @@ struct ChFetchV {
 #pragma unroll
         for (int i = 0; i < N; ++i) {
             const int rl = threadIdx.x / ACROSS + i * APART;
-            F4 u = load4(reinterpret_cast<const __nv_bfloat16*>(&x[i]));
-            bool fine = true;
+            F4 u = load4(reinterpret_cast<const __nv_bfloat16*>(&x[i])), none{{0.f, 0.f, 0.f, 0.f}};
+            if (SILU) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (SILU) u.v[e] = ch_silu(u.v[e]);
-                fine &= fs_finite(u.v[e]);
+                for (int e = 0; e < 4; ++e) u.v[e] = ch_silu(u.v[e]);
             }
-            if (!fine && odd != nullptr) {
-                atomicOr(odd + ((at + rl) >> 5), 1u << ((at + rl) & 31));
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (!fs_finite(u.v[e])) u.v[e] = 0.f;
-            }
+            ch_leave_out(u, none, at + rl, odd);
             uint2 part[3];
             ch_split(u, part);
             unsigned char* to = dst + c / 64 * (64 * 128) + rl * 128 + (((c & 63) >> 3 ^ (rl & 7)) << 4) + (c & 4) * 2;
@@ -265,6 +273,30 @@ struct ChMma {
     }
 };
 
+// The way of numbers without parts, as FMAs: one channel of a row, activated and turned; q_row k_row or q_row S.
+__device__ __forceinline__ float ch_value(const ChRows& m, int row, int c) {
+    const __nv_bfloat16* p = m.p + static_cast<size_t>(row) * m.stride;
+    float x = __bfloat162float(p[c]);
+    if (m.silu) x = ch_silu(x);
+    if (m.cs == nullptr || c >= 2 * m.half) return x;
+    const bool low = c < m.half;
+    const float other = __bfloat162float(p[low ? c + m.half : c - m.half]);
+    const float2 t = m.cs[static_cast<size_t>(row) * m.half + (low ? c : c - m.half)];
+    return low ? fmaf(x, t.x, -(other * t.y)) : fmaf(x, t.x, other * t.y);
+}
+__device__ __forceinline__ float ch_dot(const ChRows& q, int row, float q_scale, const ChRows& k, int k_row, int channels) {
+    float dot = 0.f;
+#pragma unroll 1
+    for (int c = 0; c < channels; ++c) dot = fmaf(ch_value(q, row, c) * q_scale, ch_value(k, k_row, c), dot);
+    return dot;
+}
+__device__ __forceinline__ float ch_dot(const ChRows& q, int row, float q_scale, const float* state, int channels) {
+    float dot = 0.f;
+#pragma unroll 1
+    for (int c = 0; c < channels; ++c) dot = fmaf(ch_value(q, row, c) * q_scale, state[c], dot);
+    return dot;
+}
+
 // U [tile][head][value channel][key channel].  A CTA per (tile, head), two on an SM: 64 rows at a time, k in parts and v; D = V^T K with
 // the rows as the products' K, both operands as the rows lie; the halves' sums in two accumulators.
 template <int D, bool SILU>
@@ -276,6 +308,7 @@ chunk_update_kernel(ChRows k, ChRows v, const float* __restrict__ decay, ChTiles
     unsigned char* vs = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ch_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     unsigned char* ks = vs + PV * PLANE;                  // (with 64 channels an MMA reads 64 more of v: into k, and not used)
     __shared__ float pow_s[kChRows];
+    __shared__ uint32_t odd_s[kChRows / 32];
     __shared__ __align__(8) unsigned long long bar_s;
     __shared__ uint32_t tmem_s;
     pdl_launch_dependents();
@@ -286,6 +319,7 @@ chunk_update_kernel(ChRows k, ChRows v, const float* __restrict__ decay, ChTiles
         return;
     }
     ChMma mma;
+    if (threadIdx.x < kChRows / 32) odd_s[threadIdx.x] = 0;
     mma.start(&bar_s, &tmem_s);
     pdl_wait();
     if (threadIdx.x < kChRows) pow_s[threadIdx.x] = powf(decay[h], static_cast<float>(threadIdx.x));
@@ -299,8 +333,8 @@ chunk_update_kernel(ChRows k, ChRows v, const float* __restrict__ decay, ChTiles
     fv.fetch(v, row0, 0, rows);
     for (int i = 0; i < halves; ++i) {
         if (i > 0) mma.wait();                            // the first half's operands have been read
-        fv.put(vs, PLANE, 64 * i, nullptr);
-        fk.template put<0, false>(ks, PLANE, k.silu, 64 * i, [&](int r) { return pow_s[max(rows - 1 - r, 0)]; });
+        fv.put(vs, PLANE, 64 * i, odd_s);
+        fk.template put<0, false>(ks, PLANE, k.silu, 64 * i, [&](int r) { return pow_s[max(rows - 1 - r, 0)]; }, odd_s);
         if (i + 1 < halves) {
             fk.fetch({&k}, row0, 64, rows, 0);
             fv.fetch(v, row0, 64, rows);
@@ -335,6 +369,19 @@ chunk_update_kernel(ChRows k, ChRows v, const float* __restrict__ decay, ChTiles
 #pragma unroll
             for (int e = 0; e < 32; e += 4)
                 *reinterpret_cast<float4*>(own + lane * PITCH + c + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
+        }
+        if (odd_s[0] | odd_s[1] | odd_s[2] | odd_s[3]) {
+            const int c_v = (warp & 3) * 32 + lane;
+#pragma unroll 1
+            for (int s = 0; s < rows; ++s) {
+                if (!(odd_s[s >> 5] >> (s & 31) & 1)) continue;
+                const float x = ch_value(v, row0 + s, c_v);
+#pragma unroll 1
+                for (int c = 0; c < COLS; ++c) {
+                    const float z = ch_value(k, row0 + s, (warp >> 2) * COLS + c) * pow_s[rows - 1 - s];
+                    if (!fs_has_parts(x) || !fs_has_parts(z)) own[lane * PITCH + c] = fmaf(z, x, own[lane * PITCH + c]);
+                }
+            }
         }
         __syncwarp();
         float* dst = u + (static_cast<size_t>(blockIdx.x) * heads + h) * D * D + (warp & 3) * 32 * D + (warp >> 2) * COLS;
@@ -384,28 +431,15 @@ chunk_states_kernel(float* __restrict__ u, const float* __restrict__ decay, cons
     store4(own, s);
 }
 
-// One channel of a row, activated and turned (the way of numbers that are not finite).
-__device__ float ch_value(const ChRows& m, int row, int c) {
-    const __nv_bfloat16* p = m.p + static_cast<size_t>(row) * m.stride;
-    float x = __bfloat162float(p[c]);
-    if (m.silu) x = ch_silu(x);
-    if (m.cs == nullptr || c >= 2 * m.half) return x;
-    const bool low = c < m.half;
-    const float other = __bfloat162float(p[low ? c + m.half : c - m.half]);
-    const float2 t = m.cs[static_cast<size_t>(row) * m.half + (low ? c : c - m.half)];
-    return low ? fmaf(x, t.x, -(other * t.y)) : fmaf(x, t.x, other * t.y);
-}
-
 // y of a chunk.  A CTA per (tile, head), two on an SM.  q S and scores q k^T, for 64 channels at a time; then a thread takes half
 // a row of scores, masks and decays them and writes them as parts for their product with v, 64 keys at a time.  Every sum
 // of 64 terms has an accumulator of its own and they are added in registers (gemm_f32_split.cuh says why: with 128 terms
 // in one, y of 28 heads of 128 was off by 6.6e-7, with 64 by 1.7e-7, as FMAs by 2.4e-7).  With 128 channels two of them fill
-// the CTA's half of tensor memory: so q S comes first, its two sums go to the state's own place, whose only reader this CTA is, and q's first
-// 64 channels are split once more for the scores.
+// the CTA's half of tensor memory: so q S comes first, its two sums wait in y, and q's first 64 channels are split once more for the scores.
 template <int D, bool SILU>
 __global__ void __launch_bounds__(kChThreads, 2)
 chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* __restrict__ decay,
-                     ChTiles tiles, float* __restrict__ states, int heads, int group,
+                     ChTiles tiles, const float* __restrict__ states, int heads, int group,
                      float* __restrict__ y) {
     constexpr int PLANE = kChRows * 128, VPLANE = 64 * D * 2, PV = SILU ? 3 : 1, PARTS = D / 64;
     extern __shared__ unsigned char ch_raw[];
@@ -430,7 +464,7 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
     k.p += static_cast<size_t>(h / group) * D;
     v.p += static_cast<size_t>(h) * D;
     if (threadIdx.x <= kChRows) pow_s[threadIdx.x] = powf(decay[h], static_cast<float>(threadIdx.x));
-    float* st = states + (static_cast<size_t>(blockIdx.x) * heads + h) * D * D;
+    const float* st = states + (static_cast<size_t>(blockIdx.x) * heads + h) * D * D;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, halves = rows > 64 ? 2 : 1;
     const uint32_t first = mma.tmem, second = mma.tmem + 128;
     const uint64_t xd = t5::desc_kmajor(smem_u32(xs)), yd = t5::desc_kmajor(smem_u32(ys));
@@ -473,7 +507,9 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
     const int t = (warp & 3) * 32 + lane, s0 = (warp >> 2) * 64;         // the thread's row, its scores' first key
     const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;
     constexpr int COLS = D / 2, PITCH = COLS + 4;
-    const int col0 = (warp >> 2) * COLS;
+    const int col0 = (warp >> 2) * COLS, live = rows - (warp & 3) * 32;  // (of the warp's 32 rows)
+    float* dst = y + static_cast<size_t>(row0 + (warp & 3) * 32) * heads * D + static_cast<size_t>(h) * D + col0;
+    bool fine = true;
     ChFetch<kChRows, 8, 2> f;
     float p[64];
     if constexpr (PARTS == 1) {
@@ -494,21 +530,33 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
             multiply(i == 0 ? second : first, D);
         }
         mma.wait();
+        constexpr int WIDE = 32 + 4;
+        float* turn_s = reinterpret_cast<float*>(ys) + warp * 32 * WIDE;
 #pragma unroll
-        for (int c = 0; c < COLS; c += 32) {             // g^(t + 1) q S of this thread's row and half, where it finds it again
-            float a[32], b[32];
+        for (int c = 0; c < COLS; c += 32) {             // g^(t + 1) q S of this thread's row and half, to y
+            float a[32], b[32], most = 0.f;
             t5::ld32(second + lanes + col0 + c, a);
             t5::ld32(first + lanes + col0 + c, b);
 #pragma unroll
-            for (int e = 0; e < 32; e += 4) {
-                F4 z;
-#pragma unroll
-                for (int x = 0; x < 4; ++x) z.v[x] = (a[e + x] + b[e + x]) * pow_s[t + 1];
-                store4(st + ((c + e) / 4 * kChThreads + threadIdx.x) * 4, z);
+            for (int e = 0; e < 32; ++e) {
+                a[e] = (a[e] + b[e]) * pow_s[t + 1];
+                most = fs_largest(most, a[e]);
             }
+            fine &= fs_finite(most);
+#pragma unroll
+            for (int e = 0; e < 32; e += 4)
+                *reinterpret_cast<float4*>(turn_s + lane * WIDE + e) = make_float4(a[e], a[e + 1], a[e + 2], a[e + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int i = lane; i < 32 * 8; i += 32)
+                if (i / 8 < live)
+                    *reinterpret_cast<float4*>(dst + static_cast<size_t>(i / 8) * heads * D + c + i % 8 * 4) =
+                        *reinterpret_cast<const float4*>(turn_s + i / 8 * WIDE + i % 8 * 4);
+            __syncwarp();
         }
         ChFetch<kChRows, 8, 1> fk;
         fk.fetch({&k}, row0, 0, rows, 8);                // (q's second half is there)
+        __syncthreads();
         fk.template put<0, true>(ys, PLANE, k.silu, 0, [](int) { return 1.f; });
         multiply(first, kChRows);
         f.fetch({&q, &k}, row0, 0, rows, 0);
@@ -563,6 +611,7 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
     // y = g^(t + 1) q S + P v: half of a row's columns a thread, through shared memory to whole rows
     float* own = reinterpret_cast<float*>(xs) + warp * 32 * PITCH;
     const uint32_t odd = odd_s[0] | odd_s[1] | odd_s[2] | odd_s[3];
+    float most = 0.f;
 #pragma unroll
     for (int c = 0; c < COLS; c += 32) {
         float o[32];
@@ -578,39 +627,48 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
             t5::ld32(second + lanes + col0 + c, z);
 #pragma unroll
             for (int e = 0; e < 32; ++e) o[e] = fmaf(z[e], pow_s[t + 1], o[e]);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 32; e += 4) {
-                const F4 z = load4(st + ((c + e) / 4 * kChThreads + threadIdx.x) * 4);
-#pragma unroll
-                for (int x = 0; x < 4; ++x) o[e + x] += z.v[x];
-            }
         }
+#pragma unroll
+        for (int e = 0; e < 32; ++e) most = fs_largest(most, o[e]);
 #pragma unroll
         for (int e = 0; e < 32; e += 4)
             *reinterpret_cast<float4*>(own + lane * PITCH + c + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
     }
-    if (odd != 0 && t < rows) {                           // values that are not finite: to the rows that see them
+    fine &= fs_finite(most);
+    // what v left out goes to the rows that see it; what came out infinite or NaN is summed again, as FMAs
+    if ((odd != 0 || !fine) && t < rows) {
+        float* mine = own + lane * PITCH;
+        float* carried = dst + static_cast<size_t>(lane) * heads * D;
+        unsigned long long again = 0;
+#pragma unroll 1
+        for (int c = 0; c < COLS; ++c) {
+            if (fs_finite(mine[c]) && (PARTS == 1 || fs_finite(carried[c]))) continue;
+            again |= 1ull << c;
+            const float z = ch_dot(q, row0 + t, q_scale, st + (col0 + c) * D, D) * pow_s[t + 1];
+            mine[c] = PARTS == 1 ? z : 0.f;
+            if (PARTS == 2) carried[c] = z;
+        }
 #pragma unroll 1
         for (int s = 0; s <= t; ++s) {
-            if (!(odd_s[s >> 5] >> (s & 31) & 1)) continue;
-            float dot = 0.f;
-            for (int c = 0; c < D; ++c) dot = fmaf(ch_value(q, row0 + t, c) * q_scale, ch_value(k, row0 + s, c), dot);
-            dot *= pow_s[t - s];
+            const bool left_out = odd_s[s >> 5] >> (s & 31) & 1;
+            if (again == 0 && !left_out) continue;
+            const float score = ch_dot(q, row0 + t, q_scale, k, row0 + s, D) * pow_s[t - s];
+#pragma unroll 1
             for (int c = 0; c < COLS; ++c) {
                 const float x = ch_value(v, row0 + s, col0 + c);
-                if (!fs_finite(x)) own[lane * PITCH + c] = fmaf(dot, x, own[lane * PITCH + c]);
+                if ((again >> c & 1) || (left_out && !fs_has_parts(x))) mine[c] = fmaf(score, x, mine[c]);
             }
         }
     }
     __syncwarp();
-    float* dst = y + static_cast<size_t>(row0 + (warp & 3) * 32) * heads * D + static_cast<size_t>(h) * D + col0;
-    const int live = rows - (warp & 3) * 32;
 #pragma unroll 4
     for (int i = lane; i < 32 * (COLS / 4); i += 32) {
         const int r = i / (COLS / 4), c = i % (COLS / 4) * 4;
-        if (r < live)
-            *reinterpret_cast<float4*>(dst + static_cast<size_t>(r) * heads * D + c) = *reinterpret_cast<const float4*>(own + r * PITCH + c);
+        if (r >= live) continue;
+        float4 o = *reinterpret_cast<const float4*>(own + r * PITCH + c);
+        float4* to = reinterpret_cast<float4*>(dst + static_cast<size_t>(r) * heads * D + c);
+        if (PARTS == 2) o = make_float4(o.x + to->x, o.y + to->y, o.z + to->z, o.w + to->w);
+        *to = o;
     }
     mma.end();
 }

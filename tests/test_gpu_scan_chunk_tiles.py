@@ -1,5 +1,7 @@
 """The recurrence in chunks of 128 rows at the bounds of its tiles of 64 rows and of its chunks, and the norm of parts behind it."""
 
+import math
+
 import pytest
 import torch
 
@@ -82,6 +84,77 @@ def test_what_is_not_finite_reaches_the_rows_that_see_it(ops, d, silu, what):
             assert not z[at:, :d].isfinite().any() and torch.equal(u[0, :, :, 6:], s[0, :, :, 6:])
         else:
             assert not z[at, :d].isfinite().any() and torch.equal(z[at + 1:], y[at + 1:]) and torch.equal(u, s)
+
+
+def same_kind(got, want):
+    """The same infinities and NaN, and finite numbers as near as float32 sums are."""
+    fine = want.isfinite()
+    assert torch.equal(got.isfinite(), fine) and torch.equal(got[~fine].nan_to_num(0, 1, -1), want[~fine].nan_to_num(0, 1, -1))
+    assert (got - want)[fine].norm() <= 1e-6 * want[fine].norm()
+
+
+@pytest.mark.parametrize("d,silu", [(64, False), (64, True), (128, False), (128, True)])
+@pytest.mark.parametrize("what", ["k", "v", "both"])
+def test_states_of_infinite_inputs(ops, d, silu, what):
+    """Infinities in k and v of rows 3, 70 and 200 leave infinities of the products' signs in the state (NaN where they
+    meet zeros or each other), as step by step."""
+    H, T = 2, 300
+    x = torch.randn(T, 3 * H * d, generator=torch.Generator().manual_seed(2)).bfloat16().cuda()
+    for at, value in ((3, float("inf")), (70, float("-inf")), (200, float("inf"))):
+        if what != "v":
+            x[at, H * d + 5 + at % 7] = value
+        if what != "k":
+            x[at, 2 * H * d + 9 + at % 5] = value
+    (_, got), (_, want) = run(ops, x, [T], H, d, silu), run(ops, x, [T], H, d, silu, prepare=True)
+    assert want.isinf().any()
+    same_kind(got, want)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_infinities_of_an_earlier_state(ops, d):
+    """One infinity and one NaN a head in the state that earlier rows left: every row's y has them with q's sign, as step by step."""
+    H, T = 2, 300
+    g = torch.Generator().manual_seed(3)
+    x, decay = torch.randn(T, 3 * H * d, generator=g).bfloat16().cuda(), torch.tensor([0.99, 0.9], device="cuda")
+    out = []
+    for prepare in (None, True):
+        steps = Steps(ops, 1, state=StateNeeds({"s": ((H, d, d), torch.float32)}), dtype=torch.bfloat16)
+        batch, _ = steps.step({0: T})
+        state, y = steps.mgr.view(0).state["s"], torch.empty(T, H * d, device="cuda")
+        slot = int(batch.host.state_slot[0])
+        state[slot, :, 7, 11], state[slot, 0, d - 3, 1], state[slot, 1, 2, d - 2] = float("inf"), float("-inf"), float("nan")
+        ops.matrix_state_scan(x[:, :H * d], x[:, H * d:2 * H * d], x[:, 2 * H * d:], state, batch, y, H, H, d, d, decay=decay, prepare=prepare)
+        out.append((y.double(), state[slot].double()))
+    assert (out[1][0] == float("inf")).any() and (out[1][0] == float("-inf")).any()
+    for got, want in zip(*out):
+        same_kind(got, want)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_a_turned_key_without_parts(ops, d):
+    """A key that the rotation leaves between what bfloat16 and what float32 holds, and small values beside it: y and the state are
+    finite, as step by step."""
+    H, T, at = 2, 300, 150
+    g = torch.Generator().manual_seed(4)
+    x = torch.randn(T, 3 * H * d, generator=g).bfloat16()
+    large = torch.tensor(3.1e38).bfloat16()
+    freq = torch.zeros(d // 2, dtype=torch.float64)
+    freq[5] = (math.asin(3.4e38 / float(large) / 2 ** 0.5) - math.pi / 4) / at        # (cos + sin) large = 3.4e38
+    x[at, H * d + 5], x[at, H * d + 5 + d // 2] = large, large
+    x[at, 2 * H * d:] *= 0.01
+    x = x.cuda()
+    out = []
+    for prepare in (None, True):
+        steps = Steps(ops, 1, state=StateNeeds({"s": ((H, d, d), torch.float32)}), dtype=torch.bfloat16)
+        batch, _ = steps.step({0: T})
+        state, y = steps.mgr.view(0).state["s"], torch.empty(T, H * d, device="cuda")
+        ops.matrix_state_scan(x[:, :H * d], x[:, H * d:2 * H * d], x[:, 2 * H * d:], state, batch, y, H, H, d, d, q_scale=1e-3,
+                              decay=torch.tensor([0.99, 0.9], device="cuda"), rotary=(batch.positions, freq.cuda(), d), prepare=prepare)
+        out.append((y.double(), state[int(batch.host.state_slot[0])].double()))
+    assert all(t.isfinite().all() for pair in out for t in pair) and out[1][1].abs().max() > 1e35
+    for got, want in zip(*out):
+        same_kind(got, want)
+    assert (out[0][0] - out[1][0])[:at].norm() <= 1e-6 * out[1][0][:at].norm()
 
 
 @pytest.mark.parametrize("T", [1, 3, 41, 400])
