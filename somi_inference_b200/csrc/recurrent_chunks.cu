@@ -718,7 +718,7 @@ SOMI_API int somi_matrix_state_chunks(const void* q, const void* k, const void* 
         return SOMI_ERR_UNSUPPORTED;
     if ((D != 64 && D != 128) || heads <= 0 || heads > 65535 || n_req > 65535 || group <= 0 || heads % group ||
         ((q_stride | k_stride | v_stride) & 3) || (bits & 7) || rot < 0 || rot > D || rot % 8 || (rot > 0 && (silu & 1)) ||
-        ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(u)) & 15) || (reinterpret_cast<uintptr_t>(angles) & 15))
+        ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(y)) & 15) || (reinterpret_cast<uintptr_t>(angles) & 15))
         return SOMI_ERR_UNSUPPORTED;
     float2* cs = rot > 0 ? reinterpret_cast<float2*>(angles) : nullptr;
     const int half = rot / 2, n = n_rows * half;

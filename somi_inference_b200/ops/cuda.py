@@ -1765,8 +1765,8 @@ class CudaOps:
             _check(pos, freq)
             assert pos.dtype == torch.int32 and freq.dtype == torch.float64 and freq.numel() >= rot // 2
         runs = ((0, batch.num_requests, 0),)
-        if prepare is None and self.scan_in_chunks(q, k, v, batch, heads, qk_heads, dk, dv, act_silu, unit_eps, beta,
-                                                   decay_logits, rotary):
+        if prepare is None and y.data_ptr() % 16 == 0 and self.scan_in_chunks(
+                q, k, v, batch, heads, qk_heads, dk, dv, act_silu, unit_eps, beta, decay_logits, rotary):
             runs = self.scan_runs(batch, heads, dk)
         for run in runs:
             if run[2]:

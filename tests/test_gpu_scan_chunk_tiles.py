@@ -157,6 +157,22 @@ def test_a_turned_key_without_parts(ops, d):
     assert (out[0][0] - out[1][0])[:at].norm() <= 1e-6 * out[1][0][:at].norm()
 
 
+def test_rows_that_cannot_be_stored_sixteen_bytes_at_a_time(ops):
+    """The chunks' kernels store y four floats at a time: a y that stands between goes step by step."""
+    H, d, T = 2, 64, 200
+    x = torch.randn(T, 3 * H * d, generator=torch.Generator().manual_seed(6)).bfloat16().cuda()
+    parts, decay, out = (x[:, :H * d], x[:, H * d:2 * H * d], x[:, 2 * H * d:]), torch.tensor([0.99, 0.9], device="cuda"), []
+    for offset, prepare in ((1, None), (0, True)):
+        steps = Steps(ops, 1, state=StateNeeds({"s": ((H, d, d), torch.float32)}), dtype=torch.bfloat16)
+        batch, _ = steps.step({0: T})
+        y = torch.zeros(T * H * d + 8, device="cuda")
+        state = steps.mgr.view(0).state["s"]
+        ops.matrix_state_scan(*parts, state, batch, y[offset:offset + T * H * d].view(T, H * d), H, H, d, d, decay=decay, prepare=prepare)
+        assert not y[:offset].any() and not y[offset + T * H * d:].any()
+        out.append((y[offset:offset + T * H * d], state))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
 @pytest.mark.parametrize("T", [1, 3, 41, 400])
 @pytest.mark.parametrize("groups,n", [(14, 64), (28, 128), (5, 32), (3, 48), (2, 256)])
 def test_norm_of_parts(ops, T, groups, n):

@@ -88,11 +88,12 @@ def test_the_chunks_launcher_refuses_null_arguments():
     lib = ctypes.CDLL(build(verbose=False))
     at = P(1 << 16)
 
-    def call(decay=at, positions=at, freq=at, angles=at, rot=16):
+    def call(decay=at, positions=at, freq=at, angles=at, rot=16, y=at):
         return lib.somi_matrix_state_chunks(at, at, at, L(256), L(256), L(256), I(0), F(1), decay, at, at, at, at, I(1), I(1),
-                                            I(64), I(2), I(1), I(64), positions, freq, I(rot), angles, at, at, I(0), P(0))
+                                            I(64), I(2), I(1), I(64), positions, freq, I(rot), angles, at, y, I(0), P(0))
     assert call(decay=P(0)) == call(decay=P(0), rot=0) == cuda.ERR_UNSUPPORTED
     assert call(positions=P(0)) == call(freq=P(0)) == call(angles=P(0)) == cuda.ERR_UNSUPPORTED
+    assert call(y=P((1 << 16) + 4)) == cuda.ERR_UNSUPPORTED          # (rows are stored 16 bytes at a time)
 
 
 @pytest.mark.parametrize("n,nq,nkv,hd,positions,window", [(64, 40, 8, 128, 32768, None), (64, 40, 8, 128, 32768, 1024),
