@@ -76,12 +76,14 @@ struct FsArgs {
     long long ldx, ldy, bsx, bsw, bsy;
 };
 
+constexpr long long kFsMostApart = 0x7fffffffll / 144;
+
 // Whether this way takes the product: from 512 terms on (64 terms in one chain have an error of 6.5e-8 here and of 4.4e-8
 // as FMAs, 256 terms 7.4e-8 and 7.7e-8), up to what a cluster's shared memory holds of a row's blocks, with outputs for at
-// least half a tile, and rows that can be read 16 bytes at a time.  Never by the number of rows: a row's bits must
-// not depend on it.
+// least half a tile, and rows that can be read 16 bytes at a time and lie no more than `kFsMostApart` floats apart (a tile's
+// are found by 32-bit offsets).  Never by the number of rows: a row's bits must not depend on it.
 inline bool fs_takes(const FsArgs& a) {
-    return a.K >= 512 && a.K <= 20480 && a.N >= 64 && ((a.K | a.ldx | a.bsx | a.bsw) & 3) == 0 &&
+    return a.ldx <= kFsMostApart && a.K >= 512 && a.K <= 20480 && a.N >= 64 && ((a.K | a.ldx | a.bsx | a.bsw) & 3) == 0 &&
            ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) & 15) == 0;
 }
 int fs_launch_rows(const FsArgs& a, cudaStream_t stream);    // up to 16 rows (gemm_f32_rows.cu)

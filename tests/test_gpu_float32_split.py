@@ -66,3 +66,14 @@ def test_products_of_a_batch_and_strided_rows(ops):
         y = ops.head_product(x, w, heads_first=True)
         for h in range(H):
             assert torch.equal(y[h], ops.gemm_f32(x[:, h].contiguous(), w[h]))
+
+
+def test_rows_that_lie_far_apart(ops):
+    """Rows 68 MB apart, of which a tile's last are more than 2^31 floats behind its first."""
+    T, K, N, apart = 140, 512, 128, 17_000_000
+    x = torch.empty(T * apart, device="cuda").as_strided((T, 1, K), (apart, K, 1))
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x.copy_(torch.randn(T, 1, K, generator=g, device="cuda"))
+    w = torch.randn(1, N, K, generator=g, device="cuda")
+    want = x[:, 0].double() @ w[0].double().T
+    assert (ops.head_product(x, w, heads_first=True)[0].double() - want).norm() <= 2e-7 * want.norm()
