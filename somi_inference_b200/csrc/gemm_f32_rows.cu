@@ -3,10 +3,17 @@
 // tokens on its N side; the warps of a CTA (and CTAs of a cluster) share the blocks of the same features.
 //
 // What bounds it: reading the weights, if they arrive all the time and the splitting (about 260 instructions for a block's
-// 4 KB) runs under it.  Hence the walking kernel for few rows by many features, and parts of the rows kept in
-// registers.  In chains of products over weights that are not in L2, FMA kernel before / now, us: 1 row by 151,936 x 896
-// 95.9 / 86.4 (6.3 TB/s), 5 rows 114 / 86.8; 9,728 x 896, 1, 4, 8 and 16 rows 7.4, 8.9, 12.1, 16.3 / 8.6, 8.9, 9.4, 16.7;
-// 896 x 4,864 8.5, 10.1, 14.3, 14.6 / 7.6, 8.0, 8.1, 11.2; 1,152 x 896 4.0, 4.4, 5.3, 5.7 / 3.8, 4.2, 4.4, 5.3.
+// 4 KB) runs under it.  Hence the stream, whose CTAs stay, and deep stages where the chip is not full.  In chains of products
+// over weights that are not in L2, FMA kernel before / now, us (what `fr_launch` measured between kernels stands there):
+//     151,936 x 896, 1, 4, 8, 16 rows   96, 104, 116, 150   / 82, 85, 85, 129   (6.6 TB/s)
+//     152,064 x 3,584                   379, 398, 441, 584  / 309, 315, 330, 496 (7.1 TB/s)
+//     22,016 x 2,048                    39, 48, 69, 81      / 29, 29, 30, 48
+//     9,728 x 896                       7.4, 8.7, 12.1, 17  / 8.0, 8.2, 8.3, 15.6
+//     896 x 4,864                       8.4, 9.7, 13.4, 14  / 7.5, 7.9, 8.1, 11.1
+//     2,048 x 2,048                     5.9, 7.3, 11.9, 12  / 5.4, 5.7, 5.8, 7.8
+//     1,152 x 896                       3.9, 4.4, 5.3, 5.6  / 3.2, 3.6, 3.5, 4.9
+// One or two rows are up to 10 % slower than as FMAs where 5,000 to 10,000 features have few terms: there the FMA kernel's smaller CTAs
+// let more of the next product's weights be under way.
 #include <cooperative_groups.h>
 
 #include "gemm_f32_split.cuh"
@@ -198,98 +205,132 @@ f32_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, const 
     cluster.sync();                                      // no CTA leaves while its sums are read
 }
 
-// Up to 8 rows and 16 blocks by many features: the CTAs that fill the chip walk through the tiles.  A warp keeps its (one
-// or two) blocks' parts of the rows in registers for good, and each of its stages is filled again, with the next tile's weights, as
-// soon as it has been read: weights arrive all the time.  (With a CTA a tile, those of an SM wait for their weights
-// together and multiply together.)
-__global__ void __launch_bounds__(kFrThreads, 2)
-f32_rows_walk_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
-                     float* __restrict__ y, int M, int N, int K, int blocks, int range_blocks, int tiles, long long ldx,
-                     long long ldy, long long bsx, long long bsw, long long bsy, int w_constant) {
-    constexpr int OUT = kFrFeatures * 8, TILE = 8 * kFrPitch, BLOCK = kFrFeatures * kFsBK;
-    extern __shared__ __align__(128) float fr_buf[];     // [warp][stage][BLOCK], twice [block][TILE]
+// The same by CTAs that fill the chip and walk through the tiles: a warp takes a whole range of a tile, adds its blocks in registers, and
+// each of its stages is filled again as soon as it has been read, with a later block or the next tile's first: weights arrive all the time.
+// RANGES warps a CTA, `CTAS` of them an SM.
+template <int MT, int STAGES, int RANGES, int CTAS>
+__global__ void __launch_bounds__(32 * RANGES, CTAS)
+f32_rows_stream_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+                       float* __restrict__ y, int M, int N, int K, int blocks, int range_blocks, int tiles, long long ldx,
+                       long long ldy, long long bsx, long long bsw, long long bsy, int w_constant) {
+    constexpr int OUT = kFrFeatures * 8 * MT, TILE = 8 * MT * kFrPitch, BLOCK = kFrFeatures * kFsBK;
+    extern __shared__ __align__(128) float fr_buf[];     // [warp][stage][BLOCK], twice [warp][TILE]
     pdl_launch_dependents();
     x += blockIdx.z * bsx;
     w += blockIdx.z * bsw;
     y += blockIdx.z * bsy;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    float* ring = fr_buf + warp * 2 * BLOCK;
-    float* sums = fr_buf + kFrWarps * 2 * BLOCK;
+    const int b0 = min(blocks, warp * range_blocks), b1 = min(blocks, b0 + range_blocks);
+    float* ring = fr_buf + warp * STAGES * BLOCK;
+    float* sums = fr_buf + RANGES * STAGES * BLOCK;
     const int q16 = lane & 15, row0 = lane >> 4;
     const float* w_src = w + static_cast<long long>(row0) * K + 4 * q16;
     const uint32_t w_dst = smem_u32(ring + row0 * kFsBK + 4 * ((q16 & 8) | ((q16 ^ (q16 >> 3 << 1) ^ (row0 << 2)) & 7)));
-    auto fetch = [&](int tile, int i) {                  // this warp's block i of a tile into stage i
-        const int b = warp + i * kFrWarps, n0 = tile * kFrFeatures;
-        if (b < blocks && tile < tiles) {
-            const float* src = w_src + static_cast<long long>(n0) * K + b * kFsBK;
-            const uint32_t dst = w_dst + i * (BLOCK * 4);
-            if ((b + 1) * kFsBK <= K && n0 + kFrFeatures <= N) {
+    // the next block to fetch: blocks b0 .. of a tile, then of the CTA's next one
+    int next_tile = blockIdx.x, next = b0;
+    auto fetch = [&](int stage) {
+        if (next_tile < tiles && next < b1) {
+            const int n0 = next_tile * kFrFeatures;
+            const float* src = w_src + static_cast<long long>(n0) * K + next * kFsBK;
+            const uint32_t dst = w_dst + stage * (BLOCK * 4);
+            if ((next + 1) * kFsBK <= K && n0 + kFrFeatures <= N) {
 #pragma unroll
                 for (int r = 0; r < 8; ++r)
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + r * 2 * kFsBK * 4), "l"(src + r * 2 * K));
             } else {
-                const bool in = b * kFsBK + 4 * q16 < K;
+                const bool in = next * kFsBK + 4 * q16 < K;
                 for (int r = 0; r < 8; ++r) {
                     const bool live = in && n0 + row0 + 2 * r < N;
                     cp_async_16(dst + r * 2 * kFsBK * 4, live ? src + r * 2 * K : w, live ? 16 : 0);
                 }
             }
+            if (++next == b1) {
+                next = b0;
+                next_tile += gridDim.x;
+            }
         }
         cp_async_commit();
     };
-    int tile = blockIdx.x;
-    if (!w_constant) pdl_wait();
-    fetch(tile, 0);                                      // [constant], or behind the wait
-    fetch(tile, 1);
-    pdl_wait();
-    uint2 parts[2][4][3];
-    const float* x_src = x + min(g, M - 1) * ldx + (t < 2 ? 4 * t : 24 + 4 * t);   // (rows behind the last repeat it)
+    float4 xq[MT][4];
+    const int quad = t < 2 ? 4 * t : 24 + 4 * t;
+    const float* x_src[MT];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int m = 0; m < MT; ++m) x_src[m] = x + min(8 * m + g, M - 1) * ldx + quad;
+    auto load_x = [&](int b) {
+        if ((b + 1) * kFsBK <= K) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int k = (warp + i * kFrWarps) * kFsBK + 8 * j;
-            const float4 q = k + (t < 2 ? 4 * t : 24 + 4 * t) < K ? *reinterpret_cast<const float4*>(x_src + k)
-                                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-            fs_split(q.x, q.y, parts[i][j][0].x, parts[i][j][1].x, parts[i][j][2].x);
-            fs_split(q.z, q.w, parts[i][j][0].y, parts[i][j][1].y, parts[i][j][2].y);
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) xq[m][j] = *reinterpret_cast<const float4*>(x_src[m] + b * kFsBK + 8 * j);
+        } else {
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int k = b * kFsBK + 8 * j;
+                    xq[m][j] = k + quad < K ? *reinterpret_cast<const float4*>(x_src[m] + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
         }
+    };
+    if (!w_constant) pdl_wait();
+#pragma unroll
+    for (int i = 0; i < STAGES; ++i) fetch(i);           // [constant], or behind the wait
+    pdl_wait();
+    if (b0 < b1) load_x(b0);
+    int stage = 0, odd = 0;
     const int ranges = (blocks + range_blocks - 1) / range_blocks;
-    for (int odd = 0; tile < tiles; tile += gridDim.x, odd ^= 1) {
-        float* tile_sums = sums + odd * blocks * TILE;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int b = warp + i * kFrWarps;
-            cp_async_wait<1>();                          // (the other stage's copies may be under way)
-            __syncwarp();
-            if (b < blocks) {
-                float acc[1][4];
-                fr_multiply<1>(acc, ring + i * BLOCK, [&](int, int j, uint2& c0, uint2& c1, uint2& c2) {
-                    c0 = parts[i][j][0];
-                    c1 = parts[i][j][1];
-                    c2 = parts[i][j][2];
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, odd ^= 1) {
+        float* own = sums + (odd * RANGES + warp) * TILE;
+        if (b0 < b1) {
+            float sum[MT][4];
+#pragma unroll 1
+            for (int b = b0; b < b1; ++b) {
+                cp_async_wait<STAGES - 1>();
+                __syncwarp();
+                float acc[MT][4];
+                fr_multiply<MT>(acc, ring + stage * BLOCK, [&](int m, int j, uint2& c0, uint2& c1, uint2& c2) {
+                    fs_split(xq[m][j].x, xq[m][j].y, c0.x, c1.x, c2.x);
+                    fs_split(xq[m][j].z, xq[m][j].w, c0.y, c1.y, c2.y);
                 });
-                float* dst = tile_sums + b * TILE + 2 * t * kFrPitch + g;
+                load_x(b + 1 < b1 ? b + 1 : b0);
+                __syncwarp();                            // the stage has been read
+                fetch(stage);
+                stage = stage + 1 == STAGES ? 0 : stage + 1;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) dst[(e & 1) * kFrPitch + 8 * (e >> 1)] = acc[0][e];
+                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) sum[m][e] = b == b0 ? acc[m][e] : __fadd_rn(sum[m][e], acc[m][e]);
             }
-            __syncwarp();                                // the stage has been read
-            fetch(tile + gridDim.x, i);
+            float* dst = own + 2 * t * kFrPitch + g;
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dst[(8 * m + (e & 1)) * kFrPitch + 8 * (e >> 1)] = sum[m][e];
         }
         __syncthreads();
-        const int m = threadIdx.x / kFrFeatures, n = tile * kFrFeatures + threadIdx.x % kFrFeatures;
-        if (m < M && n < N) {
-            const float* src = tile_sums + m * kFrPitch + threadIdx.x % kFrFeatures;
-            float v = 0.f;
-            for (int r = 0, i = 0; r < ranges; ++r) {
-                float s = src[i++ * TILE];
-                for (const int end = min(blocks, (r + 1) * range_blocks); i < end; ++i) s = __fadd_rn(s, src[i * TILE]);
-                v = r == 0 ? s : __fadd_rn(v, s);
-            }
+        for (int o = threadIdx.x; o < OUT; o += 32 * RANGES) {
+            const int m = o / kFrFeatures, n = tile * kFrFeatures + o % kFrFeatures;
+            if (m >= M || n >= N) continue;
+            const float* src = sums + odd * RANGES * TILE + m * kFrPitch + o % kFrFeatures;
+            float v = src[0];
+            for (int r = 1; r < ranges; ++r) v = __fadd_rn(v, src[r * TILE]);
             if (!fs_finite(v)) v = fs_plain_sum(x + m * ldx, w + static_cast<long long>(n) * K, K);
             y[m * ldy + n] = bias ? __fadd_rn(v, bias[n]) : v;
         }
     }
+}
+
+template <int MT, int STAGES, int RANGES, int CTAS>
+int fr_launch_stream(const FsArgs& a, int blocks, int range_blocks, cudaStream_t stream) {
+    constexpr auto kernel = f32_rows_stream_kernel<MT, STAGES, RANGES, CTAS>;
+    constexpr int smem = 4 * (RANGES * STAGES * kFrFeatures * kFsBK + 2 * RANGES * 8 * MT * kFrPitch);
+    static_assert(CTAS * (smem + 1024) <= 228 * 1024, "the CTAs of an SM share its 228 KB");
+    allow_smem<kernel>(smem);
+    const int tiles = (a.N + kFrFeatures - 1) / kFrFeatures, ctas = (148 * CTAS + a.batch - 1) / a.batch;
+    launch_pdl(kernel, dim3(tiles < ctas ? tiles : ctas, 1, a.batch), dim3(32 * RANGES), smem, stream, a.x, a.w, a.bias, a.y, a.M, a.N,
+               a.K, blocks, range_blocks, tiles, a.ldx, a.ldy, a.bsx, a.bsw, a.bsy, a.w_constant);
+    return launch_status();
 }
 
 template <int MT, int STAGES, bool IN_PLACE, bool CLUSTER>
@@ -304,33 +345,44 @@ int fr_launch_one(const FsArgs& a, int cluster, int blocks, int range_blocks, in
     return launch_status();
 }
 
+// Which kernel.  A tile's ranges are the warps of a CTA of the stream, so it wants as many tiles as CTAs fill the chip, and where
+// they fill it little more than once, so many an SM that one round takes them all (1 row, 5,120 x 5,120, 320 tiles: two an SM 24.0 us,
+// three 20.9; 9,728 x 896, 608: four 9.6, five 8.0; more tiles: 152,064 x 3,584 306 and 321, 17,920 x 1,536 19.0 and 21.5).  With fewer
+// tiles than SMs deeper stages (2,048 x 11,008, 128: two 27.4, four 19.2; 1,152 x 896, 72: two 3.8, six 3.2).  A cluster shares a tile's
+// blocks out where that leaves each of its CTAs few of many (896 x 4,864, 56 tiles: 7.5 us and 8.5; 512 x 8,960 7.9 and 14.1; but 896 x 2,048
+// 5.6 and 4.0, 896 x 8,960, 36 blocks a CTA, 15.1 and 14.4), and for 9 to 16 rows from fewer blocks on (960 x 3,584 8.8 and 10.0; 2,048 x
+// 1,536 7.6 and 8.7).
 template <int MT>
 int fr_launch(const FsArgs& a, cudaStream_t stream) {
     const int blocks = (a.K + kFsBK - 1) / kFsBK, range_blocks = fs_range_blocks(blocks);
     const int ranges = (blocks + range_blocks - 1) / range_blocks;
     const long long tiles = static_cast<long long>((a.N + kFrFeatures - 1) / kFrFeatures) * a.batch;
-    // more tiles than the chip holds CTAs, and registers for the rows' parts (151,936 x 896, 1 row: a CTA a tile 103 us,
-    // walking 86; 9,728 x 896, 8 rows: 12.1 and 9.4)
-    if (MT == 1 && blocks <= 2 * kFrWarps && tiles > 148 * 2) {
-        const int smem = 4 * (kFrWarps * 2 * kFrFeatures * kFsBK + 2 * blocks * 8 * kFrPitch);
-        allow_smem<f32_rows_walk_kernel>(kFrMostSmem);
-        const int all = (a.N + kFrFeatures - 1) / kFrFeatures, ctas = (148 * 2 + a.batch - 1) / a.batch;
-        launch_pdl(f32_rows_walk_kernel, dim3(all < ctas ? all : ctas, 1, a.batch), dim3(kFrThreads), smem, stream, a.x, a.w,
-                   a.bias, a.y, a.M, a.N, a.K, blocks, range_blocks, all, a.ldx, a.ldy, a.bsx, a.bsw, a.bsy, a.w_constant);
-        return launch_status();
-    }
-    // at most 40 blocks a CTA, five a warp, whose sums stand in shared memory; fewer while the chip has room for more CTAs
+    // at most 40 blocks a CTA of a cluster, five a warp, whose sums stand in shared memory; fewer while the chip has room for more CTAs
     // (896 x 4,864, 8 rows: 112 CTAs of a cluster of two 10.9 us, 224 of four 8.0)
     int cluster = 1;
     while (blocks > 40 * cluster || (blocks > 20 * cluster && cluster < 8 && 2 * cluster * tiles <= 148 * 2)) cluster *= 2;
     const int own = (ranges + cluster - 1) / cluster * range_blocks, most = own < blocks ? own : blocks;
+    if (blocks >= 32) {                                  // (eight ranges)
+        const bool shared = cluster * tiles <= 148 * 2 && (MT == 1 ? blocks >= 64 && (own <= 24 || cluster == 8) : blocks >= 48);
+        if (!shared && tiles <= 148) return fr_launch_stream<MT, 4, 8, 1>(a, blocks, range_blocks, stream);
+        if constexpr (MT == 1)
+            if (tiles > 148 * 2 && tiles <= 148 * 3) return fr_launch_stream<MT, 2, 8, 3>(a, blocks, range_blocks, stream);
+        if (!shared) return fr_launch_stream<MT, 2, 8, 2>(a, blocks, range_blocks, stream);
+    } else {
+        if constexpr (MT == 1) {
+            if (tiles > 148 * 4 && tiles <= 148 * 5) return fr_launch_stream<MT, 2, 4, 5>(a, blocks, range_blocks, stream);
+            if (tiles <= 148 * 2) return fr_launch_stream<MT, 6, 4, 2>(a, blocks, range_blocks, stream);
+        }
+        if (MT == 1 || tiles > 148 * 2) return fr_launch_stream<MT, 2, 4, 4>(a, blocks, range_blocks, stream);
+    }
 #define SOMI_FR(STAGES, IN_PLACE) \
-    return cluster > 1 ? fr_launch_one<MT, STAGES, IN_PLACE, true>(a, cluster, blocks, range_blocks, own, stream) \
-                       : fr_launch_one<MT, STAGES, IN_PLACE, false>(a, 1, blocks, range_blocks, own, stream)
-    if (most <= 2 * kFrWarps) SOMI_FR(2, true);
-    if (most <= 3 * kFrWarps) SOMI_FR(3, true);
-    SOMI_FR(3, false);
+    if (cluster > 1) return fr_launch_one<MT, STAGES, IN_PLACE, true>(a, cluster, blocks, range_blocks, own, stream); \
+    if constexpr (MT == 2) return fr_launch_one<MT, STAGES, IN_PLACE, false>(a, 1, blocks, range_blocks, own, stream)
+    if (most <= 2 * kFrWarps) { SOMI_FR(2, true); }
+    else if (most <= 3 * kFrWarps) { SOMI_FR(3, true); }
+    else { SOMI_FR(3, false); }
 #undef SOMI_FR
+    return SOMI_ERR_UNSUPPORTED;                          // (64 blocks and more are at least two CTAs')
 }
 
 int fs_launch_rows(const FsArgs& a, cudaStream_t stream) { return a.M <= 8 ? fr_launch<1>(a, stream) : fr_launch<2>(a, stream); }

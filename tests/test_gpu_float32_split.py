@@ -30,6 +30,26 @@ def test_rows_and_error(ops, N, K):
     ops.check_errors()
 
 
+@pytest.mark.parametrize("N,K", [(60, 2048), (16, 2112), (1000, 2112), (2360, 1988), (2384, 2048), (4720, 2052), (4750, 2048), (7120, 2112),
+                                 (80, 516), (4720, 1300), (4750, 576), (9480, 516), (9500, 640), (11850, 512), (30000, 900),
+                                 (512, 8960), (640, 4868), (900, 3588)])
+def test_few_rows_of_every_form(ops, N, K):
+    """Forms of the kernels for few rows: with 4 and 8 ranges (the last of them short or empty), tiles that fill the chip once, a
+    little more, several times, and clusters.  The bits are those of the kernel for many rows, the batch's those of each."""
+    g = torch.Generator(device="cuda").manual_seed(N * K)
+    N = max(N, 64)
+    x = torch.randn(24, K, generator=g, device="cuda")
+    w, b = torch.randn(N, K, generator=g, device="cuda"), torch.randn(N, generator=g, device="cuda")
+    whole = ops.gemm_f32(x, w, b)
+    assert (whole.double() - (x.double() @ w.double().T + b.double())).norm() <= 2e-7 * whole.double().norm()
+    for m in (1, 3, 8, 9, 16):
+        assert torch.equal(ops.gemm_f32(x[24 - m:].contiguous(), w, b, constant=True), whole[24 - m:]), m
+    if N <= 4800:
+        y = ops.head_product(x[:14].view(7, 2, K), torch.stack([w, w.flip(0)]), heads_first=True)
+        assert torch.equal(y[1, :5], ops.gemm_f32(x[1:10:2].contiguous(), w.flip(0))) and torch.equal(y[0], ops.gemm_f32(x[:14:2].contiguous(), w))
+    ops.check_errors()
+
+
 @pytest.mark.parametrize("M", [3, 11, 40, 300, 1500])
 @pytest.mark.parametrize("N", [80, 6000])
 def test_operands_without_parts(ops, M, N):
