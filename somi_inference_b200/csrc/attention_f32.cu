@@ -894,8 +894,12 @@ f32_single(int at, int kvh, int i, const float* __restrict__ qkv, int row_stride
     }
 }
 
+// A CTA's work is a chain of loads and small products, so CTAs beside each other hide it, and five an SM in 96 registers (which cost
+// 120 bytes of spills), three with 128 columns, are faster than the three and two that take what registers they like.  Layers in us, as
+// FMAs / three or two an SM / now: 14 heads over 2 of 64, 1 token behind 8,000 30.9 / 39.0 / 32.7, 16 behind 4,000 57.9 / 59.8 / 51.7, 64 behind 2,000
+// 95.1 / 102.6 / 85.1; 28 over 4 of 128, 8 behind 2,048 98.8 / 85.2 / 78.4.
 template <int HD>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, HD == 64 ? 5 : 3)
 attention_f32_split_kernel(const float* __restrict__ qkv, int row_stride, int row_base, int req_base,
                            const float* __restrict__ kcache, const float* __restrict__ vcache,
                            const int* __restrict__ block_table, int bt_stride, const int* __restrict__ ctx_len,
