@@ -41,15 +41,21 @@ __global__ void chunk_angles_kernel(const int* __restrict__ positions, const dou
     if (i < n) cs[i] = turn_by(static_cast<double>(positions[i / half]), freq[i % half]);
 }
 
+// The place in u of the first chunk of request r of a run, which begins `row` rows behind the run's first: its n rows' chunks end in
+// front of the next request's place, (row + n + 127 + 127 r) / 128, and nobody sums over the requests in front.
+__device__ __forceinline__ int ch_place(int row, int r) { return (row + (kChRows - 1) * r) / kChRows; }
+
 // The chunks of a run of requests, as its tiles of 64 rows give them: each pair of a request's tiles, at the pair's first.
 struct ChTiles {
     const int *tiles, *cu_q;          // (request, first row, rows); the run's requests' first rows
     int first;                        // the run's first request
-    // The chunk that begins with tile i: its first row, and how many it has (0: the tile is another chunk's second).
-    __device__ __forceinline__ int rows_of(int i, int& row0) const {
+    // The chunk that begins with tile i: its first row, its place in u, and how many rows it has (0: the tile is another chunk's second).
+    __device__ __forceinline__ int rows_of(int i, int& row0, int& place) const {
         const int r = ld_step(tiles + 3 * i) - first;     // [descriptor]
         row0 = ld_step(tiles + 3 * i + 1);
-        return (row0 - ld_step(cu_q + r)) / kChTile & 1 ? 0 : min(kChRows, ld_step(cu_q + r + 1) - row0);
+        const int begin = ld_step(cu_q + r);
+        place = ch_place(begin - ld_step(cu_q), r) + (row0 - begin) / kChRows;
+        return (row0 - begin) / kChTile & 1 ? 0 : min(kChRows, ld_step(cu_q + r + 1) - row0);
     }
 };
 
@@ -297,7 +303,7 @@ __device__ __forceinline__ float ch_dot(const ChRows& q, int row, float q_scale,
     return dot;
 }
 
-// U [tile][head][value channel][key channel].  A CTA per (tile, head), two on an SM: 64 rows at a time, k in parts and v; D = V^T K with
+// U [chunk][head][value channel][key channel].  A CTA per (tile, head), two on an SM: 64 rows at a time, k in parts and v; D = V^T K with
 // the rows as the products' K, both operands as the rows lie; the halves' sums in two accumulators.
 template <int D, bool SILU>
 __global__ void __launch_bounds__(kChThreads, 2)
@@ -312,8 +318,8 @@ chunk_update_kernel(ChRows k, ChRows v, const float* __restrict__ decay, ChTiles
     __shared__ __align__(8) unsigned long long bar_s;
     __shared__ uint32_t tmem_s;
     pdl_launch_dependents();
-    int row0;
-    const int rows = tiles.rows_of(blockIdx.x, row0), h = blockIdx.y;
+    int row0, place;
+    const int rows = tiles.rows_of(blockIdx.x, row0, place), h = blockIdx.y;
     if (rows == 0) {
         pdl_wait();
         return;
@@ -384,7 +390,7 @@ chunk_update_kernel(ChRows k, ChRows v, const float* __restrict__ decay, ChTiles
             }
         }
         __syncwarp();
-        float* dst = u + (static_cast<size_t>(blockIdx.x) * heads + h) * D * D + (warp & 3) * 32 * D + (warp >> 2) * COLS;
+        float* dst = u + (static_cast<size_t>(place) * heads + h) * D * D + (warp & 3) * 32 * D + (warp >> 2) * COLS;
 #pragma unroll 4
         for (int i = lane; i < 32 * (COLS / 4); i += 32) {
             const int r = i / (COLS / 4), c = i % (COLS / 4) * 4;
@@ -403,15 +409,14 @@ chunk_states_kernel(float* __restrict__ u, const float* __restrict__ decay, cons
     pdl_launch_dependents();
     pdl_wait();
     const int h = blockIdx.y, r = blockIdx.z;
-    int tile = 0;                                         // the request's first
-    for (int i = 0; i < r; ++i) tile += (cu_q[i + 1] - cu_q[i] + kChTile - 1) / kChTile;
+    const int place = ch_place(cu_q[r] - cu_q[0], r);
     const int rows = cu_q[r + 1] - cu_q[r], n = (rows + kChRows - 1) / kChRows;
     const float g = decay[h], full = powf(g, static_cast<float>(kChRows));
     const float tail = powf(g, static_cast<float>(rows - (n - 1) * kChRows));
     const int at = (blockIdx.x * kChThreads + threadIdx.x) * 4;
     float* own = state + (static_cast<size_t>(state_slot[r]) * heads + h) * D * D + at;
-    float* p = u + (static_cast<size_t>(tile) * heads + h) * D * D + at;
-    const size_t step = static_cast<size_t>(kChRows / kChTile) * heads * D * D;
+    float* p = u + (static_cast<size_t>(place) * heads + h) * D * D + at;
+    const size_t step = static_cast<size_t>(heads) * D * D;
     F4 s = load4(own);
     constexpr int AHEAD = 8;                              // loads in flight
     for (int c0 = 0; c0 < n; c0 += AHEAD) {
@@ -450,8 +455,8 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
     __shared__ __align__(8) unsigned long long bar_s;
     __shared__ uint32_t tmem_s;
     pdl_launch_dependents();
-    int row0;
-    const int rows = tiles.rows_of(blockIdx.x, row0), h = blockIdx.y;
+    int row0, place;
+    const int rows = tiles.rows_of(blockIdx.x, row0, place), h = blockIdx.y;
     if (rows == 0) {
         pdl_wait();
         return;
@@ -464,7 +469,7 @@ chunk_outputs_kernel(ChRows q, ChRows k, ChRows v, float q_scale, const float* _
     k.p += static_cast<size_t>(h / group) * D;
     v.p += static_cast<size_t>(h) * D;
     if (threadIdx.x <= kChRows) pow_s[threadIdx.x] = powf(decay[h], static_cast<float>(threadIdx.x));
-    const float* st = states + (static_cast<size_t>(blockIdx.x) * heads + h) * D * D;
+    const float* st = states + (static_cast<size_t>(place) * heads + h) * D * D;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, halves = rows > 64 ? 2 : 1;
     const uint32_t first = mma.tmem, second = mma.tmem + 128;
     const uint64_t xd = t5::desc_kmajor(smem_u32(xs)), yd = t5::desc_kmajor(smem_u32(ys));
@@ -704,7 +709,8 @@ using namespace somi;
 // q, k: bfloat16 rows of heads / group heads of D elements, `stride` apart; v: of `heads` heads; D = 64 or 128.
 // `silu`: q and k (bit 0) and v (bit 1) pass SiLU.  rot > 0: the pairs (i, i + rot / 2) of q and k turn by
 // positions * rot_freq; angles: float32 scratch [portions' rows, rot].  `tiles`: int32 [n_tiles, 3] = (request,
-// first row, rows <= 64) over the n_req multi-token requests, in order, request numbers from `first` on.  u: float32 scratch [n_tiles, heads, D, D].
+// first row, rows <= 64) over the n_req multi-token requests, in order, request numbers from `first` on.  u: float32 scratch
+// [(64 n_tiles + 127 n_req) / 128, heads, D, D].
 // state: float32 [slots, heads, D, D] (value channel, key channel); y: float32 rows of heads * D.
 SOMI_API int somi_matrix_state_chunks(const void* q, const void* k, const void* v, long long q_stride,
                                       long long k_stride, long long v_stride, int silu, float q_scale,

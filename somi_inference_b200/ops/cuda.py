@@ -1780,7 +1780,8 @@ class CudaOps:
         first, end, n_tiles = run
         rows = int(batch.host.cu_q[end])                     # (angles of the rows in front are made too)
         tiles, _ = self._tiles_of(batch, self.prefill_q_tile, first, end)
-        n_u = n_tiles * heads * dk * dk                      # the chunks' states, and the angles behind them
+        # a place for the state of every chunk of 128 rows (at most this many, whichever the requests' lengths), and the angles behind them
+        n_u = (64 * n_tiles + 127 * (end - first)) // 128 * heads * dk * dk
         u = torch.empty(n_u + rows * rot, dtype=torch.float32, device=q.device)
         rc = self.lib.somi_matrix_state_chunks(
             _ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(q.stride(0)), ctypes.c_longlong(k.stride(0)),

@@ -292,3 +292,25 @@ def test_the_chunks_workspace_is_bounded(ops):
     runs = ops.scan_runs(portions((0, 10000), (0, 10000), (0, 20000), singles=(4,)), heads, d)
     assert runs == ((0, 1, 157), (1, 2, 157), (2, 4, 0))
     assert all(n * heads * d * d * 4 <= 1 << 29 for _, _, n in runs)
+
+
+def test_the_chunks_workspace_has_a_place_for_every_chunk(ops, monkeypatch):
+    """The states' scratch is one per chunk of 128 rows, at most one more a request; the kernels' places in it ((rows in front + 127 r) / 128 for
+    request r's first chunk) are each a chunk's own and lie inside."""
+    sizes, calls, heads, d, rng = [], [], 2, 64, random.Random(5)
+    ops.lib.somi_matrix_state_chunks = lambda *args: calls.append([getattr(a, "value", a) for a in args]) or 0
+    ops.use_scan_chunks, ops.prefill_q_tile = True, 64
+    real = torch.empty
+    monkeypatch.setattr(cuda.torch, "empty", lambda size, **kw: sizes.append(size) or real(1, **kw))
+    for _ in range(200):
+        lengths = [rng.choice((96, 97, 127, 128, 129, 192, 193, 256, 257, rng.randrange(96, 2000))) for _ in range(rng.randrange(1, 9))]
+        batch = portions(*((0, n) for n in lengths))
+        qkv = on_device(batch.num_tokens, 3 * heads * d, dtype=torch.bfloat16)
+        sizes.clear(), calls.clear()
+        ops.matrix_state_scan(qkv[:, :heads * d], qkv[:, heads * d:2 * heads * d], qkv[:, 2 * heads * d:], on_device(len(lengths), heads, d, d),
+                              batch, on_device(batch.num_tokens, heads * d), heads, heads, d, d, decay=on_device(heads))
+        chunks = [-(-n // 128) for n in lengths]
+        assert len(sizes) == len(calls) == 1 and sizes[0] <= (sum(chunks) + len(lengths)) * heads * d * d
+        starts = [(sum(lengths[:r]) + 127 * r) // 128 for r in range(len(lengths))]
+        places = [s + c for s, n in zip(starts, chunks) for c in range(n)]
+        assert len(set(places)) == len(places) and (max(places) + 1) * heads * d * d <= sizes[0]
