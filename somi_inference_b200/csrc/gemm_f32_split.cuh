@@ -1,9 +1,9 @@
 // A float32 product on tensor cores: every operand is the exact sum of three bfloat16 numbers
-// (a0 = a rounded, a1 = a - a0 rounded, a2 = the rest: 3 x 8 bits hold float32's 24), and of the nine
-// products of parts the six down to 2^-18 of the whole are summed, in float32 accumulators.  What is left
-// out is below 2^-26 of a term; what bounds the error is the accumulator, which drops what falls off
-// its end instead of rounding: so it never holds more than 64 terms, the parts' small products come first
-// and the four steps of a0 b0 last, and everything above 64 terms is added in registers, rounded.
+// (a0 = a rounded, a1 = a - a0 rounded, a2 = the rest: 3 x 8 bits hold float32's 24; Henry, Tang and Heinecke, "Leveraging the bfloat16
+// Artificial Intelligence Datatype For Higher-Precision Computations", 2019), and of the nine products of parts six are summed, in float32
+// accumulators.  What is left out (a1 b2, a2 b1, a2 b2) is at most 2^-24 of a term and 5.7e-9 of a whole product's norm; what bounds
+// the error is the accumulator, which drops what falls off its end instead of rounding: so it never holds more than 64 terms, the
+// parts' small products come first and the four steps of a0 b0 last, and everything above 64 terms is added in registers, rounded.
 //
 // The order of an output's sum depends on K alone: K is cut into blocks of 64, blocks into up to 4 or 8
 // ranges (`fs_range_blocks`); a block is one chain of MMA steps of 16 terms (for each of its four steps
@@ -16,7 +16,8 @@
 // Relative error of whole products of normal numbers against 64 bits, float32 FMA chains / this: 896 terms 2.0e-7 / 9.7e-8,
 // 4,864 terms 3.2e-7 / 1.15e-7.  One chain of 16 steps instead of four would have 2.3e-7 by itself, all of
 // it towards zero.  What this cannot hold are operands below about 2^-109: their third parts are less than bfloat16's
-// smallest number, and what is lost is at most 2^-134.
+// smallest number, and what is lost of an operand is at most 2^-134 (of 1e-38 some seven bits are left).  That goes for all that
+// multiply parts: this product, attention_f32.cu and recurrent_chunks.cu.
 #pragma once
 
 #include "mma.cuh"

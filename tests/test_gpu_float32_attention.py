@@ -61,7 +61,9 @@ def test_kernels_give_the_same_bits(ops, hd, window, infinite):
         for part in out.split(q):
             same = (part == got[0]) | (part.isnan() & got[0].isnan())
             assert same.all()
-    if infinite:
+    if not infinite:
+        assert got[0].isfinite().all()                   # (what is not written stays NaN)
+    else:
         pos, x = torch.arange(131, 131 + q), rows[0][:, :nq * hd].view(q, nq, hd)
         sees = (pos >= 150) & (pos < 150 + (window or 10 ** 6))
         # +infinity takes all (NaN), -infinity takes nothing

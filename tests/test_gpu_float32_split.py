@@ -16,15 +16,18 @@ def ops():
 @pytest.mark.parametrize("K", [512, 516, 896, 1024, 1088, 2044, 4864, 20480])
 @pytest.mark.parametrize("N", [64, 333, 1152, 5000])
 def test_rows_and_error(ops, N, K):
-    """One error bound for all forms: six products of parts leave out less than 2^-25 of a term; a block's last four steps (and
+    """Two error bounds for all forms.  An output's: six products of parts leave out at most 2^-24 of a term; a block's last four steps (and
     20 that are 2^-8 as large) lose less than two units of 2^-24 of the terms' magnitudes each, and the sums over
-    blocks and ranges round K / 64 + 9 times.  Each row gives the bits that it gives alone."""
+    blocks and ranges round K / 64 + 9 times.  The whole product's, as a share of its norm: a block is off by 6.5e-8 (measured against 64 bits), and
+    each of the K / 64 + 9 sums by up to 2^-25 of what it has so far, which add as random signs do; without a
+    third part, or without x1 w1, it would be 2.4e-6 or more at every size (computed on the CPU from the parts).  Each row gives the bits that it gives alone."""
     g = torch.Generator(device="cuda").manual_seed(N + K)
     x = torch.randn(700, K, generator=g, device="cuda")
     w, b = torch.randn(N, K, generator=g, device="cuda"), torch.randn(N, generator=g, device="cuda")
     whole = ops.gemm_f32(x, w, b)
     want, size = x.double() @ w.double().T + b.double(), x.double().abs() @ w.double().abs().T + b.double().abs()
     assert ((whole.double() - want).abs() <= (K / 64 + 9 + 8 + 2) * 2.0 ** -24 * size).all()
+    assert (whole.double() - want).norm() <= (6.5e-8 + 2.0 ** -25 * (K / 64 + 9) ** 0.5) * want.norm()
     for m in (1, 8, 9, 16, 17, 64, 65, 129, 207, 257, 513):
         assert torch.equal(ops.gemm_f32(x[700 - m:].contiguous(), w, b), whole[700 - m:]), m
     ops.check_errors()
@@ -97,3 +100,15 @@ def test_rows_that_lie_far_apart(ops):
     w = torch.randn(1, N, K, generator=g, device="cuda")
     want = x[:, 0].double() @ w[0].double().T
     assert (ops.head_product(x, w, heads_first=True)[0].double() - want).norm() <= 2e-7 * want.norm()
+
+
+def test_more_rows_than_a_grid_has_tiles(ops):
+    """A launch of the kernel for many rows has at most 65,535 tiles of up to 128 rows; the rows behind them are another launch's."""
+    M, K, N = 65535 * 128 + 300, 512, 64
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x, w = torch.zeros(M, K, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    at = torch.cat([torch.arange(40), torch.arange(65535 * 128 - 70, M)]).cuda()
+    x[at] = torch.randn(at.numel(), K, generator=g, device="cuda")
+    y = ops.gemm_f32(x, w)
+    assert torch.equal(y[at], ops.gemm_f32(x[at], w)) and not y[40:65535 * 128 - 70].any()
+    ops.check_errors()
