@@ -95,11 +95,11 @@ template <int NB>
 __host__ __device__ constexpr int ft_columns() { return 3 * NB <= 128 ? 128 : (3 * NB <= 256 ? 256 : 512); }
 
 // The 128 rows are features and the NB columns tokens, or (TOKENS) the other way round.  A cluster of
-// `cluster_size` CTAs shares a tile's ranges, one each; else the CTA walks through all of them.
+// `cluster_size` CTAs shares a tile's ranges, `own_ranges` (one or two) each; else the CTA walks through all of them.
 template <int NB, bool TOKENS>
 __global__ void __launch_bounds__(kFtThreads, 1)
 f32_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
-                 float* __restrict__ y, int M, int N, int K, int blocks, int range_blocks, int cluster_size,
+                 float* __restrict__ y, int M, int N, int K, int blocks, int range_blocks, int cluster_size, int own_ranges,
                  long long ldx, long long ldy, long long bsx, long long bsw, long long bsy, int w_constant) {
     constexpr int PLANE_B = NB * kFsBK * 2, STAGE = 3 * (kFtTile + PLANE_B);
     constexpr int LB = (NB + 31) / 32, HALF = NB / 2;    // rows of the NB side a thread loads; columns it sums
@@ -134,8 +134,8 @@ f32_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w, const
     y += blockIdx.z * bsy;
     const int rank = blockIdx.x % cluster_size;
     const int n0 = blockIdx.x / cluster_size * (TOKENS ? NB : 128), m0 = blockIdx.y * (TOKENS ? 128 : NB);
-    const int b0 = cluster_size > 1 ? min(blocks, rank * range_blocks) : 0;
-    const int n_blocks = (cluster_size > 1 ? min(blocks, b0 + range_blocks) : blocks) - b0;
+    const int b0 = cluster_size > 1 ? min(blocks, rank * own_ranges * range_blocks) : 0;
+    const int n_blocks = (cluster_size > 1 ? min(blocks, b0 + own_ranges * range_blocks) : blocks) - b0;
     namespace cg = cooperative_groups;
     const cg::cluster_group cluster = cg::this_cluster();
 
@@ -273,9 +273,9 @@ f32_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w, const
             t5::fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&free_bar[s]));
-            if (--left == 0 || i + 1 == n_blocks) {      // the range is complete: onto the sum of those before
+            if (--left == 0 || i + 1 == n_blocks) {      // the range is complete: onto the sum of those before (or beside it)
                 const bool last = i + 1 == n_blocks;
-                if (closed > 0) ft_add<HALF>(own + 2 * NB, acc2);
+                if (closed > 0 && cluster_size == 1) ft_add<HALF>(own + 2 * NB, acc2);
                 if (!last) {
 #pragma unroll
                     for (int c = 0; c < HALF; c += 8) {
@@ -296,11 +296,23 @@ f32_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w, const
         const int row = (warp & 3) * 32 + lane, col0 = half * HALF;
         if (cluster_size > 1) {                          // (the last MMA has read the stages)
             float* tile = reinterpret_cast<float*>(stages);
+            if (closed > 1) {
+#pragma unroll
+                for (int c = 0; c < HALF; c += 8) {
+                    uint64_t v[4];
+                    ft_ld8(own + 2 * NB + c, v);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        unpair_f32(v[e], tile[(col0 + c + 2 * e) * 128 + row], tile[(col0 + c + 2 * e + 1) * 128 + row]);
+                }
+                tile += NB * 128;
+            }
 #pragma unroll
             for (int c = 0; c < HALF; ++c) tile[(col0 + c) * 128 + row] = acc[c];
-            // the ranges' tiles [column][128 rows], each in its CTA's shared memory: every CTA adds up a share of the
+            // the ranges' tiles [column][128 rows], one or two in a CTA's shared memory: every CTA adds up a share of the
             // elements in the order of the ranges
             cluster.sync();
+            const int ranges = (blocks + range_blocks - 1) / range_blocks;
             const int step = cluster_size * kFtGroup;
             for (int i0 = rank * kFtGroup + tid - kFtGroup; i0 < NB * 32; i0 += 2 * step) {
                 float4 part[2][8];                       // two elements' loads in flight
@@ -311,7 +323,9 @@ f32_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w, const
                     const float4* mine = reinterpret_cast<const float4*>(stages) + i;
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
-                        if (k < cluster_size) part[u][k] = *cluster.map_shared_rank(mine, k);
+                        if (k < ranges)
+                            part[u][k] = own_ranges == 1 ? *cluster.map_shared_rank(mine, k)
+                                                         : *cluster.map_shared_rank(mine + k % 2 * NB * 32, k / 2);
                 }
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
@@ -320,7 +334,7 @@ f32_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w, const
                     float v[4] = {part[u][0].x, part[u][0].y, part[u][0].z, part[u][0].w};
 #pragma unroll
                     for (int k = 1; k < 8; ++k)
-                        if (k < cluster_size) {
+                        if (k < ranges) {
                             v[0] = __fadd_rn(v[0], part[u][k].x);
                             v[1] = __fadd_rn(v[1], part[u][k].y);
                             v[2] = __fadd_rn(v[2], part[u][k].z);
@@ -406,13 +420,15 @@ f32_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w, const
 // tensor pipe takes 51 cycles for a step of up to 64 columns and one for two columns from there on).  It need not be exact, only
 // tell a nearly empty last wave: 207 rows by 9,728 features are 152 tiles of 128 features by 112 rows, two waves, or 136 of
 // 144 features by 128 rows, one wave (41 and 31 us).
+// With eight ranges a CTA may take two: 32 rows by 4,096 x 2,048 are three waves of clusters of eight or one of clusters of four (26.4 and
+// 13.9 us; FMAs 20.0), 203 by 2,048 x 11,008 108 and 68; one a CTA stays ahead where it saves no wave (48 by 5,120 x 2,048 28.4 and 30.0).
 struct FtForm {
-    int nb, tokens, cluster;
+    int nb, tokens, cluster, own;
     long long cost;
 };
 
 template <int NB, bool TOKENS>
-int ft_launch_one(const FsArgs& a, int cluster, int blocks, int range_blocks, cudaStream_t stream) {
+int ft_launch_one(const FsArgs& a, int cluster, int own, int blocks, int range_blocks, cudaStream_t stream) {
     constexpr auto kernel = f32_tiles_kernel<NB, TOKENS>;
     allow_smem<kernel>(ft_smem<NB>());
     constexpr int TN = TOKENS ? NB : 128, TM = TOKENS ? 128 : NB;
@@ -420,7 +436,7 @@ int ft_launch_one(const FsArgs& a, int cluster, int blocks, int range_blocks, cu
         const int rows = a.M - m < 65535 * TM ? a.M - m : 65535 * TM;
         launch_pdl_cluster(kernel, dim3((a.N + TN - 1) / TN * cluster, (rows + TM - 1) / TM, a.batch), dim3(kFtThreads),
                            ft_smem<NB>(), cluster, stream, a.x + m * a.ldx, a.w, a.bias, a.y + m * a.ldy, rows, a.N, a.K,
-                           blocks, range_blocks, cluster, a.ldx, a.ldy, a.bsx, a.bsw, a.bsy, a.w_constant);
+                           blocks, range_blocks, cluster, own, a.ldx, a.ldy, a.bsx, a.bsw, a.bsy, a.w_constant);
         m += rows;
     }
     return launch_status();
@@ -429,25 +445,27 @@ int ft_launch_one(const FsArgs& a, int cluster, int blocks, int range_blocks, cu
 int fs_launch_tiles(const FsArgs& a, cudaStream_t stream) {
     const int blocks = (a.K + kFsBK - 1) / kFsBK, range_blocks = fs_range_blocks(blocks);
     const int ranges = (blocks + range_blocks - 1) / range_blocks;
-    FtForm best{0, 0, 0, 0};
-    auto consider = [&](int nb, int tokens, int cluster) {
+    FtForm best{0, 0, 0, 0, 0};
+    auto consider = [&](int nb, int tokens, int own) {   // (own: ranges of a CTA, 0 for all)
+        const int cluster = own == 0 ? 1 : (ranges + own - 1) / own;
         const long long tiles = static_cast<long long>(tokens ? (a.N + nb - 1) / nb : (a.N + 127) / 128) *
                                 (tokens ? (a.M + 127) / 128 : (a.M + nb - 1) / nb) * a.batch;
         const int step = nb / 2 > 51 ? nb / 2 : 51;
         // (clusters of seven or eight leave a few SMs of every GPC idle)
         const int slots = cluster == 1 ? 148 : (cluster <= 4 ? 132 : 112) / cluster;
         const long long waves = (tiles + slots - 1) / slots;
-        const long long cost = waves * (24ll * step * (cluster == 1 ? blocks : range_blocks) + (cluster == 1 ? 4000 : 6000));
-        if (best.nb == 0 || cost < best.cost) best = FtForm{nb, tokens, cluster, cost};
+        const long long cost = waves * (24ll * step * (cluster == 1 ? blocks : own * range_blocks) + (cluster == 1 ? 4000 : 4000 + 2000 * own));
+        if (best.nb == 0 || cost < best.cost) best = FtForm{nb, tokens, cluster, own, cost};
     };
     constexpr int kTokenTiles[] = {32, 64, 96, 112, 128}, kFeatureTiles[] = {96, 112, 128, 144};
     for (int nb : kTokenTiles) {
-        consider(nb, 0, 1);
-        if (ranges > 1) consider(nb, 0, ranges);
+        consider(nb, 0, 0);
+        if (ranges > 1) consider(nb, 0, 1);
+        if (ranges > 4) consider(nb, 0, 2);
     }
-    for (int nb : kFeatureTiles) consider(nb, 1, 1);
+    for (int nb : kFeatureTiles) consider(nb, 1, 0);
 #define SOMI_FT(NB, T) \
-    if (best.nb == NB && best.tokens == T) return ft_launch_one<NB, T>(a, best.cluster, blocks, range_blocks, stream)
+    if (best.nb == NB && best.tokens == T) return ft_launch_one<NB, T>(a, best.cluster, best.own, blocks, range_blocks, stream)
     SOMI_FT(32, 0);
     SOMI_FT(64, 0);
     SOMI_FT(96, 0);

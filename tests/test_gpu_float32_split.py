@@ -53,6 +53,19 @@ def test_few_rows_of_every_form(ops, N, K):
     ops.check_errors()
 
 
+@pytest.mark.parametrize("N,K", [(4096, 2048), (4100, 2112), (6144, 3588), (5000, 5000)])
+@pytest.mark.parametrize("M", [17, 32, 65, 100])
+def test_two_ranges_of_a_cluster(ops, M, N, K):
+    """Clusters whose CTAs have two ranges each (the last of them one, where there are seven): the bits of few rows."""
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    b = torch.randn(N, generator=g, device="cuda")
+    y = ops.gemm_f32(x, w, b)
+    for at in range(0, M, 16):
+        assert torch.equal(y[at:at + 16], ops.gemm_f32(x[at:at + 16].contiguous(), w, b))
+    ops.check_errors()
+
+
 @pytest.mark.parametrize("M", [3, 11, 40, 300, 1500])
 @pytest.mark.parametrize("N", [80, 6000])
 def test_operands_without_parts(ops, M, N):
