@@ -910,7 +910,7 @@ attention_f32_split_kernel(const float* __restrict__ qkv, int row_stride, int ro
 }
 
 // Portions and single tokens of a step in one launch (head size 64): the portions' CTAs first, then one per (chunk, kv head, request), whose
-// upper four warps have nothing to do.
+// upper four warps have nothing to do.  Both parts' registers are more than 128: 72 to 92 bytes are spilled.
 template <int RI>
 __global__ void __launch_bounds__(256, 2)
 attention_f32_mixed_kernel(const float* __restrict__ qkv, int row_stride, const float* __restrict__ kcache,

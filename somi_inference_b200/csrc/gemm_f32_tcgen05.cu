@@ -11,8 +11,8 @@
 // faster (207 rows by 9,728 features 31.8 us, 64 rows 23.1).  Issuing the next block's loads one by one between the splits took 4,500 cycles a block, with
 // every load behind all splits the loads' latency was added to them; so they go in two groups, a and b.
 // In chains of products, FMA kernel before / now, us: 9,728 x 896, 17, 64, 207, 1,024 and 4,096 rows 22, 37, 115, 424, 1,623 /
-// 17.7, 19.7, 30.8, 113, 411 (174 TFLOP/s of float32 products); 896 x 4,864 21, 39, 65, 255, 950 / 15.0, 15.5, 20.6, 83, 222;
-// 1,152 x 896 7.9, 11.0, 17.7, 66, 230 / 7.9, 8.1, 11.1, 19.9, 52.
+// 17.7, 19.7, 30.0, 111, 398 (179 TFLOP/s of float32 products); 896 x 4,864 21, 39, 65, 255, 950 / 14.8, 15.0, 20.1, 72, 225;
+// 1,152 x 896 7.9, 11.0, 17.7, 66, 230 / 7.7, 7.8, 11.4, 20.2, 50.
 #include <cooperative_groups.h>
 
 #include "gemm_f32_split.cuh"

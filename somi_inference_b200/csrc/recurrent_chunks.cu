@@ -12,11 +12,12 @@
 // Why: step by step, a portion is one chain of rows per (head, 16 columns) with two sums over a warp each:
 // 224 CTAs for 28 heads of 128, 522 us for 2,048 rows behind 43 us of preparation.  In chunks nothing
 // waits for anything but the second kernel.  As FMAs on the CUDA cores, in chunks of 64 rows, the products took U 70 and y 123 us
-// (25 TFLOP/s); on tensor cores, with half as many states in between, the same rows take: angles 3, U 28, states 18 (36), y 66 us,
-// each with nothing in L2.  What bounds them now: a CTA's phases (load and split, multiply, load and split, ..) one behind the
-// other, two CTAs to an SM, with the tensor pipe busy a quarter of the time, and 448 CTAs in two rounds of 296.  Fetching
-// a phase ahead did not shorten y, U by 1 us.
-// The layer with it, 28 heads of 128, 2,048 rows: step by step 796, FMAs 462, now 365 us.
+// (25 TFLOP/s); on tensor cores, with half as many states in between, the same rows take: angles 3, U 29, states 18 (36), y 88 us,
+// each with nothing in L2 (y 65 with 128 terms in an accumulator, whose error was 2.7 times the FMAs').  What bounds y: a CTA's phases (load
+// and split, multiply, load and split, ..) one behind the other, two CTAs to an SM, 448 CTAs in two rounds of 296: 41 % of a warp's
+// time is waiting for loads, 16 % for instructions, the tensor pipe is busy 14 % of the cycles.  In 128 registers y spills 16 to 150 bytes;
+// fetching a phase ahead did not shorten it, U by 1 us.
+// The layer with it, 28 heads of 128, 2,048 rows: step by step 796, FMAs 462, now 385 us.
 #include "gemm_f32_split.cuh"
 #include "rotation.cuh"
 #include "tcgen05.cuh"

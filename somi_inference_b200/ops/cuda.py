@@ -1703,8 +1703,8 @@ class CudaOps:
     SCAN_TURN_ROWS = 4          # the most rows a request may have where the scan itself rotates q and k
 
     # A portion goes in chunks from rows = this * state width on.  The layer in us, captured, step by step / in chunks:
-    # 14 heads of 64: 96 rows 45.1 / 37.7, 128 51.3 / 38.3, 256 77.9 / 40.1, 512 131 / 45.1; 28 of 128: 192 rows 111 / 92.1,
-    # 256 130 / 97.0, 512 219 / 122.  Step by step is 38.3 at 64 rows of the first and 91.2 at 128 of the second, where chunks
+    # 14 heads of 64: 96 rows 45.1 / 36.9, 128 51.3 / 37.0, 256 77.9 / 39.0, 512 131 / 45.5; 28 of 128: 192 rows 112 / 106,
+    # 256 131 / 112, 512 220 / 135.  Step by step is 38.9 at 64 rows of the first and 94.8 at 128 of the second, where chunks
     # are at best the same.  Launched one by one both are bound by the host up to about 256 rows (130 / 120).
     SCAN_CHUNK_ROWS = 1.5
     SCAN_CHUNK_BYTES = 1 << 29  # the most that the chunks' states of a run of portions may take

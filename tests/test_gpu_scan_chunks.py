@@ -1,4 +1,4 @@
-"""The recurrence with a constant decay in chunks of 64 rows, against the recurrence itself in 64 bits and
+"""The recurrence with a constant decay in chunks of 128 rows, against the recurrence itself in 64 bits and
 against the step by step kernel: portions that end around a chunk, states that an earlier step left, single
 tokens beside them, rotated or activated inputs, grouped query and key heads."""
 
