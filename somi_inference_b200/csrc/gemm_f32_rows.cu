@@ -12,8 +12,9 @@
 //     896 x 4,864                       8.4, 9.7, 13.4, 14  / 7.5, 7.9, 8.1, 11.1
 //     2,048 x 2,048                     5.9, 7.3, 11.9, 12  / 5.4, 5.7, 5.8, 7.8
 //     1,152 x 896                       3.9, 4.4, 5.3, 5.6  / 3.2, 3.6, 3.5, 4.9
-// One or two rows are up to 10 % slower than as FMAs where 5,000 to 10,000 features have few terms: there the FMA kernel's smaller CTAs
-// let more of the next product's weights be under way.
+// One or two rows are up to 10 % slower than as FMAs where the tiles fill the chip little more than once (9,728 x 896, 5,120 x 5,120,
+// 2,560 x 2,048): there the FMA kernel's smaller CTAs let more of the next product's weights be under way; and for few features of many
+// terms (256 x 3,584, 768 x 8,960), where a warp's range is a chain.
 #include <cooperative_groups.h>
 
 #include "gemm_f32_split.cuh"
